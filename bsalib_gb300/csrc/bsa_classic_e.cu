@@ -285,22 +285,26 @@ namespace ecls {
 // 2 F14, 3 K_iii, 4 K_v, 5 F35, 6 K_ii, 7 K_vi, 8 F26, each kept at the lane's (a, b) and j).
 __global__ void k_e_reduce(int nm, int W, int MT, int grid, const double *__restrict__ part,
                            double *__restrict__ m3mf, double *__restrict__ m3mr) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int x = blockIdx.x * 32 + threadIdx.x;
     const int nm3 = nm * nm * nm;
-    if (x >= nm3) return;
-    const int m = x % nm, n = (x / nm) % nm, o = x / (nm * nm);
+    const int xe = x < nm3 ? x : 0;
+    const int m = xe % nm, n = (xe / nm) % nm, o = xe / (nm * nm);
     auto sum = [&](int kind, int a, int b, int j) {
         const int R = a * nm + b, mtile = R / 128, lane = R % 128;
         double s = 0.0;
-        for (int g = mtile; g < grid; g += MT) s += part[(((size_t)g * kKinds + kind) * W + j) * 128 + lane];
+        for (int g = mtile + MT * threadIdx.y; g < grid; g += MT * kRedLanes)
+            s += part[(((size_t)g * kKinds + kind) * W + j) * 128 + lane];
         return s;
     };
-    const double mr = sum(0, m, n, o) + sum(1, m, o, n) + sum(3, o, n, m) + sum(4, n, o, m) + sum(6, n, m, o) +
+    double mr = sum(0, m, n, o) + sum(1, m, o, n) + sum(3, o, n, m) + sum(4, n, o, m) + sum(6, n, m, o) +
                       sum(7, o, m, n);
-    const double mf = sum(2, m, n, o) + sum(2, m, o, n) + sum(5, o, n, m) + sum(5, n, o, m) + sum(8, n, m, o) +
+    double mf = sum(2, m, n, o) + sum(2, m, o, n) + sum(5, o, n, m) + sum(5, n, o, m) + sum(8, n, m, o) +
                       sum(8, o, m, n);
-    m3mr[x] = 2.0 * mr;  // B_F = 2 (T1 + T2 + T3)
-    m3mf[x] = 2.0 * mf;
+    red_lanes(mr, mf);
+    if (threadIdx.y == 0 && x < nm3) {
+        m3mr[x] = 2.0 * mr;  // B_F = 2 (T1 + T2 + T3)
+        m3mf[x] = 2.0 * mf;
+    }
 }
 
 template <int NMT, int JH, bool SAMPLE = false>
@@ -434,7 +438,7 @@ int Engine::contract_e(const PointSrc &ps, double *m3mf, double *m3mr, const ESa
     }
     if ((e = dOut.reserve(sizeof(double) * (3 * (size_t)nm * nm + 2 * (size_t)nm3)))) return cuda_fail(e, "out");
     double *o = dOut.as<double>() + 3 * (size_t)nm * nm;
-    k_e_reduce<<<(unsigned)((nm3 + 127) / 128), 128, 0, stream>>>(nm, W, MT, grid, prm.part, o, o + nm3);
+    k_e_reduce<<<(unsigned)((nm3 + 31) / 32), dim3(32, kRedLanes), 0, stream>>>(nm, W, MT, grid, prm.part, o, o + nm3);
     if ((e = cudaGetLastError())) return cuda_fail(e, "BF16x3 reduction");
     kernels += 2;
     std::vector<double> h(2 * (size_t)nm3);

@@ -127,6 +127,28 @@ __device__ __forceinline__ void get_point(const PointSrc &ps, long long p, int &
     }
 }
 
+// Lanes (threadIdx.y) that share the partials of one third moment in the reduction kernels of the
+// split Classic forms: one lane walking every CTA's partial of seven kinds was a chain of dependent
+// loads (0.20 ms for the 64 moments of a 4-mode structure).
+constexpr int kRedLanes = 16;
+
+// Sum of a and b over the lanes threadIdx.y of a 32 x kRedLanes block, into lane 0 (fixed order).
+__device__ __forceinline__ void red_lanes(double &a, double &b) {
+    __shared__ double red[2][kRedLanes][33];
+    const int x = threadIdx.x, y = threadIdx.y;
+    red[0][y][x] = a;
+    red[1][y][x] = b;
+    for (int h = kRedLanes / 2; h > 0; h >>= 1) {
+        __syncthreads();
+        if (y < h) {
+            red[0][y][x] += red[0][y + h][x];
+            red[1][y][x] += red[1][y + h][x];
+        }
+    }
+    a = red[0][0][x];
+    b = red[1][0][x];
+}
+
 // Two FP32 lanes in one 64-bit register.  The paired FP32 instructions of sm_100 and later
 // (fma.rn.f32x2, mul.rn.f32x2) run both lanes from one issue slot, each lane rounded as the
 // scalar fma.rn / mul.rn would round it.

@@ -460,14 +460,15 @@ __global__ void k_prep_h(int nf, int nm, int NMT, const double *__restrict__ f, 
 // with the symmetric D1 (kinds 7) term 1's mirror, kept at (m, o, n).
 __global__ void k_mixed_reduce(int nm, int NMT, int MT, int grid, int kinds, const double *__restrict__ part,
                                double *__restrict__ m3mf, double *__restrict__ m3mr) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int x = blockIdx.x * 32 + threadIdx.x;
     const int nm3 = nm * nm * nm;
-    if (x >= nm3) return;
-    const int m = x % nm, n = (x / nm) % nm, o = x / (nm * nm);
+    const int xe = x < nm3 ? x : 0;
+    const int m = xe % nm, n = (xe / nm) % nm, o = xe / (nm * nm);
     auto sum = [&](int kind, int a, int b, int j) {
         const int R = a * nm + b, mtile = R / 128, lane = R % 128;
         double s = 0.0;
-        for (int g = mtile; g < grid; g += MT) s += part[(((size_t)g * kinds + kind) * NMT + j) * 128 + lane];
+        for (int g = mtile + MT * threadIdx.y; g < grid; g += MT * kRedLanes)
+            s += part[(((size_t)g * kinds + kind) * NMT + j) * 128 + lane];
         return s;
     };
     double mr = sum(0, m, n, o) + sum(1, o, n, m) + sum(2, n, o, m);
@@ -476,8 +477,11 @@ __global__ void k_mixed_reduce(int nm, int NMT, int MT, int grid, int kinds, con
         mr += sum(5, m, o, n);
         mf += sum(6, m, o, n);
     }
-    m3mr[x] = 2.0 * mr;  // B_F = 2 * (term1 + term2 + term3)
-    m3mf[x] = 2.0 * mf;
+    red_lanes(mr, mf);
+    if (threadIdx.y == 0 && x < nm3) {
+        m3mr[x] = 2.0 * mr;  // B_F = 2 * (term1 + term2 + term3)
+        m3mf[x] = 2.0 * mf;
+    }
 }
 
 cudaError_t prep_u(cudaStream_t st, int nf, int nm, int K, int Kp, int Mp, const float *A, const double *Q,
@@ -611,7 +615,7 @@ int Engine::contract_mixed(const PointSrc &ps, long long npts, double *m3mf, dou
     const long long nm3 = (long long)nm * nm * nm;
     if ((e = dOut.reserve(sizeof(double) * (3 * (size_t)nm * nm + 2 * (size_t)nm3)))) return cuda_fail(e, "out");
     double *o = dOut.as<double>() + 3 * (size_t)nm * nm;
-    k_mixed_reduce<<<(unsigned)((nm3 + 127) / 128), 128, 0, stream>>>(nm, W, MT, grid, kinds, prm.part, o, o + nm3);
+    k_mixed_reduce<<<(unsigned)((nm3 + 31) / 32), dim3(32, kRedLanes), 0, stream>>>(nm, W, MT, grid, kinds, prm.part, o, o + nm3);
     if ((e = cudaGetLastError())) return cuda_fail(e, "BF16x3 reduction");
     kernels += 2;
     std::vector<double> h(2 * (size_t)nm3);
