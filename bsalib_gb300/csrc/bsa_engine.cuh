@@ -189,6 +189,8 @@ struct Engine {
                     double *br_host, std::vector<double> *grid_out);
     int classic_export(PointSrc ps, const std::vector<double> &f, double *m3mf, double *m3mr);
     int contract(const PointSrc &ps, long long npts, double *m3mf, double *m3mr, double *bf_host, double *br_host);
+    // the whole Classic grid in FP64 over distinct frequency pairs (bsa_pair64.cu); grid +-N df
+    int contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr);
     int contract_mixed(const PointSrc &ps, long long npts, double *m3mf, double *m3mr);
     int contract_e(const PointSrc &ps, double *m3mf, double *m3mr, const ESample *smp = nullptr);  // bsa_classic_e.cu
     // bsa_gpu_clsBispectraAt: Classic bispectra at listed grid points in the selected precision

@@ -494,6 +494,19 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
     // The split-precision contraction reduces to moments only; it reads an FP32 A table.
     const bool mixed = !diagonal && precision == BSA_PREC_BF16X3 && !bf_host && !br_host;
     if (mixed && nme > 64) return fail(BSA_ERR_UNSUPPORTED, "BF16x3 contraction supports at most 64 kept modes");
+    // FP64 moments of the whole grid f = -N..N come from the products of distinct |f| pairs
+    // (bsa_pair64.cu), on the A rows of f >= 0 alone.  Row shards, materialised or exported bispectra
+    // and the frequency convention's one-sided grid (its truncated sum reads another row than
+    // |f1 + f2|) keep the point kernel.
+    const bool pair64 = !diagonal && !mixed && !bf_host && !br_host && !export_fn && !brm_file_wanted(true) &&
+                        set.defsc == 1 && (nf & 1) && r0 == 0 && r1 == nf;
+    const int half = (nf - 1) / 2;
+    const double df_grid = f[half + 1] - f[half];  // the step itself (f[half] = 0): f[1] - f[0] is rounded
+    if (pair64) {
+        ftab.assign(f.begin() + half, f.end());
+        if (analytic)
+            for (int s = half + 1; s <= 2 * half; ++s) ftab.push_back(s * df_grid);
+    }
     cudaError_t e;
     if ((e = cudaEventRecord(ev0, stream))) return cuda_fail(e, "event");
     if ((rc = diagonal ? build_psd(ftab) : build_atable(ftab, mixed))) return rc;
@@ -501,18 +514,24 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
     if (set.ipsd && (m2mf || m2mr || m2o2mr)) {
         std::vector<double> wf(nf, scalar ? delta : delta);
         if (!scalar) { wf[0] = delta / 2; wf[nf - 1] = delta / 2; }
+        // f and -f contribute the same (Re[H_o conj H_n] is even)
+        const int np = pair64 ? half + 1 : nf;
+        if (pair64) {
+            wf.erase(wf.begin(), wf.begin() + half);
+            for (int k = 1; k < np; ++k) wf[k] *= 2.0;
+        }
         if ((e = upload(dWf, wf, stream))) return cuda_fail(e, "weights");
         if ((e = dPsdF.reserve(sizeof(double) * (size_t)nf * nm2))) return cuda_fail(e, "psd");
         if ((e = dOut.reserve(sizeof(double) * (3 * (size_t)nm2 + 2 * (size_t)dim_bisp()))))
             return cuda_fail(e, "out");
-        e = diagonal ? launch_force_psd_diag(stream, nf, K, nme, dS.as<double>(), dWd2.as<double>(), dPsdF.as<double>())
+        e = diagonal ? launch_force_psd_diag(stream, np, K, nme, dS.as<double>(), dWd2.as<double>(), dPsdF.as<double>())
             : mixed  ? launch_force_psd32(stream, nf, (int)set.tc.size(), in.nnl, nme, dL32.as<float>(),
                                           dA32.as<float>(), dPsdF.as<double>())
-                     : launch_force_psd(stream, nf, (int)set.tc.size(), in.nnl, nme, dL.as<double>(), dA.as<double>(),
+                     : launch_force_psd(stream, np, (int)set.tc.size(), in.nnl, nme, dL.as<double>(), dA.as<double>(),
                                         dPsdF.as<double>());
         if (e) return cuda_fail(e, "force PSD kernel");
         double *o = dOut.as<double>();
-        if ((e = launch_m2(stream, r0, r1, nme, diagonal ? 1 : 0, dFreq.as<double>(), dWf.as<double>(),
+        if ((e = launch_m2(stream, pair64 ? 0 : r0, pair64 ? np : r1, nme, diagonal ? 1 : 0, dFreq.as<double>(), dWf.as<double>(),
                            dPsdF.as<double>(), frf(), o, o + nm2, o + 2 * nm2)))
             return cuda_fail(e, "m2 kernel");
         kernels += 2;
@@ -573,6 +592,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
         } else {
             rc = diagonal ? contract_diag(ps, npts, 0, m3mf, m3mr, bf_host, br_host)
                  : mixed  ? contract_mixed(ps, npts, m3mf, m3mr)
+                 : pair64 ? contract_pair64(half, df_grid, analytic, !scalar, delta * delta, m3mf, m3mr)
                           : contract(ps, npts, m3mf, m3mr, bf_host, br_host);
         }
         if (rc) return rc;

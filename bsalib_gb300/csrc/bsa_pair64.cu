@@ -1,0 +1,443 @@
+// bsa_pair64.cu -- the Classic FP64 analysis over distinct frequency pairs.
+//
+// Every nodal quantity of the path depends on |f| (the spectra and c^|f|), so on the grid
+// f_i = i df, i = -N .. N, A(f_i) = A(f_-i): N + 1 distinct rows.  With
+// E(x, y)[(a, b), j] = sum_k Q[k][a] A(x)[k][b] A(y)[k][j], the three terms of the BFM at a grid
+// point (functionsImpl.F90:1494-1538) are elements of E at two of |f1|, |f2|, |f1 + f2|
+//   T1(f1, f2)[m, n, o] = E(f1, f2)[(m, n), o]
+//   T2(f1, f2)[m, n, o] = E(f1 + f2, f2)[(n, m), o]
+//   T3(f1, f2)[m, n, o] = E(f1, f1 + f2)[(o, n), m]
+// and E(x, y)[(a, b), j] = E(y, x)[(a, j), b].  The whole grid therefore needs E(x, y) for
+// 0 <= x <= y only: (N + 1)(N + 2) / 2 products of 2 K NM^3 flop instead of (2 N + 1)^2 points of
+// 4 K NM^3 (one sixteenth of the flop; GB300 issues two FP64 FMAs an SM and clock, so the flop
+// count is the time).  The analytic S(f1 + f2) (classic_trunc off) adds the rows N + 1 .. 2 N and
+// the pairs (x, y) with y > N, y - x <= N.
+//
+// The products go to HBM in chunks of first rows x (k_pair_gemm), then k_pair_moments adds each
+// element into the third moments with the FRF products and weights of every grid point that reads
+// it.  B(-f1, -f2) = B(f1, f2) on the grid, so half of the points stand for both (weight 2).
+// With Hx = H(x), Hy = H(y), P = H(x + y), D = H(y - x) and, per row (a, b) and column j,
+//   alpha = Re[Hx_a Hy_b conj P_j],  beta = Re[Hx_a conj Hy_b D_j],
+//   gamma = Re[Hy_a conj P_b Hx_j],  delta = Re[Hy_a conj D_b conj Hx_j]
+// the twelve contributions of an element are
+//   T1 at (x, +-y):      (m, n, o) = (a, b, j)   w1 (alpha + beta)
+//   T1 at (y, +-x):                  (a, j, b)   w1 (gamma + delta)
+//   T2 at (x -+ y, +-y):             (b, a, j)   w2m gamma + w2p delta
+//   T3 at (y, +-x - y):              (b, j, a)   w2m alpha + w2p beta
+//   T3 at (x, +-y - x):              (j, b, a)   w3m gamma + w3p delta
+//   T2 at (y -+ x, +-x):             (j, a, b)   w3m alpha + w3p beta
+// with w1 the weight of the grid points (x, +-y), w2p / w2m of (x - y, y) / (x + y, -y) and
+// w3p / w3m of (x, y - x) / (x, -x - y), zero beyond the grid (two contributions share a weight
+// because the weights are symmetric under f1 <-> f2 and under the central symmetry).  A product
+// with x = y feeds all at half weight (its transpose is in the same product), x = 0 has no minus
+// partners.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "../../include/bsa_gpu.h"
+#include "bsa_engine.cuh"
+#include "bsa_kernels.cuh"
+
+namespace bsa {
+namespace p64 {
+
+constexpr int kTM = 128, kTN = 32;  // product tile: rows (x, a, b) by columns (y, j)
+constexpr int kKT = 16;
+constexpr int kKinds = 9;           // K1 .. K6 (the order above: abj, ajb, baj, jba, jab, bja), M1, M2, M3
+constexpr int kBatch = 8;           // pairs a thread takes between two barriers
+
+// A chunk of products: rows r = (x - x0) nm^2 + a nm + b of the first rows x in [x0, x1), in tiles
+// of kTM; row tile mt holds the column tiles ct0[mt] .. ct0[mt] + nct[mt] of c = y nm + j, row-major
+// from base[mt].
+struct RowTile {
+    int ct0, nct;
+    long long base;   // first element in E
+    long long item0;  // product tiles before this row tile
+};
+
+struct Chunk {
+    int x0, x1, nm, K, hi, ntiles;
+    const RowTile *rt;
+    double *E;
+};
+
+// E of one product tile: 256 threads, 4 x 4 elements each, K staged 16 at a time; the row operand
+// Q[k][a] A(x)[k][b] is formed while staging.  FP64-pipe bound: 16 FMAs a thread and k against one
+// product in 32 for the staging.
+__global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__restrict__ A, const double *__restrict__ Q) {
+    __shared__ double As[kKT][kTM], Bs[kKT][kTN];
+    const int t = threadIdx.x, nm = c.nm, nm2 = nm * nm, K = c.K;
+    const long long item = blockIdx.x;
+    int lo = 0, up = c.ntiles - 1;
+    while (lo < up) {
+        const int mid = (lo + up + 1) >> 1;
+        if (c.rt[mid].item0 <= item) lo = mid; else up = mid - 1;
+    }
+    const RowTile rt = c.rt[lo];
+    const int ct = rt.ct0 + (int)(item - rt.item0);
+    const int r0 = lo * kTM, rows = (c.x1 - c.x0) * nm2;
+    // this thread's staging row and column
+    const int sr = t & (kTM - 1), kr = t >> 7;           // As: 2 k rows of 128 rows at a time
+    const bool rv = r0 + sr < rows;
+    const int rr = rv ? r0 + sr : 0, x = c.x0 + rr / nm2, ab = rr % nm2, a = ab / nm, b = ab % nm;
+    const double *Qa = Q + a, *Ab = A + (size_t)x * K * nm + b;
+    const int sc = t & (kTN - 1), kc = t >> 5;           // Bs: 8 k rows of 32 columns at a time
+    const int col = ct * kTN + sc, y = col / nm, j = col - y * nm;
+    const bool cv = y <= c.hi;
+    const double *Aj = A + (size_t)(cv ? y : 0) * K * nm + j;
+    const int tr = (t >> 3) * 4, tc = (t & 7) * 4;
+    double acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[i][q] = 0.0;
+    for (int k0 = 0; k0 < K; k0 += kKT) {
+        const int kn = min(kKT, K - k0);
+#pragma unroll
+        for (int u = 0; u < kKT / 2; ++u) {
+            const int k = kr + 2 * u;
+            As[k][sr] = (rv && k < kn) ? Qa[(size_t)(k0 + k) * nm] * Ab[(size_t)(k0 + k) * nm] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kKT / 8; ++u) {
+            const int k = kc + 8 * u;
+            Bs[k][sc] = (cv && k < kn) ? Aj[(size_t)(k0 + k) * nm] : 0.0;
+        }
+        __syncthreads();
+        for (int k = 0; k < kn; ++k) {
+            double ar[4], br[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ar[i] = As[k][tr + i];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) br[q] = Bs[k][tc + q];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[i][q] = fma(ar[i], br[q], acc[i][q]);
+        }
+        __syncthreads();
+    }
+    const size_t ld = (size_t)rt.nct * kTN;
+    double *out = c.E + rt.base + (size_t)(ct - rt.ct0) * kTN + tc;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) out[(size_t)(tr + i) * ld + q] = acc[i][q];
+}
+
+// H of the kept modes at i df, i = 0 .. 2 N.
+__global__ void k_frf_rows(int n, int nm, double df, FrfPar frf, double2 *__restrict__ H) {
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= n * nm) return;
+    const int m = u % nm;
+    double hr, hi;
+    frf_eval(frf.M[m], frf.K[m], frf.C[m], (double)(u / nm) * df * kPi2, hr, hi);
+    H[u] = make_double2(hr, hi);
+}
+
+struct MomPar {
+    int N, vect;            // vect: edge weights of intgSpectraVect_, else uniform
+    long long npairs;       // pairs (x, y) of the chunk
+    const long long *pre;   // pairs before first row x0 + i, and the total
+    const double2 *H;       // [2 N + 1][nm]
+    double w4;              // weight of an interior pair: 2 (the BFM's factor) x 2 (both points) x d^2
+    double *part;           // [groups][kKinds][nm^2][nm]
+    int first;              // first chunk: the partials are written, not added to
+    int RT, PL;             // rows (a, b) of a block, pair lanes
+};
+
+// Relative weight of grid point (i1, i2) (BsaClassicImpl.F90:596-632, vertex -1/2), 0 beyond it.
+__device__ __forceinline__ double wrel(int i1, int i2, int N, int vect) {
+    const int u = abs(i1), v = abs(i2);
+    if (u > N || v > N) return 0.0;
+    if (!vect) return 1.0;
+    return u == N ? (v == N ? -0.5 : 0.5) : (v == N ? 0.5 : 1.0);
+}
+
+struct PairInfo {
+    int x, y, region;        // 0: every weight 1; 1: w1 = w2p = w3p = 1, w2m = w3m = 0; 2: general
+    double w1, w2p, w2m, w3p, w3m, wm1, wm2, wm3;
+};
+
+// One block per (tile of RT rows (a, b), group of pairs); a thread holds one element (a, b, j) and
+// takes the pairs of its lane.  Per batch of kBatch x PL pairs: the pairs and weights, then the
+// products of the row factors (8 doubles a row) and the columns' FRF values in shared memory, then
+// 9 (all weights one), 14 (no sums on the grid) or 27 FP64 operations an element and pair.
+__global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
+    extern __shared__ double sm[];
+    const int t = threadIdx.x, nm = c.nm, nm2 = nm * nm;
+    const int PB = kBatch * P.PL, RT = P.RT, EL = RT * nm;
+    double *rowf = sm;                                 // [PB][RT][8]
+    double2 *colf = (double2 *)(rowf + (size_t)PB * RT * 8);  // [PB][nm][3]: Hx, P, D
+    PairInfo *info = (PairInfo *)(colf + (size_t)PB * nm * 3);
+    const int pl = t / EL, el = t - pl * EL;
+    const int rl = el / nm, j = el - rl * nm, ab = blockIdx.x * RT + rl;
+    const bool live = pl < P.PL && ab < nm2;
+    const int G = gridDim.y;
+    double K1 = 0, K2 = 0, K3 = 0, K4 = 0, K5 = 0, K6 = 0, M1 = 0, M2 = 0, M3 = 0;
+    double Kc = 0, Kd = 0, Mc = 0, K56 = 0, K34 = 0, M23 = 0;
+    for (long long p0 = (long long)blockIdx.y * PB; p0 < P.npairs; p0 += (long long)G * PB) {
+        const int np = (int)min((long long)PB, P.npairs - p0);
+        __syncthreads();
+        if (t < np) {
+            const long long p = p0 + t;
+            int lo = 0, up = c.x1 - c.x0 - 1;
+            while (lo < up) {
+                const int mid = (lo + up + 1) >> 1;
+                if (P.pre[mid] <= p) lo = mid; else up = mid - 1;
+            }
+            PairInfo f;
+            f.x = c.x0 + lo;
+            f.y = f.x + (int)(p - P.pre[lo]);
+            const int x = f.x, y = f.y, N = P.N;
+            const double s = (x == y ? 0.5 : 1.0) * (x == 0 && y == 0 ? 0.5 : 1.0), sm_ = x == 0 ? 0.0 : s;
+            // plus partners (x, y), (x - y, y), (x, y - x); minus partners (x, -y), (x + y, -y), (x, -x - y)
+            const double a1 = wrel(x, y, N, P.vect);
+            f.w1 = s * a1;
+            f.w2p = s * wrel(x - y, y, N, P.vect);
+            f.w3p = s * wrel(x, y - x, N, P.vect);
+            f.w2m = sm_ * wrel(x + y, y, N, P.vect);
+            f.w3m = sm_ * wrel(x, x + y, N, P.vect);
+            f.wm1 = f.w1 + sm_ * a1;
+            f.wm2 = f.w2p + f.w2m;
+            f.wm3 = f.w3p + f.w3m;
+            f.region = 2;
+            if (x > 0 && x < y && f.w1 == 1.0 && f.w2p == 1.0 && f.w3p == 1.0) {
+                if (f.w2m == 1.0 && f.w3m == 1.0) f.region = 0;
+                else if (f.w2m == 0.0 && f.w3m == 0.0) f.region = 1;
+            }
+            info[t] = f;
+        }
+        __syncthreads();
+        double e[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int s = u * P.PL + pl;
+            e[u] = 0.0;
+            if (live && s < np) {
+                const int r = (info[s].x - c.x0) * nm2 + ab, mt = r / kTM;
+                const RowTile rt = c.rt[mt];
+                e[u] = c.E[rt.base + (size_t)(r - mt * kTM) * rt.nct * kTN + (info[s].y * nm + j - rt.ct0 * kTN)];
+            }
+        }
+        for (int q = t; q < np * nm * 3; q += 256) {
+            const int s = q / (nm * 3), z = q - s * nm * 3, w = z / nm, m = z - w * nm;
+            const int x = info[s].x, y = info[s].y;
+            const int i = w == 0 ? x : w == 1 ? x + y : y - x;
+            // x + y <= 2 N wherever its value is used (a pair with y > N has w1 = 0, w2m = w3m = 0 beyond)
+            colf[((size_t)s * nm + m) * 3 + w] = P.H[(size_t)min(i, 2 * P.N) * nm + m];
+        }
+        for (int q = t; q < np * RT; q += 256) {
+            const int s = q / RT, rr = blockIdx.x * RT + (q - s * RT);
+            if (rr >= nm2) continue;
+            const int a = rr / nm, b = rr - a * nm, x = info[s].x, y = info[s].y;
+            const double2 xa = P.H[(size_t)x * nm + a], ya = P.H[(size_t)y * nm + a], yb = P.H[(size_t)y * nm + b];
+            const double2 pb = P.H[(size_t)min(x + y, 2 * P.N) * nm + b], db = P.H[(size_t)(y - x) * nm + b];
+            double *o = rowf + (size_t)q * 8;
+            o[0] = xa.x * yb.x - xa.y * yb.y;  // q1 = Hx_a Hy_b
+            o[1] = xa.x * yb.y + xa.y * yb.x;
+            o[2] = xa.x * yb.x + xa.y * yb.y;  // q2 = Hx_a conj Hy_b
+            o[3] = xa.y * yb.x - xa.x * yb.y;
+            o[4] = ya.x * pb.x + ya.y * pb.y;  // c = Hy_a conj P_b
+            o[5] = ya.y * pb.x - ya.x * pb.y;
+            o[6] = ya.x * db.x + ya.y * db.y;  // d = Hy_a conj D_b
+            o[7] = ya.y * db.x - ya.x * db.y;
+        }
+        __syncthreads();
+        if (live) {
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const int s = u * P.PL + pl;
+                if (s >= np) continue;
+                const PairInfo &f = info[s];
+                const double *o = rowf + ((size_t)s * RT + rl) * 8;
+                const double2 *h = colf + ((size_t)s * nm + j) * 3;
+                const double2 hx = h[0], hp = h[1], hd = h[2];
+                const double v = e[u];
+                const double beta = fma(o[2], hd.x, -(o[3] * hd.y));
+                if (f.region == 0) {
+                    const double ab_ = fma(o[0], hp.x, fma(o[1], hp.y, beta));
+                    // gamma + delta
+                    const double gd = fma(o[4] + o[6], hx.x, (o[7] - o[5]) * hx.y);
+                    Kc = fma(v, ab_, Kc);
+                    Kd = fma(v, gd, Kd);
+                    Mc += v;
+                } else if (f.region == 1) {
+                    const double ab_ = fma(o[0], hp.x, fma(o[1], hp.y, beta));
+                    const double dl = fma(o[6], hx.x, o[7] * hx.y);
+                    const double gd = fma(o[4], hx.x, fma(-o[5], hx.y, dl));
+                    K1 = fma(v, ab_, K1);
+                    K56 = fma(v, beta, K56);
+                    K2 = fma(v, gd, K2);
+                    K34 = fma(v, dl, K34);
+                    M1 = fma(v, 2.0, M1);
+                    M23 += v;
+                } else {
+                    const double al = fma(o[0], hp.x, o[1] * hp.y);
+                    const double dl = fma(o[6], hx.x, o[7] * hx.y);
+                    const double ga = fma(o[4], hx.x, -(o[5] * hx.y));
+                    const double w1m = f.wm1 - f.w1;
+                    const double va = v * al, vb = v * beta, vg = v * ga, vd = v * dl;
+                    K1 = fma(f.w1, va, fma(w1m, vb, K1));
+                    K2 = fma(f.w1, vg, fma(w1m, vd, K2));
+                    K3 = fma(f.w2p, vd, fma(f.w2m, vg, K3));
+                    K6 = fma(f.w2p, vb, fma(f.w2m, va, K6));
+                    K4 = fma(f.w3p, vd, fma(f.w3m, vg, K4));
+                    K5 = fma(f.w3p, vb, fma(f.w3m, va, K5));
+                    M1 = fma(f.wm1, v, M1);
+                    M2 = fma(f.wm2, v, M2);
+                    M3 = fma(f.wm3, v, M3);
+                }
+            }
+        }
+    }
+    double k[kKinds] = {K1 + Kc,         K2 + Kd,         K3 + Kd + K34,       K4 + Kd + K34,      K5 + Kc + K56,
+                        K6 + Kc + K56,   M1 + 2.0 * Mc,   M2 + 2.0 * Mc + M23, M3 + 2.0 * Mc + M23};
+    // lanes of one element, then the block's partial
+    double *red = sm;
+#pragma unroll
+    for (int q = 0; q < kKinds; ++q) {
+        double s = k[q];
+        if (P.PL > 1) {
+            __syncthreads();
+            if (pl < P.PL) red[t] = s;
+            __syncthreads();
+            if (pl == 0)
+                for (int z = 1; z < P.PL; ++z) s += red[z * EL + el];
+        }
+        if (pl == 0 && ab < nm2) {
+            double *o = P.part + (((size_t)blockIdx.y * kKinds + q) * nm2 + ab) * nm + j;
+            *o = P.first ? s : *o + s;
+        }
+    }
+}
+
+// m3[m + nm n + nm^2 o] from the summed kinds [kKinds][(a, b)][j].
+__global__ void k_pair_finish(int nm, double w4, const double *__restrict__ S, double *__restrict__ m3mf,
+                              double *__restrict__ m3mr) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, nm2 = nm * nm, nm3 = nm2 * nm;
+    if (x >= nm3) return;
+    const int m = x % nm, n = (x / nm) % nm, o = x / nm2;
+    auto at = [&](int kind, int a, int b, int j) { return S[((size_t)kind * nm2 + a * nm + b) * nm + j]; };
+    m3mr[x] = w4 * (at(0, m, n, o) + at(1, m, o, n) + at(2, n, m, o) + at(3, o, n, m) + at(4, n, o, m) + at(5, o, m, n));
+    m3mf[x] = w4 * (at(6, m, n, o) + at(6, m, o, n) + at(7, n, m, o) + at(7, o, m, n) + at(8, o, n, m) + at(8, n, o, m));
+}
+
+}  // namespace p64
+
+// Third moments of the whole Classic grid (circular-frequency convention, every row) in FP64 from
+// the products of distinct frequency pairs; dA holds the A rows of i df, i = 0 .. N (truncated
+// S(f1 + f2)) or 0 .. 2 N (analytic).
+int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr) {
+    using namespace p64;
+    const int nm = nme, nm2 = nm * nm, hi = analytic ? 2 * N : N;
+    const long long nm3 = (long long)nm2 * nm;
+    cudaError_t e;
+    auto ylast = [&](int x) { return analytic ? std::min(hi, x + N) : N; };  // last partner of first row x
+    int RT = std::max(1, std::min(nm2, 256 / nm)), PL = std::max(1, std::min(8, 256 / (RT * nm)));
+    const int tiles = (nm2 + RT - 1) / RT;
+    // about four blocks an SM; a group holds at least one batch of pairs
+    const long long pairs_all = (long long)(N + 1) * (N + 2) / 2 + (analytic ? (long long)N * (N + 1) / 2 : 0);
+    const int G = (int)std::max(1LL, std::min<long long>((608 + tiles - 1) / tiles,
+                                                         (pairs_all + kBatch * PL - 1) / (kBatch * PL)));
+    // chunks of first rows: at most 4 GB of products each (all of a 400-row, 24-mode grid in one)
+    const long long cap = 1LL << 29;
+    struct Plan { int x0, x1, ntiles; long long items, elems, npairs; size_t rt0, pre0; };
+    std::vector<Plan> plans;
+    std::vector<RowTile> rts;
+    std::vector<long long> pre;
+    for (int x0 = 0; x0 <= N;) {
+        Plan p{x0, x0, 0, 0, 0, 0, rts.size(), pre.size()};
+        auto rows_of = [&](int x1) {  // row tiles of [x0, x1), appended at p.rt0
+            rts.resize(p.rt0);
+            p.items = p.elems = 0;
+            const long long rows = (long long)(x1 - x0) * nm2;
+            for (long long r = 0; r < rows; r += kTM) {
+                const int xa = x0 + (int)(r / nm2), xb = x0 + (int)((std::min(rows, r + kTM) - 1) / nm2);
+                RowTile t;
+                t.ct0 = xa * nm / kTN;
+                t.nct = (int)(((long long)(ylast(xb) + 1) * nm + kTN - 1) / kTN) - t.ct0;
+                t.base = p.elems;
+                t.item0 = p.items;
+                p.items += t.nct;
+                p.elems += (long long)t.nct * kTN * kTM;
+                rts.push_back(t);
+            }
+        };
+        // rows of equal partner counts fill a chunk evenly: estimate, then one exact list
+        long long el = 0;
+        int x1 = x0;
+        while (x1 <= N) {
+            const long long add = (long long)nm2 * ((ylast(x1) - x1 + 1) * (long long)nm + 2 * kTN);
+            if (x1 > x0 && el + add > cap) break;
+            el += add;
+            ++x1;
+        }
+        rows_of(x1);
+        p.x1 = x1;
+        p.ntiles = (int)(rts.size() - p.rt0);
+        for (int x = x0; x < x1; ++x) {
+            pre.push_back(p.npairs);
+            p.npairs += ylast(x) - x + 1;
+        }
+        plans.push_back(p);
+        x0 = x1;
+    }
+    long long emax = 0;
+    for (const Plan &p : plans) emax = std::max(emax, p.elems);
+    const size_t rtb = sizeof(RowTile) * rts.size(), preb = sizeof(long long) * pre.size();
+    const size_t hb = sizeof(double2) * (size_t)(2 * N + 1) * nm;
+    if ((e = dMixA.reserve(sizeof(double) * (size_t)emax)) || (e = dMixH.reserve(hb)) || (e = dMshIdx.reserve(rtb + preb)) ||
+        (e = dPartF.reserve(sizeof(double) * (size_t)G * kKinds * nm3)) ||
+        (e = dPartR.reserve(sizeof(double) * (size_t)kKinds * nm3)) ||
+        (e = dOut.reserve(sizeof(double) * (3 * (size_t)nm2 + 2 * (size_t)nm3))))
+        return cuda_fail(e, "allocating pair products");
+    char *idx = (char *)dMshIdx.p;
+    if ((e = cudaMemcpyAsync(idx, rts.data(), rtb, cudaMemcpyHostToDevice, stream)) ||
+        (e = cudaMemcpyAsync(idx + rtb, pre.data(), preb, cudaMemcpyHostToDevice, stream)))
+        return cuda_fail(e, "pair lists");
+    h2d += (double)(rtb + preb);
+    if ((e = cudaEventRecord(ev2, stream)) || (e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
+    const int nh = (2 * N + 1) * nm;
+    k_frf_rows<<<(nh + 127) / 128, 128, 0, stream>>>(2 * N + 1, nm, df, frf(), dMixH.as<double2>());
+    const int PB = kBatch * PL;
+    const size_t smem = std::max((size_t)256 * sizeof(double), sizeof(double) * (size_t)PB * RT * 8 +
+                                 sizeof(double2) * (size_t)PB * nm * 3 + sizeof(PairInfo) * (size_t)PB);
+    if ((e = cudaFuncSetAttribute(k_pair_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
+        return cuda_fail(e, "pair moments kernel");
+    for (size_t q = 0; q < plans.size(); ++q) {
+        const Plan &p = plans[q];
+        Chunk c{p.x0, p.x1, nm, K, hi, p.ntiles, (const RowTile *)idx + p.rt0, dMixA.as<double>()};
+        k_pair_gemm<<<(unsigned)p.items, 256, 0, stream>>>(c, dA.as<double>(), dQ.as<double>());
+        MomPar mp{N, vect ? 1 : 0, p.npairs, (const long long *)(idx + rtb) + p.pre0, dMixH.as<double2>(), 4.0 * wval,
+                  dPartF.as<double>(), q == 0 ? 1 : 0, RT, PL};
+        k_pair_moments<<<dim3((unsigned)tiles, (unsigned)G), 256, smem, stream>>>(c, mp);
+        kernels += 2;
+    }
+    if ((e = cudaGetLastError())) return cuda_fail(e, "pair contraction kernels");
+    if ((e = cudaEventRecord(evg1, stream))) return cuda_fail(e, "event");
+    double *o = dOut.as<double>() + 3 * (size_t)nm2;
+    if ((e = launch_reduce_groups(stream, G, kKinds * nm3, dPartF.as<double>(), dPartR.as<double>(), nullptr, nullptr)))
+        return cuda_fail(e, "reduction kernel");
+    k_pair_finish<<<(unsigned)((nm3 + 127) / 128), 128, 0, stream>>>(nm, 4.0 * wval, dPartR.as<double>(), o, o + nm3);
+    if ((e = cudaGetLastError())) return cuda_fail(e, "reduction kernel");
+    kernels += 3;
+    std::vector<double> h(2 * (size_t)nm3);
+    if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
+        (e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream)))
+        return cuda_fail(e, "moment copy");
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ev2, ev1);
+    last_ms_contraction = ms;
+    cudaEventElapsedTime(&ms, evg0, evg1);
+    last_ms_gemm = ms;
+    d2h += (double)sizeof(double) * h.size();
+    if (m3mf) std::memcpy(m3mf, h.data(), sizeof(double) * nm3);
+    if (m3mr) std::memcpy(m3mr, h.data() + nm3, sizeof(double) * nm3);
+    return BSA_OK;
+}
+
+}  // namespace bsa

@@ -1,0 +1,49 @@
+"""The FP64 Classic analysis over distinct frequency pairs (bsa_pair64.cu) against the point kernel.
+
+A row range that leaves nothing out but is set explicitly in two shards keeps the point kernel, so
+the sum of two row shards is the point kernel's whole grid.  Both evaluate the same sums in FP64 in
+another order: 1e-12 of the largest moment (about 1e4 roundings of 1e-16)."""
+import numpy as np
+import pytest
+
+from bsalib_gb300 import api
+from bsalib_gb300.problem import random_structure, tall_building
+
+pytestmark = pytest.mark.gpu
+
+
+def _run(prob, rows=None, trunc=True, sym=False):
+    s = api.BsaSession(prob, classic_truncation=trunc)
+    try:
+        if rows:
+            s.set_rows(*rows)
+        if sym:
+            s.set_symmetry(True)
+        return s.run()
+    finally:
+        s.close()
+
+
+def _close(a, b, tol=1e-12):
+    for k in ("m2mf_cls", "m2mr_cls", "m2o2mr_cls", "m3mf_cls", "m3mr_cls"):
+        assert np.max(np.abs(a[k] - b[k])) <= tol * np.max(np.abs(b[k])), k
+
+
+# modes at and around the tiles of the moment kernel (rows per block, pair lanes) and of the products
+@pytest.mark.parametrize("modes,nodes,nfreqs", [(1, 3, 2), (2, 5, 3), (3, 17, 9), (5, 16, 12), (7, 33, 10), (16, 9, 8),
+                                                (17, 40, 6), (33, 12, 5), (64, 70, 3)])
+@pytest.mark.parametrize("trunc,scalar", [(True, 0), (False, 0), (True, 1), (False, 1)])
+def test_pairs_against_points(bsalib, modes, nodes, nfreqs, trunc, scalar):
+    p = tall_building(nodes=nodes, modes=modes, nfreqs=nfreqs, df=2.0 / nfreqs, seed=modes)
+    p.settings.scalar = scalar
+    nf = p.classic_nf()
+    whole = _run(p, trunc=trunc)
+    a, b = _run(p, (0, 1), trunc), _run(p, (1, nf), trunc)
+    _close(whole, {k: a[k] + b[k] for k in a})
+    _close(_run(p, trunc=trunc, sym=True), whole)
+
+
+def test_pairs_one_component(bsalib):
+    p = random_structure(11, nodes=(37, 37), modes=(9, 9), nfreq_grid=(41, 41))
+    a, b = _run(p, (0, 20)), _run(p, (20, 41))
+    _close(_run(p), {k: a[k] + b[k] for k in a})
