@@ -331,6 +331,7 @@ int Engine::upload_problem() {
     if ((rc = ensure_stream())) return rc;
     if (dev_uploaded) return BSA_OK;
     cudaError_t e;
+    if ((e = dLogc.reserve(log_coh_bytes(hCoh.size())))) return cuda_fail(e, "uploading problem data");
     if ((e = upload(dL, hL, stream)) || (e = upload(dQ, hQ, stream)) || (e = upload(dLogc, hCoh, stream)) ||
         (e = upload(dPsdPar, hPsd, stream)) || (e = upload(dFrfM, hM, stream)) || (e = upload(dFrfK, hK, stream)) ||
         (e = upload(dFrfC, hC, stream)) || (e = upload(dWd3, hWd3, stream)) || (e = upload(dWd2, hWd2, stream)) ||
@@ -339,7 +340,7 @@ int Engine::upload_problem() {
     // log c in place (FP64) and its FP32 copy
     if ((e = launch_log_coh(stream, hCoh.size(), dLogc.as<double>(), dLogc32.as<float>())))
         return cuda_fail(e, "coherence table");
-    kernels += 1;
+    kernels += 2;
     dev_uploaded = true;
     return BSA_OK;
 }
@@ -354,13 +355,13 @@ int Engine::build_psd(const std::vector<double> &freqs) {
 }
 
 // Nodal PSD table S[f][k] for the nf frequencies already in dFreq (fp32: the formulas
-// evaluated in FP32, for the split-precision A tables).
-int Engine::build_psd_dev(int nf, bool fp32) {
+// evaluated in FP32, for the split-precision A tables; root: sqrt(S)).
+int Engine::build_psd_dev(int nf, bool fp32, bool root) {
     const int ntc = (int)set.tc.size();
     cudaError_t e;
     if ((e = dS.reserve(sizeof(double) * (size_t)nf * ntc * in.nnl))) return cuda_fail(e, "allocating S");
     if ((e = launch_nodal_psd(stream, nf, dFreq.as<double>(), ntc, set.tc.data(), in.nnl, dPsdPar.as<PsdNode>(),
-                              in.psd_type, set.defsc, dS.as<double>(), fp32)))
+                              in.psd_type, set.defsc, dS.as<double>(), fp32, root)))
         return cuda_fail(e, "nodal PSD kernel");
     kernels += 1;
     return BSA_OK;
@@ -378,7 +379,7 @@ int Engine::build_atable(const std::vector<double> &freqs, bool fp32, bool msh) 
 int Engine::build_atable_dev(int nf, bool fp32) {
     const int ntc = (int)set.tc.size();
     cudaError_t e;
-    int rc = build_psd_dev(nf, fp32);
+    int rc = build_psd_dev(nf, fp32, !fp32);  // the FP64 table reads sqrt(S)
     if (rc) return rc;
     if (fp32) {
         // FP32 table on the tensor cores (tf32 hi/lo split, FP32-level accuracy)
@@ -704,7 +705,7 @@ int Engine::run_points(const double *fi, const double *fj, const double *w, doub
     int rc = upload_problem();
     if (rc) return rc;
     if (npts <= 0) return fail(BSA_ERR_ARG, "empty point set");
-    // Distinct frequencies: f1, f2 and f1+f2 of every point share one A table.
+    // Distinct |f|: f1, f2 and f1+f2 of every point share one A table (every quantity is even in f).
     std::vector<double> ftab;
     ftab.reserve(3 * (size_t)npts);
     std::vector<int> ix(npts), iy(npts), iz(npts);
@@ -712,9 +713,9 @@ int Engine::run_points(const double *fi, const double *fj, const double *w, doub
         std::vector<std::pair<double, int>> key;
         key.reserve(3 * (size_t)npts);
         for (long long p = 0; p < npts; ++p) {
-            key.push_back({fi[p], (int)(3 * p)});
-            key.push_back({fj[p], (int)(3 * p + 1)});
-            key.push_back({fi[p] + fj[p], (int)(3 * p + 2)});
+            key.push_back({std::fabs(fi[p]), (int)(3 * p)});
+            key.push_back({std::fabs(fj[p]), (int)(3 * p + 1)});
+            key.push_back({std::fabs(fi[p] + fj[p]), (int)(3 * p + 2)});
         }
         std::sort(key.begin(), key.end());
         int row = -1;

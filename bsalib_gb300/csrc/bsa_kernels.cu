@@ -18,7 +18,7 @@ namespace bsa {
 // ------------------------------------------------------------------------------------
 template <typename R>
 __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 tcs, int nnl,
-                            const PsdNode *__restrict__ par, int psd_type, int scaling,
+                            const PsdNode *__restrict__ par, int psd_type, int scaling, int root,
                             double *__restrict__ S) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long tot = (long long)nf * ntc * nnl;
@@ -66,20 +66,20 @@ __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 
         v = 0;
     }
     if (scaling == 1) v = v / R(kPi4);
-    S[t] = (double)v;
+    S[t] = root ? sqrt((double)v) : (double)v;
 }
 
 cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, const int *tcs_host,
-                             int nnl, const PsdNode *par, int psd_type, int scaling, double *S, bool fp32) {
+                             int nnl, const PsdNode *par, int psd_type, int scaling, double *S, bool fp32, bool root) {
     const long long tot = (long long)nf * ntc * nnl;
     if (tot == 0) return cudaSuccess;
     int4 tcs = make_int4(tcs_host[0], ntc > 1 ? tcs_host[1] : 0, ntc > 2 ? tcs_host[2] : 0, 0);
     const int blk = 256;
     const unsigned grid = (unsigned)((tot + blk - 1) / blk);
     if (fp32)
-        k_nodal_psd<float><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, S);
+        k_nodal_psd<float><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, root ? 1 : 0, S);
     else
-        k_nodal_psd<double><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, S);
+        k_nodal_psd<double><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, root ? 1 : 0, S);
     return cudaGetLastError();
 }
 
@@ -87,58 +87,90 @@ cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, 
 // Stage (a)+(b) factor: A(f)[(itc,i)][m] = sqrt(S_i) sum_j c_ij^|f| sqrt(S_j) L[(itc,j)][m].
 // The coherent cross-PSD c_ij^|f| sqrt(S_i S_j) (functionsImpl.F90:1450-1477,
 // getFullNodalPSD WindPSDImpl.F90:76-108) is generated on the fly from log c_ij and never
-// stored as an NNL^2 x NF tensor.  Block: 32 rows i x all modes, j streamed in tiles of
-// 32 through shared memory.  c^0 = 1 for every c (Fortran 0**0 = 1).
+// stored as an NNL^2 x NF tensor.  c^0 = 1 for every c (Fortran 0**0 = 1).
+//
+// Bound by the FP64 pipe (two FMAs an SM and clock): per (i, j) one exponential and nm FMAs.  Block:
+// 64 rows i x all modes, j streamed in tiles of 32; a thread holds one row and every fourth mode,
+// MPT of them, so nm is padded to a multiple of 4 only (8 threads a row and 8 slots each, tested
+// one by one, cost 12 modes a third of the pipe).  The exponential is expc, 10 FP64 instructions
+// where exp() spends about 25, and sqrt(S) comes from k_nodal_psd.  150 nodes, 12 modes, 3333
+// frequencies: 13.1 -> 3.9 ms.
 // ------------------------------------------------------------------------------------
+constexpr int kExpTab = 256;  // 2^(k / 256), k = 0 .. 255
+
+// e^x by table and polynomial (P. T. P. Tang, ACM TOMS 15, 1989): x = (256 q + k) ln2 / 256 + r,
+// |r| <= ln2 / 512, e^x = 2^q T[k] (1 + r + r^2/2 + r^3/6 + r^4/24); the next term is below 2^-54.
+// ln2 / 256 = hi + lo with hi of 25 bits, so that its product with the integer (18 bits) is exact.
+// Beyond |x| = 700, for infinities and for NaN: exp().
+__device__ __forceinline__ double expc(double x, const double *T) {
+    if (!(fabs(x) < 700.0)) return exp(x);
+    constexpr double kInv = 256.0 / 0.693147180559945309417232121458;
+    constexpr double kHi = 23258160.0 / 8589934592.0;  // round(2^33 ln2 / 256) / 2^33
+    constexpr double kLo = -7.4400558592100307755539978e-12;
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52: adding it rounds to an integer
+    const double z = fma(x, kInv, kMagic);
+    const int n = __double2loint(z);
+    const double kd = z - kMagic;
+    double r = fma(kd, -kHi, x);
+    r = fma(kd, -kLo, r);
+    double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
+    p = fma(p, r, 0.5);
+    p = fma(p, r * r, r);
+    const double t = T[n & (kExpTab - 1)];
+    const double v = fma(t, p, t);
+    return __hiloint2double(__double2hiint(v) + ((n >> 8) << 20), __double2loint(v));
+}
+
+template <int MPT>
 __global__ __launch_bounds__(256) void k_atable(int nf, const double *__restrict__ f, int ntc, int nnl,
                                                 int nm, const double *__restrict__ logc,
-                                                const double *__restrict__ S,
+                                                const double *__restrict__ expt,
+                                                const double *__restrict__ rootS,
                                                 const double *__restrict__ L, double *__restrict__ A) {
+    constexpr int RI = 64, JT = 32, NML = 4 * MPT;
     const int fi = blockIdx.x / ntc, itc = blockIdx.x % ntc;
-    const int i0 = blockIdx.y * 32;
-    __shared__ double Gs[32][33];
-    __shared__ double Ls[32][64];
+    const int i0 = blockIdx.y * RI;
+    __shared__ double T[kExpTab];
+    __shared__ double Gs[JT][RI + 1];
+    __shared__ double Ls[JT][NML];
     const double af = fabs(f[fi]);
-    const double *Sf = S + ((size_t)fi * ntc + itc) * nnl;
+    const double *Sf = rootS + ((size_t)fi * ntc + itc) * nnl;
     const double *lc = logc + (size_t)itc * nnl * nnl;
     const double *Lt = L + (size_t)itc * nnl * nm;
-    const int t = threadIdx.x, il = t >> 3, mg = t & 7;
-    double acc[8];
+    const int t = threadIdx.x, il = t >> 2, mg = t & 3;
+    T[t] = expt[t];
+    double acc[MPT];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) acc[u] = 0.0;
-    for (int j0 = 0; j0 < nnl; j0 += 32) {
-        for (int e = t; e < 32 * 32; e += 256) {
-            const int ii = e >> 5, jj = e & 31, gi = i0 + ii, gj = j0 + jj;
+    for (int u = 0; u < MPT; ++u) acc[u] = 0.0;
+    __syncthreads();
+    for (int j0 = 0; j0 < nnl; j0 += JT) {
+#pragma unroll
+        for (int u = 0; u < RI * JT / 256; ++u) {
+            const int e = t + 256 * u, ii = e >> 5, jj = e & 31, gi = i0 + ii, gj = j0 + jj;
             double g = 0.0;
-            if (gi < nnl && gj < nnl) {
-                const double l = lc[(size_t)gi * nnl + gj];
-                g = (af == 0.0) ? 1.0 : exp(af * l);
-            }
-            Gs[ii][jj] = g;
+            if (gi < nnl && gj < nnl) g = (af == 0.0) ? 1.0 : expc(af * lc[(size_t)gi * nnl + gj], T);
+            Gs[jj][ii] = g;
         }
-        for (int e = t; e < 32 * nm; e += 256) {
-            const int jj = e / nm, m = e % nm, gj = j0 + jj;
-            Ls[jj][m] = gj < nnl ? sqrt(Sf[gj]) * Lt[(size_t)gj * nm + m] : 0.0;
+        for (int e = t; e < JT * NML; e += 256) {
+            const int jj = e / NML, m = e % NML, gj = j0 + jj;
+            Ls[jj][m] = (gj < nnl && m < nm) ? Sf[gj] * Lt[(size_t)gj * nm + m] : 0.0;
         }
         __syncthreads();
 #pragma unroll 4
-        for (int jj = 0; jj < 32; ++jj) {
-            const double g = Gs[il][jj];
+        for (int jj = 0; jj < JT; ++jj) {
+            const double g = Gs[jj][il];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int m = mg + 8 * u;
-                if (m < nm) acc[u] = fma(g, Ls[jj][m], acc[u]);
-            }
+            for (int u = 0; u < MPT; ++u) acc[u] = fma(g, Ls[jj][mg + 4 * u], acc[u]);
         }
         __syncthreads();
     }
     const int gi = i0 + il;
     if (gi < nnl) {
-        const double si = sqrt(Sf[gi]);
+        const double si = Sf[gi];
         double *out = A + (((size_t)fi * ntc + itc) * nnl + gi) * nm;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int m = mg + 8 * u;
+        for (int u = 0; u < MPT; ++u) {
+            const int m = mg + 4 * u;
             if (m < nm) out[m] = si * acc[u];
         }
     }
@@ -152,19 +184,41 @@ __global__ void k_log_coh(size_t n, double *__restrict__ lc, float *__restrict__
     lc32[x] = (float)v;
 }
 
+__global__ void k_exp_tab(double *__restrict__ expt) { expt[threadIdx.x] = exp2((double)threadIdx.x / kExpTab); }
+
 cudaError_t launch_log_coh(cudaStream_t st, size_t n, double *lc, float *lc32) {
     if (n == 0) return cudaSuccess;
     k_log_coh<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, lc, lc32);
+    k_exp_tab<<<1, kExpTab, 0, st>>>(lc + n);
     return cudaGetLastError();
 }
 
+size_t log_coh_bytes(size_t n) { return sizeof(double) * (n + kExpTab); }
+
 cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm,
-                          const double *logc, const double *S, const double *L, double *A) {
+                          const double *logc, const double *rootS, const double *L, double *A) {
     if (nf == 0) return cudaSuccess;
     if (nm > 64) return cudaErrorInvalidValue;
-    dim3 grid((unsigned)nf * ntc, (unsigned)((nnl + 31) / 32));
-    k_atable<<<grid, 256, 0, st>>>(nf, f, ntc, nnl, nm, logc, S, L, A);
-    return cudaGetLastError();
+    const dim3 grid((unsigned)nf * ntc, (unsigned)((nnl + 63) / 64));
+    const double *expt = logc + (size_t)ntc * nnl * nnl;
+#define BSA_AT_CASE(V)                                                                          \
+    if (nm <= 4 * V) {                                                                          \
+        k_atable<V><<<grid, 256, 0, st>>>(nf, f, ntc, nnl, nm, logc, expt, rootS, L, A);        \
+        return cudaGetLastError();                                                              \
+    }
+    BSA_AT_CASE(1)
+    BSA_AT_CASE(2)
+    BSA_AT_CASE(3)
+    BSA_AT_CASE(4)
+    BSA_AT_CASE(5)
+    BSA_AT_CASE(6)
+    BSA_AT_CASE(8)
+    BSA_AT_CASE(10)
+    BSA_AT_CASE(12)
+    BSA_AT_CASE(14)
+    BSA_AT_CASE(16)
+#undef BSA_AT_CASE
+    return cudaErrorInvalidValue;
 }
 
 // ------------------------------------------------------------------------------------

@@ -5,16 +5,20 @@
 namespace bsa {
 
 // Nodal PSD S[f][itc][i] for nf frequencies (evalPSD_ and the model functions,
-// src/wind/WindPSDImpl.F90:123-316).  tcs: turbulent component ids (1..3) per itc.
+// src/wind/WindPSDImpl.F90:123-316).  tcs: turbulent component ids (1..3) per itc.  root: sqrt(S).
 cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, const int *tcs_host,
-                             int nnl, const PsdNode *par, int psd_type, int scaling, double *S, bool fp32 = false);
+                             int nnl, const PsdNode *par, int psd_type, int scaling, double *S, bool fp32 = false,
+                             bool root = false);
 
-// A[f][k][m] = sqrt(S_i(f)) sum_j c_ij^|f| sqrt(S_j(f)) L[(itc,j)][m]  (FP64).
-// lc[x] = log(lc[x]) in place (FP64) and lc32[x] = (float)lc[x]: the coherence table log c.
+// lc[x] = log(lc[x]) in place (FP64) and lc32[x] = (float)lc[x], x < n: the coherence table log c,
+// followed in lc by the table of the A kernel's exponential (log_coh_bytes(n) in all).
+size_t log_coh_bytes(size_t n);
 cudaError_t launch_log_coh(cudaStream_t st, size_t n, double *lc, float *lc32);
 
+// A[f][k][m] = sqrt(S_i(f)) sum_j c_ij^|f| sqrt(S_j(f)) L[(itc,j)][m]  (FP64); rootS = sqrt(S), logc
+// as launch_log_coh leaves it (n = ntc nnl^2).
 cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm,
-                          const double *logc, const double *S, const double *L, double *A);
+                          const double *logc, const double *rootS, const double *L, double *A);
 
 
 // The FP32 table on the tensor cores (bsa_atable_tc.cu): tf32 hi/lo split, FP32 accumulation;
