@@ -225,24 +225,34 @@ cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int
 // Second-order path: force PSD and m2 moments (functionsImpl.F90:1548-1560, 1653-1676;
 // BsaClassicImpl.F90:149-154, 197-210).
 // ------------------------------------------------------------------------------------
-template <class TA>
-__global__ void k_force_psd(int ntc, int nnl, int nm, const double *__restrict__ L, const TA *__restrict__ A,
-                            double *__restrict__ psd) {
-    const int fi = blockIdx.x;
-    const int nm2 = nm * nm, K = ntc * nnl;
-    const TA *Af = A + (size_t)fi * K * nm;
-    for (int pr = threadIdx.x; pr < nm2; pr += blockDim.x) {
-        const int n = pr % nm, o = pr / nm;
-        double s = 0.0;
-        for (int k = 0; k < K; ++k) s = fma(L[(size_t)k * nm + o], (double)Af[(size_t)k * nm + n], s);
-        psd[(size_t)fi * nm2 + pr] = s;
+// psd[f][n + nm o] = sum_k L[k][o] A[f][k][n]: 32 pairs (n, o) by 8 lanes over k per block, the lanes'
+// sums added in shared memory in a fixed order.  One thread a pair walking all k, in one block a
+// frequency, was bound by load latency: 65 rows of the 400-node, 24-mode building 0.56 -> 0.06 ms.
+__global__ __launch_bounds__(256) void k_force_psd(int ntc, int nnl, int nm, const double *__restrict__ L,
+                                                   const double *__restrict__ A, double *__restrict__ psd) {
+    __shared__ double red[8][32];
+    const int fi = blockIdx.x, nm2 = nm * nm, K = ntc * nnl;
+    const int pr = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
+    const int n = pr % nm, o = pr / nm;
+    const double *Af = A + (size_t)fi * K * nm + n, *Lo = L + o;
+    double s = 0.0;
+    if (pr < nm2)
+#pragma unroll 4
+        for (int k = lane; k < K; k += 8) s = fma(Lo[(size_t)k * nm], Af[(size_t)k * nm], s);
+    red[lane][threadIdx.x & 31] = s;
+    __syncthreads();
+    if (lane == 0 && pr < nm2) {
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v += red[q][threadIdx.x];
+        psd[(size_t)fi * nm2 + pr] = v;
     }
 }
 
 cudaError_t launch_force_psd(cudaStream_t st, int nf, int ntc, int nnl, int nm, const double *L,
                              const double *A, double *psd) {
     if (nf == 0) return cudaSuccess;
-    k_force_psd<double><<<nf, 256, 0, st>>>(ntc, nnl, nm, L, A, psd);
+    k_force_psd<<<dim3(nf, (nm * nm + 31) / 32), 256, 0, st>>>(ntc, nnl, nm, L, A, psd);
     return cudaGetLastError();
 }
 
