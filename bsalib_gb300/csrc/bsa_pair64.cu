@@ -40,29 +40,14 @@
 #include "../../include/bsa_gpu.h"
 #include "bsa_engine.cuh"
 #include "bsa_kernels.cuh"
+#include "bsa_pair64.cuh"
 
 namespace bsa {
 namespace p64 {
 
-constexpr int kTM = 128, kTN = 32;  // product tile: rows (x, a, b) by columns (y, j)
 constexpr int kKT = 16;
 constexpr int kKinds = 9;           // K1 .. K6 (the order above: abj, ajb, baj, jba, jab, bja), M1, M2, M3
 constexpr int kBatch = 8;           // pairs a thread takes between two barriers
-
-// A chunk of products: rows r = (x - x0) nm^2 + a nm + b of the first rows x in [x0, x1), in tiles
-// of kTM; row tile mt holds the column tiles ct0[mt] .. ct0[mt] + nct[mt] of c = y nm + j, row-major
-// from base[mt].
-struct RowTile {
-    int ct0, nct;
-    long long base;   // first element in E
-    long long item0;  // product tiles before this row tile
-};
-
-struct Chunk {
-    int x0, x1, nm, K, hi, ntiles;
-    const RowTile *rt;
-    double *E;
-};
 
 // E of one product tile: 256 threads, 4 x 4 elements each, K staged 16 at a time; the row operand
 // Q[k][a] A(x)[k][b] is formed while staging.  FP64-pipe bound: 16 FMAs a thread and k against one
@@ -71,11 +56,7 @@ __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__rest
     __shared__ double As[kKT][kTM], Bs[kKT][kTN];
     const int t = threadIdx.x, nm = c.nm, nm2 = nm * nm, K = c.K;
     const long long item = blockIdx.x;
-    int lo = 0, up = c.ntiles - 1;
-    while (lo < up) {
-        const int mid = (lo + up + 1) >> 1;
-        if (c.rt[mid].item0 <= item) lo = mid; else up = mid - 1;
-    }
+    const int lo = tile_row(c, item);
     const RowTile rt = c.rt[lo];
     const int ct = rt.ct0 + (int)(item - rt.item0);
     const int r0 = lo * kTM, rows = (c.x1 - c.x0) * nm2;
@@ -343,8 +324,14 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     const long long pairs_all = (long long)(N + 1) * (N + 2) / 2 + (analytic ? (long long)N * (N + 1) / 2 : 0);
     const int G = (int)std::max(1LL, std::min<long long>((608 + tiles - 1) / tiles,
                                                          (pairs_all + kBatch * PL - 1) / (kBatch * PL)));
-    // chunks of first rows: at most 4 GB of products each (all of a 400-row, 24-mode grid in one)
+    // Products on the tensor cores (bsa_pair64_tc.cu) where they outweigh the digits' preparation.
+    // Measured contraction, FP64 pipe / tensor cores: 4.1e6 FMAs, K = 30: 0.097 / 0.108 ms; 7.3e6,
+    // K = 60: 0.126 / 0.109; 1.9e7, K = 20: 0.137 / 0.167; 5.4e7, K = 12: 0.353 / 0.447; 6.9e7,
+    // K = 30: 0.285 / 0.240 (K is padded to 16, and the moments do not get faster).
+    const bool tensor = K >= 24 && pairs_all * nm3 * K >= 7000000LL;
+    // chunks of first rows: at most 4 GB of products and of row digits each
     const long long cap = 1LL << 29;
+    const int Kd = (K + 63) / 64 * 64 * 2;  // digits of a row in doubles
     struct Plan { int x0, x1, ntiles; long long items, elems, npairs; size_t rt0, pre0; };
     std::vector<Plan> plans;
     std::vector<RowTile> rts;
@@ -371,7 +358,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
         long long el = 0;
         int x1 = x0;
         while (x1 <= N) {
-            const long long add = (long long)nm2 * ((ylast(x1) - x1 + 1) * (long long)nm + 2 * kTN);
+            const long long add = (long long)nm2 * std::max((ylast(x1) - x1 + 1) * (long long)nm + 2 * kTN, (long long)Kd);
             if (x1 > x0 && el + add > cap) break;
             el += add;
             ++x1;
@@ -386,14 +373,20 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
         plans.push_back(p);
         x0 = x1;
     }
-    long long emax = 0;
-    for (const Plan &p : plans) emax = std::max(emax, p.elems);
+    long long emax = 0, rmax = 0;
+    for (const Plan &p : plans) {
+        emax = std::max(emax, p.elems);
+        rmax = std::max(rmax, (long long)(p.x1 - p.x0) * nm2);
+    }
     const size_t rtb = sizeof(RowTile) * rts.size(), preb = sizeof(long long) * pre.size();
     const size_t hb = sizeof(double2) * (size_t)(2 * N + 1) * nm;
     if ((e = dMixA.reserve(sizeof(double) * (size_t)emax)) || (e = dMixH.reserve(hb)) || (e = dMshIdx.reserve(rtb + preb)) ||
         (e = dPartF.reserve(sizeof(double) * (size_t)G * kKinds * nm3)) ||
         (e = dPartR.reserve(sizeof(double) * (size_t)kKinds * nm3)) ||
         (e = dOut.reserve(sizeof(double) * (3 * (size_t)nm2 + 2 * (size_t)nm3))))
+        return cuda_fail(e, "allocating pair products");
+    if (tensor && ((e = dMixB.reserve(tc_col_bytes(hi + 1, nm, K))) || (e = dMshT.reserve(tc_row_bytes(rmax, K))) ||
+                   (e = dFlag.reserve(256))))
         return cuda_fail(e, "allocating pair products");
     char *idx = (char *)dMshIdx.p;
     if ((e = cudaMemcpyAsync(idx, rts.data(), rtb, cudaMemcpyHostToDevice, stream)) ||
@@ -408,10 +401,20 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
                                  sizeof(double2) * (size_t)PB * nm * 3 + sizeof(PairInfo) * (size_t)PB);
     if ((e = cudaFuncSetAttribute(k_pair_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
         return cuda_fail(e, "pair moments kernel");
+    if (tensor && ((e = cudaMemsetAsync(dFlag.p, 0, sizeof(int), stream)) ||
+                   (e = tc_prep_cols(stream, hi + 1, nm, K, dA.as<double>(), dMixB.p))))
+        return cuda_fail(e, "pair product operands");
+    if (tensor) kernels += 2;
     for (size_t q = 0; q < plans.size(); ++q) {
         const Plan &p = plans[q];
-        Chunk c{p.x0, p.x1, nm, K, hi, p.ntiles, (const RowTile *)idx + p.rt0, dMixA.as<double>()};
-        k_pair_gemm<<<(unsigned)p.items, 256, 0, stream>>>(c, dA.as<double>(), dQ.as<double>());
+        Chunk c{p.x0, p.x1, nm, K, hi, p.ntiles, p.items, (const RowTile *)idx + p.rt0, dMixA.as<double>()};
+        if (tensor) {
+            if ((e = tc_products(stream, c, hi + 1, dA.as<double>(), dQ.as<double>(), dMixB.p, dMshT.p, dFlag.as<int>())))
+                return cuda_fail(e, "pair product kernel");
+            kernels += 2;
+        } else {
+            k_pair_gemm<<<(unsigned)p.items, 256, 0, stream>>>(c, dA.as<double>(), dQ.as<double>());
+        }
         MomPar mp{N, vect ? 1 : 0, p.npairs, (const long long *)(idx + rtb) + p.pre0, dMixH.as<double2>(), 4.0 * wval,
                   dPartF.as<double>(), q == 0 ? 1 : 0, RT, PL};
         k_pair_moments<<<dim3((unsigned)tiles, (unsigned)G), 256, smem, stream>>>(c, mp);
@@ -426,9 +429,12 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     if ((e = cudaGetLastError())) return cuda_fail(e, "reduction kernel");
     kernels += 3;
     std::vector<double> h(2 * (size_t)nm3);
+    int herr = 0;
     if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
+        (tensor && (e = cudaMemcpyAsync(&herr, dFlag.p, sizeof(int), cudaMemcpyDeviceToHost, stream))) ||
         (e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream)))
         return cuda_fail(e, "moment copy");
+    if (herr) return fail(BSA_ERR_TIMEOUT, "pair product kernel: a pipeline wait ran out of its budget (role %d)", herr);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev2, ev1);
     last_ms_contraction = ms;

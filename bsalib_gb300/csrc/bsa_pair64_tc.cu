@@ -1,0 +1,428 @@
+// bsa_pair64_tc.cu -- FP64 products on the tensor cores, by error-free splitting (K. Ozaki,
+// T. Ogita, S. Oishi, S. M. Rump, Numer. Algorithms 59, 2012; on half-precision tensor cores:
+// D. Mukunoki, K. Ozaki, T. Ogita, T. Imamura, ISC 2020).
+//
+// Each operand row (fixed x, a, b or y, j; contiguous k) is scaled by a power of two above its
+// largest magnitude, rounded to a 56-bit integer and cut into eight balanced base-128 digits
+// |d| <= 64, stored as bf16 (exact).  The digit products s + t = l < 8 are summed in FP32 in TMEM:
+// at most 8 x 512 products of at most 2^12, so every partial sum is an integer within 2^24 and
+// exact; longer K is cut into passes of 512 whose sums meet in 64-bit integers.  The eight level
+// sums combine exactly in integers and round once to FP64, with no FP64 instruction (the pipe is
+// two lanes an SM and clock).  Rounding the rows at 2^-55 of their scale and leaving out the levels
+// s + t >= 8 is an error of about sqrt(8 K) 2^-57 of the row scales' product, below that of K
+// FP64 FMAs.
+//
+// Cost: 36 digit products of bf16 against the DFMA kernel's one FP64 FMA: 36 / 4096 clocks of an SM
+// against 1 / 2.  Tile: 128 rows by 32 columns; the B digits of the tile are stacked along N (256
+// rows), so A digit s meets B digits 0 .. 7 - s in one MMA of N = (8 - s) 32 whose columns land on
+// levels s .. 7: 8 MMAs a K step instead of 36, and 512 TMEM columns hold two tiles.
+// 400 nodes x 2 components, 24 modes, 65 rows: FP64 pipe 40.5 ms; 1.33 ms here (8.5e11 digit FMAs,
+// 0.65 of the bf16 rate), row digits 0.35 ms.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "bsa_pair64.cuh"
+#include "bsa_tc.cuh"
+
+namespace bsa {
+namespace p64 {
+
+using namespace tc;
+
+constexpr int kDig = 8;                  // digits per operand
+constexpr int kPassK = 512 / kBK;        // K blocks of one exact pass
+constexpr int kRingA = 8;                // A digit tiles in flight (16 KB each)
+constexpr int kRingB = 2;                // B tiles in flight (32 KB each)
+constexpr int kTileA = kTM * 128, kTileB = kDig * kTN * 128;
+constexpr int kTcThreads = 192;
+constexpr size_t kTcSmem = 1024 + (size_t)kRingA * kTileA + (size_t)kRingB * kTileB + 512;
+constexpr int kBad = 1 << 20;            // row exponent of a row that holds an infinity or a NaN
+constexpr int kNone = -(1 << 20);        // of a row of zeros
+
+// Biased exponent field (0 for zeros and denormals, 2047 for infinities and NaN).
+__device__ __forceinline__ int expo(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+
+// Sixteen values of one row, scaled by 2^(55 - e), as digits: dst[s plane + 0 .. 15].
+__device__ __forceinline__ void put_digits(const double *v, int e, __nv_bfloat16 *dst, size_t plane) {
+    uint32_t w[kDig][8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        uint32_t f[2][kDig];
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+            const double x = v[2 * q + z];
+            const int ex = expo(x), sh = 3 + (ex - 1023) - e;
+            unsigned long long m = ((unsigned long long)__double_as_longlong(x) & 0xfffffffffffffull) | 0x10000000000000ull;
+            if (sh >= 0) m <<= sh;
+            else if (sh > -60) m = (m + (1ull << (-sh - 1))) >> -sh;
+            else m = 0;
+            if (ex == 0) m = 0;
+            // balanced digits: add 64 to every digit, cut into 7 bits, take 64 away
+            constexpr unsigned long long kHalf = 64ull * ((1ull << 56) - 1) / 127ull;
+            const unsigned long long u = (__double2hiint(x) < 0 ? 0ull - m : m) + kHalf;
+#pragma unroll
+            for (int s = 0; s < kDig; ++s) {
+                const int sft = 7 * (kDig - 1 - s);
+                const uint32_t d = s == 0 ? (uint32_t)(u >> sft) : (uint32_t)(u >> sft) & 127u;
+                // integer d - 64 as a float (exact in bf16: its low half is zero)
+                f[z][s] = __float_as_uint(__uint_as_float(0x4B400000u + d - 64u) - 12582912.f);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < kDig; ++s) w[s][q] = __byte_perm(f[0][s], f[1][s], 0x7632);
+    }
+#pragma unroll
+    for (int s = 0; s < kDig; ++s) {
+        uint4 *o = reinterpret_cast<uint4 *>(dst + s * plane);
+        o[0] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+        o[1] = make_uint4(w[s][4], w[s][5], w[s][6], w[s][7]);
+    }
+}
+
+// Column operand: exponent e[c] with |A[y][k][j]| < 2^e[c], c = y nm + j.
+__global__ void k_col_exp(int nm, int K, const double *__restrict__ A, int *__restrict__ ec) {
+    __shared__ int mx[64];
+    const int y = blockIdx.x;
+    if (threadIdx.x < 64) mx[threadIdx.x] = 0;
+    __syncthreads();
+    const double *a = A + (size_t)y * K * nm;
+    for (int q = threadIdx.x; q < K * nm; q += blockDim.x) atomicMax(&mx[q % nm], expo(a[q]));
+    __syncthreads();
+    if ((int)threadIdx.x < nm) {
+        const int m = mx[threadIdx.x];
+        ec[y * nm + threadIdx.x] = m == 2047 ? kBad : m == 0 ? kNone : m - 1022;
+    }
+}
+
+// Row operand: |Q[k][a] A(x)[k][b]| < 2^e[r] from the factors' exponents (at most a bit above).
+// 32 rows by 8 lanes over k per block.
+__global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restrict__ A, const double *__restrict__ Q,
+                                                 int *__restrict__ er) {
+    __shared__ int mx[8][32];
+    const int nm = c.nm, nm2 = nm * nm, ab = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
+    const int x = c.x0 + blockIdx.x, a = ab / nm, b = ab - a * nm;
+    const int *q = reinterpret_cast<const int *>(Q + a) + 1, *p = reinterpret_cast<const int *>(A + (size_t)x * c.K * nm + b) + 1;
+    int m = 0;
+    if (ab < nm2)
+#pragma unroll 8
+        for (int k = lane; k < c.K; k += 8) {
+            const int u = (q[(size_t)2 * k * nm] >> 20) & 0x7ff, v = (p[(size_t)2 * k * nm] >> 20) & 0x7ff;
+            m = max(m, (u == 2047 || v == 2047) ? kBad : (u && v) ? u + v : 0);
+        }
+    mx[lane][threadIdx.x & 31] = m;
+    __syncthreads();
+    if (lane == 0 && ab < nm2) {
+#pragma unroll
+        for (int z = 1; z < 8; ++z) m = max(m, mx[z][threadIdx.x]);
+        er[(size_t)blockIdx.x * nm2 + ab] = m == kBad ? kBad : m == 0 ? kNone : m - 2044;
+    }
+}
+
+// Column digits [ct][digit][32 columns][Kp]; block: one column tile, 128 k.
+__global__ __launch_bounds__(256) void k_col_digits(int nr, int nm, int K, int Kp, const double *__restrict__ A,
+                                                    const int *__restrict__ ec, __nv_bfloat16 *__restrict__ D) {
+    const int ct = blockIdx.x, col = threadIdx.x & 31, k0 = blockIdx.y * 128 + (threadIdx.x >> 5) * 16;
+    if (k0 >= Kp) return;
+    const int c = ct * kTN + col, y = c / nm, j = c - y * nm;
+    const bool ok = y < nr;
+    const int e = ok ? ec[c] : kNone;
+    const bool some = e != kNone && e != kBad;
+    double v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = (some && k0 + i < K) ? A[((size_t)y * K + k0 + i) * nm + j] : 0.0;
+    put_digits(v, some ? e : 0, D + ((size_t)ct * kDig * kTN + col) * Kp + k0, (size_t)kTN * Kp);
+}
+
+// Row digits [mt][digit][128 rows][Kp]; block: one x, 64 k, every (a, b).
+__global__ __launch_bounds__(256) void k_row_digits(Chunk c, int Kp, const double *__restrict__ A,
+                                                    const double *__restrict__ Q, const int *__restrict__ er,
+                                                    __nv_bfloat16 *__restrict__ D) {
+    extern __shared__ double sm[];
+    const int nm = c.nm, nm2 = nm * nm, K = c.K, xl = blockIdx.x, kb = blockIdx.y * 64;
+    double *As = sm, *Qs = sm + 64 * nm;
+    const int n = max(0, min(64, K - kb)) * nm;
+    const double *a = A + ((size_t)(c.x0 + xl) * K + kb) * nm, *q = Q + (size_t)kb * nm;
+    for (int i = threadIdx.x; i < 64 * nm; i += 256) {
+        As[i] = i < n ? a[i] : 0.0;
+        Qs[i] = i < n ? q[i] : 0.0;
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < nm2 * 4; w += 256) {
+        const int kq = w / nm2, ab = w - kq * nm2, ia = ab / nm, ib = ab - ia * nm;
+        const long long r = (long long)xl * nm2 + ab;
+        const int e = er[r];
+        const bool some = e != kNone && e != kBad;
+        double v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int k = kq * 16 + i;
+            v[i] = some ? Qs[k * nm + ia] * As[k * nm + ib] : 0.0;
+        }
+        put_digits(v, some ? e : 0, D + ((r / kTM) * kDig * kTM + r % kTM) * (size_t)Kp + kb + kq * 16, (size_t)kTM * Kp);
+    }
+}
+
+__device__ __forceinline__ void mma_n(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr));
+}
+
+// (hi 2^28 + lo) 2^ex rounded once to FP64, in integer instructions.
+__device__ __forceinline__ double combine(long long hi, long long lo, int ex) {
+    long long h = hi + (lo >> 28);
+    uint32_t l = (uint32_t)lo & 0xfffffffu;
+    const bool neg = h < 0;
+    if (neg) {
+        h = -h - (l != 0);
+        l = (0x10000000u - l) & 0xfffffffu;
+    }
+    if (h == 0 && l == 0) return 0.0;
+    const int lz = __clzll(h), E = 91 - lz + ex;
+    if (lz > 35 || E < -1022 || E > 1022) {  // small sums (28 bits of h at least otherwise) and the ends of the range
+        const double v = scalbn(fma((double)h, 268435456.0, (double)l), ex);
+        return neg ? -v : v;
+    }
+    const unsigned long long w = ((unsigned long long)h << lz) |
+                                 (lz >= 28 ? (unsigned long long)l << (lz - 28) : (unsigned long long)(l >> (28 - lz)));
+    // top bit of w at 63: 53 bits and the rounding bit
+    unsigned long long b = (w >> 11) + ((w >> 10) & 1ull) + ((unsigned long long)(E + 1022) << 52);
+    if (neg) b |= 0x8000000000000000ull;
+    return __longlong_as_double((long long)b);
+}
+
+__global__ void __launch_bounds__(kTcThreads, 1)
+    k_pair_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Chunk c, int nk,
+              int ks_last, const int *__restrict__ er, const int *__restrict__ ec, int *err) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t *sa = smem, *sb = smem + (size_t)kRingA * kTileA;
+    uint64_t *bars = (uint64_t *)(sb + (size_t)kRingB * kTileB);
+    uint64_t *fa = bars, *ea = fa + kRingA, *fb = ea + kRingA, *eb = fb + kRingB, *tfull = eb + kRingB, *tempty = tfull + 2,
+             *done = tempty + 2;
+    uint32_t *tmem_slot = (uint32_t *)(done + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kRingA; ++s) {
+            mbar_init(&fa[s], 1);
+            mbar_init(&ea[s], 1);
+        }
+        for (int s = 0; s < kRingB; ++s) {
+            mbar_init(&fb[s], 1);
+            mbar_init(&eb[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&tfull[b], 1);
+            mbar_init(&tempty[b], 128);
+        }
+        mbar_init(done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(su32(tmem_slot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        // ---------------- TMA producer ----------------
+        if (lane == 0) {
+            uint32_t ia = 0, ib = 0;
+            bool ok = true;
+            for (long long item = blockIdx.x; item < c.items && ok; item += gridDim.x) {
+                const int mt = tile_row(c, item);
+                const int ct = c.rt[mt].ct0 + (int)(item - c.rt[mt].item0);
+                for (int kb = 0; kb < nk && ok; ++kb, ++ib) {
+                    const int sB = ib % kRingB;
+                    if (!mbar_wait(&eb[sB], ((ib / kRingB) & 1u) ^ 1u, err, 1)) { ok = false; break; }
+                    mbar_expect_tx(&fb[sB], kTileB);
+                    tma_2d(sb + sB * kTileB, &tmB, &fb[sB], kb * kBK, ct * kDig * kTN);
+                    for (int s = 0; s < kDig; ++s, ++ia) {
+                        const int sA = ia % kRingA;
+                        if (!mbar_wait(&ea[sA], ((ia / kRingA) & 1u) ^ 1u, err, 1)) { ok = false; break; }
+                        mbar_expect_tx(&fa[sA], kTileA);
+                        tma_2d(sa + sA * kTileA, &tmA, &fa[sA], kb * kBK, (mt * kDig + s) * kTM);
+                    }
+                }
+            }
+            // copies in flight land before the block leaves
+            for (uint32_t q = (ia > (uint32_t)kRingA ? ia - kRingA : 0); q < ia; ++q) {
+                const uint64_t t0 = gtime();
+                while (!mbar_try(&fa[q % kRingA], (q / kRingA) & 1u) && gtime() - t0 < kWaitNs) {
+                }
+            }
+            for (uint32_t q = (ib > (uint32_t)kRingB ? ib - kRingB : 0); q < ib; ++q) {
+                const uint64_t t0 = gtime();
+                while (!mbar_try(&fb[q % kRingB], (q / kRingB) & 1u) && gtime() - t0 < kWaitNs) {
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ---------------- MMA issuer ----------------
+        if (lane == 0) {
+            uint32_t ia = 0, ib = 0, tile = 0;
+            bool ok = true;
+            for (long long item = blockIdx.x; item < c.items && ok; item += gridDim.x) {
+                for (int k0 = 0; k0 < nk && ok; k0 += kPassK, ++tile) {
+                    const int buf = tile & 1;
+                    if (!mbar_wait(&tempty[buf], ((tile >> 1) & 1u) ^ 1u, err, 2)) { ok = false; break; }
+                    fence_after();
+                    const uint32_t d = tmem + buf * 256;
+                    const int k1 = min(nk, k0 + kPassK);
+                    for (int kb = k0; kb < k1 && ok; ++kb, ++ib) {
+                        const int sB = ib % kRingB;
+                        if (!mbar_wait(&fb[sB], (ib / kRingB) & 1u, err, 3)) { ok = false; break; }
+                        const uint32_t bb = su32(sb + sB * kTileB);
+                        const int nks = kb == nk - 1 ? ks_last : kBK / 16;
+                        // unrolled: with the loops kept, issuing took longer than the MMAs (a product
+                        // of 400 nodes x 2 components, 24 modes, 65 rows 1.80 ms, unrolled 1.33 ms)
+#pragma unroll
+                        for (int s = 0; s < kDig; ++s, ++ia) {
+                            const int sA = ia % kRingA;
+                            if (!mbar_wait(&fa[sA], (ia / kRingA) & 1u, err, 3)) { ok = false; break; }
+                            fence_after();
+                            const uint32_t ab = su32(sa + sA * kTileA);
+                            // N = (8 - s) 32 columns from level s on
+                            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                                                   ((uint32_t)((kDig - s) * kTN >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
+#pragma unroll
+                            for (int ks = 0; ks < kBK / 16; ++ks)
+                                if (ks < nks)
+                                    mma_n(d + s * kTN, sdesc(ab + ks * 32), sdesc(bb + ks * 32), idesc,
+                                          (kb > k0 || ks > 0 || s > 0) ? 1u : 0u);
+                            mma_commit(&ea[sA]);
+                        }
+                        if (ok) mma_commit(&eb[sB]);
+                    }
+                    if (ok) mma_commit(&tfull[buf]);
+                }
+            }
+            mma_commit(done);
+            const uint64_t t0 = gtime();
+            while (!mbar_try(done, 0) && gtime() - t0 < kWaitNs) {
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---------------- epilogue: 128 rows, one a thread ----------------
+        const int quarter = warp & 3, row = quarter * 32 + lane;
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+        const int nrows = (c.x1 - c.x0) * c.nm * c.nm, ncols = (c.hi + 1) * c.nm;
+        uint32_t tile = 0;
+        bool ok = true;
+        for (long long item = blockIdx.x; item < c.items && ok; item += gridDim.x) {
+            const int mt = tile_row(c, item);
+            const RowTile rt = c.rt[mt];
+            const int ct = rt.ct0 + (int)(item - rt.item0);
+            long long hi[kTN], lo[kTN];
+#pragma unroll
+            for (int q = 0; q < kTN; ++q) hi[q] = lo[q] = 0;
+            for (int k0 = 0; k0 < nk && ok; k0 += kPassK, ++tile) {
+                const int buf = tile & 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (tile >> 1) & 1u, err, 4));
+                if (!ok) break;
+                fence_after();
+#pragma unroll
+                for (int cg = 0; cg < kTN / 8; ++cg) {
+                    uint32_t v[kDig][8];
+#pragma unroll
+                    for (int l = 0; l < kDig; ++l) tmem_ld8(lane_base + buf * 256 + l * kTN + cg * 8, v[l]);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        int D[kDig];
+#pragma unroll
+                        for (int l = 0; l < kDig; ++l) D[l] = __float2int_rn(__uint_as_float(v[l][q]));
+                        hi[cg * 8 + q] += (((long long)D[0] * 128 + D[1]) * 128 + D[2]) * 128 + D[3];
+                        lo[cg * 8 + q] += (((long long)D[4] * 128 + D[5]) * 128 + D[6]) * 128 + D[7];
+                    }
+                }
+                fence_before();
+                mbar_arrive(&tempty[buf]);
+            }
+            const int r = mt * kTM + row;
+            if (ok && r < nrows) {
+                const int eu = er[r];
+                double *o = c.E + rt.base + (size_t)row * rt.nct * kTN + (size_t)(ct - rt.ct0) * kTN;
+#pragma unroll
+                for (int q = 0; q < kTN; q += 2) {
+                    double2 p;
+#pragma unroll
+                    for (int z = 0; z < 2; ++z) {
+                        const int col = ct * kTN + q + z, ev = col < ncols ? ec[col] : kNone;
+                        // value = 2^(er + ec - 61) (hi 2^28 + lo)
+                        const double s = (eu == kBad || ev == kBad) ? __longlong_as_double(0x7ff8000000000000ll)
+                                         : (eu == kNone || ev == kNone) ? 0.0
+                                                                        : combine(hi[q + z], lo[q + z], eu + ev - 61);
+                        (z ? p.y : p.x) = s;
+                    }
+                    *reinterpret_cast<double2 *>(o + q) = p;
+                }
+            }
+        }
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+static int kpad(int K) { return (K + kBK - 1) / kBK * kBK; }
+static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+// [digits][exponents]
+size_t tc_col_bytes(int nr, int nm, int K) {
+    const size_t ct = ((size_t)nr * nm + kTN - 1) / kTN;
+    return up256(ct * kDig * kTN * kpad(K) * 2) + up256(sizeof(int) * (size_t)nr * nm);
+}
+size_t tc_row_bytes(long long nrows, int K) {
+    const size_t mt = (size_t)((nrows + kTM - 1) / kTM);
+    return up256(mt * kDig * kTM * kpad(K) * 2) + up256(sizeof(int) * (size_t)nrows);
+}
+
+cudaError_t tc_prep_cols(cudaStream_t st, int nr, int nm, int K, const double *A, void *cols) {
+    const int Kp = kpad(K), nct = (nr * nm + kTN - 1) / kTN;
+    int *ec = (int *)((char *)cols + up256((size_t)nct * kDig * kTN * Kp * 2));
+    k_col_exp<<<nr, 256, 0, st>>>(nm, K, A, ec);
+    k_col_digits<<<dim3(nct, (Kp + 127) / 128), 256, 0, st>>>(nr, nm, K, Kp, A, ec, (__nv_bfloat16 *)cols);
+    return cudaGetLastError();
+}
+
+cudaError_t tc_products(cudaStream_t st, const Chunk &c, int nr, const double *A, const double *Q, void *cols,
+                        void *rows, int *err) {
+    const int Kp = kpad(c.K), nm2 = c.nm * c.nm, nx = c.x1 - c.x0;
+    const size_t nct = ((size_t)nr * c.nm + kTN - 1) / kTN, nmt = (size_t)c.ntiles;
+    int *ec = (int *)((char *)cols + up256(nct * kDig * kTN * Kp * 2));
+    int *er = (int *)((char *)rows + up256(nmt * kDig * kTM * Kp * 2));
+    k_row_exp<<<dim3(nx, (nm2 + 31) / 32), 256, 0, st>>>(c, A, Q, er);
+    const size_t sm = sizeof(double) * 2 * 64 * c.nm;
+    cudaError_t e = cudaFuncSetAttribute(k_row_digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k_row_digits<<<dim3(nx, Kp / 64), 256, sm, st>>>(c, Kp, A, Q, er, (__nv_bfloat16 *)rows);
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, rows, Kp, (uint64_t)nmt * kDig * kTM, kTM) ||
+        !make_map(&mb, cols, Kp, (uint64_t)nct * kDig * kTN, kDig * kTN))
+        return cudaErrorInvalidValue;
+    if ((e = cudaFuncSetAttribute(k_pair_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem))) return e;
+    int dev = 0, nsm = 0;
+    if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev))) return e;
+    const int nk = Kp / kBK, ks_last = (c.K - (nk - 1) * kBK + 15) / 16;
+    k_pair_tc<<<(unsigned)std::min<long long>(nsm, c.items), kTcThreads, kTcSmem, st>>>(ma, mb, c, nk, ks_last, er, ec, err);
+    return cudaGetLastError();
+}
+
+}  // namespace p64
+}  // namespace bsa

@@ -47,3 +47,36 @@ def test_pairs_one_component(bsalib):
     p = random_structure(11, nodes=(37, 37), modes=(9, 9), nfreq_grid=(41, 41))
     a, b = _run(p, (0, 20)), _run(p, (20, 41))
     _close(_run(p), {k: a[k] + b[k] for k in a})
+
+
+# tensor-core products: K around a 16-wide step, a 64-wide block and the 512-wide exact pass; rows that
+# share a tile and rows that span several
+@pytest.mark.parametrize("nodes,modes,nfreqs", [(12, 33, 9), (32, 9, 33), (33, 7, 40), (256, 5, 40), (257, 5, 40),
+                                                (550, 3, 34), (20, 64, 4)])
+@pytest.mark.parametrize("trunc", [True, False])
+def test_tensor_pairs_against_points(bsalib, nodes, modes, nfreqs, trunc):
+    p = tall_building(nodes=nodes, modes=modes, nfreqs=nfreqs, df=2.0 / nfreqs, seed=modes)
+    nf = p.classic_nf()
+    whole = _run(p, trunc=trunc)
+    a, b = _run(p, (0, nf // 2), trunc), _run(p, (nf // 2, nf), trunc)
+    _close(whole, {k: a[k] + b[k] for k in a})
+
+
+def test_tensor_pairs_wide_range(bsalib):
+    """Mode shapes over twelve decades along the height and modes scaled apart by 1e60: a row's small
+    entries lie far below its scale, whole rows far apart from each other."""
+    p = tall_building(nodes=64, modes=8, nfreqs=40, df=0.05, seed=5)
+    p.wfc[0, :3, :] *= np.logspace(0, -12, p.nn)
+    p.phi[:, 3] *= np.where(np.abs(p.phi[:, 3]) == 1.0, 1.0, 1e-60)
+    nf = p.classic_nf()
+    a, b = _run(p, (0, 20)), _run(p, (20, nf))
+    _close(_run(p), {k: a[k] + b[k] for k in a})
+
+
+def test_tensor_pairs_not_finite(bsalib):
+    p = tall_building(nodes=64, modes=8, nfreqs=40, df=0.05, seed=5)
+    p.wfc[0, 0, 7] = np.inf
+    nf = p.classic_nf()
+    whole, a, b = _run(p), _run(p, (0, 20)), _run(p, (20, nf))
+    for k in ("m3mf_cls", "m3mr_cls"):
+        assert np.array_equal(np.isfinite(whole[k]), np.isfinite(a[k] + b[k]))
