@@ -499,7 +499,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
     // (bsa_pair64.cu), on the A rows of f >= 0 alone.  Row shards, materialised or exported bispectra
     // and the frequency convention's one-sided grid (its truncated sum reads another row than
     // |f1 + f2|) keep the point kernel.
-    const bool pair64 = !diagonal && !mixed && !bf_host && !br_host && !export_fn && !brm_file_wanted(true) &&
+    const bool pair64 = !mixed && !bf_host && !br_host && !export_fn && !brm_file_wanted(true) &&
                         set.defsc == 1 && (nf & 1) && r0 == 0 && r1 == nf;
     const int half = (nf - 1) / 2;
     const double df_grid = f[half + 1] - f[half];  // the step itself (f[half] = 0): f[1] - f[0] is rounded
@@ -591,10 +591,10 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
             if (r0 != 0 || r1 != nf) return fail(BSA_ERR_ARG, "the bispectrum export needs the full grid");
             rc = classic_export(ps, f, m3mf, m3mr);
         } else {
-            rc = diagonal ? contract_diag(ps, npts, 0, m3mf, m3mr, bf_host, br_host)
-                 : mixed  ? contract_mixed(ps, npts, m3mf, m3mr)
-                 : pair64 ? contract_pair64(half, df_grid, analytic, !scalar, delta * delta, m3mf, m3mr)
-                          : contract(ps, npts, m3mf, m3mr, bf_host, br_host);
+            rc = pair64     ? contract_pair64(half, df_grid, analytic, !scalar, delta * delta, m3mf, m3mr)
+                 : diagonal ? contract_diag(ps, npts, 0, m3mf, m3mr, bf_host, br_host)
+                 : mixed    ? contract_mixed(ps, npts, m3mf, m3mr)
+                            : contract(ps, npts, m3mf, m3mr, bf_host, br_host);
         }
         if (rc) return rc;
         last_points = (double)npts;

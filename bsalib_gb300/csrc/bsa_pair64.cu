@@ -54,21 +54,21 @@ constexpr int kBatch = 8;           // pairs a thread takes between two barriers
 // product in 32 for the staging.
 __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__restrict__ A, const double *__restrict__ Q) {
     __shared__ double As[kKT][kTM], Bs[kKT][kTN];
-    const int t = threadIdx.x, nm = c.nm, nm2 = nm * nm, K = c.K;
+    const int t = threadIdx.x, qn = c.qn, an = c.an, rx = c.rx(), K = c.K;
     const long long item = blockIdx.x;
     const int lo = tile_row(c, item);
     const RowTile rt = c.rt[lo];
     const int ct = rt.ct0 + (int)(item - rt.item0);
-    const int r0 = lo * kTM, rows = (c.x1 - c.x0) * nm2;
+    const int r0 = lo * kTM, rows = (c.x1 - c.x0) * rx;
     // this thread's staging row and column
     const int sr = t & (kTM - 1), kr = t >> 7;           // As: 2 k rows of 128 rows at a time
     const bool rv = r0 + sr < rows;
-    const int rr = rv ? r0 + sr : 0, x = c.x0 + rr / nm2, ab = rr % nm2, a = ab / nm, b = ab % nm;
-    const double *Qa = Q + a, *Ab = A + (size_t)x * K * nm + b;
+    const int rr = rv ? r0 + sr : 0, x = c.x0 + rr / rx, ab = rr % rx, a = ab / an, b = ab % an;
+    const double *Qa = Q + a, *Ab = A + (size_t)x * K * an + b;
     const int sc = t & (kTN - 1), kc = t >> 5;           // Bs: 8 k rows of 32 columns at a time
-    const int col = ct * kTN + sc, y = col / nm, j = col - y * nm;
+    const int col = ct * kTN + sc, y = col / an, j = col - y * an;
     const bool cv = y <= c.hi;
-    const double *Aj = A + (size_t)(cv ? y : 0) * K * nm + j;
+    const double *Aj = A + (size_t)(cv ? y : 0) * K * an + j;
     const int tr = (t >> 3) * 4, tc = (t & 7) * 4;
     double acc[4][4];
 #pragma unroll
@@ -80,12 +80,12 @@ __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__rest
 #pragma unroll
         for (int u = 0; u < kKT / 2; ++u) {
             const int k = kr + 2 * u;
-            As[k][sr] = (rv && k < kn) ? Qa[(size_t)(k0 + k) * nm] * Ab[(size_t)(k0 + k) * nm] : 0.0;
+            As[k][sr] = (rv && k < kn) ? Qa[(size_t)(k0 + k) * qn] * Ab[(size_t)(k0 + k) * an] : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < kKT / 8; ++u) {
             const int k = kc + 8 * u;
-            Bs[k][sc] = (cv && k < kn) ? Aj[(size_t)(k0 + k) * nm] : 0.0;
+            Bs[k][sc] = (cv && k < kn) ? Aj[(size_t)(k0 + k) * an] : 0.0;
         }
         __syncthreads();
         for (int k = 0; k < kn; ++k) {
@@ -124,7 +124,6 @@ struct MomPar {
     long long npairs;       // pairs (x, y) of the chunk
     const long long *pre;   // pairs before first row x0 + i, and the total
     const double2 *H;       // [2 N + 1][nm]
-    double w4;              // weight of an interior pair: 2 (the BFM's factor) x 2 (both points) x d^2
     double *part;           // [groups][kKinds][nm^2][nm]
     int first;              // first chunk: the partials are written, not added to
     int RT, PL;             // rows (a, b) of a block, pair lanes
@@ -143,13 +142,36 @@ struct PairInfo {
     double w1, w2p, w2m, w3p, w3m, wm1, wm2, wm3;
 };
 
+__device__ __forceinline__ PairInfo pair_info(int x, int y, int N, int vect) {
+    PairInfo f;
+    f.x = x;
+    f.y = y;
+    const double s = (x == y ? 0.5 : 1.0) * (x == 0 && y == 0 ? 0.5 : 1.0), sm = x == 0 ? 0.0 : s;
+    // plus partners (x, y), (x - y, y), (x, y - x); minus partners (x, -y), (x + y, -y), (x, -x - y)
+    const double a1 = wrel(x, y, N, vect);
+    f.w1 = s * a1;
+    f.w2p = s * wrel(x - y, y, N, vect);
+    f.w3p = s * wrel(x, y - x, N, vect);
+    f.w2m = sm * wrel(x + y, y, N, vect);
+    f.w3m = sm * wrel(x, x + y, N, vect);
+    f.wm1 = f.w1 + sm * a1;
+    f.wm2 = f.w2p + f.w2m;
+    f.wm3 = f.w3p + f.w3m;
+    f.region = 2;
+    if (x > 0 && x < y && f.w1 == 1.0 && f.w2p == 1.0 && f.w3p == 1.0) {
+        if (f.w2m == 1.0 && f.w3m == 1.0) f.region = 0;
+        else if (f.w2m == 0.0 && f.w3m == 0.0) f.region = 1;
+    }
+    return f;
+}
+
 // One block per (tile of RT rows (a, b), group of pairs); a thread holds one element (a, b, j) and
 // takes the pairs of its lane.  Per batch of kBatch x PL pairs: the pairs and weights, then the
 // products of the row factors (8 doubles a row) and the columns' FRF values in shared memory, then
 // 9 (all weights one), 14 (no sums on the grid) or 27 FP64 operations an element and pair.
 __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
     extern __shared__ double sm[];
-    const int t = threadIdx.x, nm = c.nm, nm2 = nm * nm;
+    const int t = threadIdx.x, nm = c.an, nm2 = nm * nm;
     const int PB = kBatch * P.PL, RT = P.RT, EL = RT * nm;
     double *rowf = sm;                                 // [PB][RT][8]
     double2 *colf = (double2 *)(rowf + (size_t)PB * RT * 8);  // [PB][nm][3]: Hx, P, D
@@ -170,26 +192,8 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
                 const int mid = (lo + up + 1) >> 1;
                 if (P.pre[mid] <= p) lo = mid; else up = mid - 1;
             }
-            PairInfo f;
-            f.x = c.x0 + lo;
-            f.y = f.x + (int)(p - P.pre[lo]);
-            const int x = f.x, y = f.y, N = P.N;
-            const double s = (x == y ? 0.5 : 1.0) * (x == 0 && y == 0 ? 0.5 : 1.0), sm_ = x == 0 ? 0.0 : s;
-            // plus partners (x, y), (x - y, y), (x, y - x); minus partners (x, -y), (x + y, -y), (x, -x - y)
-            const double a1 = wrel(x, y, N, P.vect);
-            f.w1 = s * a1;
-            f.w2p = s * wrel(x - y, y, N, P.vect);
-            f.w3p = s * wrel(x, y - x, N, P.vect);
-            f.w2m = sm_ * wrel(x + y, y, N, P.vect);
-            f.w3m = sm_ * wrel(x, x + y, N, P.vect);
-            f.wm1 = f.w1 + sm_ * a1;
-            f.wm2 = f.w2p + f.w2m;
-            f.wm3 = f.w3p + f.w3m;
-            f.region = 2;
-            if (x > 0 && x < y && f.w1 == 1.0 && f.w2p == 1.0 && f.w3p == 1.0) {
-                if (f.w2m == 1.0 && f.w3m == 1.0) f.region = 0;
-                else if (f.w2m == 0.0 && f.w3m == 0.0) f.region = 1;
-            }
+            const int x = c.x0 + lo;
+            PairInfo f = pair_info(x, x + (int)(p - P.pre[lo]), P.N, P.vect);
             info[t] = f;
         }
         __syncthreads();
@@ -296,7 +300,8 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
     }
 }
 
-// m3[m + nm n + nm^2 o] from the summed kinds [kKinds][(a, b)][j].
+// m3[m + nm n + nm^2 o] from the summed kinds [kKinds][(a, b)][j]; w4 = 2 (the BFM's factor) x 2 (a
+// point and its mirror) x d^2.
 __global__ void k_pair_finish(int nm, double w4, const double *__restrict__ S, double *__restrict__ m3mf,
                               double *__restrict__ m3mr) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, nm2 = nm * nm, nm3 = nm2 * nm;
@@ -307,28 +312,73 @@ __global__ void k_pair_finish(int nm, double w4, const double *__restrict__ S, d
     m3mf[x] = w4 * (at(6, m, n, o) + at(6, m, o, n) + at(7, n, m, o) + at(7, o, m, n) + at(8, o, n, m) + at(8, n, o, m));
 }
 
+// Diagonal-only spectra: the products are P_m(x, y) = sum_k Q_km L_km^2 S_k(x) S_k(y), rows (x, m),
+// columns y, and with a = b = j = m the twelve contributions collapse to
+// 2 (w1 + w2m + w3m) alpha + 2 (w1- + w2p + w3p) beta.  One block per (mode, group of x), a warp per
+// x with its lanes over y; part[group][0: force, 1: response][m].
+__global__ __launch_bounds__(256) void k_pair_moments_diag(Chunk c, int N, int analytic, int vect, double w4,
+                                                           const double2 *__restrict__ H, double *__restrict__ part) {
+    __shared__ double red[2][8];
+    const int m = blockIdx.x, nm = c.qn, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double sf = 0.0, sr = 0.0;
+    for (int x = c.x0 + blockIdx.y * 8 + warp; x < c.x1; x += 8 * gridDim.y) {
+        const int r = (x - c.x0) * nm + m, mt = r / kTM, y1 = analytic ? min(c.hi, x + N) : N;
+        const RowTile rt = c.rt[mt];
+        const double *e = c.E + rt.base + (size_t)(r - mt * kTM) * rt.nct * kTN - rt.ct0 * kTN;
+        const double2 hx = H[(size_t)x * nm + m];
+        for (int y = x + lane; y <= y1; y += 32) {
+            const PairInfo f = pair_info(x, y, N, vect);
+            const double2 hy = H[(size_t)y * nm + m], p = H[(size_t)min(x + y, 2 * N) * nm + m], d = H[(size_t)(y - x) * nm + m];
+            const double qr = hx.x * hy.x, qi = hx.y * hy.y, ur = hx.x * hy.y, ui = hx.y * hy.x;
+            const double al = (qr - qi) * p.x + (ur + ui) * p.y, be = (qr + qi) * d.x - (ui - ur) * d.y;
+            const double g = (f.w1 + f.w2m + f.w3m) * al + (f.wm1 - f.w1 + f.w2p + f.w3p) * be;
+            const double v = 2.0 * e[y];
+            sr = fma(v, g, sr);
+            sf = fma(v, f.wm1 + f.wm2 + f.wm3, sf);
+        }
+    }
+    for (int h = 16; h > 0; h >>= 1) {
+        sf += __shfl_down_sync(0xffffffffu, sf, h);
+        sr += __shfl_down_sync(0xffffffffu, sr, h);
+    }
+    if (lane == 0) {
+        red[0][warp] = sf;
+        red[1][warp] = sr;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double s = 0.0;
+        for (int w = 0; w < 8; ++w) s += red[threadIdx.x][w];
+        part[((size_t)blockIdx.y * 2 + threadIdx.x) * nm + m] = w4 * s;
+    }
+}
+
 }  // namespace p64
 
 // Third moments of the whole Classic grid (circular-frequency convention, every row) in FP64 from
-// the products of distinct frequency pairs; dA holds the A rows of i df, i = 0 .. N (truncated
-// S(f1 + f2)) or 0 .. 2 N (analytic).
+// the products of distinct frequency pairs; dA (dS for the diagonal-only spectra) holds the rows of
+// i df, i = 0 .. N (truncated S(f1 + f2)) or 0 .. 2 N (analytic).
 int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr) {
     using namespace p64;
-    const int nm = nme, nm2 = nm * nm, hi = analytic ? 2 * N : N;
-    const long long nm3 = (long long)nm2 * nm;
+    const bool diag = set.onlyd != 0;
+    const int nm = nme, an = diag ? 1 : nm, rx = nm * an, hi = analytic ? 2 * N : N;
+    const long long nb = dim_bisp();  // outputs: nm^3, or nm
+    const double *A = diag ? dS.as<double>() : dA.as<double>(), *Q = diag ? dWd3.as<double>() : dQ.as<double>();
     cudaError_t e;
     auto ylast = [&](int x) { return analytic ? std::min(hi, x + N) : N; };  // last partner of first row x
-    int RT = std::max(1, std::min(nm2, 256 / nm)), PL = std::max(1, std::min(8, 256 / (RT * nm)));
-    const int tiles = (nm2 + RT - 1) / RT;
-    // about four blocks an SM; a group holds at least one batch of pairs
     const long long pairs_all = (long long)(N + 1) * (N + 2) / 2 + (analytic ? (long long)N * (N + 1) / 2 : 0);
-    const int G = (int)std::max(1LL, std::min<long long>((608 + tiles - 1) / tiles,
-                                                         (pairs_all + kBatch * PL - 1) / (kBatch * PL)));
+    // moment kernel: rows of a block, pair lanes, groups (about four blocks an SM; a group holds at
+    // least one batch of pairs)
+    const int RT = std::max(1, std::min(rx, 256 / nm)), PL = std::max(1, std::min(8, 256 / (RT * nm)));
+    const int tiles = (rx + RT - 1) / RT;
+    const int G = diag ? std::min(64, (N + 8) / 8)
+                       : (int)std::max(1LL, std::min<long long>((608 + tiles - 1) / tiles,
+                                                                (pairs_all + kBatch * PL - 1) / (kBatch * PL)));
     // Products on the tensor cores (bsa_pair64_tc.cu) where they outweigh the digits' preparation.
     // Measured contraction, FP64 pipe / tensor cores: 4.1e6 FMAs, K = 30: 0.097 / 0.108 ms; 7.3e6,
     // K = 60: 0.126 / 0.109; 1.9e7, K = 20: 0.137 / 0.167; 5.4e7, K = 12: 0.353 / 0.447; 6.9e7,
     // K = 30: 0.285 / 0.240 (K is padded to 16, and the moments do not get faster).
-    const bool tensor = K >= 24 && pairs_all * nm3 * K >= 7000000LL;
+    const bool tensor = K >= 24 && pairs_all * nb * K >= 7000000LL;
     // chunks of first rows: at most 4 GB of products and of row digits each
     const long long cap = 1LL << 29;
     const int Kd = (K + 63) / 64 * 64 * 2;  // digits of a row in doubles
@@ -336,56 +386,46 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     std::vector<Plan> plans;
     std::vector<RowTile> rts;
     std::vector<long long> pre;
+    long long emax = 0, rmax = 0;
     for (int x0 = 0; x0 <= N;) {
         Plan p{x0, x0, 0, 0, 0, 0, rts.size(), pre.size()};
-        auto rows_of = [&](int x1) {  // row tiles of [x0, x1), appended at p.rt0
-            rts.resize(p.rt0);
-            p.items = p.elems = 0;
-            const long long rows = (long long)(x1 - x0) * nm2;
-            for (long long r = 0; r < rows; r += kTM) {
-                const int xa = x0 + (int)(r / nm2), xb = x0 + (int)((std::min(rows, r + kTM) - 1) / nm2);
-                RowTile t;
-                t.ct0 = xa * nm / kTN;
-                t.nct = (int)(((long long)(ylast(xb) + 1) * nm + kTN - 1) / kTN) - t.ct0;
-                t.base = p.elems;
-                t.item0 = p.items;
-                p.items += t.nct;
-                p.elems += (long long)t.nct * kTN * kTM;
-                rts.push_back(t);
-            }
-        };
-        // rows of equal partner counts fill a chunk evenly: estimate, then one exact list
         long long el = 0;
-        int x1 = x0;
-        while (x1 <= N) {
-            const long long add = (long long)nm2 * std::max((ylast(x1) - x1 + 1) * (long long)nm + 2 * kTN, (long long)Kd);
-            if (x1 > x0 && el + add > cap) break;
+        while (p.x1 <= N) {
+            const long long add = (long long)rx * std::max((ylast(p.x1) - p.x1 + 1) * (long long)an + 2 * kTN, (long long)Kd);
+            if (p.x1 > x0 && el + add > cap) break;
             el += add;
-            ++x1;
-        }
-        rows_of(x1);
-        p.x1 = x1;
-        p.ntiles = (int)(rts.size() - p.rt0);
-        for (int x = x0; x < x1; ++x) {
             pre.push_back(p.npairs);
-            p.npairs += ylast(x) - x + 1;
+            p.npairs += ylast(p.x1) - p.x1 + 1;
+            ++p.x1;
         }
-        plans.push_back(p);
-        x0 = x1;
-    }
-    long long emax = 0, rmax = 0;
-    for (const Plan &p : plans) {
+        const long long rows = (long long)(p.x1 - x0) * rx;
+        for (long long r = 0; r < rows; r += kTM) {
+            const int xa = x0 + (int)(r / rx), xb = x0 + (int)((std::min(rows, r + kTM) - 1) / rx);
+            RowTile t;
+            t.ct0 = xa * an / kTN;
+            t.nct = (int)(((long long)(ylast(xb) + 1) * an + kTN - 1) / kTN) - t.ct0;
+            t.base = p.elems;
+            t.item0 = p.items;
+            p.items += t.nct;
+            p.elems += (long long)t.nct * kTN * kTM;
+            rts.push_back(t);
+        }
+        p.ntiles = (int)(rts.size() - p.rt0);
         emax = std::max(emax, p.elems);
-        rmax = std::max(rmax, (long long)(p.x1 - p.x0) * nm2);
+        rmax = std::max(rmax, rows);
+        plans.push_back(p);
+        x0 = p.x1;
     }
     const size_t rtb = sizeof(RowTile) * rts.size(), preb = sizeof(long long) * pre.size();
-    const size_t hb = sizeof(double2) * (size_t)(2 * N + 1) * nm;
+    const size_t hb = sizeof(double2) * (size_t)(2 * N + 1) * nm, nparts = diag ? G * plans.size() : G;
+    const long long plen = diag ? 2 * nb : kKinds * nb;
+    double *o = nullptr;
     if ((e = dMixA.reserve(sizeof(double) * (size_t)emax)) || (e = dMixH.reserve(hb)) || (e = dMshIdx.reserve(rtb + preb)) ||
-        (e = dPartF.reserve(sizeof(double) * (size_t)G * kKinds * nm3)) ||
-        (e = dPartR.reserve(sizeof(double) * (size_t)kKinds * nm3)) ||
-        (e = dOut.reserve(sizeof(double) * (3 * (size_t)nm2 + 2 * (size_t)nm3))))
+        (e = dPartF.reserve(sizeof(double) * nparts * plen)) || (e = dPartR.reserve(sizeof(double) * (size_t)plen)) ||
+        (e = dOut.reserve(sizeof(double) * (3 * (size_t)dim_psd() + 2 * (size_t)nb))))
         return cuda_fail(e, "allocating pair products");
-    if (tensor && ((e = dMixB.reserve(tc_col_bytes(hi + 1, nm, K))) || (e = dMshT.reserve(tc_row_bytes(rmax, K))) ||
+    o = dOut.as<double>() + 3 * (size_t)dim_psd();
+    if (tensor && ((e = dMixB.reserve(tc_col_bytes(hi + 1, an, K))) || (e = dMshT.reserve(tc_row_bytes(rmax, K))) ||
                    (e = dFlag.reserve(256))))
         return cuda_fail(e, "allocating pair products");
     char *idx = (char *)dMshIdx.p;
@@ -399,36 +439,40 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     const int PB = kBatch * PL;
     const size_t smem = std::max((size_t)256 * sizeof(double), sizeof(double) * (size_t)PB * RT * 8 +
                                  sizeof(double2) * (size_t)PB * nm * 3 + sizeof(PairInfo) * (size_t)PB);
-    if ((e = cudaFuncSetAttribute(k_pair_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
+    if (!diag && (e = cudaFuncSetAttribute(k_pair_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
         return cuda_fail(e, "pair moments kernel");
     if (tensor && ((e = cudaMemsetAsync(dFlag.p, 0, sizeof(int), stream)) ||
-                   (e = tc_prep_cols(stream, hi + 1, nm, K, dA.as<double>(), dMixB.p))))
+                   (e = tc_prep_cols(stream, hi + 1, an, K, A, dMixB.p))))
         return cuda_fail(e, "pair product operands");
     if (tensor) kernels += 2;
     for (size_t q = 0; q < plans.size(); ++q) {
         const Plan &p = plans[q];
-        Chunk c{p.x0, p.x1, nm, K, hi, p.ntiles, p.items, (const RowTile *)idx + p.rt0, dMixA.as<double>()};
+        Chunk c{p.x0, p.x1, nm, an, K, hi, p.ntiles, p.items, (const RowTile *)idx + p.rt0, dMixA.as<double>()};
         if (tensor) {
-            if ((e = tc_products(stream, c, hi + 1, dA.as<double>(), dQ.as<double>(), dMixB.p, dMshT.p, dFlag.as<int>())))
+            if ((e = tc_products(stream, c, hi + 1, A, Q, dMixB.p, dMshT.p, dFlag.as<int>())))
                 return cuda_fail(e, "pair product kernel");
             kernels += 2;
         } else {
-            k_pair_gemm<<<(unsigned)p.items, 256, 0, stream>>>(c, dA.as<double>(), dQ.as<double>());
+            k_pair_gemm<<<(unsigned)p.items, 256, 0, stream>>>(c, A, Q);
         }
-        MomPar mp{N, vect ? 1 : 0, p.npairs, (const long long *)(idx + rtb) + p.pre0, dMixH.as<double2>(), 4.0 * wval,
-                  dPartF.as<double>(), q == 0 ? 1 : 0, RT, PL};
-        k_pair_moments<<<dim3((unsigned)tiles, (unsigned)G), 256, smem, stream>>>(c, mp);
+        if (diag) {
+            k_pair_moments_diag<<<dim3(nm, G), 256, 0, stream>>>(c, N, analytic ? 1 : 0, vect ? 1 : 0, 4.0 * wval,
+                                                                  dMixH.as<double2>(), dPartF.as<double>() + q * G * plen);
+        } else {
+            MomPar mp{N, vect ? 1 : 0, p.npairs, (const long long *)(idx + rtb) + p.pre0, dMixH.as<double2>(),
+                      dPartF.as<double>(), q == 0 ? 1 : 0, RT, PL};
+            k_pair_moments<<<dim3((unsigned)tiles, (unsigned)G), 256, smem, stream>>>(c, mp);
+        }
         kernels += 2;
     }
     if ((e = cudaGetLastError())) return cuda_fail(e, "pair contraction kernels");
     if ((e = cudaEventRecord(evg1, stream))) return cuda_fail(e, "event");
-    double *o = dOut.as<double>() + 3 * (size_t)nm2;
-    if ((e = launch_reduce_groups(stream, G, kKinds * nm3, dPartF.as<double>(), dPartR.as<double>(), nullptr, nullptr)))
+    if ((e = launch_reduce_groups(stream, (int)nparts, plen, dPartF.as<double>(), diag ? o : dPartR.as<double>(), nullptr, nullptr)))
         return cuda_fail(e, "reduction kernel");
-    k_pair_finish<<<(unsigned)((nm3 + 127) / 128), 128, 0, stream>>>(nm, 4.0 * wval, dPartR.as<double>(), o, o + nm3);
+    if (!diag) k_pair_finish<<<(unsigned)((nb + 127) / 128), 128, 0, stream>>>(nm, 4.0 * wval, dPartR.as<double>(), o, o + nb);
     if ((e = cudaGetLastError())) return cuda_fail(e, "reduction kernel");
-    kernels += 3;
-    std::vector<double> h(2 * (size_t)nm3);
+    kernels += diag ? 2 : 3;
+    std::vector<double> h(2 * (size_t)nb);
     int herr = 0;
     if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
         (tensor && (e = cudaMemcpyAsync(&herr, dFlag.p, sizeof(int), cudaMemcpyDeviceToHost, stream))) ||
@@ -441,8 +485,8 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     cudaEventElapsedTime(&ms, evg0, evg1);
     last_ms_gemm = ms;
     d2h += (double)sizeof(double) * h.size();
-    if (m3mf) std::memcpy(m3mf, h.data(), sizeof(double) * nm3);
-    if (m3mr) std::memcpy(m3mr, h.data() + nm3, sizeof(double) * nm3);
+    if (m3mf) std::memcpy(m3mf, h.data(), sizeof(double) * nb);
+    if (m3mr) std::memcpy(m3mr, h.data() + nb, sizeof(double) * nb);
     return BSA_OK;
 }
 

@@ -10,9 +10,10 @@ namespace p64 {
 
 constexpr int kTM = 128, kTN = 32;  // product tile: rows (x, a, b) by columns (y, j)
 
-// A chunk of products: rows r = (x - x0) nm^2 + a nm + b of the first rows x in [x0, x1), in tiles
-// of kTM; row tile mt holds the column tiles ct0[mt] .. ct0[mt] + nct[mt] of c = y nm + j, row-major
-// from base[mt].
+// A chunk of products sum_k Q[k][a] A(x)[k][b] A(y)[k][j], Q of qn and A of an columns (nm and nm;
+// nm and 1 for the diagonal-only spectra): rows r = (x - x0) qn an + a an + b of the first rows x in
+// [x0, x1), in tiles of kTM; row tile mt holds the column tiles ct0[mt] .. ct0[mt] + nct[mt] of
+// c = y an + j, row-major from base[mt].
 struct RowTile {
     int ct0, nct;
     long long base;   // first element in E
@@ -20,10 +21,11 @@ struct RowTile {
 };
 
 struct Chunk {
-    int x0, x1, nm, K, hi, ntiles;
+    int x0, x1, qn, an, K, hi, ntiles;
     long long items;
     const RowTile *rt;
     double *E;
+    __host__ __device__ int rx() const { return qn * an; }  // rows of one x
 };
 
 // Row tile of a product tile.
@@ -39,9 +41,9 @@ __device__ __forceinline__ int tile_row(const Chunk &c, long long item) {
 // Tensor-core products.  tc_col_bytes / tc_row_bytes: scratch of the column operand (nr rows of the A
 // table) and of the row operand of nrows product rows.  tc_prep_cols once per analysis, then
 // tc_products per chunk.  err receives a nonzero code if a pipeline wait ran out of its budget.
-size_t tc_col_bytes(int nr, int nm, int K);
+size_t tc_col_bytes(int nr, int an, int K);
 size_t tc_row_bytes(long long nrows, int K);
-cudaError_t tc_prep_cols(cudaStream_t st, int nr, int nm, int K, const double *A, void *cols);
+cudaError_t tc_prep_cols(cudaStream_t st, int nr, int an, int K, const double *A, void *cols);
 cudaError_t tc_products(cudaStream_t st, const Chunk &c, int nr, const double *A, const double *Q, void *cols,
                         void *rows, int *err);
 

@@ -82,18 +82,23 @@ __device__ __forceinline__ void put_digits(const double *v, int e, __nv_bfloat16
     }
 }
 
-// Column operand: exponent e[c] with |A[y][k][j]| < 2^e[c], c = y nm + j.
-__global__ void k_col_exp(int nm, int K, const double *__restrict__ A, int *__restrict__ ec) {
+// Column operand: exponent e[c] with |A[y][k][j]| < 2^e[c], c = y an + j.
+__global__ __launch_bounds__(256) void k_col_exp(int an, int K, const double *__restrict__ A, int *__restrict__ ec) {
     __shared__ int mx[64];
     const int y = blockIdx.x;
     if (threadIdx.x < 64) mx[threadIdx.x] = 0;
     __syncthreads();
-    const double *a = A + (size_t)y * K * nm;
-    for (int q = threadIdx.x; q < K * nm; q += blockDim.x) atomicMax(&mx[q % nm], expo(a[q]));
+    const double *a = A + (size_t)y * K * an;
+    // a thread keeps one column: 256 / an lanes over k
+    const int lanes = 256 / an, j = threadIdx.x % an, lane = threadIdx.x / an;
+    int m = 0;
+    if (lane < lanes)
+        for (int k = lane; k < K; k += lanes) m = max(m, expo(a[(size_t)k * an + j]));
+    atomicMax(&mx[j], m);
     __syncthreads();
-    if ((int)threadIdx.x < nm) {
-        const int m = mx[threadIdx.x];
-        ec[y * nm + threadIdx.x] = m == 2047 ? kBad : m == 0 ? kNone : m - 1022;
+    if ((int)threadIdx.x < an) {
+        const int e = mx[threadIdx.x];
+        ec[y * an + threadIdx.x] = e == 2047 ? kBad : e == 0 ? kNone : e - 1022;
     }
 }
 
@@ -102,37 +107,37 @@ __global__ void k_col_exp(int nm, int K, const double *__restrict__ A, int *__re
 __global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restrict__ A, const double *__restrict__ Q,
                                                  int *__restrict__ er) {
     __shared__ int mx[8][32];
-    const int nm = c.nm, nm2 = nm * nm, ab = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
-    const int x = c.x0 + blockIdx.x, a = ab / nm, b = ab - a * nm;
-    const int *q = reinterpret_cast<const int *>(Q + a) + 1, *p = reinterpret_cast<const int *>(A + (size_t)x * c.K * nm + b) + 1;
+    const int qn = c.qn, an = c.an, rx = c.rx(), ab = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
+    const int x = c.x0 + blockIdx.x, a = ab / an, b = ab - a * an;
+    const int *q = reinterpret_cast<const int *>(Q + a) + 1, *p = reinterpret_cast<const int *>(A + (size_t)x * c.K * an + b) + 1;
     int m = 0;
-    if (ab < nm2)
+    if (ab < rx)
 #pragma unroll 8
         for (int k = lane; k < c.K; k += 8) {
-            const int u = (q[(size_t)2 * k * nm] >> 20) & 0x7ff, v = (p[(size_t)2 * k * nm] >> 20) & 0x7ff;
+            const int u = (q[(size_t)2 * k * qn] >> 20) & 0x7ff, v = (p[(size_t)2 * k * an] >> 20) & 0x7ff;
             m = max(m, (u == 2047 || v == 2047) ? kBad : (u && v) ? u + v : 0);
         }
     mx[lane][threadIdx.x & 31] = m;
     __syncthreads();
-    if (lane == 0 && ab < nm2) {
+    if (lane == 0 && ab < rx) {
 #pragma unroll
         for (int z = 1; z < 8; ++z) m = max(m, mx[z][threadIdx.x]);
-        er[(size_t)blockIdx.x * nm2 + ab] = m == kBad ? kBad : m == 0 ? kNone : m - 2044;
+        er[(size_t)blockIdx.x * rx + ab] = m == kBad ? kBad : m == 0 ? kNone : m - 2044;
     }
 }
 
 // Column digits [ct][digit][32 columns][Kp]; block: one column tile, 128 k.
-__global__ __launch_bounds__(256) void k_col_digits(int nr, int nm, int K, int Kp, const double *__restrict__ A,
+__global__ __launch_bounds__(256) void k_col_digits(int nr, int an, int K, int Kp, const double *__restrict__ A,
                                                     const int *__restrict__ ec, __nv_bfloat16 *__restrict__ D) {
     const int ct = blockIdx.x, col = threadIdx.x & 31, k0 = blockIdx.y * 128 + (threadIdx.x >> 5) * 16;
     if (k0 >= Kp) return;
-    const int c = ct * kTN + col, y = c / nm, j = c - y * nm;
+    const int c = ct * kTN + col, y = c / an, j = c - y * an;
     const bool ok = y < nr;
     const int e = ok ? ec[c] : kNone;
     const bool some = e != kNone && e != kBad;
     double v[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = (some && k0 + i < K) ? A[((size_t)y * K + k0 + i) * nm + j] : 0.0;
+    for (int i = 0; i < 16; ++i) v[i] = (some && k0 + i < K) ? A[((size_t)y * K + k0 + i) * an + j] : 0.0;
     put_digits(v, some ? e : 0, D + ((size_t)ct * kDig * kTN + col) * Kp + k0, (size_t)kTN * Kp);
 }
 
@@ -141,25 +146,23 @@ __global__ __launch_bounds__(256) void k_row_digits(Chunk c, int Kp, const doubl
                                                     const double *__restrict__ Q, const int *__restrict__ er,
                                                     __nv_bfloat16 *__restrict__ D) {
     extern __shared__ double sm[];
-    const int nm = c.nm, nm2 = nm * nm, K = c.K, xl = blockIdx.x, kb = blockIdx.y * 64;
-    double *As = sm, *Qs = sm + 64 * nm;
-    const int n = max(0, min(64, K - kb)) * nm;
-    const double *a = A + ((size_t)(c.x0 + xl) * K + kb) * nm, *q = Q + (size_t)kb * nm;
-    for (int i = threadIdx.x; i < 64 * nm; i += 256) {
-        As[i] = i < n ? a[i] : 0.0;
-        Qs[i] = i < n ? q[i] : 0.0;
-    }
+    const int qn = c.qn, an = c.an, rx = c.rx(), K = c.K, xl = blockIdx.x, kb = blockIdx.y * 64;
+    double *As = sm, *Qs = sm + 64 * an;
+    const int n = max(0, min(64, K - kb));
+    const double *a = A + ((size_t)(c.x0 + xl) * K + kb) * an, *q = Q + (size_t)kb * qn;
+    for (int i = threadIdx.x; i < 64 * an; i += 256) As[i] = i < n * an ? a[i] : 0.0;
+    for (int i = threadIdx.x; i < 64 * qn; i += 256) Qs[i] = i < n * qn ? q[i] : 0.0;
     __syncthreads();
-    for (int w = threadIdx.x; w < nm2 * 4; w += 256) {
-        const int kq = w / nm2, ab = w - kq * nm2, ia = ab / nm, ib = ab - ia * nm;
-        const long long r = (long long)xl * nm2 + ab;
+    for (int w = threadIdx.x; w < rx * 4; w += 256) {
+        const int kq = w / rx, ab = w - kq * rx, ia = ab / an, ib = ab - ia * an;
+        const long long r = (long long)xl * rx + ab;
         const int e = er[r];
         const bool some = e != kNone && e != kBad;
         double v[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int k = kq * 16 + i;
-            v[i] = some ? Qs[k * nm + ia] * As[k * nm + ib] : 0.0;
+            v[i] = some ? Qs[k * qn + ia] * As[k * an + ib] : 0.0;
         }
         put_digits(v, some ? e : 0, D + ((r / kTM) * kDig * kTM + r % kTM) * (size_t)Kp + kb + kq * 16, (size_t)kTM * Kp);
     }
@@ -320,7 +323,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // ---------------- epilogue: 128 rows, one a thread ----------------
         const int quarter = warp & 3, row = quarter * 32 + lane;
         const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
-        const int nrows = (c.x1 - c.x0) * c.nm * c.nm, ncols = (c.hi + 1) * c.nm;
+        const int nrows = (c.x1 - c.x0) * c.rx(), ncols = (c.hi + 1) * c.an;
         uint32_t tile = 0;
         bool ok = true;
         for (long long item = blockIdx.x; item < c.items && ok; item += gridDim.x) {
@@ -384,31 +387,31 @@ static int kpad(int K) { return (K + kBK - 1) / kBK * kBK; }
 static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 // [digits][exponents]
-size_t tc_col_bytes(int nr, int nm, int K) {
-    const size_t ct = ((size_t)nr * nm + kTN - 1) / kTN;
-    return up256(ct * kDig * kTN * kpad(K) * 2) + up256(sizeof(int) * (size_t)nr * nm);
+size_t tc_col_bytes(int nr, int an, int K) {
+    const size_t ct = ((size_t)nr * an + kTN - 1) / kTN;
+    return up256(ct * kDig * kTN * kpad(K) * 2) + up256(sizeof(int) * (size_t)nr * an);
 }
 size_t tc_row_bytes(long long nrows, int K) {
     const size_t mt = (size_t)((nrows + kTM - 1) / kTM);
     return up256(mt * kDig * kTM * kpad(K) * 2) + up256(sizeof(int) * (size_t)nrows);
 }
 
-cudaError_t tc_prep_cols(cudaStream_t st, int nr, int nm, int K, const double *A, void *cols) {
-    const int Kp = kpad(K), nct = (nr * nm + kTN - 1) / kTN;
+cudaError_t tc_prep_cols(cudaStream_t st, int nr, int an, int K, const double *A, void *cols) {
+    const int Kp = kpad(K), nct = (nr * an + kTN - 1) / kTN;
     int *ec = (int *)((char *)cols + up256((size_t)nct * kDig * kTN * Kp * 2));
-    k_col_exp<<<nr, 256, 0, st>>>(nm, K, A, ec);
-    k_col_digits<<<dim3(nct, (Kp + 127) / 128), 256, 0, st>>>(nr, nm, K, Kp, A, ec, (__nv_bfloat16 *)cols);
+    k_col_exp<<<nr, 256, 0, st>>>(an, K, A, ec);
+    k_col_digits<<<dim3(nct, (Kp + 127) / 128), 256, 0, st>>>(nr, an, K, Kp, A, ec, (__nv_bfloat16 *)cols);
     return cudaGetLastError();
 }
 
 cudaError_t tc_products(cudaStream_t st, const Chunk &c, int nr, const double *A, const double *Q, void *cols,
                         void *rows, int *err) {
-    const int Kp = kpad(c.K), nm2 = c.nm * c.nm, nx = c.x1 - c.x0;
-    const size_t nct = ((size_t)nr * c.nm + kTN - 1) / kTN, nmt = (size_t)c.ntiles;
+    const int Kp = kpad(c.K), nx = c.x1 - c.x0;
+    const size_t nct = ((size_t)nr * c.an + kTN - 1) / kTN, nmt = (size_t)c.ntiles;
     int *ec = (int *)((char *)cols + up256(nct * kDig * kTN * Kp * 2));
     int *er = (int *)((char *)rows + up256(nmt * kDig * kTM * Kp * 2));
-    k_row_exp<<<dim3(nx, (nm2 + 31) / 32), 256, 0, st>>>(c, A, Q, er);
-    const size_t sm = sizeof(double) * 2 * 64 * c.nm;
+    k_row_exp<<<dim3(nx, (c.rx() + 31) / 32), 256, 0, st>>>(c, A, Q, er);
+    const size_t sm = sizeof(double) * 64 * (c.qn + c.an);
     cudaError_t e = cudaFuncSetAttribute(k_row_digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     k_row_digits<<<dim3(nx, Kp / 64), 256, sm, st>>>(c, Kp, A, Q, er, (__nv_bfloat16 *)rows);

@@ -80,3 +80,16 @@ def test_tensor_pairs_not_finite(bsalib):
     whole, a, b = _run(p), _run(p, (0, 20)), _run(p, (20, nf))
     for k in ("m3mf_cls", "m3mr_cls"):
         assert np.array_equal(np.isfinite(whole[k]), np.isfinite(a[k] + b[k]))
+
+
+# diagonal-only spectra: both product kernels, several row tiles and y lanes past a warp
+@pytest.mark.parametrize("modes,nodes,nfreqs", [(1, 3, 2), (3, 17, 9), (5, 16, 40), (24, 33, 20), (33, 130, 70), (64, 20, 34)])
+@pytest.mark.parametrize("trunc,scalar", [(True, 0), (False, 0), (True, 1)])
+def test_diagonal_pairs_against_points(bsalib, modes, nodes, nfreqs, trunc, scalar):
+    p = tall_building(nodes=nodes, modes=modes, nfreqs=nfreqs, df=2.0 / nfreqs, seed=modes)
+    p.settings.scalar, p.settings.onlyd = scalar, 1
+    nf = p.classic_nf()
+    whole = _run(p, trunc=trunc)
+    a, b = _run(p, (0, 1), trunc), _run(p, (1, nf), trunc)
+    _close(whole, {k: a[k] + b[k] for k in a})
+    _close(_run(p, trunc=trunc, sym=True), whole)
