@@ -47,3 +47,25 @@ def test_training_separable_and_deterministic(bsalib):
             net.close()
         assert loss < 0.1 and acc > 0.97
     assert np.array_equal(params[0], params[1])
+
+
+# sample tiles of 32 (gradients) and 64 (probabilities), blocks that walk several tiles, widths and
+# inputs below and at the 128 the tiles hold
+@pytest.mark.parametrize("n,din,W", [(1, 1, 1), (31, 13, 128), (32, 128, 128), (33, 5, 7), (64, 13, 127), (65, 127, 33),
+                                     (4900, 13, 128), (9800, 3, 64)])
+def test_tiles_match_oracle(bsalib, n, din, W):
+    rng = np.random.default_rng(n + din + W)
+    net = api.Mlp(din, W, seed=9)
+    try:
+        x = rng.normal(0, 1, (n, din)).astype(np.float32)
+        y = rng.uniform(size=n).astype(np.float32)
+        w = rng.uniform(0.5, 2.0, n).astype(np.float32)
+        pb = net.params(bf16=True)
+        loss, g = net.gradients(x, y, w)
+        eloss, eg = mlp_ref.loss_and_grad(pb, x, y, w, din, W)
+        assert abs(loss - eloss) <= 1e-5 * abs(eloss)
+        assert np.max(np.abs(g - eg)) <= 1e-4 * np.max(np.abs(eg))
+        logit, _ = mlp_ref.forward(pb, x, din, W)
+        assert np.max(np.abs(net.forward(x) - 1 / (1 + np.exp(-logit)))) < 1e-5
+    finally:
+        net.close()
