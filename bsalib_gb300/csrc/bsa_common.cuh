@@ -70,6 +70,11 @@ struct PointSrc {
     const double *f1, *f2;  // point frequencies (kPointsList)
     const ZoneDev *zones;   // optional (kPointsList): BRM neighbourhood of each point
     const int *zid, *zi, *zj; // zone and lattice coordinates of each point
+    // FRF tables of the zones whose lattice lies along the axes: from zoff[zone] (< 0: none) nm complex
+    // values at each frequency of the f1 direction, of the f2 direction, and at f1 + f2 of the BRM
+    // lattice, the f1 direction slowest
+    const double2 *zH;
+    const long long *zoff;
     // optional (kPointsList), listed BRM points: point p feeds entries [cptr[p], cptr[p + 1]) of
     // cq, each (f1, f2, coefficient) of a BRM point, the coefficient its integration weight
     // times the share of this BFM point in its interpolated BFM

@@ -157,7 +157,7 @@ struct Engine {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     DevBuf dL, dQ, dLogc, dPsdPar, dFrfM, dFrfK, dFrfC, dFreq, dS, dA, dPartF, dPartR, dOut, dPsdF, dWf, dPts,
         dPtsD, dBF, dBR, dMixA, dMixB, dMixH, dMixPart, dA32, dZones, dZidx, dWd3, dWd2, dMshT, dMshIdx, dLogc32, dL32,
-        dPod, dFlag, dSlot, dHash, dCptr, dCq;
+        dPod, dFlag, dSlot, dHash, dCptr, dCq, dZoneH, dZoff;
 
     // stats
     double last_ms = 0, last_ms_contraction = 0, last_ms_gemm = 0, last_points = 0;
@@ -188,7 +188,14 @@ struct Engine {
     int run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf, double *m3mr, double *bf_host,
                     double *br_host, std::vector<double> *grid_out);
     int classic_export(PointSrc ps, const std::vector<double> &f, double *m3mf, double *m3mr);
-    int contract(const PointSrc &ps, long long npts, double *m3mf, double *m3mr, double *bf_host, double *br_host);
+    // rows: the points' A rows on the host (point lists), nr rows of the table
+    struct HostRows { const int *ix = nullptr, *iy = nullptr, *iz = nullptr; int nr = 0; };
+    int contract(const PointSrc &ps, long long npts, double *m3mf, double *m3mr, double *bf_host, double *br_host,
+                 const HostRows *rows = nullptr);
+    // point lists in FP64 over pair products (bsa_list64.cu)
+    bool list64_wanted(long long npts, int nr) const;
+    int contract_list64(const PointSrc &ps, long long npts, int nr, const int *ix, const int *iy, const int *iz, int G,
+                        double *bfd, double *brd);
     // the whole Classic grid in FP64 over distinct frequency pairs (bsa_pair64.cu); grid +-N df
     int contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr);
     int contract_mixed(const PointSrc &ps, long long npts, double *m3mf, double *m3mr);

@@ -158,7 +158,7 @@ void Engine::free_device() {
     if (stream) cudaStreamSynchronize(stream);  // the blocks go back to the cache for reuse
     for (DevBuf *b : {&dL, &dQ, &dLogc, &dPsdPar, &dFrfM, &dFrfK, &dFrfC, &dFreq, &dS, &dA, &dPartF, &dPartR,
                       &dOut, &dPsdF, &dWf, &dPts, &dPtsD, &dBF, &dBR, &dMixA, &dMixB, &dMixH, &dMixPart, &dA32,
-                      &dZones, &dZidx, &dWd3, &dWd2, &dMshT, &dMshIdx, &dLogc32, &dL32, &dPod, &dFlag, &dSlot, &dHash})
+                      &dZones, &dZidx, &dWd3, &dWd2, &dMshT, &dMshIdx, &dLogc32, &dL32, &dPod, &dFlag, &dSlot, &dHash, &dCptr, &dCq, &dZoneH, &dZoff})
         b->release();
     if (stream) cudaStreamDestroy(stream);
     stream = nullptr;
@@ -340,7 +340,7 @@ int Engine::upload_problem() {
     // log c in place (FP64) and its FP32 copy
     if ((e = launch_log_coh(stream, hCoh.size(), dLogc.as<double>(), dLogc32.as<float>())))
         return cuda_fail(e, "coherence table");
-    kernels += 2;
+    kernels += 1;
     dev_uploaded = true;
     return BSA_OK;
 }
@@ -651,7 +651,7 @@ int Engine::classic_export(PointSrc ps, const std::vector<double> &f, double *m3
 
 // Contraction + FRF + reduction over a point source; dA must hold every row it names.
 int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m3mr, double *bf_host,
-                     double *br_host) {
+                     double *br_host, const HostRows *rows) {
     const long long nm3 = (long long)nme * nme * nme;
     cudaError_t e;
     const int G = bfm_fp64_groups(npts, nme);
@@ -667,22 +667,30 @@ int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m
     }
     if ((e = cudaEventRecord(ev2, stream))) return cuda_fail(e, "event");
     if ((e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
-    if ((e = launch_bfm_fp64(stream, dA.as<double>(), dQ.as<double>(), K, nme, ps, npts, frf(), G, dPartF.as<double>(),
-                             dPartR.as<double>(), bfd, brd)))
+    const bool list64 = rows && list64_wanted(npts, rows->nr);
+    if (list64) {
+        int rc = contract_list64(ps, npts, rows->nr, rows->ix, rows->iy, rows->iz, G, bfd, brd);
+        if (rc) return rc;
+    } else if ((e = launch_bfm_fp64(stream, dA.as<double>(), dQ.as<double>(), K, nme, ps, npts, frf(), G,
+                                    dPartF.as<double>(), dPartR.as<double>(), bfd, brd))) {
         return cuda_fail(e, "FP64 contraction kernel");
+    }
     if ((e = cudaEventRecord(evg1, stream))) return cuda_fail(e, "event");
     double *o = dOut.as<double>() + 3 * (size_t)nme * nme;
     if ((e = launch_reduce_groups(stream, G, nm3, dPartF.as<double>(), o, dPartR.as<double>(), o + nm3)))
         return cuda_fail(e, "reduction kernel");
     kernels += 2;
     std::vector<double> h(2 * (size_t)nm3);
-    if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)))
+    int herr = 0;
+    if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
+        (list64 && (e = cudaMemcpyAsync(&herr, dFlag.p, sizeof(int), cudaMemcpyDeviceToHost, stream))))
         return cuda_fail(e, "moment copy");
     if (bf_host && (e = cudaMemcpyAsync(bf_host, bfd, sizeof(double) * (size_t)npts * nm3, cudaMemcpyDeviceToHost, stream)))
         return cuda_fail(e, "bispectrum copy");
     if (br_host && (e = cudaMemcpyAsync(br_host, brd, sizeof(double) * (size_t)npts * nm3, cudaMemcpyDeviceToHost, stream)))
         return cuda_fail(e, "bispectrum copy");
     if ((e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream))) return cuda_fail(e, "sync");
+    if (herr) return fail(BSA_ERR_TIMEOUT, "pair product kernel: a pipeline wait ran out of its budget (role %d)", herr);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev2, ev1);
     last_ms_contraction = ms;
@@ -766,6 +774,30 @@ int Engine::run_points(const double *fi, const double *fj, const double *w, doub
         ps.zid = dzid;
         ps.zi = dzi;
         ps.zj = dzj;
+        if (!set.onlyd) {
+            // FRF tables of the zones along the axes, within 8 GB
+            const size_t nz = zones->size();
+            std::vector<long long> zoff(2 * nz);
+            long long total = 0;
+            const long long cap = (8LL << 30) / (long long)sizeof(double2);
+            for (size_t k = 0; k < nz; ++k) {
+                const ZoneDev &z = (*zones)[k];
+                const long long na = (long long)(z.ni - 1) * z.Fi + 1, nb = (long long)(z.nj - 1) * z.Fj + 1;
+                const long long need = (na * nb + na + nb) * nme;
+                const bool axes = (z.dIj == 0.0 && z.dJi == 0.0) || (z.dIi == 0.0 && z.dJj == 0.0);
+                zoff[nz + k] = total;
+                zoff[k] = axes && total + need <= cap ? total : -1;
+                if (zoff[k] >= 0) total += need;
+            }
+            if ((e = dZoff.reserve(sizeof(long long) * zoff.size())) || (e = dZoneH.reserve(sizeof(double2) * (size_t)total)) ||
+                (e = cudaMemcpyAsync(dZoff.p, zoff.data(), sizeof(long long) * zoff.size(), cudaMemcpyHostToDevice, stream)) ||
+                (e = launch_zone_frf(stream, (int)nz, nme, ps.zones, dZoff.as<long long>(), total, frf(), dZoneH.as<double2>())))
+                return cuda_fail(e, "zone FRF tables");
+            h2d += (double)(sizeof(long long) * zoff.size());
+            kernels += total > 0;
+            ps.zH = dZoneH.as<double2>();
+            ps.zoff = dZoff.as<long long>();
+        }
     }
     if (cptr) {
         const size_t ne = (size_t)cptr[n];
@@ -779,7 +811,8 @@ int Engine::run_points(const double *fi, const double *fj, const double *w, doub
         ps.cq = dCq.as<double>();
     }
     // Mesher functions: the diagonal-only form is getFM_diag_tnm_scalar_msh_'s.
-    rc = set.onlyd ? contract_diag(ps, npts, 1, m3mf, m3mr, bfm, brm) : contract(ps, npts, m3mf, m3mr, bfm, brm);
+    const HostRows rows{ix.data(), iy.data(), iz.data(), (int)ftab.size()};
+    rc = set.onlyd ? contract_diag(ps, npts, 1, m3mf, m3mr, bfm, brm) : contract(ps, npts, m3mf, m3mr, bfm, brm, &rows);
     if (rc) return rc;
     last_points = (double)npts;
     if ((e = cudaEventRecord(ev1, stream)) || (e = cudaEventSynchronize(ev1))) return cuda_fail(e, "event");
@@ -886,7 +919,8 @@ int Engine::classic_points(const int *i1, const int *i2, long long npts, double 
         ps.f1 = df1;
         ps.f2 = df2;
         std::vector<double> mf(nm3), mr(nm3);
-        if ((rc = contract(ps, npts, mf.data(), mr.data(), bf, br))) return rc;
+        const HostRows rows{i1, i2, iz.data(), (int)ftab.size()};
+        if ((rc = contract(ps, npts, mf.data(), mr.data(), bf, br, &rows))) return rc;
     }
     last_points = (double)npts;
     if ((e = cudaEventRecord(ev1, stream)) || (e = cudaEventSynchronize(ev1))) return cuda_fail(e, "event");

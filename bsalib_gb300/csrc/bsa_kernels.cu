@@ -176,20 +176,19 @@ __global__ __launch_bounds__(256) void k_atable(int nf, const double *__restrict
     }
 }
 
+// The first block also fills the exponential's table behind the log-coherences.
 __global__ void k_log_coh(size_t n, double *__restrict__ lc, float *__restrict__ lc32) {
     const size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0) lc[n + threadIdx.x] = exp2((double)threadIdx.x / kExpTab);
     if (x >= n) return;
     const double v = log(lc[x]);
     lc[x] = v;
     lc32[x] = (float)v;
 }
 
-__global__ void k_exp_tab(double *__restrict__ expt) { expt[threadIdx.x] = exp2((double)threadIdx.x / kExpTab); }
-
 cudaError_t launch_log_coh(cudaStream_t st, size_t n, double *lc, float *lc32) {
     if (n == 0) return cudaSuccess;
-    k_log_coh<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, lc, lc32);
-    k_exp_tab<<<1, kExpTab, 0, st>>>(lc + n);
+    k_log_coh<<<(unsigned)((n + kExpTab - 1) / kExpTab), kExpTab, 0, st>>>(n, lc, lc32);
     return cudaGetLastError();
 }
 
@@ -332,10 +331,12 @@ cudaError_t launch_m2(cudaStream_t st, int k0, int k1, int nm, int diag, const d
 // ------------------------------------------------------------------------------------
 constexpr int KC = 32;
 
-template <int NOT, int MT>
+// PAIR: the three terms of a point are read from products E(x, y) of its frequency pairs
+// (bsa_list64.cu) instead of formed from the A rows.
+template <int NOT, int MT, bool PAIR>
 __global__ __launch_bounds__(256) void k_bfm_fp64(const double *__restrict__ A,
                                                   const double *__restrict__ Q, int K, int nm,
-                                                  PointSrc ps, long long npts, FrfPar frf,
+                                                  PointSrc ps, long long npts, FrfPar frf, PairPts pp,
                                                   double *__restrict__ part_mf,
                                                   double *__restrict__ part_mr,
                                                   double *__restrict__ bf_out,
@@ -353,7 +354,7 @@ __global__ __launch_bounds__(256) void k_bfm_fp64(const double *__restrict__ A,
     double *Zs = Qs + KC * nm;
     double *Ps = Zs + KC * nm;
     double *Rs = Ps + KC * NOT;
-    double *Hs = Rs + KC * NOT;  // [3][nm][2]
+    double *Hs = PAIR ? sm : Rs + KC * NOT;  // [3][nm][2]
     double smf[MT], smr[MT];
 #pragma unroll
     for (int u = 0; u < MT; ++u) smf[u] = smr[u] = 0.0;
@@ -368,7 +369,28 @@ __global__ __launch_bounds__(256) void k_bfm_fp64(const double *__restrict__ A,
         double acc[MT];
 #pragma unroll
         for (int u = 0; u < MT; ++u) acc[u] = 0.0;
-        for (int k0 = 0; k0 < K; k0 += KC) {
+        if constexpr (PAIR) {
+            // T1 = E(x, y)[(m, n), o], T2 = E(z, y)[(n, m), o], T3 = E(x, z)[(o, n), m]; a product kept
+            // as E(y, x) is read with its last two indices exchanged
+            const int *e3 = pp.pe + 3 * p;
+            auto src = [&](int w) { return e3[w] >= 0 ? pp.E + (size_t)(e3[w] >> 1) * nm3 : nullptr; };
+            const double *E1 = src(0), *E2 = src(1), *E3 = src(2);
+            const int t1 = e3[0] & 1, t2 = e3[1] & 1, t3 = e3[2] & 1;
+            const int i1 = t1 ? o * nm + n : n * nm + o;           // + m nm^2
+            const int s2 = t2 ? 1 : nm, i2 = n * nm2 + (t2 ? o * nm : o);   // + m s2
+            const int s3 = t3 ? nm : 1, i3 = o * nm2 + (t3 ? n : n * nm);   // + m s3
+#pragma unroll
+            for (int u = 0; u < MT; ++u) {
+                const int m = mg + MG * u;
+                if (ok && m < nm) {
+                    double v = E1 ? E1[(size_t)m * nm2 + i1] : 0.0;
+                    if (E2) v += E2[i2 + m * s2];
+                    if (E3) v += E3[i3 + m * s3];
+                    acc[u] = v;
+                }
+            }
+        }
+        for (int k0 = 0; !PAIR && k0 < K; k0 += KC) {
             const int kc = min(KC, K - k0);
             for (int e = t; e < kc * nm; e += 256) {
                 Qs[e] = Q[(size_t)k0 * nm + e];
@@ -445,6 +467,72 @@ __global__ __launch_bounds__(256) void k_bfm_fp64(const double *__restrict__ A,
             // BRM lattice point of its bilinear support with weight lambda; accumulate
             // G = sum_q lambda_q w_q Re[H_m(w1_q) H_n(w2_q) conj H_o(w1_q + w2_q)].
             const ZoneDev z = ps.zones[ps.zid[p]];
+            const long long off = ps.zoff ? ps.zoff[ps.zid[p]] : -1;
+            if (off >= 0) {
+                // lattice along the axes: f1 changes along one lattice direction (a) only and f2 along the
+                // other (b), so G = Re sum_a H_m(a) S_no(a), S_no(a) = sum_b w_ab H_n(b) conj H_o(a, b):
+                // the inner sum once per (n, o), one a per m group at a time, the FRF values from the
+                // zone's table.  Evaluated per point and block by one warp and summed per (m, n, o), the FRF
+                // part took 3.0 ms of the 200-node, 16-mode building's 128 zones (1523 points); now 0.4.
+                const bool ax = z.dIj == 0.0 && z.dJi == 0.0;  // f1 along the I direction
+                const int la = ax ? ps.zi[p] : ps.zj[p], lb = ax ? ps.zj[p] : ps.zi[p];
+                const int Fa = ax ? z.Fi : z.Fj, Fb = ax ? z.Fj : z.Fi;
+                const int Na = ((ax ? z.ni : z.nj) - 1) * Fa, Nb = ((ax ? z.nj : z.ni) - 1) * Fb;
+                const int a0 = max(0, la * Fa + 1 - Fa), a1 = min(Na, la * Fa + Fa - 1);
+                const int b0 = max(0, lb * Fb + 1 - Fb), b1 = min(Nb, lb * Fb + Fb - 1);
+                const double2 *H1 = ps.zH + off, *H2 = H1 + (size_t)(Na + 1) * nm, *H3 = H2 + (size_t)(Nb + 1) * nm;
+                const double wz = z.sym * (z.wI / z.Fi) * (z.wJ / z.Fj), ra = 1.0 / Fa, rb = 1.0 / Fb;
+                double2 *Ss = (double2 *)Hs;  // [MG][NOT]
+                double g[MT];
+#pragma unroll
+                for (int u = 0; u < MT; ++u) g[u] = 0.0;
+                for (int ac = a0; ac <= a1; ac += MG) {
+                    const int qa = ac + mg;
+                    double sr = 0.0, si = 0.0;
+                    if (ok && qa <= a1) {
+                        for (int qb = b0; qb <= b1; ++qb) {
+                            const double wb = (1.0 - abs(qb - lb * Fb) * rb) * ((qb == 0 || qb == Nb) ? 0.5 : 1.0);
+                            const double2 h2 = H2[(size_t)qb * nm + n], h3 = H3[((size_t)qa * (Nb + 1) + qb) * nm + o];
+                            const double xr = wb * h2.x, xi = wb * h2.y;
+                            sr = fma(xr, h3.x, fma(xi, h3.y, sr));
+                            si = fma(xi, h3.x, fma(-xr, h3.y, si));
+                        }
+                        const double wa = wz * (1.0 - abs(qa - la * Fa) * ra) * ((qa == 0 || qa == Na) ? 0.5 : 1.0);
+                        sr *= wa;
+                        si *= wa;
+                    }
+                    __syncthreads();
+                    Ss[mg * NOT + nol] = make_double2(sr, si);
+                    __syncthreads();
+                    if (ok) {
+                        const int na = min(MG, a1 - ac + 1);
+                        for (int q = 0; q < na; ++q) {
+                            const double2 s2 = Ss[q * NOT + nol];
+#pragma unroll
+                            for (int u = 0; u < MT; ++u) {
+                                const int m = mg + MG * u;
+                                if (m < nm) {
+                                    const double2 h1 = H1[(size_t)(ac + q) * nm + m];
+                                    g[u] = fma(h1.x, s2.x, fma(-h1.y, s2.y, g[u]));
+                                }
+                            }
+                        }
+                    }
+                }
+                if (ok) {
+#pragma unroll
+                    for (int u = 0; u < MT; ++u) {
+                        const int m = mg + MG * u;
+                        if (m < nm) {
+                            const double bfv = 2.0 * acc[u];
+                            smf[u] = fma(w, bfv, smf[u]);
+                            smr[u] = fma(g[u], bfv, smr[u]);
+                        }
+                    }
+                }
+                __syncthreads();
+                continue;
+            }
             const int li = ps.zi[p], lj = ps.zj[p];
             const int NI = (z.ni - 1) * z.Fi, NJ = (z.nj - 1) * z.Fj;  // last BRM index
             double g[MT];
@@ -529,8 +617,8 @@ __global__ __launch_bounds__(256) void k_bfm_fp64(const double *__restrict__ A,
             const int m = mg + MG * u;
             if (m < nm) {
                 const size_t idx = (size_t)pg * nm3 + m + (size_t)nm * no;
-                part_mf[idx] = smf[u];
-                part_mr[idx] = smr[u];
+                part_mf[idx] = PAIR && !pp.first ? part_mf[idx] + smf[u] : smf[u];
+                part_mr[idx] = PAIR && !pp.first ? part_mr[idx] + smr[u] : smr[u];
             }
         }
     }
@@ -552,27 +640,27 @@ int bfm_fp64_groups(long long npts, int nm) {
 
 template <int NOT, int MT>
 static cudaError_t launch_bfm_t(cudaStream_t st, const double *A, const double *Q, int K, int nm,
-                                const PointSrc &ps, long long npts, FrfPar frf, int n_groups,
+                                const PointSrc &ps, long long npts, FrfPar frf, const PairPts &pp, int n_groups,
                                 double *part_mf, double *part_mr, double *bf_out, double *br_out) {
-    const size_t smem = sizeof(double) * (2 * KC * nm + 2 * KC * NOT + 6 * nm);
-    cudaError_t e = cudaFuncSetAttribute(k_bfm_fp64<NOT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    const size_t smem = sizeof(double) * ((pp.E ? 0 : 2 * KC * nm + 2 * KC * NOT) + std::max(6 * nm, ps.zoff ? 2 * 256 : 0));
+    const auto kern = pp.E ? k_bfm_fp64<NOT, MT, true> : k_bfm_fp64<NOT, MT, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((nm * nm + NOT - 1) / NOT), (unsigned)n_groups);
-    k_bfm_fp64<NOT, MT><<<grid, 256, smem, st>>>(A, Q, K, nm, ps, npts, frf, part_mf, part_mr, bf_out, br_out);
+    kern<<<grid, 256, smem, st>>>(A, Q, K, nm, ps, npts, frf, pp, part_mf, part_mr, bf_out, br_out);
     return cudaGetLastError();
 }
 
 // MT = smallest supported count >= ceil(nm / MG), so no thread carries idle mode slots.
 template <int NOT>
 static cudaError_t launch_bfm_n(cudaStream_t st, const double *A, const double *Q, int K, int nm,
-                                const PointSrc &ps, long long npts, FrfPar frf, int n_groups,
+                                const PointSrc &ps, long long npts, FrfPar frf, const PairPts &pp, int n_groups,
                                 double *part_mf, double *part_mr, double *bf_out, double *br_out) {
     constexpr int MG = 256 / NOT;
     const int need = (nm + MG - 1) / MG;
-#define BSA_MT_CASE(V)                                                                                   \
-    if (need <= V)                                                                                       \
-        return launch_bfm_t<NOT, V>(st, A, Q, K, nm, ps, npts, frf, n_groups, part_mf, part_mr, bf_out, br_out);
+#define BSA_MT_CASE(V)                                                                                       \
+    if (need <= V)                                                                                           \
+        return launch_bfm_t<NOT, V>(st, A, Q, K, nm, ps, npts, frf, pp, n_groups, part_mf, part_mr, bf_out, br_out);
     BSA_MT_CASE(1)
     BSA_MT_CASE(2)
     BSA_MT_CASE(4)
@@ -584,18 +672,55 @@ static cudaError_t launch_bfm_n(cudaStream_t st, const double *A, const double *
     return cudaErrorInvalidValue;
 }
 
+// The zones' FRF tables (PointSrc::zH): a thread per value.
+__global__ void k_zone_frf(int nz, int nm, const ZoneDev *__restrict__ zones, const long long *__restrict__ zoff,
+                           long long total, FrfPar frf, double2 *__restrict__ H) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= total) return;
+    int lo = 0, up = nz - 1;  // last zone that has a table starting at or before t (zoff[nz + k]: running starts)
+    while (lo < up) {
+        const int mid = (lo + up + 1) >> 1;
+        if (zoff[nz + mid] <= t) lo = mid; else up = mid - 1;
+    }
+    const ZoneDev z = zones[lo];
+    const bool ax = z.dIj == 0.0 && z.dJi == 0.0;
+    const int Fa = ax ? z.Fi : z.Fj, Fb = ax ? z.Fj : z.Fi;
+    const int Na = ((ax ? z.ni : z.nj) - 1) * Fa + 1, Nb = ((ax ? z.nj : z.ni) - 1) * Fb + 1;
+    const long long r = (t - zoff[nz + lo]) / nm;
+    const int m = (int)((t - zoff[nz + lo]) - r * nm);
+    auto f1 = [&](int a) { return (z.fi0 + (double)a / Fa * (ax ? z.dIi : z.dJi)) * kPi2; };
+    auto f2 = [&](int b) { return (z.fj0 + (double)b / Fb * (ax ? z.dJj : z.dIj)) * kPi2; };
+    double w;
+    if (r < Na) w = f1((int)r);
+    else if (r < Na + Nb) w = f2((int)(r - Na));
+    else {
+        const long long q = r - Na - Nb;
+        w = f1((int)(q / Nb)) + f2((int)(q % Nb));
+    }
+    double hr, hi;
+    frf_eval(frf.M[m], frf.K[m], frf.C[m], w, hr, hi);
+    H[t] = make_double2(hr, hi);
+}
+
+cudaError_t launch_zone_frf(cudaStream_t st, int nz, int nm, const ZoneDev *zones, const long long *zoff, long long total,
+                            FrfPar frf, double2 *H) {
+    if (total == 0) return cudaSuccess;
+    k_zone_frf<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(nz, nm, zones, zoff, total, frf, H);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_bfm_fp64(cudaStream_t st, const double *A, const double *Q, int K, int nm,
                             const PointSrc &ps, long long npts, FrfPar frf, int n_groups,
-                            double *part_mf, double *part_mr, double *bf_out, double *br_out) {
+                            double *part_mf, double *part_mr, double *bf_out, double *br_out, const PairPts &pp) {
     if (nm > 64 || nm < 1) return cudaErrorInvalidValue;
     if (npts == 0) return cudaSuccess;
     switch (not_for(nm)) {
     case 64:
-        return launch_bfm_n<64>(st, A, Q, K, nm, ps, npts, frf, n_groups, part_mf, part_mr, bf_out, br_out);
+        return launch_bfm_n<64>(st, A, Q, K, nm, ps, npts, frf, pp, n_groups, part_mf, part_mr, bf_out, br_out);
     case 32:
-        return launch_bfm_n<32>(st, A, Q, K, nm, ps, npts, frf, n_groups, part_mf, part_mr, bf_out, br_out);
+        return launch_bfm_n<32>(st, A, Q, K, nm, ps, npts, frf, pp, n_groups, part_mf, part_mr, bf_out, br_out);
     default:
-        return launch_bfm_n<16>(st, A, Q, K, nm, ps, npts, frf, n_groups, part_mf, part_mr, bf_out, br_out);
+        return launch_bfm_n<16>(st, A, Q, K, nm, ps, npts, frf, pp, n_groups, part_mf, part_mr, bf_out, br_out);
     }
 }
 

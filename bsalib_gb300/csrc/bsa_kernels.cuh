@@ -50,10 +50,23 @@ cudaError_t launch_force_psd_diag(cudaStream_t st, int nf, int K, int nm, const 
 //   of functionsImpl.F90:1494-1538), B_R = B_F * Re[H_m(w1) H_n(w2) conj H_o(w1+w2)].
 // part_mf / part_mr receive one nm^3 partial per point group (n_groups of them);
 // bf_out / br_out (optional) receive B_F / B_R per point, (nm^3, npts).
+// pp.E set: the points' terms from pair products E[pair][a nm + b][j] instead of A and Q; point p reads
+// pairs pp.pe[3 p + 0 .. 2] (f1 f2, f1+f2 f2, f1 f1+f2) = 2 pair + (product kept with its two
+// frequencies exchanged), or -1 for a zero term; !pp.first: the partials are added to.
+struct PairPts {
+    const double *E = nullptr;
+    const int *pe = nullptr;
+    int first = 1;
+};
 cudaError_t launch_bfm_fp64(cudaStream_t st, const double *A, const double *Q, int K, int nm,
                             const PointSrc &ps, long long npts, FrfPar frf, int n_groups,
-                            double *part_mf, double *part_mr, double *bf_out, double *br_out);
+                            double *part_mf, double *part_mr, double *bf_out, double *br_out, const PairPts &pp = PairPts());
 int bfm_fp64_groups(long long npts, int nm);
+
+// The FRF tables of PointSrc::zH (total values): zoff holds nz offsets (< 0: zone without a table), then
+// the nz running starts.
+cudaError_t launch_zone_frf(cudaStream_t st, int nz, int nm, const ZoneDev *zones, const long long *zoff, long long total,
+                            FrfPar frf, double2 *H);
 
 // out[x] = sum_g part[g * len + x] (fixed order); optional second array.
 cudaError_t launch_reduce_groups(cudaStream_t st, int n_groups, long long len, const double *part,

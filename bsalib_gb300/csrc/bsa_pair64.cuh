@@ -25,8 +25,22 @@ struct Chunk {
     long long items;
     const RowTile *rt;
     double *E;
+    int rpad;         // rows of one x in the row operand (rx, or whole tiles in a pair list)
+    const int *xmap;  // pair list: A row of x (x0 = 0); null: x itself
     __host__ __device__ int rx() const { return qn * an; }  // rows of one x
 };
+
+// A list of products instead (point sets, bsa_list64.cu): the columns of an A row come in np blocks
+// of bw (a multiple of 8, at most 32), kSlots(bw) blocks to a product tile.  Item i multiplies row tile
+// items[i].x with the blocks blk[items[i].y] .. (items[i].z of them); product pair[e] of entry e goes
+// to E[pair][a nm + b][j].
+struct PairList {
+    const int4 *items;
+    const int *blk, *pair;
+    int np, bw, tiles_x;  // row tiles of one x
+};
+__host__ __device__ inline int blocks_of(int nm) { return (nm + kTN - 1) / kTN; }
+__host__ __device__ inline int block_width(int nm) { return ((nm + blocks_of(nm) - 1) / blocks_of(nm) + 7) / 8 * 8; }
 
 // Row tile of a product tile.
 __device__ __forceinline__ int tile_row(const Chunk &c, long long item) {
@@ -46,6 +60,12 @@ size_t tc_row_bytes(long long nrows, int K);
 cudaError_t tc_prep_cols(cudaStream_t st, int nr, int an, int K, const double *A, void *cols);
 cudaError_t tc_products(cudaStream_t st, const Chunk &c, int nr, const double *A, const double *Q, void *cols,
                         void *rows, int *err);
+
+// The same for a pair list: column blocks of nr A rows, then the products of c.x1 rows (c.items items).
+size_t tc_block_bytes(int nr, int nm, int K);
+cudaError_t tc_prep_blocks(cudaStream_t st, int nr, int nm, int K, const double *A, void *cols);
+cudaError_t tc_list_products(cudaStream_t st, const Chunk &c, const PairList &l, int nr, const double *A, const double *Q,
+                             void *cols, void *rows, int *err);
 
 }  // namespace p64
 }  // namespace bsa

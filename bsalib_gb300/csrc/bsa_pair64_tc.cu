@@ -108,7 +108,7 @@ __global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restri
                                                  int *__restrict__ er) {
     __shared__ int mx[8][32];
     const int qn = c.qn, an = c.an, rx = c.rx(), ab = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
-    const int x = c.x0 + blockIdx.x, a = ab / an, b = ab - a * an;
+    const int x = c.xmap ? c.xmap[blockIdx.x] : c.x0 + blockIdx.x, a = ab / an, b = ab - a * an;
     const int *q = reinterpret_cast<const int *>(Q + a) + 1, *p = reinterpret_cast<const int *>(A + (size_t)x * c.K * an + b) + 1;
     int m = 0;
     if (ab < rx)
@@ -122,7 +122,7 @@ __global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restri
     if (lane == 0 && ab < rx) {
 #pragma unroll
         for (int z = 1; z < 8; ++z) m = max(m, mx[z][threadIdx.x]);
-        er[(size_t)blockIdx.x * rx + ab] = m == kBad ? kBad : m == 0 ? kNone : m - 2044;
+        er[(size_t)blockIdx.x * c.rpad + ab] = m == kBad ? kBad : m == 0 ? kNone : m - 2044;
     }
 }
 
@@ -141,6 +141,23 @@ __global__ __launch_bounds__(256) void k_col_digits(int nr, int an, int K, int K
     put_digits(v, some ? e : 0, D + ((size_t)ct * kDig * kTN + col) * Kp + k0, (size_t)kTN * Kp);
 }
 
+// Column digits of a pair list [block][digit][bw columns][Kp]; exponents [block][32].
+__global__ __launch_bounds__(256) void k_block_digits(int nm, int np, int bw, int K, int Kp, const double *__restrict__ A,
+                                                      const int *__restrict__ ec, int *__restrict__ eb,
+                                                      __nv_bfloat16 *__restrict__ D) {
+    const int blk = blockIdx.x, col = threadIdx.x & 31, k0 = blockIdx.y * 128 + (threadIdx.x >> 5) * 16;
+    const int y = blk / np, j = (blk - y * np) * bw + col;
+    const bool ok = col < bw && j < nm;
+    const int e = ok ? ec[y * nm + j] : kNone;
+    if (blockIdx.y == 0 && threadIdx.x < 32) eb[blk * 32 + col] = e;
+    if (k0 >= Kp || col >= bw) return;
+    const bool some = e != kNone && e != kBad;
+    double v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = (some && k0 + i < K) ? A[((size_t)y * K + k0 + i) * nm + j] : 0.0;
+    put_digits(v, some ? e : 0, D + ((size_t)blk * kDig * bw + col) * Kp + k0, (size_t)bw * Kp);
+}
+
 // Row digits [mt][digit][128 rows][Kp]; block: one x, 64 k, every (a, b).
 __global__ __launch_bounds__(256) void k_row_digits(Chunk c, int Kp, const double *__restrict__ A,
                                                     const double *__restrict__ Q, const int *__restrict__ er,
@@ -149,13 +166,13 @@ __global__ __launch_bounds__(256) void k_row_digits(Chunk c, int Kp, const doubl
     const int qn = c.qn, an = c.an, rx = c.rx(), K = c.K, xl = blockIdx.x, kb = blockIdx.y * 64;
     double *As = sm, *Qs = sm + 64 * an;
     const int n = max(0, min(64, K - kb));
-    const double *a = A + ((size_t)(c.x0 + xl) * K + kb) * an, *q = Q + (size_t)kb * qn;
+    const double *a = A + ((size_t)(c.xmap ? c.xmap[xl] : c.x0 + xl) * K + kb) * an, *q = Q + (size_t)kb * qn;
     for (int i = threadIdx.x; i < 64 * an; i += 256) As[i] = i < n * an ? a[i] : 0.0;
     for (int i = threadIdx.x; i < 64 * qn; i += 256) Qs[i] = i < n * qn ? q[i] : 0.0;
     __syncthreads();
     for (int w = threadIdx.x; w < rx * 4; w += 256) {
         const int kq = w / rx, ab = w - kq * rx, ia = ab / an, ib = ab - ia * an;
-        const long long r = (long long)xl * rx + ab;
+        const long long r = (long long)xl * c.rpad + ab;
         const int e = er[r];
         const bool some = e != kNone && e != kBad;
         double v[16];
@@ -203,9 +220,11 @@ __device__ __forceinline__ double combine(long long hi, long long lo, int ex) {
     return __longlong_as_double((long long)b);
 }
 
+// LIST: the items and column blocks of a pair list instead of the chunk's tile rows.
+template <bool LIST>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    k_pair_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Chunk c, int nk,
-              int ks_last, const int *__restrict__ er, const int *__restrict__ ec, int *err) {
+    k_pair_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Chunk c, PairList pl,
+              int nk, int ks_last, const int *__restrict__ er, const int *__restrict__ ec, int *err) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *sa = smem, *sb = smem + (size_t)kRingA * kTileA;
@@ -245,13 +264,30 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             uint32_t ia = 0, ib = 0;
             bool ok = true;
             for (long long item = blockIdx.x; item < c.items && ok; item += gridDim.x) {
-                const int mt = tile_row(c, item);
-                const int ct = c.rt[mt].ct0 + (int)(item - c.rt[mt].item0);
+                int mt, ct = 0;
+                int4 it = make_int4(0, 0, 0, 0);
+                if (LIST) {
+                    it = pl.items[item];
+                    mt = it.x;
+                } else {
+                    mt = tile_row(c, item);
+                    ct = c.rt[mt].ct0 + (int)(item - c.rt[mt].item0);
+                }
                 for (int kb = 0; kb < nk && ok; ++kb, ++ib) {
                     const int sB = ib % kRingB;
                     if (!mbar_wait(&eb[sB], ((ib / kRingB) & 1u) ^ 1u, err, 1)) { ok = false; break; }
-                    mbar_expect_tx(&fb[sB], kTileB);
-                    tma_2d(sb + sB * kTileB, &tmB, &fb[sB], kb * kBK, ct * kDig * kTN);
+                    if (LIST) {
+                        // blocks side by side within each digit's 32 rows; columns past them hold what was there
+                        mbar_expect_tx(&fb[sB], (uint32_t)(it.z * kDig * pl.bw * 128));
+                        for (int q = 0; q < it.z; ++q) {
+                            const int y = pl.blk[it.y + q] * kDig * pl.bw;
+                            for (int t = 0; t < kDig; ++t)
+                                tma_2d(sb + sB * kTileB + (t * kTN + q * pl.bw) * 128, &tmB, &fb[sB], kb * kBK, y + t * pl.bw);
+                        }
+                    } else {
+                        mbar_expect_tx(&fb[sB], kTileB);
+                        tma_2d(sb + sB * kTileB, &tmB, &fb[sB], kb * kBK, ct * kDig * kTN);
+                    }
                     for (int s = 0; s < kDig; ++s, ++ia) {
                         const int sA = ia % kRingA;
                         if (!mbar_wait(&ea[sA], ((ia / kRingA) & 1u) ^ 1u, err, 1)) { ok = false; break; }
@@ -327,9 +363,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         uint32_t tile = 0;
         bool ok = true;
         for (long long item = blockIdx.x; item < c.items && ok; item += gridDim.x) {
-            const int mt = tile_row(c, item);
-            const RowTile rt = c.rt[mt];
-            const int ct = rt.ct0 + (int)(item - rt.item0);
+            int mt, ct = 0;
+            RowTile rt{};
+            int4 it = make_int4(0, 0, 0, 0);
+            if (LIST) {
+                it = pl.items[item];
+                mt = it.x;
+            } else {
+                mt = tile_row(c, item);
+                rt = c.rt[mt];
+                ct = rt.ct0 + (int)(item - rt.item0);
+            }
             long long hi[kTN], lo[kTN];
 #pragma unroll
             for (int q = 0; q < kTN; ++q) hi[q] = lo[q] = 0;
@@ -356,23 +400,36 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 fence_before();
                 mbar_arrive(&tempty[buf]);
             }
+            // value = 2^(er + ec - 61) (hi 2^28 + lo)
+            auto value = [&](int q, int eu, int ev) {
+                return (eu == kBad || ev == kBad)     ? __longlong_as_double(0x7ff8000000000000ll)
+                       : (eu == kNone || ev == kNone) ? 0.0
+                                                      : combine(hi[q], lo[q], eu + ev - 61);
+            };
+            if (LIST) {
+                const int nm = c.an, r = (mt % pl.tiles_x) * kTM + row;
+                if (ok && r < c.rx()) {
+                    const int eu = er[mt * kTM + row];
+#pragma unroll
+                    for (int q = 0; q < kTN; ++q) {
+                        const int s = (q >= pl.bw) + (q >= 2 * pl.bw) + (q >= 3 * pl.bw);
+                        if (s >= it.z) continue;
+                        const int blk = pl.blk[it.y + s], cq = q - s * pl.bw, j = (blk % pl.np) * pl.bw + cq;
+                        if (j < nm)
+                            c.E[((size_t)pl.pair[it.y + s] * c.rx() + r) * nm + j] = value(q, eu, ec[blk * 32 + cq]);
+                    }
+                }
+                continue;
+            }
             const int r = mt * kTM + row;
             if (ok && r < nrows) {
                 const int eu = er[r];
                 double *o = c.E + rt.base + (size_t)row * rt.nct * kTN + (size_t)(ct - rt.ct0) * kTN;
 #pragma unroll
                 for (int q = 0; q < kTN; q += 2) {
-                    double2 p;
-#pragma unroll
-                    for (int z = 0; z < 2; ++z) {
-                        const int col = ct * kTN + q + z, ev = col < ncols ? ec[col] : kNone;
-                        // value = 2^(er + ec - 61) (hi 2^28 + lo)
-                        const double s = (eu == kBad || ev == kBad) ? __longlong_as_double(0x7ff8000000000000ll)
-                                         : (eu == kNone || ev == kNone) ? 0.0
-                                                                        : combine(hi[q + z], lo[q + z], eu + ev - 61);
-                        (z ? p.y : p.x) = s;
-                    }
-                    *reinterpret_cast<double2 *>(o + q) = p;
+                    const int col = ct * kTN + q;
+                    *reinterpret_cast<double2 *>(o + q) = make_double2(value(q, eu, col < ncols ? ec[col] : kNone),
+                                                                       value(q + 1, eu, col + 1 < ncols ? ec[col + 1] : kNone));
                 }
             }
         }
@@ -404,27 +461,62 @@ cudaError_t tc_prep_cols(cudaStream_t st, int nr, int an, int K, const double *A
     return cudaGetLastError();
 }
 
-cudaError_t tc_products(cudaStream_t st, const Chunk &c, int nr, const double *A, const double *Q, void *cols,
-                        void *rows, int *err) {
+// Row digits and the product kernel; rows_total rows in whole tiles.
+template <bool LIST>
+static cudaError_t products(cudaStream_t st, const Chunk &c, const PairList &l, size_t ntiles, const CUtensorMap &mb,
+                            const double *A, const double *Q, const int *ec, void *rows, int *err) {
     const int Kp = kpad(c.K), nx = c.x1 - c.x0;
-    const size_t nct = ((size_t)nr * c.an + kTN - 1) / kTN, nmt = (size_t)c.ntiles;
-    int *ec = (int *)((char *)cols + up256(nct * kDig * kTN * Kp * 2));
-    int *er = (int *)((char *)rows + up256(nmt * kDig * kTM * Kp * 2));
+    int *er = (int *)((char *)rows + up256(ntiles * kDig * kTM * Kp * 2));
     k_row_exp<<<dim3(nx, (c.rx() + 31) / 32), 256, 0, st>>>(c, A, Q, er);
     const size_t sm = sizeof(double) * 64 * (c.qn + c.an);
     cudaError_t e = cudaFuncSetAttribute(k_row_digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     k_row_digits<<<dim3(nx, Kp / 64), 256, sm, st>>>(c, Kp, A, Q, er, (__nv_bfloat16 *)rows);
-    CUtensorMap ma, mb;
-    if (!make_map(&ma, rows, Kp, (uint64_t)nmt * kDig * kTM, kTM) ||
-        !make_map(&mb, cols, Kp, (uint64_t)nct * kDig * kTN, kDig * kTN))
-        return cudaErrorInvalidValue;
-    if ((e = cudaFuncSetAttribute(k_pair_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem))) return e;
+    CUtensorMap ma;
+    if (!make_map(&ma, rows, Kp, (uint64_t)ntiles * kDig * kTM, kTM)) return cudaErrorInvalidValue;
+    if ((e = cudaFuncSetAttribute(k_pair_tc<LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem))) return e;
     int dev = 0, nsm = 0;
     if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev))) return e;
     const int nk = Kp / kBK, ks_last = (c.K - (nk - 1) * kBK + 15) / 16;
-    k_pair_tc<<<(unsigned)std::min<long long>(nsm, c.items), kTcThreads, kTcSmem, st>>>(ma, mb, c, nk, ks_last, er, ec, err);
+    k_pair_tc<LIST><<<(unsigned)std::min<long long>(nsm, c.items), kTcThreads, kTcSmem, st>>>(ma, mb, c, l, nk, ks_last, er,
+                                                                                             ec, err);
     return cudaGetLastError();
+}
+
+cudaError_t tc_products(cudaStream_t st, const Chunk &c, int nr, const double *A, const double *Q, void *cols,
+                        void *rows, int *err) {
+    const int Kp = kpad(c.K);
+    const size_t nct = ((size_t)nr * c.an + kTN - 1) / kTN;
+    const int *ec = (const int *)((char *)cols + up256(nct * kDig * kTN * Kp * 2));
+    CUtensorMap mb;
+    if (!make_map(&mb, cols, Kp, (uint64_t)nct * kDig * kTN, kDig * kTN)) return cudaErrorInvalidValue;
+    return products<false>(st, c, PairList{}, (size_t)c.ntiles, mb, A, Q, ec, rows, err);
+}
+
+// [digits][block exponents][row exponents]
+size_t tc_block_bytes(int nr, int nm, int K) {
+    const size_t nb = (size_t)nr * blocks_of(nm);
+    return up256(nb * kDig * block_width(nm) * kpad(K) * 2) + up256(nb * 32 * sizeof(int)) + up256(sizeof(int) * (size_t)nr * nm);
+}
+
+cudaError_t tc_prep_blocks(cudaStream_t st, int nr, int nm, int K, const double *A, void *cols) {
+    const int Kp = kpad(K), np = blocks_of(nm), bw = block_width(nm);
+    const size_t nb = (size_t)nr * np;
+    int *eb = (int *)((char *)cols + up256(nb * kDig * bw * Kp * 2));
+    int *ec = (int *)((char *)eb + up256(nb * 32 * sizeof(int)));
+    k_col_exp<<<nr, 256, 0, st>>>(nm, K, A, ec);
+    k_block_digits<<<dim3((unsigned)nb, (Kp + 127) / 128), 256, 0, st>>>(nm, np, bw, K, Kp, A, ec, eb, (__nv_bfloat16 *)cols);
+    return cudaGetLastError();
+}
+
+cudaError_t tc_list_products(cudaStream_t st, const Chunk &c, const PairList &l, int nr, const double *A, const double *Q,
+                             void *cols, void *rows, int *err) {
+    const int Kp = kpad(c.K);
+    const size_t nb = (size_t)nr * l.np;
+    const int *eb = (const int *)((char *)cols + up256(nb * kDig * l.bw * Kp * 2));
+    CUtensorMap mb;
+    if (!make_map(&mb, cols, Kp, (uint64_t)nb * kDig * l.bw, (uint32_t)l.bw)) return cudaErrorInvalidValue;
+    return products<true>(st, c, l, (size_t)c.x1 * l.tiles_x, mb, A, Q, eb, rows, err);
 }
 
 }  // namespace p64
