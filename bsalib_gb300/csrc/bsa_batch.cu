@@ -646,7 +646,9 @@ struct BatchCase {
     int nnl = 0, psd_type = 0, nme = 0, K = 0;
     bool trunc = true;
     std::vector<int> modes;
-    std::vector<double> hL, hQ, hCoh, hM, hK, hC, hWd3, hWd2;
+    std::vector<double> hL, hQ, hCorr, hM, hK, hC, hWd3, hWd2;
+    std::vector<int> hNodes;
+    int hNn = 0;
     std::vector<float> hL32;
     std::vector<PsdNode> hPsd;
     std::vector<double> f;  // Classic grid
@@ -670,7 +672,7 @@ int Engine::batch_add(int *id) {
     c.K = K;
     c.trunc = classic_trunc;
     c.modes = modes;
-    c.hL = hL; c.hQ = hQ; c.hCoh = hCoh; c.hM = hM; c.hK = hK; c.hC = hC; c.hWd3 = hWd3; c.hWd2 = hWd2;
+    c.hL = hL; c.hQ = hQ; c.hCorr = hCorr; c.hNodes = hNodes; c.hNn = hNn; c.hM = hM; c.hK = hK; c.hC = hC; c.hWd3 = hWd3; c.hWd2 = hWd2;
     c.hL32 = hL32; c.hPsd = hPsd;
     g_batch.push_back(std::move(c));
     if (id) *id = (int)g_batch.size() - 1;
@@ -687,7 +689,7 @@ void Engine::batch_install(const BatchCase &c) {
     nme = c.nme;
     K = c.K;
     modes = c.modes;
-    hL = c.hL; hQ = c.hQ; hCoh = c.hCoh; hM = c.hM; hK = c.hK; hC = c.hC; hWd3 = c.hWd3; hWd2 = c.hWd2;
+    hL = c.hL; hQ = c.hQ; hCorr = c.hCorr; hNodes = c.hNodes; hNn = c.hNn; hM = c.hM; hK = c.hK; hC = c.hC; hWd3 = c.hWd3; hWd2 = c.hWd2;
     hL32 = c.hL32; hPsd = c.hPsd;
     derived_ok = true;
     dev_uploaded = false;
@@ -746,7 +748,7 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
     saved.K = K;
     saved.trunc = classic_trunc;
     saved.modes = modes;
-    saved.hL = hL; saved.hQ = hQ; saved.hCoh = hCoh; saved.hM = hM; saved.hK = hK; saved.hC = hC;
+    saved.hL = hL; saved.hQ = hQ; saved.hCorr = hCorr; saved.hNodes = hNodes; saved.hNn = hNn; saved.hM = hM; saved.hK = hK; saved.hC = hC;
     saved.hWd3 = hWd3; saved.hWd2 = hWd2; saved.hL32 = hL32; saved.hPsd = hPsd;
     const Inputs saved_in = in;
     const bool saved_ok = derived_ok;

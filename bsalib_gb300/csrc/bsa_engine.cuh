@@ -147,7 +147,9 @@ struct Engine {
     std::vector<int> modes;
     int nme = 0, K = 0;
     std::vector<double> phitc, hL, hQ, hM, hK, hC;
-    std::vector<double> hCoh;          // coherence bases c_ij [comp][i][j]; log c formed on the device
+    std::vector<double> hCorr;         // packed coherences of the components [comp][ncorr]; log c_ij formed on the device
+    std::vector<int> hNodes;           // loaded nodes
+    int hNn = 0;                       // nodes the packing counts
     std::vector<double> hWd3, hWd2;  // diagonal-only weights Q L^2 and L^2, [k][m]
     std::vector<float> hL32;         // FP32 copy of L for the split-precision A(f) table
     std::vector<PsdNode> hPsd;
@@ -157,7 +159,7 @@ struct Engine {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     DevBuf dL, dQ, dLogc, dPsdPar, dFrfM, dFrfK, dFrfC, dFreq, dS, dA, dPartF, dPartR, dOut, dPsdF, dWf, dPts,
         dPtsD, dBF, dBR, dMixA, dMixB, dMixH, dMixPart, dA32, dZones, dZidx, dWd3, dWd2, dMshT, dMshIdx, dLogc32, dL32,
-        dPod, dFlag, dSlot, dHash, dCptr, dCq, dZoneH, dZoff;
+        dPod, dFlag, dSlot, dHash, dCptr, dCq, dZoneH, dZoff, dCorr;
 
     // stats
     double last_ms = 0, last_ms_contraction = 0, last_ms_gemm = 0, last_points = 0;
@@ -178,7 +180,7 @@ struct Engine {
     int build_atable(const std::vector<double> &freqs, bool fp32 = false, bool msh = false);
     int pod_atable(const std::vector<double> &freqs, bool fp32);
     int build_psd(const std::vector<double> &freqs);
-    int build_psd_dev(int nf, bool fp32 = false, bool root = false);  // the nf frequencies already in dFreq
+    int build_psd_dev(int nf, bool fp32 = false, double *expt = nullptr);  // the nf frequencies already in dFreq
     int build_atable_dev(int nf, bool fp32);   // the same, A table (not the truncated POD form)
     // dimM_psd_ / dimM_bisp_ (src/bsa/BsaLibImpl.F90:313-355): nm / nm for the diagonal-only
     // spectra, nm^2 / nm^3 otherwise.

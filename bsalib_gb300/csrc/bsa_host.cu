@@ -158,7 +158,7 @@ void Engine::free_device() {
     if (stream) cudaStreamSynchronize(stream);  // the blocks go back to the cache for reuse
     for (DevBuf *b : {&dL, &dQ, &dLogc, &dPsdPar, &dFrfM, &dFrfK, &dFrfC, &dFreq, &dS, &dA, &dPartF, &dPartR,
                       &dOut, &dPsdF, &dWf, &dPts, &dPtsD, &dBF, &dBR, &dMixA, &dMixB, &dMixH, &dMixPart, &dA32,
-                      &dZones, &dZidx, &dWd3, &dWd2, &dMshT, &dMshIdx, &dLogc32, &dL32, &dPod, &dFlag, &dSlot, &dHash, &dCptr, &dCq, &dZoneH, &dZoff})
+                      &dZones, &dZidx, &dWd3, &dWd2, &dMshT, &dMshIdx, &dLogc32, &dL32, &dPod, &dFlag, &dSlot, &dHash, &dCptr, &dCq, &dZoneH, &dZoff, &dCorr})
         b->release();
     if (stream) cudaStreamDestroy(stream);
     stream = nullptr;
@@ -181,12 +181,6 @@ int Engine::ensure_stream() {
     if ((e = cudaEventCreate(&evg0)) != cudaSuccess) return cuda_fail(e, "cudaEventCreate");
     if ((e = cudaEventCreate(&evg1)) != cudaSuccess) return cuda_fail(e, "cudaEventCreate");
     return BSA_OK;
-}
-
-static long corr_index(int ni, int nj, int tot) {
-    // util_getCorrVectIndex, src/utils/utility.F90:60-71 (1-based)
-    if (nj >= ni) return (long)(ni - 1) * tot + nj - ((long)ni * ni - ni) / 2;
-    return (long)(nj - 1) * tot + ni - ((long)nj * nj - nj) / 2;
 }
 
 // validateAll_ (src/bsa/BsaLibImpl.F90:469-535) restricted to what the BFM path reads:
@@ -286,14 +280,28 @@ int Engine::validate() {
         hWd2[x] = hL[x] * hL[x];
     }
     const long ncorr = (long)I.ncorr;
-    hCoh.assign((size_t)ntc * nnl * nnl, 0.0);
-    for (int itc = 0; itc < ntc; ++itc)
-        for (int i = 0; i < nnl; ++i)
-            for (int j = 0; j < nnl; ++j) {
-                const long id = corr_index(I.n_load[i], I.n_load[j], I.nn);
-                const double c = I.corr[(size_t)(id - 1) + (size_t)ncorr * (set.tc[itc] - 1)];
-                hCoh[((size_t)itc * nnl + i) * nnl + j] = c;
-            }
+    hNodes.assign(I.n_load, I.n_load + nnl);
+    hNn = I.nn;
+    if (I.nn <= 2 * nnl) {  // the whole packed triangle is at most twice the loaded nodes' square
+        hCorr.resize((size_t)ntc * ncorr);
+        for (int itc = 0; itc < ntc; ++itc)
+            std::memcpy(hCorr.data() + (size_t)itc * ncorr, I.corr + (size_t)ncorr * (set.tc[itc] - 1), sizeof(double) * ncorr);
+    } else {  // few of many nodes loaded: their own packed triangle
+        const size_t nc = (size_t)nnl * (nnl + 1) / 2;
+        hCorr.resize(ntc * nc);
+        for (int itc = 0; itc < ntc; ++itc) {
+            const double *col = I.corr + (size_t)ncorr * (set.tc[itc] - 1);
+            double *out = hCorr.data() + itc * nc;
+            for (int i = 0; i < nnl; ++i)
+                for (int j = i; j < nnl; ++j) {
+                    // util_getCorrVectIndex, src/utils/utility.F90:60-71 (1-based)
+                    const long u = std::min(hNodes[i], hNodes[j]), v = std::max(hNodes[i], hNodes[j]);
+                    *out++ = col[(u - 1) * I.nn + v - (u * u - u) / 2 - 1];
+                }
+        }
+        for (int i = 0; i < nnl; ++i) hNodes[i] = i + 1;
+        hNn = nnl;
+    }
     hL32.assign(hL.begin(), hL.end());
     const int idir = set.dirs.empty() ? 1 : set.dirs[0];
     hPsd.assign((size_t)ntc * nnl, PsdNode{});
@@ -331,14 +339,20 @@ int Engine::upload_problem() {
     if ((rc = ensure_stream())) return rc;
     if (dev_uploaded) return BSA_OK;
     cudaError_t e;
-    if ((e = dLogc.reserve(log_coh_bytes(hCoh.size())))) return cuda_fail(e, "uploading problem data");
-    if ((e = upload(dL, hL, stream)) || (e = upload(dQ, hQ, stream)) || (e = upload(dLogc, hCoh, stream)) ||
-        (e = upload(dPsdPar, hPsd, stream)) || (e = upload(dFrfM, hM, stream)) || (e = upload(dFrfK, hK, stream)) ||
-        (e = upload(dFrfC, hC, stream)) || (e = upload(dWd3, hWd3, stream)) || (e = upload(dWd2, hWd2, stream)) ||
-        (e = upload(dL32, hL32, stream)) || (e = dLogc32.reserve(sizeof(float) * hCoh.size())))
+    const int ntc = (int)set.tc.size(), nnl = (int)hNodes.size();
+    const size_t ncoh = (size_t)ntc * nnl * nnl, nb = (sizeof(int) * nnl + 255) / 256 * 256;
+    if ((e = dCorr.reserve(nb + sizeof(double) * hCorr.size())) || (e = dLogc.reserve(log_coh_bytes(ncoh))) ||
+        (e = cudaMemcpyAsync(dCorr.p, hNodes.data(), sizeof(int) * nnl, cudaMemcpyHostToDevice, stream)) ||
+        (e = cudaMemcpyAsync((char *)dCorr.p + nb, hCorr.data(), sizeof(double) * hCorr.size(), cudaMemcpyHostToDevice, stream)) ||
+        (e = upload(dL, hL, stream)) || (e = upload(dQ, hQ, stream)) || (e = upload(dPsdPar, hPsd, stream)) ||
+        (e = upload(dFrfM, hM, stream)) || (e = upload(dFrfK, hK, stream)) || (e = upload(dFrfC, hC, stream)) ||
+        (e = upload(dWd3, hWd3, stream)) || (e = upload(dWd2, hWd2, stream)) || (e = upload(dL32, hL32, stream)) ||
+        (e = dLogc32.reserve(sizeof(float) * ncoh)))
         return cuda_fail(e, "uploading problem data");
-    // log c in place (FP64) and its FP32 copy
-    if ((e = launch_log_coh(stream, hCoh.size(), dLogc.as<double>(), dLogc32.as<float>())))
+    h2d += (double)(sizeof(int) * nnl + sizeof(double) * hCorr.size());
+    // log c in FP64 and its FP32 copy
+    if ((e = launch_log_coh(stream, ntc, nnl, hNn, (long long)(hCorr.size() / ntc), dCorr.as<int>(),
+                            (const double *)((char *)dCorr.p + nb), dLogc.as<double>(), dLogc32.as<float>())))
         return cuda_fail(e, "coherence table");
     kernels += 1;
     dev_uploaded = true;
@@ -355,13 +369,13 @@ int Engine::build_psd(const std::vector<double> &freqs) {
 }
 
 // Nodal PSD table S[f][k] for the nf frequencies already in dFreq (fp32: the formulas
-// evaluated in FP32, for the split-precision A tables; root: sqrt(S)).
-int Engine::build_psd_dev(int nf, bool fp32, bool root) {
+// evaluated in FP32, for the split-precision A tables; expt: sqrt(S) and the exponential's table).
+int Engine::build_psd_dev(int nf, bool fp32, double *expt) {
     const int ntc = (int)set.tc.size();
     cudaError_t e;
     if ((e = dS.reserve(sizeof(double) * (size_t)nf * ntc * in.nnl))) return cuda_fail(e, "allocating S");
     if ((e = launch_nodal_psd(stream, nf, dFreq.as<double>(), ntc, set.tc.data(), in.nnl, dPsdPar.as<PsdNode>(),
-                              in.psd_type, set.defsc, dS.as<double>(), fp32, root)))
+                              in.psd_type, set.defsc, dS.as<double>(), fp32, expt)))
         return cuda_fail(e, "nodal PSD kernel");
     kernels += 1;
     return BSA_OK;
@@ -379,7 +393,8 @@ int Engine::build_atable(const std::vector<double> &freqs, bool fp32, bool msh) 
 int Engine::build_atable_dev(int nf, bool fp32) {
     const int ntc = (int)set.tc.size();
     cudaError_t e;
-    int rc = build_psd_dev(nf, fp32, !fp32);  // the FP64 table reads sqrt(S)
+    // the FP64 table reads sqrt(S) and the exponential's table behind log c
+    int rc = build_psd_dev(nf, fp32, fp32 ? nullptr : dLogc.as<double>() + (size_t)ntc * in.nnl * in.nnl);
     if (rc) return rc;
     if (fp32) {
         // FP32 table on the tensor cores (tf32 hi/lo split, FP32-level accuracy)

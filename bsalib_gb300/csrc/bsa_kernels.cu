@@ -7,6 +7,8 @@
 
 namespace bsa {
 
+constexpr int kExpTab = 256;  // 2^(k / 256), k = 0 .. 255
+
 // ------------------------------------------------------------------------------------
 // Stage (a): nodal turbulence PSD.  One thread per (f, itc, node), node fastest so the
 // stores are coalesced.  Model formulas: vonKarmanPSD_ (WindPSDImpl.F90:149-226, u form
@@ -18,10 +20,12 @@ namespace bsa {
 // ------------------------------------------------------------------------------------
 template <typename R>
 __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 tcs, int nnl,
-                            const PsdNode *__restrict__ par, int psd_type, int scaling, int root,
-                            double *__restrict__ S) {
+                            const PsdNode *__restrict__ par, int psd_type, int scaling, double *__restrict__ S,
+                            double *__restrict__ expt) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long tot = (long long)nf * ntc * nnl;
+    // expt (FP64 only): sqrt(S) instead of S, and the A kernel's exponential table
+    if (sizeof(R) == 8 && expt && blockIdx.x == 0) expt[threadIdx.x] = exp2((double)threadIdx.x / kExpTab);
     if (t >= tot) return;
     const int i = (int)(t % nnl);
     const long long r = t / nnl;
@@ -66,20 +70,20 @@ __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 
         v = 0;
     }
     if (scaling == 1) v = v / R(kPi4);
-    S[t] = root ? sqrt((double)v) : (double)v;
+    S[t] = (sizeof(R) == 8 && expt) ? sqrt((double)v) : (double)v;
 }
 
 cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, const int *tcs_host,
-                             int nnl, const PsdNode *par, int psd_type, int scaling, double *S, bool fp32, bool root) {
+                             int nnl, const PsdNode *par, int psd_type, int scaling, double *S, bool fp32, double *expt) {
     const long long tot = (long long)nf * ntc * nnl;
     if (tot == 0) return cudaSuccess;
     int4 tcs = make_int4(tcs_host[0], ntc > 1 ? tcs_host[1] : 0, ntc > 2 ? tcs_host[2] : 0, 0);
-    const int blk = 256;
+    const int blk = kExpTab;
     const unsigned grid = (unsigned)((tot + blk - 1) / blk);
     if (fp32)
-        k_nodal_psd<float><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, root ? 1 : 0, S);
+        k_nodal_psd<float><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, S, expt);
     else
-        k_nodal_psd<double><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, root ? 1 : 0, S);
+        k_nodal_psd<double><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, S, expt);
     return cudaGetLastError();
 }
 
@@ -96,8 +100,6 @@ cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, 
 // where exp() spends about 25, and sqrt(S) comes from k_nodal_psd.  150 nodes, 12 modes, 3333
 // frequencies: 13.1 -> 3.9 ms.
 // ------------------------------------------------------------------------------------
-constexpr int kExpTab = 256;  // 2^(k / 256), k = 0 .. 255
-
 // e^x by table and polynomial (P. T. P. Tang, ACM TOMS 15, 1989): x = (256 q + k) ln2 / 256 + r,
 // |r| <= ln2 / 512, e^x = 2^q T[k] (1 + r + r^2/2 + r^3/6 + r^4/24); the next term is below 2^-54.
 // ln2 / 256 = hi + lo with hi of 25 bits, so that its product with the integer (18 bits) is exact.
@@ -176,19 +178,25 @@ __global__ __launch_bounds__(256) void k_atable(int nf, const double *__restrict
     }
 }
 
-// The first block also fills the exponential's table behind the log-coherences.
-__global__ void k_log_coh(size_t n, double *__restrict__ lc, float *__restrict__ lc32) {
-    const size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.x == 0) lc[n + threadIdx.x] = exp2((double)threadIdx.x / kExpTab);
-    if (x >= n) return;
-    const double v = log(lc[x]);
+// log c_ij of every loaded node pair from the packed upper triangle (util_getCorrVectIndex,
+// src/utils/utility.F90:60-71), in FP64 and FP32; the host side of this expansion and its copy were
+// 0.6 ms of a 400-node, two-component analysis.
+__global__ void k_log_coh(int ntc, int nnl, int nn, long long ncorr, const int *__restrict__ nodes,
+                          const double *__restrict__ corr, double *__restrict__ lc, float *__restrict__ lc32) {
+    const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= (long long)ntc * nnl * nnl) return;
+    const int j = (int)(x % nnl), i = (int)(x / nnl % nnl), c = (int)(x / nnl / nnl);
+    const long long a = min(nodes[i], nodes[j]), b = max(nodes[i], nodes[j]);
+    const double v = log(corr[c * ncorr + (a - 1) * nn + b - (a * a - a) / 2 - 1]);
     lc[x] = v;
     lc32[x] = (float)v;
 }
 
-cudaError_t launch_log_coh(cudaStream_t st, size_t n, double *lc, float *lc32) {
+cudaError_t launch_log_coh(cudaStream_t st, int ntc, int nnl, int nn, long long ncorr, const int *nodes, const double *corr,
+                           double *lc, float *lc32) {
+    const long long n = (long long)ntc * nnl * nnl;
     if (n == 0) return cudaSuccess;
-    k_log_coh<<<(unsigned)((n + kExpTab - 1) / kExpTab), kExpTab, 0, st>>>(n, lc, lc32);
+    k_log_coh<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ntc, nnl, nn, ncorr, nodes, corr, lc, lc32);
     return cudaGetLastError();
 }
 

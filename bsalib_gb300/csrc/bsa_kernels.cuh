@@ -5,18 +5,21 @@
 namespace bsa {
 
 // Nodal PSD S[f][itc][i] for nf frequencies (evalPSD_ and the model functions,
-// src/wind/WindPSDImpl.F90:123-316).  tcs: turbulent component ids (1..3) per itc.  root: sqrt(S).
+// src/wind/WindPSDImpl.F90:123-316).  tcs: turbulent component ids (1..3) per itc.  expt
+// (FP64): sqrt(S) instead, and the A kernel's exponential table into expt.
 cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, const int *tcs_host,
                              int nnl, const PsdNode *par, int psd_type, int scaling, double *S, bool fp32 = false,
-                             bool root = false);
+                             double *expt = nullptr);
 
-// lc[x] = log(lc[x]) in place (FP64) and lc32[x] = (float)lc[x], x < n: the coherence table log c,
-// followed in lc by the table of the A kernel's exponential (log_coh_bytes(n) in all).
+// log c_ij [itc][i][j] of the loaded nodes (1-based ids) from the packed coherences corr[itc][ncorr] of
+// nn nodes, in FP64 and FP32.  lc has room for the A kernel's exponential table behind it
+// (log_coh_bytes(n), n = ntc nnl^2).
 size_t log_coh_bytes(size_t n);
-cudaError_t launch_log_coh(cudaStream_t st, size_t n, double *lc, float *lc32);
+cudaError_t launch_log_coh(cudaStream_t st, int ntc, int nnl, int nn, long long ncorr, const int *nodes, const double *corr,
+                           double *lc, float *lc32);
 
 // A[f][k][m] = sqrt(S_i(f)) sum_j c_ij^|f| sqrt(S_j(f)) L[(itc,j)][m]  (FP64); rootS = sqrt(S), logc
-// as launch_log_coh leaves it (n = ntc nnl^2).
+// followed by the exponential's table (launch_nodal_psd's expt).
 cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm,
                           const double *logc, const double *rootS, const double *L, double *A);
 

@@ -47,3 +47,27 @@ def test_atable_through_force_moments(bsalib, nodes, modes):
     w[[0, -1]] /= 2
     ref = np.einsum("f,fon->on", w, _reference(p, f)).ravel()
     assert np.max(np.abs(m2 - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("nodes,loaded", [(9, (9, 2, 5)), (7, (7, 1, 4, 6)), (6, (2, 4, 6, 1, 3, 5)), (40, (40, 1))])
+def test_loaded_nodes_in_any_order(bsalib, nodes, loaded):
+    """Few of many nodes loaded, and out of order: the coherences are those of the loaded nodes."""
+    import dataclasses
+    p = random_structure(nodes, nodes=(nodes, nodes), modes=(3, 3), nfreq_grid=(9, 9))
+    p.settings.ibisp = 0
+    ix = np.array(loaded) - 1
+    q = dataclasses.replace(p, n_load=np.array(loaded, dtype=np.int32), wfc=np.asfortranarray(p.wfc[:, :, ix]))
+    s = api.BsaSession(q)
+    try:
+        m2 = s.run()["m2mf_cls"]
+    finally:
+        s.close()
+    # the same with zero forces on the other nodes
+    w = np.zeros_like(p.wfc)
+    w[:, :, ix] = p.wfc[:, :, ix]
+    s = api.BsaSession(dataclasses.replace(p, wfc=np.asfortranarray(w)))
+    try:
+        ref = s.run()["m2mf_cls"]
+    finally:
+        s.close()
+    assert np.max(np.abs(m2 - ref)) <= 1e-12 * np.max(np.abs(ref))
