@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <deque>
 #include <vector>
 
 #include "../../include/bsa_gpu.h"
@@ -44,6 +45,7 @@ constexpr size_t kSmem = (size_t)kStages * kStageBytes + 1024 + kBarBytes + kHBy
 struct CaseP {
     int nf, nm, Mp, MT, nk, ks_last, n_ntiles, wmode;
     double wval;
+    int ufold;        // the case's U rows are those of |r - h| (E form, every quantity is even in f)
     int u_row0;       // first U-table row of the case
     int g_row0;       // first G-table row
     int s_row0;       // first S-table row
@@ -444,7 +446,7 @@ __global__ void __launch_bounds__(ecls::ELayout<RS>::threads, 1)  // 128 registe
                 const BItem im = p.items[w];
                 const CaseP cs = p.cases[im.c];
                 const int nu = n_units(im.r, cs.n_ntiles, NC), nt0 = im.r / NC;
-                const int yu = cs.u_row0 + im.r * cs.Mp + im.mt * kBM;
+                const int yu = cs.u_row0 + (cs.ufold ? abs(im.r - (cs.nf - 1) / 2) : im.r) * cs.Mp + im.mt * kBM;
                 for (int jh = 0; jh < JH && ok; ++jh)
                 for (int u = 0; u < nu && ok; ++u)
                     for (int kc = 0; kc < cs.nk && ok; ++kc, ++it) {
@@ -679,8 +681,26 @@ int Engine::batch_add(int *id) {
     return BSA_OK;
 }
 
+// Exchanges the engine's derived tables with case c's: copies to the device read the case's own
+// vectors, which stay where they are until the sweep is over.
+void Engine::batch_swap(BatchCase &c) {
+    modes.swap(c.modes);
+    hL.swap(c.hL);
+    hQ.swap(c.hQ);
+    hCorr.swap(c.hCorr);
+    hNodes.swap(c.hNodes);
+    std::swap(hNn, c.hNn);
+    hM.swap(c.hM);
+    hK.swap(c.hK);
+    hC.swap(c.hC);
+    hWd3.swap(c.hWd3);
+    hWd2.swap(c.hWd2);
+    hL32.swap(c.hL32);
+    hPsd.swap(c.hPsd);
+}
+
 // Makes case c the engine's problem (derived tables only; no caller arrays are read).
-void Engine::batch_install(const BatchCase &c) {
+void Engine::batch_install(BatchCase &c) {
     in = Inputs();
     in.nnl = c.nnl;
     in.psd_type = c.psd_type;
@@ -688,9 +708,7 @@ void Engine::batch_install(const BatchCase &c) {
     classic_trunc = c.trunc;
     nme = c.nme;
     K = c.K;
-    modes = c.modes;
-    hL = c.hL; hQ = c.hQ; hCorr = c.hCorr; hNodes = c.hNodes; hNn = c.hNn; hM = c.hM; hK = c.hK; hC = c.hC; hWd3 = c.hWd3; hWd2 = c.hWd2;
-    hL32 = c.hL32; hPsd = c.hPsd;
+    batch_swap(c);
     derived_ok = true;
     dev_uploaded = false;
 }
@@ -727,6 +745,8 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
         return use_e_form && b.nme <= kEFormMaxModes && b.trunc && (b.f.size() & 1) != 0 &&
                plan_prefer_e(b.nme, b.K, (int)b.f.size());
     };
+    // A rows of f >= 0 stand for the whole grid (Engine::run_classic's fold)
+    auto fold_ok = [](const BatchCase &b) { return b.trunc && b.set.defsc == 1 && (b.f.size() & 1) != 0; };
     // group width: the FRF-table width of the D1 / D3 form, or of the E form (8, 16, 24; 32 and
     // 48 as two mode halves of 16 and 24)
     auto width = [&](int c) {
@@ -747,14 +767,12 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
     saved.nme = nme;
     saved.K = K;
     saved.trunc = classic_trunc;
-    saved.modes = modes;
-    saved.hL = hL; saved.hQ = hQ; saved.hCorr = hCorr; saved.hNodes = hNodes; saved.hNn = hNn; saved.hM = hM; saved.hK = hK; saved.hC = hC;
-    saved.hWd3 = hWd3; saved.hWd2 = hWd2; saved.hL32 = hL32; saved.hPsd = hPsd;
+    batch_swap(saved);
     const Inputs saved_in = in;
     const bool saved_ok = derived_ok;
     struct Restore {
         Engine &E;
-        const BatchCase &c;
+        BatchCase &c;
         const Inputs &in;
         bool ok;
         ~Restore() {
@@ -816,6 +834,7 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
             double delta = c.f[1] - c.f[0];
             if (c.set.defsc == 1) delta *= kPi2;
             q.wval = delta * delta;
+            q.ufold = eform && fold_ok(c) ? 1 : 0;
             q.u_row0 = (int)urows;
             q.g_row0 = (int)grows;
             q.s_row0 = (int)srows;
@@ -823,7 +842,7 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
             q.hs0 = (int)hs;
             q.part0 = parts;
             q.nitems = (unsigned)(nf * q.MT);
-            urows += (long long)nf * q.Mp;
+            urows += (long long)(q.ufold ? (nf + 1) / 2 : nf) * q.Mp;
             grows += (long long)JH * nf * NMT;
             if (!eform) srows += (long long)JH * (2 * nf - 1) * NMT;
             hg += (long long)nf * Wd;
@@ -859,43 +878,64 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
             (e = cudaMemsetAsync(d_cnt, 0, sizeof(unsigned) * cp.size(), stream)) ||
             (e = cudaMemsetAsync(d_tdone, 0, sizeof(unsigned long long) * (cp.size() + 1), stream)))
             return cuda_fail(e, "batch memset");
-        // per case: its tables, A(f) in FP32, operands into the group tables, m2
+        // per case: its tables, A(f) in FP32, operands into the group tables, m2; nothing waits between
+        // the cases, so what the copies read lives until the group is done
+        std::deque<std::vector<double>> hostv;
         for (size_t k = g0; k < g1; ++k) {
-            const BatchCase &c = g_batch[order[k]];
+            BatchCase &c = g_batch[order[k]];
             const CaseP &q = cp[k - g0];
-            batch_install(c);
+            struct Installed {
+                Engine &E;
+                BatchCase &c;
+                Installed(Engine &E, BatchCase &c) : E(E), c(c) { E.batch_install(c); }
+                ~Installed() { E.batch_swap(c); }
+            } installed(*this, c);
             if ((rc = upload_problem())) return rc;
             const int nf = q.nf;
-            std::vector<double> ftab = c.f;
-            if (!c.trunc)
-                for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back(2.0 * c.f[0] + s * (c.f[1] - c.f[0]));
-            if ((rc = build_atable(ftab, true))) return rc;
+            const int half = (nf - 1) / 2, fold1 = fold_ok(c) ? half + 1 : 0;
+            if (fold1) {
+                if ((e = upload(dFreq, c.f, stream))) return cuda_fail(e, "uploading frequencies");
+                rc = build_atable_dev(half + 1, true, half);
+            } else {
+                hostv.push_back(c.f);
+                std::vector<double> &ftab = hostv.back();
+                if (!c.trunc)
+                    for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back(2.0 * c.f[0] + s * (c.f[1] - c.f[0]));
+                rc = build_atable(ftab, true);
+            }
+            if (rc) return rc;
             const float *A = dA32.as<float>();
-            if ((e = mixed::prep_u(stream, nf, c.nme, c.K, Kp, q.Mp, A, dQ.as<double>(), Uh + (size_t)q.u_row0 * Kp,
-                                   Ul + (size_t)q.u_row0 * Kp)) ||
+            if ((e = mixed::prep_u(stream, q.ufold ? half + 1 : nf, c.nme, c.K, Kp, q.Mp, A, dQ.as<double>(),
+                                   Uh + (size_t)q.u_row0 * Kp, Ul + (size_t)q.u_row0 * Kp, q.ufold ? 0 : fold1)) ||
                 (e = mixed::prep_h(stream, nf, c.nme, Wd, dFreq.as<double>(), frf(), Hg + q.hg0, Hs + q.hs0, eform)))
                 return cuda_fail(e, "batch operand preparation");
             for (int jh = 0; jh < JH; ++jh) {
                 const size_t og = ((size_t)q.g_row0 + (size_t)jh * nf * NMT) * Kp;
                 const size_t os = ((size_t)q.s_row0 + (size_t)jh * (2 * nf - 1) * NMT) * Kp;
                 if ((e = mixed::prep_b(stream, nf, c.nme, NMT, jh * NMT, c.K, Kp, nf, (nf - 1) / 2, c.trunc ? 1 : 0, nf,
-                                       0, A, Gh + og, Gl + og)) ||
+                                       0, A, Gh + og, Gl + og, fold1)) ||
                     (!eform && (e = mixed::prep_b(stream, 2 * nf - 1, c.nme, NMT, jh * NMT, c.K, Kp, nf, (nf - 1) / 2,
-                                       c.trunc ? 1 : 0, nf, 1, A, Sh + os, Sl + os))))
+                                       c.trunc ? 1 : 0, nf, 1, A, Sh + os, Sl + os, fold1))))
                     return cuda_fail(e, "batch operand preparation");
             }
             // second-order moments (FP64 over the FP32 A table), rectangle or trapezoid weights
             double delta = c.f[1] - c.f[0];
             if (c.set.defsc == 1) delta *= kPi2;
-            std::vector<double> wf(nf, delta);
+            hostv.emplace_back(nf, delta);
+            std::vector<double> &wf = hostv.back();
             if (q.wmode == kWeightClassicVect) { wf[0] = delta / 2; wf[nf - 1] = delta / 2; }
+            const int np = fold1 ? half + 1 : nf;
+            if (fold1) {
+                wf.erase(wf.begin(), wf.begin() + half);
+                for (int k2 = 1; k2 < np; ++k2) wf[k2] *= 2.0;
+            }
             const int nm2 = c.nme * c.nme;
             if ((e = upload(dWf, wf, stream)) || (e = dPsdF.reserve(sizeof(double) * (size_t)nf * nm2)))
                 return cuda_fail(e, "batch m2");
             double *m2o = d_m2 + 3 * off2[order[k]];
-            if ((e = launch_force_psd32(stream, nf, (int)c.set.tc.size(), c.nnl, c.nme, dL32.as<float>(), A,
+            if ((e = launch_force_psd32(stream, np, (int)c.set.tc.size(), c.nnl, c.nme, dL32.as<float>(), A,
                                         dPsdF.as<double>())) ||
-                (e = launch_m2(stream, 0, nf, c.nme, 0, dFreq.as<double>(), dWf.as<double>(), dPsdF.as<double>(), frf(),
+                (e = launch_m2(stream, 0, np, c.nme, 0, dFreq.as<double>() + (fold1 ? half : 0), dWf.as<double>(), dPsdF.as<double>(), frf(),
                                m2o, m2o + nm2, m2o + 2 * nm2)))
                 return cuda_fail(e, "batch m2");
             kernels += 4 + (eform ? 1 : 2) * JH;
@@ -983,6 +1023,7 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
             (e = cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, stream)) ||
             (e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream)))
             return cuda_fail(e, "batch run");
+        if ((rc = atable_check())) return rc;
         if (herr) return fail(BSA_ERR_TIMEOUT, "batched kernel: a pipeline wait ran out of its budget (role %d)", herr);
         // results of this group: moments and m2 of its cases
         for (size_t k = g0; k < g1; ++k) {

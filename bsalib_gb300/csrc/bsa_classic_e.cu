@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(ELayout<RS>::threads, 1)  // 128 registers a t
                         uint8_t *st = smem + s * kStageBytes;
                         mbar_expect_tx(&full[s], tx_bytes);
                         const int x = kc * kBK;
-                        const int yu = p * P.Mp + mt * kBM;
+                        const int yu = (P.ufold ? abs(p - P.h) : p) * P.Mp + mt * kBM;
                         // G rows of mode half jh; rows past a half's columns read the next
                         // half's rows or zeros (masked in the epilogue)
                         const int yg = jh * P.nf * NMT + (nt0 + 2 * u) * BROWS;
@@ -343,7 +343,8 @@ int Engine::contract_e(const PointSrc &ps, double *m3mf, double *m3mr, const ESa
         return cuda_fail(e, "device query");
     int grid = (nsm / MT) * MT;
     if (grid < MT) grid = MT;
-    const size_t uel = (size_t)nf * Mp * Kp, gel = (size_t)JH * nf * NMT * Kp;
+    const int nfu = ps.fold1 ? ps.fold1 : nf;  // U rows: f >= 0 only where the A table is folded
+    const size_t uel = (size_t)nfu * Mp * Kp, gel = (size_t)JH * nf * NMT * Kp;
     const size_t bytesA = 2 * uel * 2, bytesB = 2 * gel * 2;
     const size_t bytesH = sizeof(float2) * (size_t)(nf + ns) * W;
     const size_t bytesP = sizeof(double) * (size_t)grid * kKinds * W * 128;
@@ -358,19 +359,19 @@ int Engine::contract_e(const PointSrc &ps, double *m3mf, double *m3mr, const ESa
     if ((e = cudaMemsetAsync(derr, 0, sizeof(int), stream))) return cuda_fail(e, "memset");
     {
         const float *A = dA32.as<float>();
-        if ((e = mixed::prep_u(stream, nf, nm, K, Kp, Mp, A, dQ.as<double>(), Uh, Ul)) ||
+        if ((e = mixed::prep_u(stream, nfu, nm, K, Kp, Mp, A, dQ.as<double>(), Uh, Ul)) ||
             (e = mixed::prep_h(stream, nf, nm, W, ps.fgrid, frf(), Hg, Hs, true)))
             return cuda_fail(e, "BF16x3 operand preparation");
         for (int jh = 0; jh < JH; ++jh) {  // G rows of mode half jh at jh nf NMT
             const size_t og = (size_t)jh * nf * NMT * Kp;
             if ((e = mixed::prep_b(stream, nf, nm, NMT, jh * NMT, K, Kp, nf, ps.n_pad, ps.trunc, ps.sum_base, 0, A,
-                                   Gh + og, Gl + og)))
+                                   Gh + og, Gl + og, ps.fold1)))
                 return cuda_fail(e, "BF16x3 operand preparation");
         }
         kernels += 2 + JH;
     }
     CUtensorMap maps[4];
-    if (!make_map(&maps[0], Uh, Kp, (uint64_t)nf * Mp, kBM) || !make_map(&maps[1], Ul, Kp, (uint64_t)nf * Mp, kBM) ||
+    if (!make_map(&maps[0], Uh, Kp, (uint64_t)nfu * Mp, kBM) || !make_map(&maps[1], Ul, Kp, (uint64_t)nfu * Mp, kBM) ||
         !make_map(&maps[2], Gh, Kp, (uint64_t)JH * nf * NMT, NC * NMT) ||
         !make_map(&maps[3], Gl, Kp, (uint64_t)JH * nf * NMT, NC * NMT))
         return fail(BSA_ERR_CUDA, "cuTensorMapEncodeTiled failed");
@@ -389,6 +390,7 @@ int Engine::contract_e(const PointSrc &ps, double *m3mf, double *m3mr, const ESa
     prm.Hs = Hs;
     prm.part = dMixPart.as<double>();
     prm.err = derr;
+    prm.ufold = ps.fold1 ? 1 : 0;
     prm.test_skip_tile1 = wait_test_tile1;
     wait_test_tile1 = 0;  // one analysis only
     if (cls_shards > 1 && !smp) {  // product rows p = rank + shards l (bsa_gpu_setClassicShard)

@@ -61,6 +61,7 @@ struct PointSrc {
     int sum_base;           // A-table row of the analytic sum table (s = i1 + i2)
     int r0, nr;             // grid rows (f1 index) of this run: i1 in [r0, r0 + nr)
     long long pbase;        // kPointsGrid: point p of the launch is grid point pbase + p
+    int fold1;              // kPointsGrid: 0, or 1 + h: the A table holds the rows of |i - h| only (even in f)
     int sym_rows;           // kPointsGrid, central symmetry: rows i1 < sym_rows weigh twice
     int wmode;
     double wval;            // uniform weight, or d^2 for the classic edge weights

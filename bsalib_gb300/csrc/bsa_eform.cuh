@@ -99,6 +99,7 @@ struct EParams {
     // Shard of the product rows (bsa_gpu_setClassicShard): rows p = p0 + (pstep_m1 + 1) l, l = 0, 1, ...
     // (zero-initialised: every row).
     int p0, pstep_m1;
+    int ufold;  // the U table holds the rows of |p - h| (every quantity is even in f)
 };
 
 // Shared-memory float2 load the compiler does not hoist (keeps the per-mode FRF values out

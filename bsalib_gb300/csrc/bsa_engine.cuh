@@ -106,6 +106,14 @@ struct ESample {
 };
 
 struct Engine {
+    // host lists of contract_list64: copies read them, so they live until the caller has waited
+    struct Lists64 {
+        std::vector<int> start, deg, other, pe, xmap, blk, pair, row_of, fill;
+        std::vector<long long> uniq;
+        std::vector<int4> items;
+        struct Ref { int hi, slot; };
+        std::vector<Ref> refs;
+    };
     Inputs in;
     Settings set;
     bool inited = false, halted = false, derived_ok = false, dev_uploaded = false;
@@ -180,8 +188,12 @@ struct Engine {
     int build_atable(const std::vector<double> &freqs, bool fp32 = false, bool msh = false);
     int pod_atable(const std::vector<double> &freqs, bool fp32);
     int build_psd(const std::vector<double> &freqs);
-    int build_psd_dev(int nf, bool fp32 = false, double *expt = nullptr);  // the nf frequencies already in dFreq
-    int build_atable_dev(int nf, bool fp32);   // the same, A table (not the truncated POD form)
+    int build_psd_dev(int nf, bool fp32 = false, double *expt = nullptr, int f0 = 0);  // the nf frequencies already in dFreq
+    int build_atable_dev(int nf, bool fp32, int f0 = 0);   // the same, A table (not the truncated POD form)
+    // The FP32 A kernel's pipeline flag, read once behind the run's own results instead of after every
+    // table.
+    bool atable_pending = false;
+    int atable_check();
     // dimM_psd_ / dimM_bisp_ (src/bsa/BsaLibImpl.F90:313-355): nm / nm for the diagonal-only
     // spectra, nm^2 / nm^3 otherwise.
     long long dim_psd() const { return set.onlyd ? nme : (long long)nme * nme; }
@@ -196,8 +208,8 @@ struct Engine {
                  const HostRows *rows = nullptr);
     // point lists in FP64 over pair products (bsa_list64.cu)
     bool list64_wanted(long long npts, int nr) const;
-    int contract_list64(const PointSrc &ps, long long npts, int nr, const int *ix, const int *iy, const int *iz, int G,
-                        double *bfd, double *brd);
+    int contract_list64(const PointSrc &ps, long long npts, const HostRows &rows, int G, double *bfd, double *brd,
+                        Lists64 &lists);
     // the whole Classic grid in FP64 over distinct frequency pairs (bsa_pair64.cu); grid +-N df
     int contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr);
     int contract_mixed(const PointSrc &ps, long long npts, double *m3mf, double *m3mr);
@@ -234,7 +246,8 @@ struct Engine {
     int br_decomp(const double *m2mf, double *bkg, double *res);
     int modal_recomb(const double *m2mr, const double *m3mr, const double *m2o2mr, double *const *outs);
     int batch_add(int *id);
-    void batch_install(const BatchCase &c);
+    void batch_install(BatchCase &c);
+    void batch_swap(BatchCase &c);
     int batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms, double *total_ms);
 };
 

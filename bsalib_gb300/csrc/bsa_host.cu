@@ -169,6 +169,7 @@ void Engine::free_device() {
     if (evg1) cudaEventDestroy(evg1);
     ev0 = ev1 = ev2 = evg0 = evg1 = nullptr;
     dev_uploaded = false;
+    atable_pending = false;
 }
 
 int Engine::ensure_stream() {
@@ -368,13 +369,13 @@ int Engine::build_psd(const std::vector<double> &freqs) {
     return build_psd_dev((int)freqs.size());
 }
 
-// Nodal PSD table S[f][k] for the nf frequencies already in dFreq (fp32: the formulas
+// Nodal PSD table S[f][k] for the nf frequencies already in dFreq from f0 on (fp32: the formulas
 // evaluated in FP32, for the split-precision A tables; expt: sqrt(S) and the exponential's table).
-int Engine::build_psd_dev(int nf, bool fp32, double *expt) {
+int Engine::build_psd_dev(int nf, bool fp32, double *expt, int f0) {
     const int ntc = (int)set.tc.size();
     cudaError_t e;
     if ((e = dS.reserve(sizeof(double) * (size_t)nf * ntc * in.nnl))) return cuda_fail(e, "allocating S");
-    if ((e = launch_nodal_psd(stream, nf, dFreq.as<double>(), ntc, set.tc.data(), in.nnl, dPsdPar.as<PsdNode>(),
+    if ((e = launch_nodal_psd(stream, nf, dFreq.as<double>() + f0, ntc, set.tc.data(), in.nnl, dPsdPar.as<PsdNode>(),
                               in.psd_type, set.defsc, dS.as<double>(), fp32, expt)))
         return cuda_fail(e, "nodal PSD kernel");
     kernels += 1;
@@ -389,37 +390,45 @@ int Engine::build_atable(const std::vector<double> &freqs, bool fp32, bool msh) 
     return build_atable_dev((int)freqs.size(), fp32);
 }
 
-// Nodal PSD + A(f) for the nf frequencies already in dFreq (not the truncated POD form).
-int Engine::build_atable_dev(int nf, bool fp32) {
+// Nodal PSD + A(f) for the nf frequencies already in dFreq from f0 on (not the truncated POD form).
+int Engine::build_atable_dev(int nf, bool fp32, int f0) {
     const int ntc = (int)set.tc.size();
     cudaError_t e;
     // the FP64 table reads sqrt(S) and the exponential's table behind log c
-    int rc = build_psd_dev(nf, fp32, fp32 ? nullptr : dLogc.as<double>() + (size_t)ntc * in.nnl * in.nnl);
+    int rc = build_psd_dev(nf, fp32, fp32 ? nullptr : dLogc.as<double>() + (size_t)ntc * in.nnl * in.nnl, f0);
     if (rc) return rc;
     if (fp32) {
         // FP32 table on the tensor cores (tf32 hi/lo split, FP32-level accuracy)
-        if ((e = dA32.reserve(sizeof(float) * (size_t)nf * K * nme)) ||
-            (e = dFlag.reserve(256 + atable_tc_scratch(ntc, in.nnl, nme))))
+        const size_t fb = 256 + atable_tc_scratch(ntc, in.nnl, nme);
+        if (fb > dFlag.bytes && (rc = atable_check())) return rc;  // the flag's block is about to move
+        if ((e = dA32.reserve(sizeof(float) * (size_t)nf * K * nme)) || (e = dFlag.reserve(fb)))
             return cuda_fail(e, "allocating A");
         int *flag = dFlag.as<int>();
-        if ((e = cudaMemsetAsync(flag, 0, sizeof(int), stream))) return cuda_fail(e, "memset");
-        e = launch_atable_tc(stream, nf, dFreq.as<double>(), ntc, in.nnl, nme, dLogc32.as<float>(), dS.as<double>(),
+        if (!atable_pending && (e = cudaMemsetAsync(flag, 0, sizeof(int), stream))) return cuda_fail(e, "memset");
+        atable_pending = true;
+        e = launch_atable_tc(stream, nf, dFreq.as<double>() + f0, ntc, in.nnl, nme, dLogc32.as<float>(), dS.as<double>(),
                              dL32.as<float>(), dA32.as<float>(), (char *)dFlag.p + 256, flag);
         if (e) return cuda_fail(e, "A-table kernel");
         kernels += 2;
-        int hflag = 0;
-        if ((e = cudaMemcpyAsync(&hflag, flag, sizeof(int), cudaMemcpyDeviceToHost, stream)) ||
-            (e = cudaStreamSynchronize(stream)))
-            return cuda_fail(e, "A-table kernel");
-        if (hflag) return fail(BSA_ERR_TIMEOUT, "A-table kernel: a pipeline wait ran out of its budget (role %d)", hflag);
         return BSA_OK;
-    } else {
-        if ((e = dA.reserve(sizeof(double) * (size_t)nf * K * nme))) return cuda_fail(e, "allocating A");
-        e = launch_atable(stream, nf, dFreq.as<double>(), ntc, in.nnl, nme, dLogc.as<double>(), dS.as<double>(),
-                          dL.as<double>(), dA.as<double>());
     }
+    if ((e = dA.reserve(sizeof(double) * (size_t)nf * K * nme))) return cuda_fail(e, "allocating A");
+    e = launch_atable(stream, nf, dFreq.as<double>() + f0, ntc, in.nnl, nme, dLogc.as<double>(), dS.as<double>(),
+                      dL.as<double>(), dA.as<double>());
     if (e) return cuda_fail(e, "A-table kernel");
     kernels += 1;
+    return BSA_OK;
+}
+
+int Engine::atable_check() {
+    if (!atable_pending) return BSA_OK;
+    atable_pending = false;
+    int hflag = 0;
+    cudaError_t e;
+    if ((e = cudaMemcpyAsync(&hflag, dFlag.p, sizeof(int), cudaMemcpyDeviceToHost, stream)) ||
+        (e = cudaStreamSynchronize(stream)))
+        return cuda_fail(e, "A-table kernel");
+    if (hflag) return fail(BSA_ERR_TIMEOUT, "A-table kernel: a pipeline wait ran out of its budget (role %d)", hflag);
     return BSA_OK;
 }
 
@@ -523,16 +532,29 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
         if (analytic)
             for (int s = half + 1; s <= 2 * half; ++s) ftab.push_back(s * df_grid);
     }
+    // The split forms read the same rows: A table (and second-order moments) of f >= 0, grid row i
+    // from row |i - half|.
+    const bool fold = mixed && !analytic && set.defsc == 1 && (nf & 1) && r0 == 0 && r1 == nf && cls_shards == 1 &&
+                      !export_fn && !brm_file_wanted(true);
     cudaError_t e;
     if ((e = cudaEventRecord(ev0, stream))) return cuda_fail(e, "event");
-    if ((rc = diagonal ? build_psd(ftab) : build_atable(ftab, mixed))) return rc;
+    if (fold) {
+        if ((e = upload(dFreq, f, stream))) return cuda_fail(e, "uploading frequencies");
+        rc = build_atable_dev(half + 1, true, half);
+    } else {
+        rc = diagonal ? build_psd(ftab) : build_atable(ftab, mixed);
+    }
+    if (rc) return rc;
     const long long nm2 = dim_psd();
-    if (set.ipsd && (m2mf || m2mr || m2o2mr)) {
-        std::vector<double> wf(nf, scalar ? delta : delta);
+    const bool m2 = set.ipsd && (m2mf || m2mr || m2o2mr);
+    std::vector<double> wf;  // read by a copy: lives until the run has waited
+    if (m2) {
+        wf.assign(nf, delta);
         if (!scalar) { wf[0] = delta / 2; wf[nf - 1] = delta / 2; }
         // f and -f contribute the same (Re[H_o conj H_n] is even)
-        const int np = pair64 ? half + 1 : nf;
-        if (pair64) {
+        const bool one = pair64 || fold;
+        const int np = one ? half + 1 : nf;
+        if (one) {
             wf.erase(wf.begin(), wf.begin() + half);
             for (int k = 1; k < np; ++k) wf[k] *= 2.0;
         }
@@ -541,24 +563,16 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
         if ((e = dOut.reserve(sizeof(double) * (3 * (size_t)nm2 + 2 * (size_t)dim_bisp()))))
             return cuda_fail(e, "out");
         e = diagonal ? launch_force_psd_diag(stream, np, K, nme, dS.as<double>(), dWd2.as<double>(), dPsdF.as<double>())
-            : mixed  ? launch_force_psd32(stream, nf, (int)set.tc.size(), in.nnl, nme, dL32.as<float>(),
+            : mixed  ? launch_force_psd32(stream, np, (int)set.tc.size(), in.nnl, nme, dL32.as<float>(),
                                           dA32.as<float>(), dPsdF.as<double>())
                      : launch_force_psd(stream, np, (int)set.tc.size(), in.nnl, nme, dL.as<double>(), dA.as<double>(),
                                         dPsdF.as<double>());
         if (e) return cuda_fail(e, "force PSD kernel");
         double *o = dOut.as<double>();
-        if ((e = launch_m2(stream, pair64 ? 0 : r0, pair64 ? np : r1, nme, diagonal ? 1 : 0, dFreq.as<double>(), dWf.as<double>(),
+        if ((e = launch_m2(stream, one ? 0 : r0, one ? np : r1, nme, diagonal ? 1 : 0, dFreq.as<double>() + (fold ? half : 0), dWf.as<double>(),
                            dPsdF.as<double>(), frf(), o, o + nm2, o + 2 * nm2)))
             return cuda_fail(e, "m2 kernel");
         kernels += 2;
-        std::vector<double> h(3 * (size_t)nm2);
-        if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
-            (e = cudaStreamSynchronize(stream)))
-            return cuda_fail(e, "m2 copy");
-        d2h += (double)sizeof(double) * h.size();
-        if (m2mf) std::memcpy(m2mf, h.data(), sizeof(double) * nm2);
-        if (m2mr) std::memcpy(m2mr, h.data() + nm2, sizeof(double) * nm2);
-        if (m2o2mr) std::memcpy(m2o2mr, h.data() + 2 * nm2, sizeof(double) * nm2);
     }
     last_points = 0;
     if (set.ibisp && (m3mf || m3mr || bf_host || br_host)) {
@@ -571,6 +585,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
         ps.wmode = scalar ? kWeightUniform : kWeightClassicVect;
         ps.wval = delta * delta;
         ps.fgrid = dFreq.as<double>();
+        ps.fold1 = fold ? half + 1 : 0;
         ps.r0 = r0;
         ps.nr = r1 - r0;
         long long npts = (long long)(r1 - r0) * nf;
@@ -614,7 +629,18 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
         if (rc) return rc;
         last_points = (double)npts;
     }
+    // the second-order moments wait on the device until here, so that nothing stops the launches
+    std::vector<double> h(m2 ? 3 * (size_t)nm2 : 0);
+    if (m2 && (e = cudaMemcpyAsync(h.data(), dOut.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)))
+        return cuda_fail(e, "m2 copy");
     if ((e = cudaEventRecord(ev1, stream)) || (e = cudaEventSynchronize(ev1))) return cuda_fail(e, "event");
+    if ((rc = atable_check())) return rc;
+    if (m2) {
+        d2h += (double)sizeof(double) * h.size();
+        if (m2mf) std::memcpy(m2mf, h.data(), sizeof(double) * nm2);
+        if (m2mr) std::memcpy(m2mr, h.data() + nm2, sizeof(double) * nm2);
+        if (m2o2mr) std::memcpy(m2o2mr, h.data() + 2 * nm2, sizeof(double) * nm2);
+    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev0, ev1);
     last_ms = ms;
@@ -683,8 +709,9 @@ int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m
     if ((e = cudaEventRecord(ev2, stream))) return cuda_fail(e, "event");
     if ((e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
     const bool list64 = rows && list64_wanted(npts, rows->nr);
+    Lists64 lists;
     if (list64) {
-        int rc = contract_list64(ps, npts, rows->nr, rows->ix, rows->iy, rows->iz, G, bfd, brd);
+        int rc = contract_list64(ps, npts, *rows, G, bfd, brd, lists);
         if (rc) return rc;
     } else if ((e = launch_bfm_fp64(stream, dA.as<double>(), dQ.as<double>(), K, nme, ps, npts, frf(), G,
                                     dPartF.as<double>(), dPartR.as<double>(), bfd, brd))) {
@@ -770,6 +797,7 @@ int Engine::run_points(const double *fi, const double *fj, const double *w, doub
         (e = cudaMemcpyAsync(df2, f2.data(), n * sizeof(double), cudaMemcpyHostToDevice, stream)) ||
         (w && (e = cudaMemcpyAsync(dw, w, n * sizeof(double), cudaMemcpyHostToDevice, stream))))
         return cuda_fail(e, "point upload");
+    std::vector<long long> zoff;
     PointSrc ps{};
     ps.mode = kPointsList;
     ps.wmode = w ? kWeightList : kWeightUniform;
@@ -792,7 +820,7 @@ int Engine::run_points(const double *fi, const double *fj, const double *w, doub
         if (!set.onlyd) {
             // FRF tables of the zones along the axes, within 8 GB
             const size_t nz = zones->size();
-            std::vector<long long> zoff(2 * nz);
+            zoff.resize(2 * nz);
             long long total = 0;
             const long long cap = (8LL << 30) / (long long)sizeof(double2);
             for (size_t k = 0; k < nz; ++k) {
@@ -888,7 +916,7 @@ int Engine::classic_points(const int *i1, const int *i2, long long npts, double 
         ps.r0 = 0;
         ps.nr = nf;
         ESample smp{dSlot.as<int>(), dBF.as<double>(), dBR.as<double>(), nslot};
-        if ((rc = contract_e(ps, nullptr, nullptr, &smp))) return rc;
+        if ((rc = contract_e(ps, nullptr, nullptr, &smp)) || (rc = atable_check())) return rc;
         std::vector<double> hf((size_t)nslot * nm3), hr((size_t)nslot * nm3);
         if ((e = cudaMemcpyAsync(hf.data(), smp.sF, sizeof(double) * hf.size(), cudaMemcpyDeviceToHost, stream)) ||
             (e = cudaMemcpyAsync(hr.data(), smp.sR, sizeof(double) * hr.size(), cudaMemcpyDeviceToHost, stream)) ||

@@ -34,11 +34,16 @@ bool Engine::list64_wanted(long long npts, int nr) const {
     return pair_ms < point_ms;
 }
 
-// Third moments (and bispectra) of a point list; nr rows of dA, ix / iy / iz the points' rows on the
-// host (iz < 0: the sum reads zero), ps the same on the device.
-int Engine::contract_list64(const PointSrc &ps, long long npts, int nr, const int *ix, const int *iy, const int *iz, int G,
-                            double *bfd, double *brd) {
+// Third moments (and bispectra) of a point list; rows: the points' A rows on the host (iz < 0: the sum
+// reads zero), ps the same on the device.
+int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &rows, int G, double *bfd, double *brd,
+                            Lists64 &lists) {
     using namespace p64;
+    const int nr = rows.nr, *ix = rows.ix, *iy = rows.iy, *iz = rows.iz;
+    auto &[start, deg, other, pe, xmap, blk, pair, row_of, fill, uniq, items, refs] = lists;
+    using Ref = Lists64::Ref;
+    deg.assign(nr, 0);
+    row_of.assign(nr, 0);
     const int nm = nme, rx = nm * nm, np = blocks_of(nm), bw = block_width(nm), slots = kTN / bw;
     const int tiles_x = (rx + kTM - 1) / kTM;
     const long long nm3 = (long long)rx * nm;
@@ -51,11 +56,6 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, int nr, const in
     if ((e = cudaMemsetAsync(dFlag.p, 0, sizeof(int), stream)) || (e = tc_prep_blocks(stream, nr, nm, K, dA.as<double>(), dMixB.p)))
         return cuda_fail(e, "pair product operands");
     kernels += 2;
-    std::vector<int> start, deg(nr), other, pe, xmap, blk, pair, row_of(nr), fill;
-    std::vector<long long> uniq;
-    std::vector<int4> items;
-    struct Ref { int hi, slot; };
-    std::vector<Ref> refs;
     for (long long p0 = 0; p0 < npts; p0 += batch) {
         const int n = (int)std::min(batch, npts - p0);
         // pairs (lo <= hi) bucketed by lo, then by hi; slot 3 p + w is the term that asks for it

@@ -372,10 +372,10 @@ __global__ void __launch_bounds__(192, 1)
 // U[(r*Mp + a*nm + b)][k] = Q[k][a] * A(f_r)[k][b]   (rows >= nm^2 and k >= K are zero).
 // Each thread writes 8 consecutive k of one row as one 16-byte store per hi / lo table.
 __global__ void k_prep_u(int nm, int K, int Kp, int Mp, const float *__restrict__ A, const double *__restrict__ Q,
-                         __nv_bfloat16 *__restrict__ Uh, __nv_bfloat16 *__restrict__ Ul) {
+                         __nv_bfloat16 *__restrict__ Uh, __nv_bfloat16 *__restrict__ Ul, int fold1) {
     const int r = blockIdx.x, k0 = blockIdx.y * 64;
     __shared__ float As[64][65], Qs[64][65];  // nm <= 64
-    const float *Ar = A + (size_t)r * K * nm;
+    const float *Ar = A + (size_t)(fold1 ? abs(r + 1 - fold1) : r) * K * nm;
     for (int e = threadIdx.x; e < 64 * nm; e += blockDim.x) {
         const int kk = e / nm, m = e % nm, k = k0 + kk;
         As[kk][m] = k < K ? Ar[(size_t)k * nm + m] : 0.f;
@@ -401,7 +401,7 @@ __global__ void k_prep_u(int nm, int K, int Kp, int Mp, const float *__restrict_
 // too).
 __global__ void k_prep_b(int nm, int NMT, int j0, int K, int Kp, int nf, int n_pad, int trunc, int sum_base,
                          int is_sum, const float *__restrict__ A, __nv_bfloat16 *__restrict__ Th,
-                         __nv_bfloat16 *__restrict__ Tl) {
+                         __nv_bfloat16 *__restrict__ Tl, int fold1) {
     const int t = blockIdx.x, k0 = blockIdx.y * 64;
     int src = t;
     if (is_sum) {
@@ -412,6 +412,7 @@ __global__ void k_prep_b(int nm, int NMT, int j0, int K, int Kp, int nf, int n_p
             src = sum_base + t;
         }
     }
+    if (fold1 && src >= 0) src = abs(src + 1 - fold1);
     __shared__ float As[64][33];
     for (int e = threadIdx.x; e < 64 * NMT; e += blockDim.x) {
         const int kk = e / NMT, jj = e % NMT, m = j0 + jj, k = k0 + kk;
@@ -485,14 +486,14 @@ __global__ void k_mixed_reduce(int nm, int NMT, int MT, int grid, int kinds, con
 }
 
 cudaError_t prep_u(cudaStream_t st, int nf, int nm, int K, int Kp, int Mp, const float *A, const double *Q,
-                   __nv_bfloat16 *Uh, __nv_bfloat16 *Ul) {
-    k_prep_u<<<dim3(nf, Kp / 64), 256, 0, st>>>(nm, K, Kp, Mp, A, Q, Uh, Ul);
+                   __nv_bfloat16 *Uh, __nv_bfloat16 *Ul, int fold1) {
+    k_prep_u<<<dim3(nf, Kp / 64), 256, 0, st>>>(nm, K, Kp, Mp, A, Q, Uh, Ul, fold1);
     return cudaGetLastError();
 }
 
 cudaError_t prep_b(cudaStream_t st, int rows, int nm, int NMT, int j0, int K, int Kp, int nf, int n_pad, int trunc,
-                   int sum_base, int is_sum, const float *A, __nv_bfloat16 *Th, __nv_bfloat16 *Tl) {
-    k_prep_b<<<dim3(rows, Kp / 64), 256, 0, st>>>(nm, NMT, j0, K, Kp, nf, n_pad, trunc, sum_base, is_sum, A, Th, Tl);
+                   int sum_base, int is_sum, const float *A, __nv_bfloat16 *Th, __nv_bfloat16 *Tl, int fold1) {
+    k_prep_b<<<dim3(rows, Kp / 64), 256, 0, st>>>(nm, NMT, j0, K, Kp, nf, n_pad, trunc, sum_base, is_sum, A, Th, Tl, fold1);
     return cudaGetLastError();
 }
 
@@ -562,15 +563,15 @@ int Engine::contract_mixed(const PointSrc &ps, long long npts, double *m3mf, dou
     {
         const float *A = dA32.as<float>();
         dim3 gu(nf, Kp / 64);
-        k_prep_u<<<gu, 256, 0, stream>>>(nm, K, Kp, Mp, A, dQ.as<double>(), Uh, Ul);
+        k_prep_u<<<gu, 256, 0, stream>>>(nm, K, Kp, Mp, A, dQ.as<double>(), Uh, Ul, ps.fold1);
         dim3 gg(nf, Kp / 64), gs(ns, Kp / 64);
         // B tables: one block of rows per mode half, modes jh NMT .. jh NMT + NMT - 1
         for (int jh = 0; jh < JH; ++jh) {
             const size_t og = (size_t)jh * nf * NMT * Kp, os = (size_t)jh * ns * NMT * Kp;
             k_prep_b<<<gg, 256, 0, stream>>>(nm, NMT, jh * NMT, K, Kp, nf, ps.n_pad, ps.trunc, ps.sum_base, 0, A,
-                                             Gh + og, Gl + og);
+                                             Gh + og, Gl + og, ps.fold1);
             k_prep_b<<<gs, 256, 0, stream>>>(nm, NMT, jh * NMT, K, Kp, nf, ps.n_pad, ps.trunc, ps.sum_base, 1, A,
-                                             Sh + os, Sl + os);
+                                             Sh + os, Sl + os, ps.fold1);
         }
         const int nh = (nf + ns) * W;
         k_prep_h<<<(nh + 255) / 256, 256, 0, stream>>>(nf, nm, W, ps.fgrid, frf(), Hg, Hs, 0);

@@ -1272,7 +1272,8 @@ int Engine::msh_mixed_batch(const std::vector<ZoneDev> &zs, std::vector<double> 
             return cuda_fail(e, "Mesher task upload");
         h2d += (double)((nU + ncol + 2 * npts) * sizeof(int) + tasks.size() * sizeof(Task) +
                         witems.size() * sizeof(int4));
-        if ((rc = build_atable(F.v, true, true))) return rc;
+        // the lists above end with this branch: wait for their copies
+        if ((rc = build_atable(F.v, true, true)) || (rc = atable_check())) return rc;
     }
     const size_t uel = (size_t)nU * Mp * Kp, gel = (size_t)ncol * NMT * Kp, sel = 2 * (size_t)npts * NMT * Kp;
     const int nm3p = (nm3 + 3) & ~3, hs = frf_row(nm);
@@ -1398,6 +1399,7 @@ int Engine::msh_mixed_batch(const std::vector<ZoneDev> &zs, std::vector<double> 
     if (graph) cudaGraphDestroy(graph);
     d2h += (double)sizeof(double) * h.size() + sizeof(int);
     if (xerr) return fail(BSA_ERR_STATE, "Mesher zone expansion: a frequency missing from its table");
+    if ((rc = atable_check())) return rc;
     if (herr) return fail(BSA_ERR_TIMEOUT, "Mesher BF16x3 kernel: a pipeline wait ran out of its budget (role %d)", herr);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, evg0, evg1);
