@@ -877,7 +877,7 @@ __global__ void k_msh_reduce(int nm, int G, const double *__restrict__ part, dou
 // Device-side expansion of a zone pass: the zone list (one ZoneX per axis-aligned zone, with
 // its offsets) becomes, on the device, the distinct frequencies (A-table rows), the distinct
 // line / column frequencies (U blocks), the point and column index tables, the tasks and the
-// work queue.  Frequencies meet in open-addressing hash tables keyed by round(f 2^40) (values
+// work queue.  Frequencies meet in open-addressing hash tables keyed by round(|f| 2^40) (values
 // equal to ~1e-12 Hz share a row); the occupied slots are then numbered in slot order.
 // ------------------------------------------------------------------------------------
 struct ZoneX {
@@ -891,7 +891,9 @@ struct ZoneX {
 
 constexpr unsigned long long kEmptyKey = 0x8080808080808080ull;  // memset pattern 0x80
 
-__device__ __forceinline__ long long fkey(double f) { return __double2ll_rn(f * 1099511627776.0); }  // 2^40
+// f and -f share a row: every quantity of the A and U tables is even in f (the bridge deck's 301 zones
+// lie on both signs).
+__device__ __forceinline__ long long fkey(double f) { return __double2ll_rn(fabs(f) * 1099511627776.0); }  // 2^40
 
 __device__ __forceinline__ unsigned long long fhash(long long q, int bits) {
     return ((unsigned long long)q * 0x9E3779B97F4A7C15ull) >> (64 - bits);
@@ -1102,7 +1104,7 @@ constexpr double kFreqTol = 1e-12;
 
 struct FreqIndex {
     std::vector<double> v;
-    void add(double f) { v.push_back(f); }
+    void add(double f) { v.push_back(std::fabs(f)); }  // every quantity is even in f
     void seal() {
         std::sort(v.begin(), v.end());
         size_t w = 0;
@@ -1110,7 +1112,8 @@ struct FreqIndex {
             if (w == 0 || v[r] - v[w - 1] > kFreqTol * (1.0 + std::fabs(v[w - 1]))) v[w++] = v[r];
         v.resize(w);
     }
-    int at(double f) const {
+    int at(double fs) const {
+        const double f = std::fabs(fs);
         const size_t i = (size_t)(std::lower_bound(v.begin(), v.end(), f) - v.begin());
         if (i == v.size()) return (int)i - 1;
         if (i > 0 && f - v[i - 1] <= v[i] - f) return (int)i - 1;
@@ -1530,8 +1533,8 @@ int Engine::run_zones_mixed(const std::vector<ZoneDev> &zones, double *m3mf, dou
                 const ZoneDev &z = axis[b1];
                 size_t nu_new = 0;
                 std::vector<double> cand;
-                for (int i = 0; i < z.ni; ++i) cand.push_back(z.fi0 + i * z.dIi);
-                for (int j = 0; j < z.nj; ++j) cand.push_back(z.fj0 + j * z.dJj);
+                for (int i = 0; i < z.ni; ++i) cand.push_back(std::fabs(z.fi0 + i * z.dIi));
+                for (int j = 0; j < z.nj; ++j) cand.push_back(std::fabs(z.fj0 + j * z.dJj));
                 for (double f : cand)
                     if (!std::binary_search(uf.begin(), uf.end(), f)) ++nu_new;
                 const double nq = (double)((z.ni - 1) * z.Fi + 1) * ((z.nj - 1) * z.Fj + 1);
