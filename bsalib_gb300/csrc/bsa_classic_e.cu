@@ -292,6 +292,7 @@ __global__ void k_e_reduce(int nm, int W, int MT, int grid, const double *__rest
     auto sum = [&](int kind, int a, int b, int j) {
         const int R = a * nm + b, mtile = R / 128, lane = R % 128;
         double s = 0.0;
+#pragma unroll 4
         for (int g = mtile + MT * threadIdx.y; g < grid; g += MT * kRedLanes)
             s += part[(((size_t)g * kKinds + kind) * W + j) * 128 + lane];
         return s;

@@ -250,10 +250,8 @@ int Engine::contract_diag(const PointSrc &ps, long long npts, int msh_form, doub
     std::vector<double> h(2 * (size_t)nme);
     if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)))
         return cuda_fail(e, "moment copy");
-    if (bf_host && (e = cudaMemcpyAsync(bf_host, bfd, sizeof(double) * (size_t)npts * nme, cudaMemcpyDeviceToHost, stream)))
-        return cuda_fail(e, "bispectrum copy");
-    if (br_host && (e = cudaMemcpyAsync(br_host, brd, sizeof(double) * (size_t)npts * nme, cudaMemcpyDeviceToHost, stream)))
-        return cuda_fail(e, "bispectrum copy");
+    if (bf_host && (e = fetch(stream, bf_host, bfd, sizeof(double) * (size_t)npts * nme))) return cuda_fail(e, "bispectrum copy");
+    if (br_host && (e = fetch(stream, br_host, brd, sizeof(double) * (size_t)npts * nme))) return cuda_fail(e, "bispectrum copy");
     if ((e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream))) return cuda_fail(e, "sync");
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev2, ev1);

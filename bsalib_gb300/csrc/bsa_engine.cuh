@@ -28,6 +28,10 @@ int plan_msh_width(int nm, int K);
 // Frees the device blocks the engine keeps for reuse after bsa_Finalise.
 void release_device_cache();
 
+// Large results to pageable host memory through a pinned block and host threads (bsa_fetch.cu).
+cudaError_t fetch(cudaStream_t st, void *dst, const void *src, size_t n);
+void release_fetch_block();
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;

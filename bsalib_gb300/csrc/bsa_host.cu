@@ -727,10 +727,8 @@ int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m
     if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
         (list64 && (e = cudaMemcpyAsync(&herr, dFlag.p, sizeof(int), cudaMemcpyDeviceToHost, stream))))
         return cuda_fail(e, "moment copy");
-    if (bf_host && (e = cudaMemcpyAsync(bf_host, bfd, sizeof(double) * (size_t)npts * nm3, cudaMemcpyDeviceToHost, stream)))
-        return cuda_fail(e, "bispectrum copy");
-    if (br_host && (e = cudaMemcpyAsync(br_host, brd, sizeof(double) * (size_t)npts * nm3, cudaMemcpyDeviceToHost, stream)))
-        return cuda_fail(e, "bispectrum copy");
+    if (bf_host && (e = fetch(stream, bf_host, bfd, sizeof(double) * (size_t)npts * nm3))) return cuda_fail(e, "bispectrum copy");
+    if (br_host && (e = fetch(stream, br_host, brd, sizeof(double) * (size_t)npts * nm3))) return cuda_fail(e, "bispectrum copy");
     if ((e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream))) return cuda_fail(e, "sync");
     if (herr) return fail(BSA_ERR_TIMEOUT, "pair product kernel: a pipeline wait ran out of its budget (role %d)", herr);
     float ms = 0.f;
@@ -1380,6 +1378,7 @@ int bsa_gpu_setClassicForm(int form) {
 
 int bsa_gpu_releaseDeviceCache(void) {
     bsa::release_device_cache();
+    bsa::release_fetch_block();
     return BSA_OK;
 }
 

@@ -468,6 +468,7 @@ __global__ void k_mixed_reduce(int nm, int NMT, int MT, int grid, int kinds, con
     auto sum = [&](int kind, int a, int b, int j) {
         const int R = a * nm + b, mtile = R / 128, lane = R % 128;
         double s = 0.0;
+#pragma unroll 4
         for (int g = mtile + MT * threadIdx.y; g < grid; g += MT * kRedLanes)
             s += part[(((size_t)g * kinds + kind) * NMT + j) * 128 + lane];
         return s;
