@@ -198,6 +198,7 @@ struct Engine {
     // table.
     bool atable_pending = false;
     int atable_check();
+    int pipeline_flags(const int *flags, bool atable, bool pairs);
     // dimM_psd_ / dimM_bisp_ (src/bsa/BsaLibImpl.F90:313-355): nm / nm for the diagonal-only
     // spectra, nm^2 / nm^3 otherwise.
     long long dim_psd() const { return set.onlyd ? nme : (long long)nme * nme; }

@@ -413,10 +413,43 @@ int Engine::build_atable_dev(int nf, bool fp32, int f0) {
         return BSA_OK;
     }
     if ((e = dA.reserve(sizeof(double) * (size_t)nf * K * nme))) return cuda_fail(e, "allocating A");
-    e = launch_atable(stream, nf, dFreq.as<double>() + f0, ntc, in.nnl, nme, dLogc.as<double>(), dS.as<double>(),
-                      dL.as<double>(), dA.as<double>());
+    const double *fp = dFreq.as<double>() + f0;
+    const int *bad = log_coh_bad(dLogc.as<double>(), (size_t)ntc * in.nnl * in.nnl);
+    // On the tensor cores from 80 nodes on.  Second-order analyses, FP64 pipe / tensor cores (ms): 40
+    // nodes, 12 modes, 65 rows 0.071 / 0.075; 64, 12, 65: 0.078 / 0.078; 100, 12, 65: 0.107 / 0.091;
+    // 150, 12, 129: 0.229 / 0.139; 400, 24, 33: 0.564 / 0.157; 520, 8, 17: 0.258 / 0.165.
+    const bool tensor = in.nnl >= 80;
+    if (tensor) {
+        // frequencies in chunks of at most 1 GB of B digits
+        const size_t per = atable64_tc_scratch(1, ntc, in.nnl, nme);
+        const int step = (int)std::max<size_t>(1, std::min<size_t>(nf, ((size_t)1 << 30) / per));
+        if (256 > dFlag.bytes && (rc = atable_check())) return rc;
+        if ((e = dMshT.reserve(atable64_tc_scratch(step, ntc, in.nnl, nme))) || (e = dFlag.reserve(256)))
+            return cuda_fail(e, "allocating A");
+        if (!atable_pending && (e = cudaMemsetAsync(dFlag.p, 0, sizeof(int), stream))) return cuda_fail(e, "memset");
+        atable_pending = true;
+        for (int q = 0; q < nf; q += step) {
+            e = launch_atable64_tc(stream, std::min(step, nf - q), fp + q, ntc, in.nnl, nme, dLogc.as<double>(),
+                                   dS.as<double>() + (size_t)q * K, dL.as<double>(), bad, dA.as<double>() + (size_t)q * K * nme,
+                                   dMshT.p, dFlag.as<int>());
+            if (e) return cuda_fail(e, "A-table kernel");
+            kernels += 3;
+        }
+    }
+    e = launch_atable(stream, nf, fp, ntc, in.nnl, nme, dLogc.as<double>(), dS.as<double>(), dL.as<double>(), dA.as<double>(),
+                      tensor ? bad : nullptr);
     if (e) return cuda_fail(e, "A-table kernel");
     kernels += 1;
+    return BSA_OK;
+}
+
+// Flags read behind a run: [0] the A kernel's, [1] the pair products'.
+int Engine::pipeline_flags(const int *flags, bool atable, bool pairs) {
+    if (atable) atable_pending = false;
+    if (atable && flags[0])
+        return fail(BSA_ERR_TIMEOUT, "A-table kernel: a pipeline wait ran out of its budget (role %d)", flags[0]);
+    if (pairs && flags[1])
+        return fail(BSA_ERR_TIMEOUT, "pair product kernel: a pipeline wait ran out of its budget (role %d)", flags[1]);
     return BSA_OK;
 }
 
@@ -710,8 +743,9 @@ int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m
     if ((e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
     const bool list64 = rows && list64_wanted(npts, rows->nr);
     Lists64 lists;
+    int rc = BSA_OK;
     if (list64) {
-        int rc = contract_list64(ps, npts, *rows, G, bfd, brd, lists);
+        rc = contract_list64(ps, npts, *rows, G, bfd, brd, lists);
         if (rc) return rc;
     } else if ((e = launch_bfm_fp64(stream, dA.as<double>(), dQ.as<double>(), K, nme, ps, npts, frf(), G,
                                     dPartF.as<double>(), dPartR.as<double>(), bfd, brd))) {
@@ -723,14 +757,15 @@ int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m
         return cuda_fail(e, "reduction kernel");
     kernels += 2;
     std::vector<double> h(2 * (size_t)nm3);
-    int herr = 0;
+    int flags[2] = {0, 0};  // A table, pair products
+    const bool pend = atable_pending;
     if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
-        (list64 && (e = cudaMemcpyAsync(&herr, dFlag.p, sizeof(int), cudaMemcpyDeviceToHost, stream))))
+        ((list64 || pend) && (e = cudaMemcpyAsync(flags, dFlag.p, sizeof flags, cudaMemcpyDeviceToHost, stream))))
         return cuda_fail(e, "moment copy");
     if (bf_host && (e = fetch(stream, bf_host, bfd, sizeof(double) * (size_t)npts * nm3))) return cuda_fail(e, "bispectrum copy");
     if (br_host && (e = fetch(stream, br_host, brd, sizeof(double) * (size_t)npts * nm3))) return cuda_fail(e, "bispectrum copy");
     if ((e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream))) return cuda_fail(e, "sync");
-    if (herr) return fail(BSA_ERR_TIMEOUT, "pair product kernel: a pipeline wait ran out of its budget (role %d)", herr);
+    if ((rc = pipeline_flags(flags, pend, list64))) return rc;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev2, ev1);
     last_ms_contraction = ms;

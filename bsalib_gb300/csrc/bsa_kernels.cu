@@ -128,7 +128,9 @@ __global__ __launch_bounds__(256) void k_atable(int nf, const double *__restrict
                                                 int nm, const double *__restrict__ logc,
                                                 const double *__restrict__ expt,
                                                 const double *__restrict__ rootS,
-                                                const double *__restrict__ L, double *__restrict__ A) {
+                                                const double *__restrict__ L, double *__restrict__ A,
+                                                const int *__restrict__ only) {
+    if (only && !*only) return;
     constexpr int RI = 64, JT = 32, NML = 4 * MPT;
     const int fi = blockIdx.x / ntc, itc = blockIdx.x % ntc;
     const int i0 = blockIdx.y * RI;
@@ -182,35 +184,43 @@ __global__ __launch_bounds__(256) void k_atable(int nf, const double *__restrict
 // src/utils/utility.F90:60-71), in FP64 and FP32; the host side of this expansion and its copy were
 // 0.6 ms of a 400-node, two-component analysis.
 __global__ void k_log_coh(int ntc, int nnl, int nn, long long ncorr, const int *__restrict__ nodes,
-                          const double *__restrict__ corr, double *__restrict__ lc, float *__restrict__ lc32) {
+                          const double *__restrict__ corr, double *__restrict__ lc, float *__restrict__ lc32,
+                          int *__restrict__ bad) {
     const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= (long long)ntc * nnl * nnl) return;
     const int j = (int)(x % nnl), i = (int)(x / nnl % nnl), c = (int)(x / nnl / nnl);
     const long long a = min(nodes[i], nodes[j]), b = max(nodes[i], nodes[j]);
-    const double v = log(corr[c * ncorr + (a - 1) * nn + b - (a * a - a) / 2 - 1]);
+    const double w = corr[c * ncorr + (a - 1) * nn + b - (a * a - a) / 2 - 1];
+    if (!(w >= 0.0 && w <= 1.0) || (i == j && w != 1.0)) *bad = 1;
+    const double v = log(w);
     lc[x] = v;
     lc32[x] = (float)v;
 }
+
+int *log_coh_bad(const double *lc, size_t n) { return (int *)(lc + n + kExpTab); }
 
 cudaError_t launch_log_coh(cudaStream_t st, int ntc, int nnl, int nn, long long ncorr, const int *nodes, const double *corr,
                            double *lc, float *lc32) {
     const long long n = (long long)ntc * nnl * nnl;
     if (n == 0) return cudaSuccess;
-    k_log_coh<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ntc, nnl, nn, ncorr, nodes, corr, lc, lc32);
+    int *bad = log_coh_bad(lc, (size_t)n);
+    cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    k_log_coh<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ntc, nnl, nn, ncorr, nodes, corr, lc, lc32, bad);
     return cudaGetLastError();
 }
 
-size_t log_coh_bytes(size_t n) { return sizeof(double) * (n + kExpTab); }
+size_t log_coh_bytes(size_t n) { return sizeof(double) * (n + kExpTab + 1); }
 
 cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm,
-                          const double *logc, const double *rootS, const double *L, double *A) {
+                          const double *logc, const double *rootS, const double *L, double *A, const int *only) {
     if (nf == 0) return cudaSuccess;
     if (nm > 64) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)nf * ntc, (unsigned)((nnl + 63) / 64));
     const double *expt = logc + (size_t)ntc * nnl * nnl;
 #define BSA_AT_CASE(V)                                                                          \
     if (nm <= 4 * V) {                                                                          \
-        k_atable<V><<<grid, 256, 0, st>>>(nf, f, ntc, nnl, nm, logc, expt, rootS, L, A);        \
+        k_atable<V><<<grid, 256, 0, st>>>(nf, f, ntc, nnl, nm, logc, expt, rootS, L, A, only);  \
         return cudaGetLastError();                                                              \
     }
     BSA_AT_CASE(1)

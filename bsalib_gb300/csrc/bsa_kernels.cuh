@@ -13,15 +13,24 @@ cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, 
 
 // log c_ij [itc][i][j] of the loaded nodes (1-based ids) from the packed coherences corr[itc][ncorr] of
 // nn nodes, in FP64 and FP32.  lc has room for the A kernel's exponential table behind it
-// (log_coh_bytes(n), n = ntc nnl^2).
+// and a flag (log_coh_bad) that says whether a coherence lies outside [0, 1] or a node's own is not 1
+// (log_coh_bytes(n) in all, n = ntc nnl^2).
 size_t log_coh_bytes(size_t n);
+int *log_coh_bad(const double *lc, size_t n);
 cudaError_t launch_log_coh(cudaStream_t st, int ntc, int nnl, int nn, long long ncorr, const int *nodes, const double *corr,
                            double *lc, float *lc32);
 
 // A[f][k][m] = sqrt(S_i(f)) sum_j c_ij^|f| sqrt(S_j(f)) L[(itc,j)][m]  (FP64); rootS = sqrt(S), logc
-// followed by the exponential's table (launch_nodal_psd's expt).
+// followed by the exponential's table (launch_nodal_psd's expt).  only: form nothing where *only is 0.
 cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm,
-                          const double *logc, const double *rootS, const double *L, double *A);
+                          const double *logc, const double *rootS, const double *L, double *A, const int *only = nullptr);
+
+// The same on the tensor cores (bsa_atable64_tc.cu); leaves A alone where *bad is set (then launch_atable
+// with only = bad forms it).  scratch: atable64_tc_scratch(nf, ntc, nnl, nm) bytes; err receives a
+// nonzero code if a pipeline wait ran out of its budget.
+size_t atable64_tc_scratch(int nf, int ntc, int nnl, int nm);
+cudaError_t launch_atable64_tc(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm, const double *logc,
+                               const double *rootS, const double *L, const int *bad, double *A, void *scratch, int *err);
 
 
 // The FP32 table on the tensor cores (bsa_atable_tc.cu): tf32 hi/lo split, FP32 accumulation;

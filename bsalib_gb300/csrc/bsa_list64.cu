@@ -53,7 +53,7 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
     const long long cap = 8LL << 30;
     const long long batch = std::max(1LL, std::min({npts, cap / (24 * nm3), cap / (2 * rowb)}));
     if ((e = dMixB.reserve(tc_block_bytes(nr, nm, K))) || (e = dFlag.reserve(256))) return cuda_fail(e, "allocating pair products");
-    if ((e = cudaMemsetAsync(dFlag.p, 0, sizeof(int), stream)) || (e = tc_prep_blocks(stream, nr, nm, K, dA.as<double>(), dMixB.p)))
+    if ((e = cudaMemsetAsync(dFlag.as<int>() + 1, 0, sizeof(int), stream)) || (e = tc_prep_blocks(stream, nr, nm, K, dA.as<double>(), dMixB.p)))
         return cuda_fail(e, "pair product operands");
     kernels += 2;
     for (long long p0 = 0; p0 < npts; p0 += batch) {
@@ -148,7 +148,7 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
         h2d += (double)(ib + 2 * lb + xb + pb);
         Chunk c{0, (int)xmap.size(), nm, nm, K, nr - 1, 0, (long long)items.size(), nullptr, dMixA.as<double>(), tiles_x * kTM, dx};
         PairList l{ditems, dblk, dpair, np, bw, tiles_x};
-        if ((e = tc_list_products(stream, c, l, nr, dA.as<double>(), dQ.as<double>(), dMixB.p, dMshT.p, dFlag.as<int>())))
+        if ((e = tc_list_products(stream, c, l, nr, dA.as<double>(), dQ.as<double>(), dMixB.p, dMshT.p, dFlag.as<int>() + 1)))
             return cuda_fail(e, "pair product kernel");
         PointSrc q = ps;
         q.ix += p0;

@@ -441,7 +441,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
                                  sizeof(double2) * (size_t)PB * nm * 3 + sizeof(PairInfo) * (size_t)PB);
     if (!diag && (e = cudaFuncSetAttribute(k_pair_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
         return cuda_fail(e, "pair moments kernel");
-    if (tensor && ((e = cudaMemsetAsync(dFlag.p, 0, sizeof(int), stream)) ||
+    if (tensor && ((e = cudaMemsetAsync(dFlag.as<int>() + 1, 0, sizeof(int), stream)) ||
                    (e = tc_prep_cols(stream, hi + 1, an, K, A, dMixB.p))))
         return cuda_fail(e, "pair product operands");
     if (tensor) kernels += 2;
@@ -449,7 +449,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
         const Plan &p = plans[q];
         Chunk c{p.x0, p.x1, nm, an, K, hi, p.ntiles, p.items, (const RowTile *)idx + p.rt0, dMixA.as<double>(), rx, nullptr};
         if (tensor) {
-            if ((e = tc_products(stream, c, hi + 1, A, Q, dMixB.p, dMshT.p, dFlag.as<int>())))
+            if ((e = tc_products(stream, c, hi + 1, A, Q, dMixB.p, dMshT.p, dFlag.as<int>() + 1)))
                 return cuda_fail(e, "pair product kernel");
             kernels += 2;
         } else {
@@ -473,12 +473,13 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     if ((e = cudaGetLastError())) return cuda_fail(e, "reduction kernel");
     kernels += diag ? 2 : 3;
     std::vector<double> h(2 * (size_t)nb);
-    int herr = 0;
+    int flags[2] = {0, 0}, rc;  // A table, pair products
+    const bool pend = atable_pending;
     if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
-        (tensor && (e = cudaMemcpyAsync(&herr, dFlag.p, sizeof(int), cudaMemcpyDeviceToHost, stream))) ||
+        ((tensor || pend) && (e = cudaMemcpyAsync(flags, dFlag.p, sizeof flags, cudaMemcpyDeviceToHost, stream))) ||
         (e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream)))
         return cuda_fail(e, "moment copy");
-    if (herr) return fail(BSA_ERR_TIMEOUT, "pair product kernel: a pipeline wait ran out of its budget (role %d)", herr);
+    if ((rc = pipeline_flags(flags, pend, tensor))) return rc;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev2, ev1);
     last_ms_contraction = ms;

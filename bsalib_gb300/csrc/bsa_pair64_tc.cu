@@ -24,63 +24,20 @@
 
 #include <algorithm>
 
+#include "bsa_digits.cuh"
 #include "bsa_pair64.cuh"
-#include "bsa_tc.cuh"
 
 namespace bsa {
 namespace p64 {
 
 using namespace tc;
 
-constexpr int kDig = 8;                  // digits per operand
 constexpr int kPassK = 512 / kBK;        // K blocks of one exact pass
 constexpr int kRingA = 8;                // A digit tiles in flight (16 KB each)
 constexpr int kRingB = 2;                // B tiles in flight (32 KB each)
 constexpr int kTileA = kTM * 128, kTileB = kDig * kTN * 128;
 constexpr int kTcThreads = 192;
 constexpr size_t kTcSmem = 1024 + (size_t)kRingA * kTileA + (size_t)kRingB * kTileB + 512;
-constexpr int kBad = 1 << 20;            // row exponent of a row that holds an infinity or a NaN
-constexpr int kNone = -(1 << 20);        // of a row of zeros
-
-// Biased exponent field (0 for zeros and denormals, 2047 for infinities and NaN).
-__device__ __forceinline__ int expo(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
-
-// Sixteen values of one row, scaled by 2^(55 - e), as digits: dst[s plane + 0 .. 15].
-__device__ __forceinline__ void put_digits(const double *v, int e, __nv_bfloat16 *dst, size_t plane) {
-    uint32_t w[kDig][8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        uint32_t f[2][kDig];
-#pragma unroll
-        for (int z = 0; z < 2; ++z) {
-            const double x = v[2 * q + z];
-            const int ex = expo(x), sh = 3 + (ex - 1023) - e;
-            unsigned long long m = ((unsigned long long)__double_as_longlong(x) & 0xfffffffffffffull) | 0x10000000000000ull;
-            if (sh >= 0) m <<= sh;
-            else if (sh > -60) m = (m + (1ull << (-sh - 1))) >> -sh;
-            else m = 0;
-            if (ex == 0) m = 0;
-            // balanced digits: add 64 to every digit, cut into 7 bits, take 64 away
-            constexpr unsigned long long kHalf = 64ull * ((1ull << 56) - 1) / 127ull;
-            const unsigned long long u = (__double2hiint(x) < 0 ? 0ull - m : m) + kHalf;
-#pragma unroll
-            for (int s = 0; s < kDig; ++s) {
-                const int sft = 7 * (kDig - 1 - s);
-                const uint32_t d = s == 0 ? (uint32_t)(u >> sft) : (uint32_t)(u >> sft) & 127u;
-                // integer d - 64 as a float (exact in bf16: its low half is zero)
-                f[z][s] = __float_as_uint(__uint_as_float(0x4B400000u + d - 64u) - 12582912.f);
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < kDig; ++s) w[s][q] = __byte_perm(f[0][s], f[1][s], 0x7632);
-    }
-#pragma unroll
-    for (int s = 0; s < kDig; ++s) {
-        uint4 *o = reinterpret_cast<uint4 *>(dst + s * plane);
-        o[0] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
-        o[1] = make_uint4(w[s][4], w[s][5], w[s][6], w[s][7]);
-    }
-}
 
 // Column operand: exponent e[c] with |A[y][k][j]| < 2^e[c], c = y an + j.
 __global__ __launch_bounds__(256) void k_col_exp(int an, int K, const double *__restrict__ A, int *__restrict__ ec) {
@@ -115,14 +72,14 @@ __global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restri
 #pragma unroll 8
         for (int k = lane; k < c.K; k += 8) {
             const int u = (q[(size_t)2 * k * qn] >> 20) & 0x7ff, v = (p[(size_t)2 * k * an] >> 20) & 0x7ff;
-            m = max(m, (u == 2047 || v == 2047) ? kBad : (u && v) ? u + v : 0);
+            m = max(m, expo_pair(u, v));
         }
     mx[lane][threadIdx.x & 31] = m;
     __syncthreads();
     if (lane == 0 && ab < rx) {
 #pragma unroll
         for (int z = 1; z < 8; ++z) m = max(m, mx[z][threadIdx.x]);
-        er[(size_t)blockIdx.x * c.rpad + ab] = m == kBad ? kBad : m == 0 ? kNone : m - 2044;
+        er[(size_t)blockIdx.x * c.rpad + ab] = expo_of_pairs(m);
     }
 }
 
@@ -183,41 +140,6 @@ __global__ __launch_bounds__(256) void k_row_digits(Chunk c, int Kp, const doubl
         }
         put_digits(v, some ? e : 0, D + ((r / kTM) * kDig * kTM + r % kTM) * (size_t)Kp + kb + kq * 16, (size_t)kTM * Kp);
     }
-}
-
-__device__ __forceinline__ void mma_n(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-                 : "r"(taddr));
-}
-
-// (hi 2^28 + lo) 2^ex rounded once to FP64, in integer instructions.
-__device__ __forceinline__ double combine(long long hi, long long lo, int ex) {
-    long long h = hi + (lo >> 28);
-    uint32_t l = (uint32_t)lo & 0xfffffffu;
-    const bool neg = h < 0;
-    if (neg) {
-        h = -h - (l != 0);
-        l = (0x10000000u - l) & 0xfffffffu;
-    }
-    if (h == 0 && l == 0) return 0.0;
-    const int lz = __clzll(h), E = 91 - lz + ex;
-    if (lz > 35 || E < -1022 || E > 1022) {  // small sums (28 bits of h at least otherwise) and the ends of the range
-        const double v = scalbn(fma((double)h, 268435456.0, (double)l), ex);
-        return neg ? -v : v;
-    }
-    const unsigned long long w = ((unsigned long long)h << lz) |
-                                 (lz >= 28 ? (unsigned long long)l << (lz - 28) : (unsigned long long)(l >> (28 - lz)));
-    // top bit of w at 63: 53 bits and the rounding bit
-    unsigned long long b = (w >> 11) + ((w >> 10) & 1ull) + ((unsigned long long)(E + 1022) << 52);
-    if (neg) b |= 0x8000000000000000ull;
-    return __longlong_as_double((long long)b);
 }
 
 // LIST: the items and column blocks of a pair list instead of the chunk's tile rows.
@@ -393,8 +315,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         int D[kDig];
 #pragma unroll
                         for (int l = 0; l < kDig; ++l) D[l] = __float2int_rn(__uint_as_float(v[l][q]));
-                        hi[cg * 8 + q] += (((long long)D[0] * 128 + D[1]) * 128 + D[2]) * 128 + D[3];
-                        lo[cg * 8 + q] += (((long long)D[4] * 128 + D[5]) * 128 + D[6]) * 128 + D[7];
+                        add_levels(D, hi[cg * 8 + q], lo[cg * 8 + q]);
                     }
                 }
                 fence_before();

@@ -28,7 +28,8 @@ def _reference(p, f):
 
 
 @pytest.mark.parametrize("nodes,modes", [(2, 1), (31, 4), (32, 5), (33, 8), (63, 9), (64, 12), (65, 13), (66, 16), (40, 17),
-                                         (40, 21), (40, 25), (40, 33), (40, 41), (40, 49), (130, 57), (70, 64)])
+                                         (40, 21), (40, 25), (40, 33), (40, 41), (40, 49), (130, 57), (70, 64),
+                                         (79, 3), (80, 3), (128, 12), (129, 32), (200, 33), (192, 8), (513, 5), (600, 40)])
 def test_atable_through_force_moments(bsalib, nodes, modes):
     p = random_structure(nodes + modes, nodes=(nodes, nodes), modes=(modes, modes), nfreq_grid=(17, 17))
     p.settings.ibisp = 0
@@ -36,6 +37,25 @@ def test_atable_through_force_moments(bsalib, nodes, modes):
     p.nod_corr[1, 0] = 0.0
     if p.nod_corr.shape[0] > 4:
         p.nod_corr[3, 0], p.nod_corr[4, 0] = 1e-300, 1e-120
+    s = api.BsaSession(p)
+    try:
+        m2 = s.run()["m2mf_cls"]
+    finally:
+        s.close()
+    h = p.settings.nfreqs - 1
+    f = np.arange(-h, h + 1) * p.settings.df
+    w = np.full(f.size, 2 * np.pi * p.settings.df)
+    w[[0, -1]] /= 2
+    ref = np.einsum("f,fon->on", w, _reference(p, f)).ravel()
+    assert np.max(np.abs(m2 - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("where,value", [(0, 0.5), (3, 1.5), (0, 0.0)])
+def test_coherences_outside_the_usual(bsalib, where, value):
+    """A node's own coherence below 1, a coherence above 1: the general kernel forms the table."""
+    p = random_structure(7, nodes=(90, 90), modes=(5, 5), nfreq_grid=(17, 17))
+    p.settings.ibisp = 0
+    p.nod_corr[where, 0] = value
     s = api.BsaSession(p)
     try:
         m2 = s.run()["m2mf_cls"]
