@@ -651,6 +651,7 @@ struct BatchCase {
     std::vector<double> hL, hQ, hCorr, hM, hK, hC, hWd3, hWd2;
     std::vector<int> hNodes;
     int hNn = 0;
+    std::vector<unsigned char> hPack;
     std::vector<float> hL32;
     std::vector<PsdNode> hPsd;
     std::vector<double> f;  // Classic grid
@@ -697,6 +698,7 @@ void Engine::batch_swap(BatchCase &c) {
     hWd2.swap(c.hWd2);
     hL32.swap(c.hL32);
     hPsd.swap(c.hPsd);
+    hPack.swap(c.hPack);
 }
 
 // Makes case c the engine's problem (derived tables only; no caller arrays are read).
@@ -1025,18 +1027,8 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
             return cuda_fail(e, "batch run");
         if ((rc = atable_check())) return rc;
         if (herr) return fail(BSA_ERR_TIMEOUT, "batched kernel: a pipeline wait ran out of its budget (role %d)", herr);
-        // results of this group: moments and m2 of its cases
-        for (size_t k = g0; k < g1; ++k) {
-            const int c = order[k];
-            const long long n3 = (long long)g_batch[c].nme * g_batch[c].nme * g_batch[c].nme;
-            const long long n2 = (long long)g_batch[c].nme * g_batch[c].nme;
-            if ((e = cudaMemcpy(h3f.data() + off3[c], o + off3[c], sizeof(double) * n3, cudaMemcpyDeviceToHost)) ||
-                (e = cudaMemcpy(h3r.data() + off3[c], o + t3 + off3[c], sizeof(double) * n3, cudaMemcpyDeviceToHost)) ||
-                (e = cudaMemcpy(h2.data() + 3 * off2[c], d_m2 + 3 * off2[c], sizeof(double) * 3 * n2,
-                                cudaMemcpyDeviceToHost)))
-                return cuda_fail(e, "batch results");
-            lat[c] = (double)(td[k - g0] - td[cp.size()]) * 1e-6;  // ms from the launch start
-        }
+        for (size_t k = g0; k < g1; ++k)
+            lat[order[k]] = (double)(td[k - g0] - td[cp.size()]) * 1e-6;  // ms from the launch start
         float ms = 0.f;
         cudaEventElapsedTime(&ms, ev2, ev1);
         total += ms;
@@ -1045,6 +1037,12 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
         for (const CaseP &q : cp) points += (double)q.nf * q.nf;
         g0 = g1;
     }
+    // every case's moments and m2, in case order on the device
+    if ((e = cudaMemcpyAsync(h3f.data(), dOut.p, sizeof(double) * (size_t)t3, cudaMemcpyDeviceToHost, stream)) ||
+        (e = cudaMemcpyAsync(h3r.data(), dOut.as<double>() + t3, sizeof(double) * (size_t)t3, cudaMemcpyDeviceToHost, stream)) ||
+        (e = cudaMemcpyAsync(h2.data(), dMshT.p, sizeof(double) * 3 * (size_t)t2, cudaMemcpyDeviceToHost, stream)) ||
+        (e = cudaStreamSynchronize(stream)))
+        return cuda_fail(e, "batch results");
     for (int c = 0; c < nc; ++c) {
         const long long n3 = (long long)g_batch[c].nme * g_batch[c].nme * g_batch[c].nme;
         const long long n2 = (long long)g_batch[c].nme * g_batch[c].nme;

@@ -41,6 +41,13 @@ struct DevBuf {
     T *as() const { return (T *)p; }
 };
 
+// Part of a device buffer.
+struct DevView {
+    void *p = nullptr;
+    template <class T>
+    T *as() const { return (T *)p; }
+};
+
 // Borrowed caller arrays (Fortran layouts), as the reference keeps pointers to them.
 struct Inputs {
     int nn = 0, nlibs = 0, ndofs = 0, phi_ndofs = 0, nnl = 0, nlibsl = 0;
@@ -162,6 +169,7 @@ struct Engine {
     std::vector<double> hCorr;         // packed coherences of the components [comp][ncorr]; log c_ij formed on the device
     std::vector<int> hNodes;           // loaded nodes
     int hNn = 0;                       // nodes the packing counts
+    std::vector<unsigned char> hPack;  // the derived tables as they go to the device, in one copy
     std::vector<double> hWd3, hWd2;  // diagonal-only weights Q L^2 and L^2, [k][m]
     std::vector<float> hL32;         // FP32 copy of L for the split-precision A(f) table
     std::vector<PsdNode> hPsd;
@@ -169,9 +177,10 @@ struct Engine {
     // device
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
-    DevBuf dL, dQ, dLogc, dPsdPar, dFrfM, dFrfK, dFrfC, dFreq, dS, dA, dPartF, dPartR, dOut, dPsdF, dWf, dPts,
-        dPtsD, dBF, dBR, dMixA, dMixB, dMixH, dMixPart, dA32, dZones, dZidx, dWd3, dWd2, dMshT, dMshIdx, dLogc32, dL32,
-        dPod, dFlag, dSlot, dHash, dCptr, dCq, dZoneH, dZoff, dCorr;
+    DevView dL, dQ, dPsdPar, dFrfM, dFrfK, dFrfC, dWd3, dWd2, dL32;  // parts of dProb
+    DevBuf dProb, dLogc, dFreq, dS, dA, dPartF, dPartR, dOut, dPsdF, dWf, dPts,
+        dPtsD, dBF, dBR, dMixA, dMixB, dMixH, dMixPart, dA32, dZones, dZidx, dMshT, dMshIdx, dLogc32,
+        dPod, dFlag, dSlot, dHash, dCptr, dCq, dZoneH, dZoff;
 
     // stats
     double last_ms = 0, last_ms_contraction = 0, last_ms_gemm = 0, last_points = 0;

@@ -156,9 +156,9 @@ void Engine::reset_inputs() {
 
 void Engine::free_device() {
     if (stream) cudaStreamSynchronize(stream);  // the blocks go back to the cache for reuse
-    for (DevBuf *b : {&dL, &dQ, &dLogc, &dPsdPar, &dFrfM, &dFrfK, &dFrfC, &dFreq, &dS, &dA, &dPartF, &dPartR,
+    for (DevBuf *b : {&dProb, &dLogc, &dFreq, &dS, &dA, &dPartF, &dPartR,
                       &dOut, &dPsdF, &dWf, &dPts, &dPtsD, &dBF, &dBR, &dMixA, &dMixB, &dMixH, &dMixPart, &dA32,
-                      &dZones, &dZidx, &dWd3, &dWd2, &dMshT, &dMshIdx, &dLogc32, &dL32, &dPod, &dFlag, &dSlot, &dHash, &dCptr, &dCq, &dZoneH, &dZoff, &dCorr})
+                      &dZones, &dZidx, &dMshT, &dMshIdx, &dLogc32, &dPod, &dFlag, &dSlot, &dHash, &dCptr, &dCq, &dZoneH, &dZoff})
         b->release();
     if (stream) cudaStreamDestroy(stream);
     stream = nullptr;
@@ -341,19 +341,29 @@ int Engine::upload_problem() {
     if (dev_uploaded) return BSA_OK;
     cudaError_t e;
     const int ntc = (int)set.tc.size(), nnl = (int)hNodes.size();
-    const size_t ncoh = (size_t)ntc * nnl * nnl, nb = (sizeof(int) * nnl + 255) / 256 * 256;
-    if ((e = dCorr.reserve(nb + sizeof(double) * hCorr.size())) || (e = dLogc.reserve(log_coh_bytes(ncoh))) ||
-        (e = cudaMemcpyAsync(dCorr.p, hNodes.data(), sizeof(int) * nnl, cudaMemcpyHostToDevice, stream)) ||
-        (e = cudaMemcpyAsync((char *)dCorr.p + nb, hCorr.data(), sizeof(double) * hCorr.size(), cudaMemcpyHostToDevice, stream)) ||
-        (e = upload(dL, hL, stream)) || (e = upload(dQ, hQ, stream)) || (e = upload(dPsdPar, hPsd, stream)) ||
-        (e = upload(dFrfM, hM, stream)) || (e = upload(dFrfK, hK, stream)) || (e = upload(dFrfC, hC, stream)) ||
-        (e = upload(dWd3, hWd3, stream)) || (e = upload(dWd2, hWd2, stream)) || (e = upload(dL32, hL32, stream)) ||
+    const size_t ncoh = (size_t)ntc * nnl * nnl;
+    // one copy for all tables (eleven small ones cost 60 us of launches)
+    DevView corr, nodes;
+    struct Part { const void *src; size_t bytes; DevView *dst; };
+    auto part = [](const auto &v, DevView &d) { return Part{v.data(), sizeof(v[0]) * v.size(), &d}; };
+    const Part parts[] = {part(hCorr, corr), part(hNodes, nodes), part(hL, dL), part(hQ, dQ), part(hPsd, dPsdPar), part(hM, dFrfM),
+                          part(hK, dFrfK), part(hC, dFrfC), part(hWd3, dWd3), part(hWd2, dWd2), part(hL32, dL32)};
+    size_t total = 0;
+    for (const Part &p : parts) total += (p.bytes + 255) & ~(size_t)255;
+    hPack.resize(total);
+    if ((e = dProb.reserve(total))) return cuda_fail(e, "uploading problem data");
+    size_t at = 0;
+    for (const Part &p : parts) {
+        if (p.bytes) std::memcpy(hPack.data() + at, p.src, p.bytes);
+        p.dst->p = (char *)dProb.p + at;
+        at += (p.bytes + 255) & ~(size_t)255;
+    }
+    if ((e = upload(dProb, hPack, stream)) || (e = dLogc.reserve(log_coh_bytes(ncoh))) ||
         (e = dLogc32.reserve(sizeof(float) * ncoh)))
         return cuda_fail(e, "uploading problem data");
-    h2d += (double)(sizeof(int) * nnl + sizeof(double) * hCorr.size());
     // log c in FP64 and its FP32 copy
-    if ((e = launch_log_coh(stream, ntc, nnl, hNn, (long long)(hCorr.size() / ntc), dCorr.as<int>(),
-                            (const double *)((char *)dCorr.p + nb), dLogc.as<double>(), dLogc32.as<float>())))
+    if ((e = launch_log_coh(stream, ntc, nnl, hNn, (long long)(hCorr.size() / ntc), nodes.as<int>(), corr.as<double>(),
+                            dLogc.as<double>(), dLogc32.as<float>())))
         return cuda_fail(e, "coherence table");
     kernels += 1;
     dev_uploaded = true;
