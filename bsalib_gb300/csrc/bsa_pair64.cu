@@ -49,19 +49,22 @@ constexpr int kKT = 16;
 constexpr int kKinds = 9;           // K1 .. K6 (the order above: abj, ajb, baj, jba, jab, bja), M1, M2, M3
 constexpr int kBatch = 8;           // pairs a thread takes between two barriers
 
-// E of one product tile: 256 threads, 4 x 4 elements each, K staged 16 at a time; the row operand
-// Q[k][a] A(x)[k][b] is formed while staging.  FP64-pipe bound: 16 FMAs a thread and k against one
-// product in 32 for the staging.
+// E of one product tile, or of a quarter of its rows: 256 threads, ROWS / 32 x 4 elements each, K staged
+// 16 at a time; the row operand Q[k][a] A(x)[k][b] is formed while staging.  FP64-pipe bound (one
+// product in 32 for the staging); a problem of few tiles spreads over more SMs by quarters (the
+// 30-node tower's 45 tiles: 40 -> 20 us).
+template <int ROWS>
 __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__restrict__ A, const double *__restrict__ Q) {
-    __shared__ double As[kKT][kTM], Bs[kKT][kTN];
+    constexpr int RPT = ROWS / 32, KS = 256 / ROWS;
+    __shared__ double As[kKT][ROWS], Bs[kKT][kTN];
     const int t = threadIdx.x, qn = c.qn, an = c.an, rx = c.rx(), K = c.K;
     const long long item = blockIdx.x;
     const int lo = tile_row(c, item);
     const RowTile rt = c.rt[lo];
     const int ct = rt.ct0 + (int)(item - rt.item0);
-    const int r0 = lo * kTM, rows = (c.x1 - c.x0) * rx;
+    const int rt0 = blockIdx.y * ROWS, r0 = lo * kTM + rt0, rows = (c.x1 - c.x0) * rx;
     // this thread's staging row and column
-    const int sr = t & (kTM - 1), kr = t >> 7;           // As: 2 k rows of 128 rows at a time
+    const int sr = t % ROWS, kr = t / ROWS;              // As: KS k rows of ROWS rows at a time
     const bool rv = r0 + sr < rows;
     const int rr = rv ? r0 + sr : 0, x = c.x0 + rr / rx, ab = rr % rx, a = ab / an, b = ab % an;
     const double *Qa = Q + a, *Ab = A + (size_t)x * K * an + b;
@@ -69,17 +72,17 @@ __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__rest
     const int col = ct * kTN + sc, y = col / an, j = col - y * an;
     const bool cv = y <= c.hi;
     const double *Aj = A + (size_t)(cv ? y : 0) * K * an + j;
-    const int tr = (t >> 3) * 4, tc = (t & 7) * 4;
-    double acc[4][4];
+    const int tr = (t >> 3) * RPT, tc = (t & 7) * 4;
+    double acc[RPT][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RPT; ++i)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[i][q] = 0.0;
     for (int k0 = 0; k0 < K; k0 += kKT) {
         const int kn = min(kKT, K - k0);
 #pragma unroll
-        for (int u = 0; u < kKT / 2; ++u) {
-            const int k = kr + 2 * u;
+        for (int u = 0; u < kKT / KS; ++u) {
+            const int k = kr + KS * u;
             As[k][sr] = (rv && k < kn) ? Qa[(size_t)(k0 + k) * qn] * Ab[(size_t)(k0 + k) * an] : 0.0;
         }
 #pragma unroll
@@ -89,13 +92,13 @@ __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__rest
         }
         __syncthreads();
         for (int k = 0; k < kn; ++k) {
-            double ar[4], br[4];
+            double ar[RPT], br[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) ar[i] = As[k][tr + i];
+            for (int i = 0; i < RPT; ++i) ar[i] = As[k][tr + i];
 #pragma unroll
             for (int q = 0; q < 4; ++q) br[q] = Bs[k][tc + q];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RPT; ++i)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) acc[i][q] = fma(ar[i], br[q], acc[i][q]);
         }
@@ -104,9 +107,9 @@ __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__rest
     const size_t ld = (size_t)rt.nct * kTN;
     double *out = c.E + rt.base + (size_t)(ct - rt.ct0) * kTN + tc;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RPT; ++i)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) out[(size_t)(tr + i) * ld + q] = acc[i][q];
+        for (int q = 0; q < 4; ++q) out[(size_t)(rt0 + tr + i) * ld + q] = acc[i][q];
 }
 
 // H of the kept modes at i df, i = 0 .. 2 N.
@@ -126,7 +129,7 @@ struct MomPar {
     const double2 *H;       // [2 N + 1][nm]
     double *part;           // [groups][kKinds][nm^2][nm]
     int first;              // first chunk: the partials are written, not added to
-    int RT, PL;             // rows (a, b) of a block, pair lanes
+    int RT, PL, PB;         // rows (a, b) of a block, pair lanes, pairs of a batch (at most kBatch PL)
 };
 
 // Relative weight of grid point (i1, i2) (BsaClassicImpl.F90:596-632, vertex -1/2), 0 beyond it.
@@ -166,13 +169,13 @@ __device__ __forceinline__ PairInfo pair_info(int x, int y, int N, int vect) {
 }
 
 // One block per (tile of RT rows (a, b), group of pairs); a thread holds one element (a, b, j) and
-// takes the pairs of its lane.  Per batch of kBatch x PL pairs: the pairs and weights, then the
+// takes the pairs of its lane.  Per batch of PB pairs: the pairs and weights, then the
 // products of the row factors (8 doubles a row) and the columns' FRF values in shared memory, then
 // 9 (all weights one), 14 (no sums on the grid) or 27 FP64 operations an element and pair.
 __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
     extern __shared__ double sm[];
     const int t = threadIdx.x, nm = c.an, nm2 = nm * nm;
-    const int PB = kBatch * P.PL, RT = P.RT, EL = RT * nm;
+    const int PB = P.PB, RT = P.RT, EL = RT * nm;
     double *rowf = sm;                                 // [PB][RT][8]
     double2 *colf = (double2 *)(rowf + (size_t)PB * RT * 8);  // [PB][nm][3]: Hx, P, D
     PairInfo *info = (PairInfo *)(colf + (size_t)PB * nm * 3);
@@ -371,9 +374,10 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     // least one batch of pairs)
     const int RT = std::max(1, std::min(rx, 256 / nm)), PL = std::max(1, std::min(8, 256 / (RT * nm)));
     const int tiles = (rx + RT - 1) / RT;
-    const int G = diag ? std::min(64, (N + 8) / 8)
-                       : (int)std::max(1LL, std::min<long long>((608 + tiles - 1) / tiles,
-                                                                (pairs_all + kBatch * PL - 1) / (kBatch * PL)));
+    // pairs of a batch: fewer for small grids, so that the groups still fill the chip
+    const long long want = (608 + tiles - 1) / tiles;
+    const int PB = PL * (int)std::max(1LL, std::min<long long>(kBatch, pairs_all / (want * PL)));
+    const int G = diag ? std::min(64, (N + 8) / 8) : (int)std::max(1LL, std::min(want, (pairs_all + PB - 1) / PB));
     // Products on the tensor cores (bsa_pair64_tc.cu) where they outweigh the digits' preparation.
     // Measured contraction, FP64 pipe / tensor cores: 4.1e6 FMAs, K = 30: 0.097 / 0.108 ms; 7.3e6,
     // K = 60: 0.126 / 0.109; 1.9e7, K = 20: 0.137 / 0.167; 5.4e7, K = 12: 0.353 / 0.447; 6.9e7,
@@ -436,7 +440,6 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     if ((e = cudaEventRecord(ev2, stream)) || (e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
     const int nh = (2 * N + 1) * nm;
     k_frf_rows<<<(nh + 127) / 128, 128, 0, stream>>>(2 * N + 1, nm, df, frf(), dMixH.as<double2>());
-    const int PB = kBatch * PL;
     const size_t smem = std::max((size_t)256 * sizeof(double), sizeof(double) * (size_t)PB * RT * 8 +
                                  sizeof(double2) * (size_t)PB * nm * 3 + sizeof(PairInfo) * (size_t)PB);
     if (!diag && (e = cudaFuncSetAttribute(k_pair_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
@@ -453,14 +456,15 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
                 return cuda_fail(e, "pair product kernel");
             kernels += 2;
         } else {
-            k_pair_gemm<<<(unsigned)p.items, 256, 0, stream>>>(c, A, Q);
+            if (p.items < 304) k_pair_gemm<32><<<dim3((unsigned)p.items, kTM / 32), 256, 0, stream>>>(c, A, Q);
+            else k_pair_gemm<kTM><<<dim3((unsigned)p.items, 1), 256, 0, stream>>>(c, A, Q);
         }
         if (diag) {
             k_pair_moments_diag<<<dim3(nm, G), 256, 0, stream>>>(c, N, analytic ? 1 : 0, vect ? 1 : 0, 4.0 * wval,
                                                                   dMixH.as<double2>(), dPartF.as<double>() + q * G * plen);
         } else {
             MomPar mp{N, vect ? 1 : 0, p.npairs, (const long long *)(idx + rtb) + p.pre0, dMixH.as<double2>(),
-                      dPartF.as<double>(), q == 0 ? 1 : 0, RT, PL};
+                      dPartF.as<double>(), q == 0 ? 1 : 0, RT, PL, PB};
             k_pair_moments<<<dim3((unsigned)tiles, (unsigned)G), 256, smem, stream>>>(c, mp);
         }
         kernels += 2;
