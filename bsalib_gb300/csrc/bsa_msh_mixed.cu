@@ -340,10 +340,12 @@ __global__ void k_prep_u_rows(int nm, int K, int Kp, int Mp, const int *__restri
     }
 }
 
-// T[(t*NMT + j)][k] = A(src[t])[k][j]   (j >= nm and k >= K are zero)
-__global__ void k_prep_b_rows(int nm, int NMT, int K, int Kp, const int *__restrict__ src, const float *__restrict__ A,
-                              __nv_bfloat16 *__restrict__ Th, __nv_bfloat16 *__restrict__ Tl) {
-    const int t = blockIdx.x, k0 = blockIdx.y * 64;
+// T[(t*NMT + j)][k] = A(src[t])[k][j]   (j >= nm and k >= K are zero); with pos the same row at pos[t]
+// too (a point's row in line and in column order from one read).
+__global__ __launch_bounds__(256) void k_prep_b_rows(int nm, int NMT, int K, int Kp, const int *__restrict__ src,
+                                                     const int *__restrict__ pos, const float *__restrict__ A,
+                                                     __nv_bfloat16 *__restrict__ Th, __nv_bfloat16 *__restrict__ Tl) {
+    const int t = blockIdx.x, k0 = blockIdx.y * 64, t2 = pos ? pos[t] : -1;
     __shared__ float As[64][65];
     const float *Ar = A + (size_t)src[t] * K * nm;
     for (int e = threadIdx.x; e < 64 * nm; e += blockDim.x) {
@@ -359,6 +361,11 @@ __global__ void k_prep_b_rows(int nm, int NMT, int K, int Kp, const int *__restr
         const size_t o = ((size_t)t * NMT + j) * Kp + k0 + kv;
         *(uint4 *)(Th + o) = *(const uint4 *)hi;
         *(uint4 *)(Tl + o) = *(const uint4 *)lo;
+        if (t2 >= 0) {
+            const size_t o2 = ((size_t)t2 * NMT + j) * Kp + k0 + kv;
+            *(uint4 *)(Th + o2) = *(const uint4 *)hi;
+            *(uint4 *)(Tl + o2) = *(const uint4 *)lo;
+        }
     }
 }
 
@@ -404,12 +411,21 @@ __global__ void k_msh_frf(int nm, int nz, const ZoneM *__restrict__ zones, int n
     const double v1 = (z.fi0 + ((double)qi / z.Fi) * z.dI) * kPi2;
     const double v2 = (z.fj0 + ((double)qj / z.Fj) * z.dJ) * kPi2;
     const double w = which == 0 ? v1 : which == 1 ? v2 : v1 + v2;
-    double hr, hi;
-    frf_eval(frf.M[m], frf.K[m], frf.C[m], w, hr, hi);
     const int hs = frf_row(nm);
     float2 *row = Hq + (size_t)q * hs;
-    row[r] = make_float2((float)hr, (float)hi);
-    if (r == 0) {
+    // H(w1) is the same along a lattice line and H(w2) along a column: the line's (column's) first point
+    // evaluates it and stores it for all (the divisions of three values a point were 2.1 ms of the
+    // bridge deck's 94 773 points, now 1.75 ms)
+    if ((which == 0 && qj != 0) || (which == 1 && qi != 0)) return;
+    double hr, hi;
+    frf_eval(frf.M[m], frf.K[m], frf.C[m], w, hr, hi);
+    const float2 h = make_float2((float)hr, (float)hi);
+    row[r] = h;
+    if (which == 0)
+        for (int j = 1; j <= NJ; ++j) row[(size_t)j * hs + r] = h;
+    if (which == 1)
+        for (int i = 1; i <= NI; ++i) row[(size_t)i * (NJ + 1) * hs + r] = h;
+    if (which == 2 && m == 0) {
         const double ti = (qi == 0 || qi == NI) ? 0.5 : 1.0, tj = (qj == 0 || qj == NJ) ? 0.5 : 1.0;
         const float wq = (float)(z.sym * (z.wI / z.Fi) * (z.wJ / z.Fj) * ti * tj);
         Wq[q] = wq;
@@ -441,6 +457,11 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 // one bulk copy per (term, corner) brings in.
 struct MomLayout {
     int JB, AR, RB, nchj;
+    // A warp covers 4 a-rows x 8 modes b of a j' where the block holds them (B8 warps side by side), so
+    // that every load of the point loop is one 128-byte wavefront; in thread order (one a-row after the
+    // other) the b-indexed loads took four.  Bridge deck, 60 modes: 41.8 -> 37.6 ms with the point loop's
+    // narrower loads.
+    int B8;
     static MomLayout make(int nm) {
         MomLayout L;
         L.AR = (nm + kMomEPT - 1) / kMomEPT;
@@ -448,12 +469,14 @@ struct MomLayout {
         L.JB = std::max(1, std::min(256 / per_j, kVY / nm));
         L.RB = L.JB > 1 ? L.AR : 256 / nm;
         L.nchj = L.JB > 1 ? 1 : (L.AR + L.RB - 1) / L.RB;
+        const int b8 = (nm + 7) / 8, a4 = (L.RB + 3) / 4;
+        L.B8 = L.JB == 1 && b8 * a4 <= 8 ? b8 : 0;
         return L;
     }
     int groups(int nm) const { return (nm + JB - 1) / JB; }
     // dynamic shared memory of k_msh_moments
     static size_t smem() {
-        return (size_t)kQB * kVY * 16 + (size_t)kQB * 64 * 16 + (size_t)kQB * kHrow * 8 + (size_t)12 * kWin * 4 + 16;
+        return (size_t)kQB * kVY * 24 + (size_t)kQB * 64 * 24 + (size_t)kQB * kHrow * 8 + (size_t)12 * kWin * 4 + 16;
     }
 };
 
@@ -574,13 +597,16 @@ __global__ __launch_bounds__(256, 2) void k_msh_moments(int nm, int nm3p, MomLay
     extern __shared__ __align__(16) unsigned char msm[];
     float4(*VY)[kVY] = reinterpret_cast<float4(*)[kVY]>(msm);                            // {Vr, Yr, Vi, Yi}
     float4(*H23)[64] = reinterpret_cast<float4(*)[64]>(msm + kQB * kVY * 16);            // {H2r, H3r, -H2i, H3i}
-    float2 *Hraw = reinterpret_cast<float2 *>(msm + kQB * kVY * 16 + kQB * 64 * 16);     // [kQB][hs]
+    // Y and H3 once more on their own: the loads by b and by a take 8 bytes of them, and the point loop is
+    // bound by the bytes its shared loads move (152 a thread and point with the 16-byte forms, now 104)
+    float2(*Ys)[kVY] = reinterpret_cast<float2(*)[kVY]>(msm + kQB * kVY * 16 + kQB * 64 * 16);
+    float2(*H3s)[64] = reinterpret_cast<float2(*)[64]>(msm + kQB * kVY * 24 + kQB * 64 * 16);
+    float2 *Hraw = reinterpret_cast<float2 *>(msm + kQB * kVY * 24 + kQB * 64 * 24);     // [kQB][hs]
     float *Cs = reinterpret_cast<float *>(Hraw + kQB * kHrow);                           // [2][2][3][kWin]
     uint64_t *bar = reinterpret_cast<uint64_t *>(Cs + 12 * kWin);
     const ulonglong2(*VYp)[kVY] = reinterpret_cast<const ulonglong2(*)[kVY]>(msm);      // the same, as pairs
     const ulonglong2(*H23p)[64] = reinterpret_cast<const ulonglong2(*)[64]>(msm + kQB * kVY * 16);
-    __shared__ ulonglong2 tq[kQB];  // {ti, ti}, {tj, tj}
-    __shared__ f2x tq2[kQB];        // {ti tj, ti tj}
+    __shared__ float2 tq[kQB];      // ti, tj
     __shared__ MomItem sit[3];      // the current item and the two after it
     const int nm2 = nm * nm, nm3 = nm2 * nm, tid = threadIdx.x, hs = frf_row(nm);
     const int grp = blockIdx.y / L.nchj, chunk = blockIdx.y % L.nchj;
@@ -599,9 +625,16 @@ __global__ __launch_bounds__(256, 2) void k_msh_moments(int nm, int nm3p, MomLay
         wlen = (((jg0 + njb) * nm2 + 3) & ~3) - win0;
     } else {
         jl = 0;
-        arow = chunk * L.RB + tid / nm;
+        int ar = tid / nm;
         b = tid % nm;
-        tval = tid < L.RB * nm && arow < L.AR;
+        if (L.B8) {
+            const int w = tid >> 5, lane = tid & 31;
+            ar = (w / L.B8) * 4 + (lane >> 3);
+            b = (w % L.B8) * 8 + (lane & 7);
+        }
+        arow = chunk * L.RB + ar;
+        tval = ar < L.RB && b < nm && arow < L.AR;
+        if (!tval) b = 0;
         const int a0 = chunk * L.RB * EPT, a1 = min(nm, (chunk + 1) * L.RB * EPT);
         win0 = (jg0 * nm2 + a0 * nm) & ~3;
         wlen = ((jg0 * nm2 + a1 * nm + 3) & ~3) - win0;
@@ -610,13 +643,16 @@ __global__ __launch_bounds__(256, 2) void k_msh_moments(int nm, int nm3p, MomLay
     const int ev0 = tval ? (jg0 + jl) * nm2 + arow * EPT * nm + b : 0;  // element u: ev0 + u nm
     const int wofs = tval ? ev0 - win0 : 0;                           // in the window
     // elements past a = nm - 1 (u >= nval) read the next staged V, Y, H entries, which lie inside
-    // the dynamic shared memory (VY is followed by H23, H23 by Hraw); their sums are never stored
+    // the dynamic shared memory (VY is followed by H23, H23 by Ys, H3s by Hraw); their sums are never stored
     const int ia0 = tval ? jl * nm + arow * EPT : 0, ih0 = tval ? arow * EPT : 0;
     const int yb = tval ? jl * nm + b : 0, bb = tval ? b : 0;
     // conversion roles: (jl, m) pairs of VY, modes of H23
     const int st = tid & (kVY - 1), sq0 = tid / kVY;
     const int sjl = st / nm, sm = st - sjl * nm;
     const bool svy = sjl < njb;
+    // (with several j' a block holds every a)
+    const int oa0 = L.JB > 1 ? 0 : chunk * L.RB * EPT, oa1 = L.JB > 1 ? nm : min(nm, (chunk + 1) * L.RB * EPT);
+    const bool sown = sm >= oa0 && sm < oa1, sown3 = st >= oa0 && st < oa1;
     const float *Ts[3] = {T1, T3, T2};
 
     // corner window of slot s (column), row r (0: i0, 1: i0 + 1), term t
@@ -736,27 +772,32 @@ __global__ __launch_bounds__(256, 2) void k_msh_moments(int nm, int nm3p, MomLay
             }
         }
         // FRF rows -> V, Y, H2, H3 of the item's points; (ti, tj)
-        for (int ql = sq0; ql < nb; ql += 256 / kVY) {
-            const float2 *h = Hraw + ql * hs;
-            if (svy) {
-                const float w = h[3 * nm].x;
-                const int jg = jg0 + sjl;
-                const float2 h1 = h[sm], h2 = h[nm + sm];
-                const float2 h1j = h[jg], h3j = h[2 * nm + jg];
-                // V = w H1(m) conj H3(j'),  Y = w H1(j') H2(m)
-                VY[ql][st] = make_float4(w * (h1.x * h3j.x + h1.y * h3j.y), w * (h1j.x * h2.x - h1j.y * h2.y),
-                                         w * (h1.y * h3j.x - h1.x * h3j.y), w * (h1j.x * h2.y + h1j.y * h2.x));
+        // (V, Y by a and H3 by a for the block's own a-rows only: the blocks of one j' share the rest)
+        if (svy || st < nm)
+            for (int ql = sq0; ql < nb; ql += 256 / kVY) {
+                const float2 *h = Hraw + ql * hs;
+                if (svy) {
+                    const float w = h[3 * nm].x;
+                    const int jg = jg0 + sjl;
+                    const float2 h2 = h[nm + sm], h1j = h[jg];
+                    // Y = w H1(j') H2(m),  V = w H1(m) conj H3(j')
+                    const float yr = w * (h1j.x * h2.x - h1j.y * h2.y), yi = w * (h1j.x * h2.y + h1j.y * h2.x);
+                    Ys[ql][st] = make_float2(yr, yi);
+                    if (sown) {
+                        const float2 h1 = h[sm], h3j = h[2 * nm + jg];
+                        VY[ql][st] = make_float4(w * (h1.x * h3j.x + h1.y * h3j.y), yr, w * (h1.y * h3j.x - h1.x * h3j.y), yi);
+                    }
+                }
+                if (st < nm) {
+                    const float2 h2 = h[nm + st], h3 = h[2 * nm + st];
+                    H23[ql][st] = make_float4(h2.x, h3.x, -h2.y, h3.y);
+                    if (sown3) H3s[ql][st] = h3;
+                }
             }
-            if (st < nm) {
-                const float2 h2 = h[nm + st], h3 = h[2 * nm + st];
-                H23[ql][st] = make_float4(h2.x, h3.x, -h2.y, h3.y);
-            }
-        }
         if (tid < nb) {
             const int qq = cur.q0 + tid, qr = qq / cur.nqj, qc = qq - qr * cur.nqj;
             const float ti = (float)qr * cur.rFi, tj = (float)qc * cur.rFj;
-            tq[tid] = make_ulonglong2(pk2(ti, ti), pk2(tj, tj));
-            tq2[tid] = pk2(ti * tj, ti * tj);
+            tq[tid] = make_float2(ti, tj);
         }
         // VY, H23 and tq ready; FRF rows and corners consumed, the item's fields read
         if (__syncthreads_or(!ok)) break;  // a copy did not arrive: leave with the error code set
@@ -765,18 +806,19 @@ __global__ __launch_bounds__(256, 2) void k_msh_moments(int nm, int nm3p, MomLay
         if (tid < 32 && nxt.valid) issue(nxt, tid);
         if (tid == 32) build(nxt, sit[(k + 2) % 3]);
         for (int ql = 0; ql < nb; ++ql) {
-            const ulonglong2 tt = tq[ql];
-            const f2x ti2 = tt.x, tj2 = tt.y, tij2 = tq2[ql];
+            const float2 tt = tq[ql];
+            const float ti = tt.x, tj = tt.y, tij = ti * tj;
+            const f2x ti2 = pk2(ti, ti), tj2 = pk2(tj, tj), tij2 = pk2(tij, tij);
             const ulonglong2 hb = H23p[ql][bb];  // {H2r(b), H3r(b)}, {-H2i(b), H3i(b)}
-            const float4 ybv = VY[ql][yb];       // .y, .w: Y_j'(b)
+            const float2 ybv = Ys[ql][yb];       // Y_j'(b)
             float f3[EPT];
 #pragma unroll
             for (int u = 0; u < EPT; ++u) {
                 const ulonglong2 va = VYp[ql][ia0 + u];  // {Vr(a), Yr(a)}, {Vi(a), Yi(a)}
-                const float4 h3a = H23[ql][ih0 + u];     // .y, .w: H3(a)
+                const float2 h3a = H3s[ql][ih0 + u];     // H3(a)
                 // {T1, T2} = {Re[H2(b) V_j'(a)], Re[Y_j'(a) conj H3(b)]}
                 const f2x f12 = fma2(hb.y, va.y, mul2(hb.x, va.x));
-                f3[u] = fmaf(ybv.w, h3a.w, ybv.y * h3a.y);  // T3 = Re[Y_j'(b) conj H3(a)]
+                f3[u] = fmaf(ybv.y, h3a.y, ybv.x * h3a.x);  // T3 = Re[Y_j'(b) conj H3(a)]
                 const f2x v = fma2(tij2, c12[u][3], fma2(tj2, c12[u][2], fma2(ti2, c12[u][1], c12[u][0])));
                 z12[u] = fma2(f12, v, z12[u]);
             }
@@ -784,7 +826,6 @@ __global__ __launch_bounds__(256, 2) void k_msh_moments(int nm, int nm3p, MomLay
                 const f2x v = fma2(tij2, c3p[3], fma2(tj2, c3p[2], fma2(ti2, c3p[1], c3p[0])));
                 z3p = fma2(pk2(f3[0], f3[1]), v, z3p);
                 if constexpr (EPT == 3) {
-                    const float ti = up2(ti2).x, tj = up2(tj2).x, tij = up2(tij2).x;
                     const float vs = fmaf(tij, c3s[3], fmaf(tj, c3s[2], fmaf(ti, c3s[1], c3s[0])));
                     z3s = fmaf(f3[EPT - 1], vs, z3s);
                 }
@@ -1051,8 +1092,8 @@ __global__ void k_fx_expand(int nz, const ZoneX *__restrict__ zx, const unsigned
             atomicCAS(err, 0, 8);
             fid = 0;
         }
-        ssrc[z.pbase + y] = fid;                                    // line order (line tasks)
-        ssrc[npts + z.pbase + (long long)j * z.ni + i] = fid;       // column order (column tasks)
+        ssrc[z.pbase + y] = fid;                                               // line order (line tasks)
+        ssrc[npts + z.pbase + y] = (int)(npts + z.pbase + (long long)j * z.ni + i);  // its place in column order
     }
     const long long nit = line_items + (long long)z.nj * MT * nic;
     for (long long y = threadIdx.x; y < nit; y += blockDim.x) {
@@ -1245,8 +1286,8 @@ int Engine::msh_mixed_batch(const std::vector<ZoneDev> &zs, std::vector<double> 
                 const double r = z.fi0 + i * z.dIi;
                 for (int j = 0; j < z.nj; ++j) {
                     const int row = F.at(r + (z.fj0 + j * z.dJj));
-                    ssrc[pb + (size_t)i * z.nj + j] = row;         // line order (kind 0)
-                    ssrc[npts + pb + (size_t)j * z.ni + i] = row;  // column order (kind 1)
+                    ssrc[pb + (size_t)i * z.nj + j] = row;  // line order (kind 0), and its place in column order (kind 1)
+                    ssrc[npts + pb + (size_t)i * z.nj + j] = (int)(npts + pb + (size_t)j * z.ni + i);
                 }
                 tasks.push_back(Task{UF.at(r) * Mp, (int)gb * NMT, (int)(pb + (long long)i * z.nj) * NMT, z.nj,
                                      (int)(pb + (long long)i * z.nj), 1, 0});
@@ -1348,9 +1389,9 @@ int Engine::msh_mixed_batch(const std::vector<ZoneDev> &zs, std::vector<double> 
         };
         k_prep_u_rows<<<dim3(nU, Kp / 32), 256, 0, stream>>>(nm, K, Kp, Mp, d_usrc, dA32.as<float>(), dQ.as<double>(),
                                                              Uh, Ul);
-        k_prep_b_rows<<<dim3((unsigned)ncol, Kp / 64), 256, 0, stream>>>(nm, NMT, K, Kp, d_gsrc, dA32.as<float>(), Gh,
+        k_prep_b_rows<<<dim3((unsigned)ncol, Kp / 64), 256, 0, stream>>>(nm, NMT, K, Kp, d_gsrc, nullptr, dA32.as<float>(), Gh,
                                                                          Gl);
-        k_prep_b_rows<<<dim3((unsigned)(2 * npts), Kp / 64), 256, 0, stream>>>(nm, NMT, K, Kp, d_ssrc, dA32.as<float>(),
+        k_prep_b_rows<<<dim3((unsigned)npts, Kp / 64), 256, 0, stream>>>(nm, NMT, K, Kp, d_ssrc, d_ssrc + npts, dA32.as<float>(),
                                                                                Sh, Sl);
         cudaError_t r = mark(evg0);
         if (r) return r;
