@@ -289,18 +289,21 @@ __global__ void k_e_reduce(int nm, int W, int MT, int grid, const double *__rest
     const int nm3 = nm * nm * nm;
     const int xe = x < nm3 ? x : 0;
     const int m = xe % nm, n = (xe / nm) % nm, o = xe / (nm * nm);
-    auto sum = [&](int kind, int a, int b, int j) {
+    auto at = [&](int kind, int a, int b, int j) {  // one loop over the CTAs of a row tile, as k_mixed_reduce
         const int R = a * nm + b, mtile = R / 128, lane = R % 128;
-        double s = 0.0;
-#pragma unroll 4
-        for (int g = mtile + MT * threadIdx.y; g < grid; g += MT * kRedLanes)
-            s += part[(((size_t)g * kKinds + kind) * W + j) * 128 + lane];
-        return s;
+        return part + (((size_t)mtile * kKinds + kind) * W + j) * 128 + lane;
     };
-    double mr = sum(0, m, n, o) + sum(1, m, o, n) + sum(3, o, n, m) + sum(4, n, o, m) + sum(6, n, m, o) +
-                      sum(7, o, m, n);
-    double mf = sum(2, m, n, o) + sum(2, m, o, n) + sum(5, o, n, m) + sum(5, n, o, m) + sum(8, n, m, o) +
-                      sum(8, o, m, n);
+    const double *p[12] = {at(0, m, n, o), at(1, m, o, n), at(3, o, n, m), at(4, n, o, m), at(6, n, m, o), at(7, o, m, n),
+                           at(2, m, n, o), at(2, m, o, n), at(5, o, n, m), at(5, n, o, m), at(8, n, m, o), at(8, o, m, n)};
+    const size_t step = (size_t)MT * kKinds * W * 128;
+    double mr = 0.0, mf = 0.0;
+    for (int i = threadIdx.y; i < grid / MT; i += kRedLanes) {
+        double v[12];
+#pragma unroll
+        for (int q = 0; q < 12; ++q) v[q] = p[q][i * step];
+        mr += ((v[0] + v[1]) + (v[2] + v[3])) + (v[4] + v[5]);
+        mf += ((v[6] + v[7]) + (v[8] + v[9])) + (v[10] + v[11]);
+    }
     red_lanes(mr, mf);
     if (threadIdx.y == 0 && x < nm3) {
         m3mr[x] = 2.0 * mr;  // B_F = 2 (T1 + T2 + T3)
