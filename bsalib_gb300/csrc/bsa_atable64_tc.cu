@@ -215,7 +215,7 @@ __global__ __launch_bounds__(256) void k_wdigits(int ntc, int n, int nm, int np,
 #pragma unroll
     for (int i = 0; i < 16; ++i)
         v[i] = (some && k0 + i < n) ? rootS[(size_t)fc * n + k0 + i] * L[((size_t)itc * n + k0 + i) * nm + m] : 0.0;
-    put_digits(v, some ? e : 0, D + ((size_t)blk * kDig * bw + col) * Kp + k0, (size_t)bw * Kp);
+    put_digits<16>(v, some ? e : 0, D + ((size_t)blk * kDig * bw + col) * Kp + k0, (size_t)bw * Kp);
 }
 
 template <int NP>

@@ -39,11 +39,12 @@ __device__ __forceinline__ void digits_of(unsigned long long x, uint32_t *f) {
     }
 }
 
-// Sixteen values of one row, scaled by 2^(55 - e), as digits: dst[s plane + 0 .. 15].
+// NV (8 or 16) values of one row, scaled by 2^(55 - e), as digits: dst[s plane + 0 .. NV - 1].
+template <int NV>
 __device__ __forceinline__ void put_digits(const double *v, int e, __nv_bfloat16 *dst, size_t plane) {
-    uint32_t w[kDig][8];
+    uint32_t w[kDig][NV / 2];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < NV / 2; ++q) {
         uint32_t f[2][kDig];
 #pragma unroll
         for (int z = 0; z < 2; ++z) {
@@ -62,8 +63,8 @@ __device__ __forceinline__ void put_digits(const double *v, int e, __nv_bfloat16
 #pragma unroll
     for (int s = 0; s < kDig; ++s) {
         uint4 *o = reinterpret_cast<uint4 *>(dst + s * plane);
-        o[0] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
-        o[1] = make_uint4(w[s][4], w[s][5], w[s][6], w[s][7]);
+#pragma unroll
+        for (int z = 0; z < NV / 8; ++z) o[z] = make_uint4(w[s][4 * z], w[s][4 * z + 1], w[s][4 * z + 2], w[s][4 * z + 3]);
     }
 }
 

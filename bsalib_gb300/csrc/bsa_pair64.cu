@@ -48,6 +48,7 @@ namespace p64 {
 constexpr int kKT = 16;
 constexpr int kKinds = 9;           // K1 .. K6 (the order above: abj, ajb, baj, jba, jab, bja), M1, M2, M3
 constexpr int kBatch = 8;           // pairs a thread takes between two barriers
+constexpr int kRow = 10;            // doubles of a row's factors
 
 // E of one product tile, or of a quarter of its rows: 256 threads, ROWS / 32 x 4 elements each, K staged
 // 16 at a time; the row operand Q[k][a] A(x)[k][b] is formed while staging.  FP64-pipe bound (one
@@ -170,14 +171,16 @@ __device__ __forceinline__ PairInfo pair_info(int x, int y, int N, int vect) {
 
 // One block per (tile of RT rows (a, b), group of pairs); a thread holds one element (a, b, j) and
 // takes the pairs of its lane.  Per batch of PB pairs: the pairs and weights, then the
-// products of the row factors (8 doubles a row) and the columns' FRF values in shared memory, then
-// 9 (all weights one), 14 (no sums on the grid) or 27 FP64 operations an element and pair.
+// products of the row factors (10 doubles a row) and the columns' FRF values in shared memory, then
+// 9 (all weights one), 13 (no sums on the grid) or 27 FP64 operations an element and pair.  Bound by
+// the FP64 pipe (84 % busy): 2145 pairs of 24 modes 0.88 ms, the sums of row factors formed
+// once a row.
 __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
     extern __shared__ double sm[];
     const int t = threadIdx.x, nm = c.an, nm2 = nm * nm;
     const int PB = P.PB, RT = P.RT, EL = RT * nm;
-    double *rowf = sm;                                 // [PB][RT][8]
-    double2 *colf = (double2 *)(rowf + (size_t)PB * RT * 8);  // [PB][nm][3]: Hx, P, D
+    double *rowf = sm;                                 // [PB][RT][kRow]
+    double2 *colf = (double2 *)(rowf + (size_t)PB * RT * kRow);  // [PB][nm][3]: Hx, P, D
     PairInfo *info = (PairInfo *)(colf + (size_t)PB * nm * 3);
     const int pl = t / EL, el = t - pl * EL;
     const int rl = el / nm, j = el - rl * nm, ab = blockIdx.x * RT + rl;
@@ -224,7 +227,7 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
             const int a = rr / nm, b = rr - a * nm, x = info[s].x, y = info[s].y;
             const double2 xa = P.H[(size_t)x * nm + a], ya = P.H[(size_t)y * nm + a], yb = P.H[(size_t)y * nm + b];
             const double2 pb = P.H[(size_t)min(x + y, 2 * P.N) * nm + b], db = P.H[(size_t)(y - x) * nm + b];
-            double *o = rowf + (size_t)q * 8;
+            double *o = rowf + (size_t)q * kRow;
             o[0] = xa.x * yb.x - xa.y * yb.y;  // q1 = Hx_a Hy_b
             o[1] = xa.x * yb.y + xa.y * yb.x;
             o[2] = xa.x * yb.x + xa.y * yb.y;  // q2 = Hx_a conj Hy_b
@@ -233,6 +236,8 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
             o[5] = ya.y * pb.x - ya.x * pb.y;
             o[6] = ya.x * db.x + ya.y * db.y;  // d = Hy_a conj D_b
             o[7] = ya.y * db.x - ya.x * db.y;
+            o[8] = o[4] + o[6];
+            o[9] = o[7] - o[5];
         }
         __syncthreads();
         if (live) {
@@ -241,7 +246,7 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
                 const int s = u * P.PL + pl;
                 if (s >= np) continue;
                 const PairInfo &f = info[s];
-                const double *o = rowf + ((size_t)s * RT + rl) * 8;
+                const double *o = rowf + ((size_t)s * RT + rl) * kRow;
                 const double2 *h = colf + ((size_t)s * nm + j) * 3;
                 const double2 hx = h[0], hp = h[1], hd = h[2];
                 const double v = e[u];
@@ -249,7 +254,7 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
                 if (f.region == 0) {
                     const double ab_ = fma(o[0], hp.x, fma(o[1], hp.y, beta));
                     // gamma + delta
-                    const double gd = fma(o[4] + o[6], hx.x, (o[7] - o[5]) * hx.y);
+                    const double gd = fma(o[8], hx.x, o[9] * hx.y);
                     Kc = fma(v, ab_, Kc);
                     Kd = fma(v, gd, Kd);
                     Mc += v;
@@ -261,7 +266,6 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
                     K56 = fma(v, beta, K56);
                     K2 = fma(v, gd, K2);
                     K34 = fma(v, dl, K34);
-                    M1 = fma(v, 2.0, M1);
                     M23 += v;
                 } else {
                     const double al = fma(o[0], hp.x, o[1] * hp.y);
@@ -283,7 +287,7 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
         }
     }
     double k[kKinds] = {K1 + Kc,         K2 + Kd,         K3 + Kd + K34,       K4 + Kd + K34,      K5 + Kc + K56,
-                        K6 + Kc + K56,   M1 + 2.0 * Mc,   M2 + 2.0 * Mc + M23, M3 + 2.0 * Mc + M23};
+                        K6 + Kc + K56,   M1 + 2.0 * (Mc + M23), M2 + 2.0 * Mc + M23, M3 + 2.0 * Mc + M23};
     // lanes of one element, then the block's partial
     double *red = sm;
 #pragma unroll
@@ -370,14 +374,24 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     cudaError_t e;
     auto ylast = [&](int x) { return analytic ? std::min(hi, x + N) : N; };  // last partner of first row x
     const long long pairs_all = (long long)(N + 1) * (N + 2) / 2 + (analytic ? (long long)N * (N + 1) / 2 : 0);
-    // moment kernel: rows of a block, pair lanes, groups (about four blocks an SM; a group holds at
-    // least one batch of pairs)
+    // moment kernel: rows of a block, pair lanes, pairs of a batch (fewer for small grids, so that the
+    // groups still fill the chip) and groups: one wave of resident blocks (a third wave of a few blocks
+    // cost 0.3 of 1.1 ms)
     const int RT = std::max(1, std::min(rx, 256 / nm)), PL = std::max(1, std::min(8, 256 / (RT * nm)));
     const int tiles = (rx + RT - 1) / RT;
-    // pairs of a batch: fewer for small grids, so that the groups still fill the chip
-    const long long want = (608 + tiles - 1) / tiles;
+    auto smem_of = [&](int PB) {
+        return std::max((size_t)256 * sizeof(double), sizeof(double) * (size_t)PB * RT * kRow +
+                        sizeof(double2) * (size_t)PB * nm * 3 + sizeof(PairInfo) * (size_t)PB);
+    };
+    int dev = 0, nsm = 0, occ = 1;
+    if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) ||
+        (e = cudaFuncSetAttribute(k_pair_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(kBatch * PL))) ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pair_moments, 256, smem_of(kBatch * PL))))
+        return cuda_fail(e, "pair moments kernel");
+    const long long want = std::max(1, std::max(1, occ) * nsm / tiles);
     const int PB = PL * (int)std::max(1LL, std::min<long long>(kBatch, pairs_all / (want * PL)));
     const int G = diag ? std::min(64, (N + 8) / 8) : (int)std::max(1LL, std::min(want, (pairs_all + PB - 1) / PB));
+    const size_t smem = smem_of(PB);
     // Products on the tensor cores (bsa_pair64_tc.cu) where they outweigh the digits' preparation.
     // Measured contraction, FP64 pipe / tensor cores: 4.1e6 FMAs, K = 30: 0.097 / 0.108 ms; 7.3e6,
     // K = 60: 0.126 / 0.109; 1.9e7, K = 20: 0.137 / 0.167; 5.4e7, K = 12: 0.353 / 0.447; 6.9e7,
@@ -440,10 +454,6 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     if ((e = cudaEventRecord(ev2, stream)) || (e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
     const int nh = (2 * N + 1) * nm;
     k_frf_rows<<<(nh + 127) / 128, 128, 0, stream>>>(2 * N + 1, nm, df, frf(), dMixH.as<double2>());
-    const size_t smem = std::max((size_t)256 * sizeof(double), sizeof(double) * (size_t)PB * RT * 8 +
-                                 sizeof(double2) * (size_t)PB * nm * 3 + sizeof(PairInfo) * (size_t)PB);
-    if (!diag && (e = cudaFuncSetAttribute(k_pair_moments, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
-        return cuda_fail(e, "pair moments kernel");
     if (tensor && ((e = cudaMemsetAsync(dFlag.as<int>() + 1, 0, sizeof(int), stream)) ||
                    (e = tc_prep_cols(stream, hi + 1, an, K, A, dMixB.p))))
         return cuda_fail(e, "pair product operands");

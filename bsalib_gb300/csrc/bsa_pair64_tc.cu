@@ -17,7 +17,7 @@
 // rows), so A digit s meets B digits 0 .. 7 - s in one MMA of N = (8 - s) 32 whose columns land on
 // levels s .. 7: 8 MMAs a K step instead of 36, and 512 TMEM columns hold two tiles.
 // 400 nodes x 2 components, 24 modes, 65 rows: FP64 pipe 40.5 ms; 1.33 ms here (8.5e11 digit FMAs,
-// 0.65 of the bf16 rate), row digits 0.35 ms.
+// 0.65 of the bf16 rate), row digits 0.11 ms.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -95,7 +95,7 @@ __global__ __launch_bounds__(256) void k_col_digits(int nr, int an, int K, int K
     double v[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = (some && k0 + i < K) ? A[((size_t)y * K + k0 + i) * an + j] : 0.0;
-    put_digits(v, some ? e : 0, D + ((size_t)ct * kDig * kTN + col) * Kp + k0, (size_t)kTN * Kp);
+    put_digits<16>(v, some ? e : 0, D + ((size_t)ct * kDig * kTN + col) * Kp + k0, (size_t)kTN * Kp);
 }
 
 // Column digits of a pair list [block][digit][bw columns][Kp]; exponents [block][32].
@@ -112,33 +112,39 @@ __global__ __launch_bounds__(256) void k_block_digits(int nm, int np, int bw, in
     double v[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = (some && k0 + i < K) ? A[((size_t)y * K + k0 + i) * nm + j] : 0.0;
-    put_digits(v, some ? e : 0, D + ((size_t)blk * kDig * bw + col) * Kp + k0, (size_t)bw * Kp);
+    put_digits<16>(v, some ? e : 0, D + ((size_t)blk * kDig * bw + col) * Kp + k0, (size_t)bw * Kp);
 }
 
-// Row digits [mt][digit][128 rows][Kp]; block: one x, 64 k, every (a, b).
+// Row digits [mt][digit][128 rows][Kp]; block: one x, 64 k, every (a, b).  Eight lanes cover a row's 64 k,
+// so that a warp's store of a digit is four whole 128-byte rows (16 bytes a row at a time, 32 rows a
+// store, ran at 1.3 TB/s: 0.36 ms for 65 x 576 rows of 800 k, now 0.11 ms).
 __global__ __launch_bounds__(256) void k_row_digits(Chunk c, int Kp, const double *__restrict__ A,
                                                     const double *__restrict__ Q, const int *__restrict__ er,
                                                     __nv_bfloat16 *__restrict__ D) {
-    extern __shared__ double sm[];
+    constexpr int LD = 66;  // [mode][64 k] with 16-byte aligned, staggered rows
+    extern __shared__ __align__(16) double sm[];
     const int qn = c.qn, an = c.an, rx = c.rx(), K = c.K, xl = blockIdx.x, kb = blockIdx.y * 64;
-    double *As = sm, *Qs = sm + 64 * an;
+    double *As = sm, *Qs = sm + LD * an;
     const int n = max(0, min(64, K - kb));
     const double *a = A + ((size_t)(c.xmap ? c.xmap[xl] : c.x0 + xl) * K + kb) * an, *q = Q + (size_t)kb * qn;
-    for (int i = threadIdx.x; i < 64 * an; i += 256) As[i] = i < n * an ? a[i] : 0.0;
-    for (int i = threadIdx.x; i < 64 * qn; i += 256) Qs[i] = i < n * qn ? q[i] : 0.0;
+    for (int i = threadIdx.x; i < 64 * an; i += 256) As[i % an * LD + i / an] = i < n * an ? a[i] : 0.0;
+    for (int i = threadIdx.x; i < 64 * qn; i += 256) Qs[i % qn * LD + i / qn] = i < n * qn ? q[i] : 0.0;
     __syncthreads();
-    for (int w = threadIdx.x; w < rx * 4; w += 256) {
-        const int kq = w / rx, ab = w - kq * rx, ia = ab / an, ib = ab - ia * an;
+    const int kq = (threadIdx.x & 7) * 8;
+    for (int ab = threadIdx.x >> 3; ab < rx; ab += 32) {
+        const int ia = ab / an, ib = ab - ia * an;
         const long long r = (long long)xl * c.rpad + ab;
         const int e = er[r];
         const bool some = e != kNone && e != kBad;
-        double v[16];
+        const double2 *pa = reinterpret_cast<const double2 *>(As + ib * LD + kq), *pq = reinterpret_cast<const double2 *>(Qs + ia * LD + kq);
+        double v[8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int k = kq * 16 + i;
-            v[i] = some ? Qs[k * qn + ia] * As[k * an + ib] : 0.0;
+        for (int i = 0; i < 4; ++i) {
+            const double2 u = pa[i], w = pq[i];
+            v[2 * i] = some ? w.x * u.x : 0.0;
+            v[2 * i + 1] = some ? w.y * u.y : 0.0;
         }
-        put_digits(v, some ? e : 0, D + ((r / kTM) * kDig * kTM + r % kTM) * (size_t)Kp + kb + kq * 16, (size_t)kTM * Kp);
+        put_digits<8>(v, some ? e : 0, D + ((r / kTM) * kDig * kTM + r % kTM) * (size_t)Kp + kb + kq, (size_t)kTM * Kp);
     }
 }
 
@@ -389,7 +395,7 @@ static cudaError_t products(cudaStream_t st, const Chunk &c, const PairList &l, 
     const int Kp = kpad(c.K), nx = c.x1 - c.x0;
     int *er = (int *)((char *)rows + up256(ntiles * kDig * kTM * Kp * 2));
     k_row_exp<<<dim3(nx, (c.rx() + 31) / 32), 256, 0, st>>>(c, A, Q, er);
-    const size_t sm = sizeof(double) * 64 * (c.qn + c.an);
+    const size_t sm = sizeof(double) * 66 * (c.qn + c.an);
     cudaError_t e = cudaFuncSetAttribute(k_row_digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
     k_row_digits<<<dim3(nx, Kp / 64), 256, sm, st>>>(c, Kp, A, Q, er, (__nv_bfloat16 *)rows);
