@@ -675,7 +675,11 @@ int Engine::batch_add(int *id) {
     c.K = K;
     c.trunc = classic_trunc;
     c.modes = modes;
-    c.hL = hL; c.hQ = hQ; c.hCorr = hCorr; c.hNodes = hNodes; c.hNn = hNn; c.hM = hM; c.hK = hK; c.hC = hC; c.hWd3 = hWd3; c.hWd2 = hWd2;
+    c.hL = hL; c.hQ = hQ; c.hCorr = hCorr;
+    if (c.hCorr.empty())  // the caller's arrays may be gone when the sweep runs
+        for (int tc : set.tc)
+            c.hCorr.insert(c.hCorr.end(), in.corr + (size_t)in.ncorr * (tc - 1), in.corr + (size_t)in.ncorr * tc);
+    c.hNodes = hNodes; c.hNn = hNn; c.hM = hM; c.hK = hK; c.hC = hC; c.hWd3 = hWd3; c.hWd2 = hWd2;
     c.hL32 = hL32; c.hPsd = hPsd;
     g_batch.push_back(std::move(c));
     if (id) *id = (int)g_batch.size() - 1;

@@ -127,7 +127,7 @@ struct Engine {
     };
     Inputs in;
     Settings set;
-    bool inited = false, halted = false, derived_ok = false, dev_uploaded = false;
+    bool inited = false, halted = false, derived_ok = false, dev_uploaded = false, coh_uploaded = false;
     std::string last_error;
     int precision = 0;          // BSA_PREC_FP64
     bool classic_trunc = true;  // S(f1+f2) beyond the classic grid reads zero
@@ -166,7 +166,7 @@ struct Engine {
     std::vector<int> modes;
     int nme = 0, K = 0;
     std::vector<double> phitc, hL, hQ, hM, hK, hC;
-    std::vector<double> hCorr;         // packed coherences of the components [comp][ncorr]; log c_ij formed on the device
+    std::vector<double> hCorr;         // packed coherences [comp][hNn (hNn + 1) / 2], or empty: the caller's array
     std::vector<int> hNodes;           // loaded nodes
     int hNn = 0;                       // nodes the packing counts
     std::vector<unsigned char> hPack;  // the derived tables as they go to the device, in one copy
@@ -177,10 +177,10 @@ struct Engine {
     // device
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
-    DevView dL, dQ, dPsdPar, dFrfM, dFrfK, dFrfC, dWd3, dWd2, dL32;  // parts of dProb
+    DevView dNodes, dL, dQ, dPsdPar, dFrfM, dFrfK, dFrfC, dWd3, dWd2, dL32;  // parts of dProb
     DevBuf dProb, dLogc, dFreq, dS, dA, dPartF, dPartR, dOut, dPsdF, dWf, dPts,
         dPtsD, dBF, dBR, dMixA, dMixB, dMixH, dMixPart, dA32, dZones, dZidx, dMshT, dMshIdx, dLogc32,
-        dPod, dFlag, dSlot, dHash, dCptr, dCq, dZoneH, dZoff;
+        dPod, dFlag, dSlot, dHash, dCptr, dCq, dZoneH, dZoff, dCorr;
 
     // stats
     double last_ms = 0, last_ms_contraction = 0, last_ms_gemm = 0, last_points = 0;
@@ -196,6 +196,7 @@ struct Engine {
     int ensure_stream();
     int validate();
     int upload_problem();
+    int upload_coherence();
     FrfPar frf() const;
     // msh: the table serves the Mesher functions, whose POD form may be truncated
     int build_atable(const std::vector<double> &freqs, bool fp32 = false, bool msh = false);

@@ -158,7 +158,7 @@ void Engine::free_device() {
     if (stream) cudaStreamSynchronize(stream);  // the blocks go back to the cache for reuse
     for (DevBuf *b : {&dProb, &dLogc, &dFreq, &dS, &dA, &dPartF, &dPartR,
                       &dOut, &dPsdF, &dWf, &dPts, &dPtsD, &dBF, &dBR, &dMixA, &dMixB, &dMixH, &dMixPart, &dA32,
-                      &dZones, &dZidx, &dMshT, &dMshIdx, &dLogc32, &dPod, &dFlag, &dSlot, &dHash, &dCptr, &dCq, &dZoneH, &dZoff})
+                      &dZones, &dZidx, &dMshT, &dMshIdx, &dLogc32, &dPod, &dFlag, &dSlot, &dHash, &dCptr, &dCq, &dZoneH, &dZoff, &dCorr})
         b->release();
     if (stream) cudaStreamDestroy(stream);
     stream = nullptr;
@@ -283,11 +283,10 @@ int Engine::validate() {
     const long ncorr = (long)I.ncorr;
     hNodes.assign(I.n_load, I.n_load + nnl);
     hNn = I.nn;
-    if (I.nn <= 2 * nnl) {  // the whole packed triangle is at most twice the loaded nodes' square
-        hCorr.resize((size_t)ntc * ncorr);
-        for (int itc = 0; itc < ntc; ++itc)
-            std::memcpy(hCorr.data() + (size_t)itc * ncorr, I.corr + (size_t)ncorr * (set.tc[itc] - 1), sizeof(double) * ncorr);
-    } else {  // few of many nodes loaded: their own packed triangle
+    hCorr.clear();
+    if (I.nn > 2 * nnl) {
+        // few of many nodes loaded: their own packed triangle (else the caller's is at most twice the loaded
+        // nodes' square and goes to the device from where it is, if a table needs it: upload_coherence)
         const size_t nc = (size_t)nnl * (nnl + 1) / 2;
         hCorr.resize(ntc * nc);
         for (int itc = 0; itc < ntc; ++itc) {
@@ -340,13 +339,10 @@ int Engine::upload_problem() {
     if ((rc = ensure_stream())) return rc;
     if (dev_uploaded) return BSA_OK;
     cudaError_t e;
-    const int ntc = (int)set.tc.size(), nnl = (int)hNodes.size();
-    const size_t ncoh = (size_t)ntc * nnl * nnl;
     // one copy for all tables (eleven small ones cost 60 us of launches)
-    DevView corr, nodes;
     struct Part { const void *src; size_t bytes; DevView *dst; };
     auto part = [](const auto &v, DevView &d) { return Part{v.data(), sizeof(v[0]) * v.size(), &d}; };
-    const Part parts[] = {part(hCorr, corr), part(hNodes, nodes), part(hL, dL), part(hQ, dQ), part(hPsd, dPsdPar), part(hM, dFrfM),
+    const Part parts[] = {part(hNodes, dNodes), part(hL, dL), part(hQ, dQ), part(hPsd, dPsdPar), part(hM, dFrfM),
                           part(hK, dFrfK), part(hC, dFrfC), part(hWd3, dWd3), part(hWd2, dWd2), part(hL32, dL32)};
     size_t total = 0;
     for (const Part &p : parts) total += (p.bytes + 255) & ~(size_t)255;
@@ -358,15 +354,33 @@ int Engine::upload_problem() {
         p.dst->p = (char *)dProb.p + at;
         at += (p.bytes + 255) & ~(size_t)255;
     }
-    if ((e = upload(dProb, hPack, stream)) || (e = dLogc.reserve(log_coh_bytes(ncoh))) ||
+    if ((e = upload(dProb, hPack, stream))) return cuda_fail(e, "uploading problem data");
+    dev_uploaded = true;
+    coh_uploaded = false;
+    return BSA_OK;
+}
+
+// The coherence table log c (FP64 and FP32), on the first use by an A table: the diagonal-only spectra
+// never read it (0.2 ms of a 400-node, two-component analysis).
+int Engine::upload_coherence() {
+    if (coh_uploaded) return BSA_OK;
+    const int ntc = (int)set.tc.size(), nnl = (int)hNodes.size();
+    const size_t ncoh = (size_t)ntc * nnl * nnl, nc = (size_t)hNn * (hNn + 1) / 2;
+    cudaError_t e;
+    if ((e = dCorr.reserve(sizeof(double) * ntc * nc)) || (e = dLogc.reserve(log_coh_bytes(ncoh))) ||
         (e = dLogc32.reserve(sizeof(float) * ncoh)))
-        return cuda_fail(e, "uploading problem data");
-    // log c in FP64 and its FP32 copy
-    if ((e = launch_log_coh(stream, ntc, nnl, hNn, (long long)(hCorr.size() / ntc), nodes.as<int>(), corr.as<double>(),
-                            dLogc.as<double>(), dLogc32.as<float>())))
+        return cuda_fail(e, "uploading coherences");
+    for (int itc = 0; itc < ntc; ++itc) {
+        const double *src = hCorr.empty() ? in.corr + (size_t)in.ncorr * (set.tc[itc] - 1) : hCorr.data() + itc * nc;
+        if ((e = cudaMemcpyAsync(dCorr.as<double>() + itc * nc, src, sizeof(double) * nc, cudaMemcpyHostToDevice, stream)))
+            return cuda_fail(e, "uploading coherences");
+    }
+    h2d += (double)(sizeof(double) * ntc * nc);
+    if ((e = launch_log_coh(stream, ntc, nnl, hNn, (long long)nc, dNodes.as<int>(), dCorr.as<double>(), dLogc.as<double>(),
+                            dLogc32.as<float>())))
         return cuda_fail(e, "coherence table");
     kernels += 1;
-    dev_uploaded = true;
+    coh_uploaded = true;
     return BSA_OK;
 }
 
@@ -404,8 +418,10 @@ int Engine::build_atable(const std::vector<double> &freqs, bool fp32, bool msh) 
 int Engine::build_atable_dev(int nf, bool fp32, int f0) {
     const int ntc = (int)set.tc.size();
     cudaError_t e;
+    int rc = upload_coherence();
+    if (rc) return rc;
     // the FP64 table reads sqrt(S) and the exponential's table behind log c
-    int rc = build_psd_dev(nf, fp32, fp32 ? nullptr : dLogc.as<double>() + (size_t)ntc * in.nnl * in.nnl, f0);
+    rc = build_psd_dev(nf, fp32, fp32 ? nullptr : dLogc.as<double>() + (size_t)ntc * in.nnl * in.nnl, f0);
     if (rc) return rc;
     if (fp32) {
         // FP32 table on the tensor cores (tf32 hi/lo split, FP32-level accuracy)

@@ -136,7 +136,7 @@ int Engine::pod_atable(const std::vector<double> &freqs, bool fp32) {
     Solver &sv = solver();
     if (!sv.load()) return fail(BSA_ERR_UNSUPPORTED, "truncated POD needs cuSOLVER (libcusolver), which could not be loaded");
     int rc = build_psd(freqs);  // nodal PSD table S[f][comp][node] into dS
-    if (rc) return rc;
+    if (rc || (rc = upload_coherence())) return rc;
     cudaError_t e;
     if (sv.set_stream(sv.h, stream) != CUSOLVER_STATUS_SUCCESS) return fail(BSA_ERR_CUDA, "cusolverDnSetStream failed");
     int lwork = 0;

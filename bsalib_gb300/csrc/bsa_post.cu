@@ -187,7 +187,7 @@ int Engine::br_decomp(const double *m2mf, double *bkg, double *res) {
                     in.phi[(size_t)(skip + in.libs_load[l] - 1) + (size_t)ndofs * (modes[im] - 1)];
     }
     cudaError_t e;
-    if ((rc = build_psd(fm))) return rc;
+    if ((rc = build_psd(fm)) || (rc = upload_coherence())) return rc;
     if ((e = upload(dMixA, aw, stream)) || (e = upload(dMixB, ph, stream)) || (e = dOut.reserve(sizeof(double) * nme)))
         return cuda_fail(e, "BR decomposition upload");
     post::k_br_sfm<<<nme, 256, 0, stream>>>(nme, ntc, nnl, nl, dFreq.as<double>(), dS.as<double>(), dLogc.as<double>(),
