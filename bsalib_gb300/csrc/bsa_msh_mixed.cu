@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -380,6 +381,7 @@ struct ZoneM {
     double fi0, fj0, dI, dJ, wI, wJ, sym;
     int ni, nj, Fi, Fj;
     int pbase, cbase, qbase;
+    int sg;    // +1, or -1: point (i, j) is tensor pbase - (i nj + j) (the zone mirrors an evaluated one)
     float wb;  // sym wI wJ rounded once: the BFM-lattice trapezoid weight of an interior point
 };
 
@@ -491,6 +493,7 @@ struct MomItem {
     // previous cell's right column, still staged (the next cell of a zone row)
     int cl, reuse;
     long long qbase, P00;
+    int sg;  // the zone's: corner (r, c) is BFM point P00 + sg (r nj + c)
     float wp[4];  // BFM lattice trapezoid weights of the corners the cell owns
     float rFi, rFj;
 };
@@ -518,7 +521,8 @@ __device__ __forceinline__ void mom_fill(const ZoneM *__restrict__ zones, int z,
     it.cl = 0;
     it.reuse = 0;
     it.qbase = Z.qbase;
-    it.P00 = (long long)Z.pbase + (long long)i0 * nj + j0;
+    it.sg = Z.sg;
+    it.P00 = (long long)Z.pbase + Z.sg * ((long long)i0 * nj + j0);
     const int ci[4] = {i0, i0, i0 + 1, i0 + 1}, cj[4] = {j0, j0 + 1, j0, j0 + 1};
     for (int k = 0; k < 4; ++k) {
         const bool own = (ci[k] == i0 || i0 == ni - 2) && (cj[k] == j0 || j0 == nj - 2);
@@ -660,7 +664,7 @@ __global__ __launch_bounds__(256, 2) void k_msh_moments(int nm, int nm3p, MomLay
     // warp 0: the copies of item it (one mbarrier phase) spread over its lanes: lane l < 16 the
     // FRF rows of the item's points on BRM lattice row r0 + l of the cell (at most 16 rows),
     // lanes 20-31 at a cell's first item the corner window (column, row, term) = lane - 20;
-    // corner (r, c) of the cell is BFM point P00 + r nj + c
+    // corner (r, c) of the cell is BFM point P00 + sg (r nj + c)
     auto issue = [&](const MomItem &it, int lane) {
         if (lane == 0) {
             uint32_t bytes = (uint32_t)it.nb * hs * 8;
@@ -679,7 +683,7 @@ __global__ __launch_bounds__(256, 2) void k_msh_moments(int nm, int nm3p, MomLay
             const int w = lane - 20, t = w >> 2, col = (w >> 1) & 1, r = w & 1;
             if (col >= it.reuse)
                 bulk_g2s(cwin(col == 0 ? it.cl : 1 - it.cl, r, t),
-                         Ts[t] + (size_t)(it.P00 + (long long)r * it.nj + col) * nm3p + win0, (uint32_t)wlen * 4, bar);
+                         Ts[t] + (size_t)(it.P00 + it.sg * ((long long)r * it.nj + col)) * nm3p + win0, (uint32_t)wlen * 4, bar);
         }
     };
     // thread 32: nx = the item after p; p's zone ends with p when nx is in another zone
@@ -871,10 +875,10 @@ __global__ void k_msh_zone_diag(int nm, size_t nm3p, const ZoneM *__restrict__ z
             const int qi = q / (NJ + 1), qj = q % (NJ + 1);
             const int i0 = min(qi / z.Fi, z.ni - 2), j0 = min(qj / z.Fj, z.nj - 2);
             const float ti = (float)(qi - i0 * z.Fi) / (float)z.Fi, tj = (float)(qj - j0 * z.Fj) / (float)z.Fj;
-            const size_t P00 = (size_t)z.pbase + (size_t)i0 * z.nj + j0, P01 = P00 + 1, P10 = P00 + z.nj,
-                         P11 = P10 + 1;
+            const long long o00 = (long long)i0 * z.nj + j0;
             float c[4];
-            const size_t P[4] = {P00, P01, P10, P11};
+            const size_t P[4] = {(size_t)(z.pbase + z.sg * o00), (size_t)(z.pbase + z.sg * (o00 + 1)),
+                                 (size_t)(z.pbase + z.sg * (o00 + z.nj)), (size_t)(z.pbase + z.sg * (o00 + z.nj + 1))};
 #pragma unroll
             for (int k = 0; k < 4; ++k)
                 c[k] = T1[P[k] * nm3p + em] + T3[P[k] * nm3p + em] + T2[P[k] * nm3p + em];
@@ -1177,17 +1181,50 @@ int Engine::msh_mixed_batch(const std::vector<ZoneDev> &zs, std::vector<double> 
     std::vector<ZoneX> zx;
     zm.reserve(zs.size());
     zx.reserve(zs.size());
-    for (const ZoneDev &z : zs) {
-        zm.push_back(ZoneM{z.fi0, z.fj0, z.dIi, z.dJj, z.wI, z.wJ, z.sym, z.ni, z.nj, z.Fi, z.Fj, (int)npts, (int)ncells,
-                           (int)nbrm, (float)(z.sym * z.wI * z.wJ)});
+    // B(-f1, -f2) = B(f1, f2), term by term and bit by bit (the tables hold |f|): a zone whose lattice is
+    // that of an earlier zone, or its mirror image through the origin, reads that zone's tensors.  A
+    // whole-plane layout has every zone twice (285 of the bridge deck's 285): half of the contraction.
+    auto line = [](const ZoneDev &z, int i) { return z.fi0 + i * z.dIi; };
+    auto colf = [](const ZoneDev &z, int j) { return z.fj0 + j * z.dJj; };
+    auto key = [](double f) { return std::llrint(std::fabs(f) * 1099511627776.0); };  // the tables' key
+    auto same = [&](const ZoneDev &u, const ZoneDev &v, bool mirror) {
+        for (int i = 0; i < u.ni; ++i) {
+            const int k = mirror ? u.ni - 1 - i : i;
+            if (key(line(u, i)) != key(line(v, k))) return false;
+            for (int j = 0; j < u.nj; ++j) {
+                const int l = mirror ? u.nj - 1 - j : j;
+                if (i == 0 && key(colf(u, j)) != key(colf(v, l))) return false;
+                if (key(line(u, i) + colf(u, j)) != key(line(v, k) + colf(v, l))) return false;
+            }
+        }
+        return true;
+    };
+    std::map<std::array<long long, 6>, std::vector<int>> seen;  // by sizes and corner frequencies, in either direction
+    const int nzones = (int)zs.size();
+    for (int k = 0; k < nzones; ++k) {
+        const ZoneDev &z = zs[k];
+        const long long r0 = key(line(z, 0)), r1 = key(line(z, z.ni - 1)), c0 = key(colf(z, 0)), c1 = key(colf(z, z.nj - 1));
+        std::vector<int> &cand = seen[{z.ni, z.nj, std::min(r0, r1), std::max(r0, r1), std::min(c0, c1), std::max(c0, c1)}];
+        int of = -1, sg = 1;
+        for (int c : cand) {
+            if (same(z, zs[c], true)) sg = -1;
+            else if (!same(z, zs[c], false)) continue;
+            of = c;
+            break;
+        }
+        const long long pb = of < 0 ? npts : sg > 0 ? zm[of].pbase : zm[of].pbase + (long long)z.ni * z.nj - 1;
+        zm.push_back(ZoneM{z.fi0, z.fj0, z.dIi, z.dJj, z.wI, z.wJ, z.sym, z.ni, z.nj, z.Fi, z.Fj, (int)pb, (int)ncells,
+                           (int)nbrm, sg, (float)(z.sym * z.wI * z.wJ)});
+        ncells += (long long)(z.ni - 1) * (z.nj - 1);
+        nbrm += (long long)((z.ni - 1) * z.Fi + 1) * ((z.nj - 1) * z.Fj + 1);
+        if (of >= 0) continue;
+        cand.push_back(k);
         zx.push_back(ZoneX{z.fi0, z.fj0, z.dIi, z.dJj, z.ni, z.nj, npts, (int)ncol, (int)ntasks, nitems});
         const long long ntl_l = (z.nj + NC - 1) / NC, ntl_c = (z.ni + NC - 1) / NC;
         nitems += (long long)z.ni * MT * ntl_l + (long long)z.nj * MT * ((ntl_c + 1) / 2);
         npts += (long long)z.ni * z.nj;
-        ncells += (long long)(z.ni - 1) * (z.nj - 1);
         ncol += z.nj;
         ntasks += z.ni + z.nj;
-        nbrm += (long long)((z.ni - 1) * z.Fi + 1) * ((z.nj - 1) * z.Fj + 1);
     }
     if (2 * npts * NMT > 0x7fffffffLL || nitems > 0x7fffffffLL || nbrm > 0x7fffffffLL)
         return fail(BSA_ERR_ARG, "Mesher zone pass too large");
@@ -1259,16 +1296,16 @@ int Engine::msh_mixed_batch(const std::vector<ZoneDev> &zs, std::vector<double> 
         // The same tables built on the host (and the frequencies of the truncated POD form,
         // whose A table is formed from host frequencies).
         FreqIndex F, UF;
-        for (const ZoneDev &z : zs) {
+        for (const ZoneX &z : zx) {
             for (int i = 0; i < z.ni; ++i) {
-                const double r = z.fi0 + i * z.dIi;
+                const double r = z.fi0 + i * z.dI;
                 F.add(r);
                 UF.add(r);
-                for (int j = 0; j < z.nj; ++j) F.add(r + (z.fj0 + j * z.dJj));
+                for (int j = 0; j < z.nj; ++j) F.add(r + (z.fj0 + j * z.dJ));
             }
             for (int j = 0; j < z.nj; ++j) {
-                F.add(z.fj0 + j * z.dJj);
-                UF.add(z.fj0 + j * z.dJj);
+                F.add(z.fj0 + j * z.dJ);
+                UF.add(z.fj0 + j * z.dJ);
             }
         }
         F.seal();
@@ -1278,14 +1315,13 @@ int Engine::msh_mixed_batch(const std::vector<ZoneDev> &zs, std::vector<double> 
         for (int u = 0; u < nU; ++u) usrc[u] = F.at(UF.v[u]);
         std::vector<Task> tasks;
         tasks.reserve(ntasks);
-        for (size_t k = 0; k < zs.size(); ++k) {
-            const ZoneDev &z = zs[k];
-            const long long pb = zx[k].pbase, gb = zx[k].gbase;
-            for (int j = 0; j < z.nj; ++j) gsrc[gb + j] = F.at(z.fj0 + j * z.dJj);
+        for (const ZoneX &z : zx) {
+            const long long pb = z.pbase, gb = z.gbase;
+            for (int j = 0; j < z.nj; ++j) gsrc[gb + j] = F.at(z.fj0 + j * z.dJ);
             for (int i = 0; i < z.ni; ++i) {
-                const double r = z.fi0 + i * z.dIi;
+                const double r = z.fi0 + i * z.dI;
                 for (int j = 0; j < z.nj; ++j) {
-                    const int row = F.at(r + (z.fj0 + j * z.dJj));
+                    const int row = F.at(r + (z.fj0 + j * z.dJ));
                     ssrc[pb + (size_t)i * z.nj + j] = row;  // line order (kind 0), and its place in column order (kind 1)
                     ssrc[npts + pb + (size_t)i * z.nj + j] = (int)(npts + pb + (size_t)j * z.ni + i);
                 }
@@ -1293,7 +1329,7 @@ int Engine::msh_mixed_batch(const std::vector<ZoneDev> &zs, std::vector<double> 
                                      (int)(pb + (long long)i * z.nj), 1, 0});
             }
             for (int j = 0; j < z.nj; ++j)
-                tasks.push_back(Task{UF.at(z.fj0 + j * z.dJj) * Mp, -1, (int)(npts + pb + (long long)j * z.ni) * NMT,
+                tasks.push_back(Task{UF.at(z.fj0 + j * z.dJ) * Mp, -1, (int)(npts + pb + (long long)j * z.ni) * NMT,
                                      z.ni, (int)(pb + j), z.nj, 1});
         }
         // work items: per task, its row tiles x N tiles (one, or two for column tasks), consecutive
