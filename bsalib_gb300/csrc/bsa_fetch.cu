@@ -3,10 +3,14 @@
 // A device-to-host copy into fresh pageable memory faults its pages in one by one behind the copy:
 // 31 MB of listed bispectra took 26 ms, 15 MB of a materialised grid 12 ms, against 0.2 ms over the
 // link.  Here the link fills a pinned block and several host threads copy it on, so the page faults
-// and the copy run on many cores.
+// and the copy run on many cores.  Memory whose pages are there already takes the plain copy (3 MB in
+// about 0.1 ms, which starting the threads alone costs).
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -17,7 +21,8 @@
 namespace bsa {
 namespace {
 
-constexpr size_t kDirect = 2 << 20;    // smaller results: one plain copy
+constexpr size_t kDirect = 1 << 20;    // smaller results: one plain copy
+constexpr size_t kThreads = 8;
 constexpr size_t kBlockMax = 64 << 20; // pinned block, at most
 
 // One pinned block for the process, grown on demand to kBlockMax; bsa_gpu_releaseDeviceCache frees it.
@@ -31,8 +36,19 @@ Pinned &pinned() {
     return b;
 }
 
+// Whether sixteen pages spread over the range are in memory.
+bool resident(const void *p, size_t n) {
+    static const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    for (int k = 0; k < 16; ++k) {
+        const uintptr_t a = ((uintptr_t)p + (n - 1) / 15 * k) & ~(page - 1);
+        unsigned char v = 0;
+        if (mincore((void *)a, page, &v) != 0 || !(v & 1)) return false;
+    }
+    return true;
+}
+
 void copy_threads(char *dst, const char *src, size_t n) {
-    const size_t nt = std::max<size_t>(1, std::min<size_t>({8, n >> 20, std::thread::hardware_concurrency()}));
+    const size_t nt = std::max<size_t>(1, std::min<size_t>({kThreads, n >> 20, std::thread::hardware_concurrency()}));
     const size_t step = ((n + nt - 1) / nt + 4095) & ~(size_t)4095;
     std::vector<std::thread> ts;
     size_t o = step;
@@ -53,8 +69,9 @@ cudaError_t fetch(cudaStream_t st, void *dst, const void *src, size_t n) {
     cudaError_t e;
     Pinned &b = pinned();
     std::unique_lock<std::mutex> lk(b.m, std::defer_lock);
-    if (n >= kDirect) lk.lock();
-    if (n >= kDirect && b.bytes < std::min(n, kBlockMax)) {
+    const bool direct = n < kDirect || resident(dst, n);
+    if (!direct) lk.lock();
+    if (!direct && b.bytes < std::min(n, kBlockMax)) {
         if (b.p) cudaFreeHost(b.p);
         b.p = nullptr;
         b.bytes = 0;
@@ -65,7 +82,7 @@ cudaError_t fetch(cudaStream_t st, void *dst, const void *src, size_t n) {
             cudaGetLastError();  // no pinned memory: plain copy
         }
     }
-    if (n < kDirect || !b.p) {
+    if (direct || !b.p) {
         if ((e = cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, st))) return e;
         return cudaStreamSynchronize(st);
     }
