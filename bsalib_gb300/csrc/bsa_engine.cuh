@@ -226,7 +226,8 @@ struct Engine {
     int contract_list64(const PointSrc &ps, long long npts, const HostRows &rows, int G, double *bfd, double *brd,
                         Lists64 &lists);
     // the whole Classic grid in FP64 over distinct frequency pairs (bsa_pair64.cu); grid +-N df
-    int contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr);
+    int contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr,
+                        double *bf_host = nullptr, double *br_host = nullptr);
     int contract_mixed(const PointSrc &ps, long long npts, double *m3mf, double *m3mr);
     int contract_e(const PointSrc &ps, double *m3mf, double *m3mr, const ESample *smp = nullptr);  // bsa_classic_e.cu
     // bsa_gpu_clsBispectraAt: Classic bispectra at listed grid points in the selected precision

@@ -579,12 +579,15 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
     const bool mixed = !diagonal && precision == BSA_PREC_BF16X3 && !bf_host && !br_host;
     if (mixed && nme > 64) return fail(BSA_ERR_UNSUPPORTED, "BF16x3 contraction supports at most 64 kept modes");
     // FP64 moments of the whole grid f = -N..N come from the products of distinct |f| pairs
-    // (bsa_pair64.cu), on the A rows of f >= 0 alone.  Row shards, materialised or exported bispectra
-    // and the frequency convention's one-sided grid (its truncated sum reads another row than
-    // |f1 + f2|) keep the point kernel.
-    const bool pair64 = !mixed && !bf_host && !br_host && !export_fn && !brm_file_wanted(true) &&
-                        set.defsc == 1 && (nf & 1) && r0 == 0 && r1 == nf;
+    // (bsa_pair64.cu), on the A rows of f >= 0 alone; materialised bispectra read the products too, where
+    // all of them fit 4 GB.  Row shards, exported bispectra and the frequency convention's one-sided
+    // grid (its truncated sum reads another row than |f1 + f2|) keep the point kernel.
     const int half = (nf - 1) / 2;
+    const bool pts = bf_host || br_host;
+    const bool pts_ok = !pts || (!diagonal && !m3mf && !m3mr && (double)nf * nf <= 2.0e9 &&
+                                 (double)(half + 2) * (half + 8) / (analytic ? 1 : 2) * (double)dim_bisp() * 10.0 <= 4.0e9);
+    const bool pair64 = !mixed && pts_ok && !export_fn && !brm_file_wanted(true) &&
+                        set.defsc == 1 && (nf & 1) && r0 == 0 && r1 == nf;
     const double df_grid = f[half + 1] - f[half];  // the step itself (f[half] = 0): f[1] - f[0] is rounded
     if (pair64) {
         ftab.assign(f.begin() + half, f.end());
@@ -680,7 +683,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
             if (r0 != 0 || r1 != nf) return fail(BSA_ERR_ARG, "the bispectrum export needs the full grid");
             rc = classic_export(ps, f, m3mf, m3mr);
         } else {
-            rc = pair64     ? contract_pair64(half, df_grid, analytic, !scalar, delta * delta, m3mf, m3mr)
+            rc = pair64     ? contract_pair64(half, df_grid, analytic, !scalar, delta * delta, m3mf, m3mr, bf_host, br_host)
                  : diagonal ? contract_diag(ps, npts, 0, m3mf, m3mr, bf_host, br_host)
                  : mixed    ? contract_mixed(ps, npts, m3mf, m3mr)
                             : contract(ps, npts, m3mf, m3mr, bf_host, br_host);

@@ -319,6 +319,48 @@ __global__ void k_pair_finish(int nm, double w4, const double *__restrict__ S, d
     m3mf[x] = w4 * (at(6, m, n, o) + at(6, m, o, n) + at(7, n, m, o) + at(7, o, m, n) + at(8, o, n, m) + at(8, n, o, m));
 }
 
+// E(x, y)[(a, b), j] of a chunk that holds every product.
+__device__ __forceinline__ double pair_at(const Chunk &c, int x, int y, int a, int b, int j) {
+    if (x > y) {
+        const int t = x;
+        x = y;
+        y = t;
+        const int u = b;
+        b = j;
+        j = u;
+    }
+    const int r = x * c.rx() + a * c.an + b, mt = r / kTM;
+    const RowTile rt = c.rt[mt];
+    return c.E[rt.base + (size_t)(r - mt * kTM) * rt.nct * kTN + (y * c.an + j - rt.ct0 * kTN)];
+}
+
+// Force and response bispectra of every grid point from the products: one block per point (i1, i2) =
+// (p % nf - N, p / nf - N), the layout and FRF product of k_bfm_fp64.  65 x 65 points of 60 nodes, 6
+// modes: 0.55 ms by three contractions a point, 0.05 ms with the products.
+__global__ __launch_bounds__(256) void k_pair_points(Chunk c, int N, const double2 *__restrict__ H, double *__restrict__ bf,
+                                                     double *__restrict__ br) {
+    __shared__ double2 h[3][64];
+    const int nm = c.an, nm2 = nm * nm, nm3 = nm2 * nm, nf = 2 * N + 1, p = blockIdx.x;
+    const int i1 = p % nf - N, i2 = p / nf - N, i3 = i1 + i2, x = abs(i1), y = abs(i2), z = abs(i3);
+    for (int q = threadIdx.x; q < 3 * nm; q += blockDim.x) {
+        const int w = q / nm, i = w == 0 ? i1 : w == 1 ? i2 : i3;
+        double2 v = H[(size_t)abs(i) * nm + (q - w * nm)];
+        if (i < 0) v.y = -v.y;
+        h[w][q - w * nm] = v;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nm3; e += blockDim.x) {
+        const int m = e % nm, n = (e / nm) % nm, o = e / nm2;
+        double v = pair_at(c, x, y, m, n, o);                                                  // T1
+        if (z <= c.hi) v += pair_at(c, z, y, n, m, o) + pair_at(c, x, z, o, n, m);             // T2 + T3
+        const double2 h1 = h[0][m], h2 = h[1][n], h3 = h[2][o];
+        const double cr = h2.x * h3.x + h2.y * h3.y, ci = h2.y * h3.x - h2.x * h3.y;
+        const double F = h1.x * cr - h1.y * ci, b = 2.0 * v;
+        if (bf) bf[(size_t)p * nm3 + e] = b;
+        if (br) br[(size_t)p * nm3 + e] = b * F;
+    }
+}
+
 // Diagonal-only spectra: the products are P_m(x, y) = sum_k Q_km L_km^2 S_k(x) S_k(y), rows (x, m),
 // columns y, and with a = b = j = m the twelve contributions collapse to
 // 2 (w1 + w2m + w3m) alpha + 2 (w1- + w2p + w3p) beta.  One block per (mode, group of x), a warp per
@@ -365,7 +407,10 @@ __global__ __launch_bounds__(256) void k_pair_moments_diag(Chunk c, int N, int a
 // Third moments of the whole Classic grid (circular-frequency convention, every row) in FP64 from
 // the products of distinct frequency pairs; dA (dS for the diagonal-only spectra) holds the rows of
 // i df, i = 0 .. N (truncated S(f1 + f2)) or 0 .. 2 N (analytic).
-int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr) {
+// With bf_host / br_host the bispectra of every grid point instead (every product in one chunk:
+// pair64_points).
+int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double wval, double *m3mf, double *m3mr,
+                            double *bf_host, double *br_host) {
     using namespace p64;
     const bool diag = set.onlyd != 0;
     const int nm = nme, an = diag ? 1 : nm, rx = nm * an, hi = analytic ? 2 * N : N;
@@ -405,12 +450,13 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     std::vector<RowTile> rts;
     std::vector<long long> pre;
     long long emax = 0, rmax = 0;
+    const bool pts = bf_host || br_host;
     for (int x0 = 0; x0 <= N;) {
         Plan p{x0, x0, 0, 0, 0, 0, rts.size(), pre.size()};
         long long el = 0;
         while (p.x1 <= N) {
             const long long add = (long long)rx * std::max((ylast(p.x1) - p.x1 + 1) * (long long)an + 2 * kTN, (long long)Kd);
-            if (p.x1 > x0 && el + add > cap) break;
+            if (!pts && p.x1 > x0 && el + add > cap) break;
             el += add;
             pre.push_back(p.npairs);
             p.npairs += ylast(p.x1) - p.x1 + 1;
@@ -443,6 +489,8 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
         (e = dOut.reserve(sizeof(double) * (3 * (size_t)dim_psd() + 2 * (size_t)nb))))
         return cuda_fail(e, "allocating pair products");
     o = dOut.as<double>() + 3 * (size_t)dim_psd();
+    const size_t ptb = sizeof(double) * (size_t)(2 * N + 1) * (2 * N + 1) * nb;
+    if (pts && ((bf_host && (e = dBF.reserve(ptb))) || (br_host && (e = dBR.reserve(ptb))))) return cuda_fail(e, "allocating bispectra");
     if (tensor && ((e = dMixB.reserve(tc_col_bytes(hi + 1, an, K))) || (e = dMshT.reserve(tc_row_bytes(rmax, K))) ||
                    (e = dFlag.reserve(256))))
         return cuda_fail(e, "allocating pair products");
@@ -469,7 +517,10 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
             if (p.items < 304) k_pair_gemm<32><<<dim3((unsigned)p.items, kTM / 32), 256, 0, stream>>>(c, A, Q);
             else k_pair_gemm<kTM><<<dim3((unsigned)p.items, 1), 256, 0, stream>>>(c, A, Q);
         }
-        if (diag) {
+        if (pts) {
+            k_pair_points<<<(2 * N + 1) * (2 * N + 1), 256, 0, stream>>>(c, N, dMixH.as<double2>(), bf_host ? dBF.as<double>() : nullptr,
+                                                                         br_host ? dBR.as<double>() : nullptr);
+        } else if (diag) {
             k_pair_moments_diag<<<dim3(nm, G), 256, 0, stream>>>(c, N, analytic ? 1 : 0, vect ? 1 : 0, 4.0 * wval,
                                                                   dMixH.as<double2>(), dPartF.as<double>() + q * G * plen);
         } else {
@@ -481,6 +532,22 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     }
     if ((e = cudaGetLastError())) return cuda_fail(e, "pair contraction kernels");
     if ((e = cudaEventRecord(evg1, stream))) return cuda_fail(e, "event");
+    if (pts) {
+        const size_t bytes = ptb;
+        int flags[2] = {0, 0};
+        const bool pend = atable_pending;
+        if (((tensor || pend) && (e = cudaMemcpyAsync(flags, dFlag.p, sizeof flags, cudaMemcpyDeviceToHost, stream))) ||
+            (bf_host && (e = fetch(stream, bf_host, dBF.p, bytes))) || (br_host && (e = fetch(stream, br_host, dBR.p, bytes))) ||
+            (e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream)))
+            return cuda_fail(e, "bispectrum copy");
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, ev2, ev1);
+        last_ms_contraction = ms;
+        cudaEventElapsedTime(&ms, evg0, evg1);
+        last_ms_gemm = ms;
+        d2h += (double)bytes * ((bf_host ? 1 : 0) + (br_host ? 1 : 0));
+        return pipeline_flags(flags, pend, tensor);
+    }
     if ((e = launch_reduce_groups(stream, (int)nparts, plen, dPartF.as<double>(), diag ? o : dPartR.as<double>(), nullptr, nullptr)))
         return cuda_fail(e, "reduction kernel");
     if (!diag) k_pair_finish<<<(unsigned)((nb + 127) / 128), 128, 0, stream>>>(nm, 4.0 * wval, dPartR.as<double>(), o, o + nb);

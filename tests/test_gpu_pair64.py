@@ -93,3 +93,20 @@ def test_diagonal_pairs_against_points(bsalib, modes, nodes, nfreqs, trunc, scal
     a, b = _run(p, (0, 1), trunc), _run(p, (1, nf), trunc)
     _close(whole, {k: a[k] + b[k] for k in a})
     _close(_run(p, trunc=trunc, sym=True), whole)
+
+
+@pytest.mark.parametrize("modes,nodes,nfreqs", [(1, 3, 2), (5, 16, 6), (9, 40, 12), (17, 33, 4), (64, 12, 3)])
+@pytest.mark.parametrize("trunc", [True, False])
+def test_bispectra_against_listed_points(bsalib, modes, nodes, nfreqs, trunc):
+    p = tall_building(nodes=nodes, modes=modes, nfreqs=nfreqs, df=2.0 / nfreqs, seed=modes)
+    s = api.BsaSession(p, classic_truncation=trunc)
+    try:
+        f, bf, br = s.classic_bispectra()
+        n = f.size
+        i1, i2 = (v.ravel() for v in np.meshgrid(np.arange(n), np.arange(n), indexing="ij"))
+        pieces = [s.classic_points(i1[k:k + 3], i2[k:k + 3]) for k in range(0, n * n, 3)]
+    finally:
+        s.close()
+    for a, k in ((bf, 0), (br, 1)):
+        b = np.concatenate([x[k] for x in pieces]).reshape(a.shape)
+        assert np.max(np.abs(a - b)) <= 1e-12 * np.max(np.abs(b))
