@@ -32,6 +32,10 @@ void release_device_cache();
 cudaError_t fetch(cudaStream_t st, void *dst, const void *src, size_t n);
 void release_fetch_block();
 
+// An optional form found no room for its scratch and has launched nothing: the caller goes on with the
+// form that needs none.
+constexpr int kNoRoom = -1000;
+
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
@@ -208,6 +212,7 @@ struct Engine {
     // table.
     bool atable_pending = false;
     int atable_check();
+    cudaError_t need(DevBuf &b, size_t bytes);
     int pipeline_flags(const int *flags, bool atable, bool pairs);
     // dimM_psd_ / dimM_bisp_ (src/bsa/BsaLibImpl.F90:313-355): nm / nm for the diagonal-only
     // spectra, nm^2 / nm^3 otherwise.

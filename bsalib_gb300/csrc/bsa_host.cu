@@ -112,8 +112,12 @@ cudaError_t DevBuf::reserve(size_t nbytes) {
         }
         e = cudaMalloc(&p, want);
     }
-    if (e == cudaSuccess) bytes = want;
-    else p = nullptr;
+    if (e == cudaSuccess) {
+        bytes = want;
+    } else {
+        p = nullptr;
+        cudaGetLastError();  // reported by the return value; a caller may go on with less
+    }
     return e;
 }
 
@@ -438,20 +442,25 @@ int Engine::build_atable_dev(int nf, bool fp32, int f0) {
         kernels += 2;
         return BSA_OK;
     }
-    if ((e = dA.reserve(sizeof(double) * (size_t)nf * K * nme))) return cuda_fail(e, "allocating A");
+    if ((e = need(dA, sizeof(double) * (size_t)nf * K * nme))) return cuda_fail(e, "allocating A");
     const double *fp = dFreq.as<double>() + f0;
     const int *bad = log_coh_bad(dLogc.as<double>(), (size_t)ntc * in.nnl * in.nnl);
     // On the tensor cores from 80 nodes on.  Second-order analyses, FP64 pipe / tensor cores (ms): 40
     // nodes, 12 modes, 65 rows 0.071 / 0.075; 64, 12, 65: 0.078 / 0.078; 100, 12, 65: 0.107 / 0.091;
     // 150, 12, 129: 0.229 / 0.139; 400, 24, 33: 0.564 / 0.157; 520, 8, 17: 0.258 / 0.165.
-    const bool tensor = in.nnl >= 80;
+    bool tensor = in.nnl >= 80;
+    int step = 0;
     if (tensor) {
-        // frequencies in chunks of at most 1 GB of B digits
+        // frequencies in chunks of at most 1 GB of B digits; without room for them the FP64 pipe
         const size_t per = atable64_tc_scratch(1, ntc, in.nnl, nme);
-        const int step = (int)std::max<size_t>(1, std::min<size_t>(nf, ((size_t)1 << 30) / per));
+        step = (int)std::max<size_t>(1, std::min<size_t>(nf, ((size_t)1 << 30) / per));
+        e = dMshT.reserve(atable64_tc_scratch(step, ntc, in.nnl, nme));
+        if (e == cudaErrorMemoryAllocation) tensor = false;
+        else if (e) return cuda_fail(e, "allocating A");
+    }
+    if (tensor) {
         if (256 > dFlag.bytes && (rc = atable_check())) return rc;
-        if ((e = dMshT.reserve(atable64_tc_scratch(step, ntc, in.nnl, nme))) || (e = dFlag.reserve(256)))
-            return cuda_fail(e, "allocating A");
+        if ((e = dFlag.reserve(256))) return cuda_fail(e, "allocating A");
         if (!atable_pending && (e = cudaMemsetAsync(dFlag.p, 0, sizeof(int), stream))) return cuda_fail(e, "memset");
         atable_pending = true;
         for (int q = 0; q < nf; q += step) {
@@ -467,6 +476,15 @@ int Engine::build_atable_dev(int nf, bool fp32, int f0) {
     if (e) return cuda_fail(e, "A-table kernel");
     kernels += 1;
     return BSA_OK;
+}
+
+// What an FP64 analysis cannot do without; the optional forms' scratch gives way to it.  Between
+// contractions only: nothing in flight but kernels of this stream.
+cudaError_t Engine::need(DevBuf &b, size_t bytes) {
+    cudaError_t e = b.reserve(bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    for (DevBuf *s : {&dMixA, &dMixB, &dMshT}) s->release();
+    return b.reserve(bytes);
 }
 
 // Flags read behind a run: [0] the A kernel's, [1] the pair products'.
@@ -683,10 +701,23 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
             if (r0 != 0 || r1 != nf) return fail(BSA_ERR_ARG, "the bispectrum export needs the full grid");
             rc = classic_export(ps, f, m3mf, m3mr);
         } else {
-            rc = pair64     ? contract_pair64(half, df_grid, analytic, !scalar, delta * delta, m3mf, m3mr, bf_host, br_host)
-                 : diagonal ? contract_diag(ps, npts, 0, m3mf, m3mr, bf_host, br_host)
-                 : mixed    ? contract_mixed(ps, npts, m3mf, m3mr)
-                            : contract(ps, npts, m3mf, m3mr, bf_host, br_host);
+            rc = kNoRoom;
+            if (pair64) {
+                rc = contract_pair64(half, df_grid, analytic, !scalar, delta * delta, m3mf, m3mr, bf_host, br_host);
+                if (rc == kNoRoom) {
+                    // no room for the products and their operands: the point kernel on the rows of every f
+                    for (DevBuf *b : {&dMixA, &dMixB, &dMshT}) b->release();
+                    ftab = f;
+                    if (analytic)
+                        for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back(2.0 * f[0] + s * (f[1] - f[0]));
+                    const int r = diagonal ? build_psd(ftab) : build_atable(ftab, false);
+                    if (r) return r;
+                }
+            }
+            if (rc == kNoRoom)
+                rc = diagonal ? contract_diag(ps, npts, 0, m3mf, m3mr, bf_host, br_host)
+                     : mixed  ? contract_mixed(ps, npts, m3mf, m3mr)
+                              : contract(ps, npts, m3mf, m3mr, bf_host, br_host);
         }
         if (rc) return rc;
         last_points = (double)npts;
@@ -758,12 +789,12 @@ int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m
     const long long nm3 = (long long)nme * nme * nme;
     cudaError_t e;
     const int G = bfm_fp64_groups(npts, nme);
-    if ((e = dPartF.reserve(sizeof(double) * (size_t)G * nm3)) || (e = dPartR.reserve(sizeof(double) * (size_t)G * nm3)))
+    if ((e = need(dPartF, sizeof(double) * (size_t)G * nm3)) || (e = need(dPartR, sizeof(double) * (size_t)G * nm3)))
         return cuda_fail(e, "allocating partial sums");
     if ((e = dOut.reserve(sizeof(double) * (3 * (size_t)nme * nme + 2 * (size_t)nm3)))) return cuda_fail(e, "out");
     double *bfd = nullptr, *brd = nullptr;
     if (bf_host || br_host) {
-        if ((e = dBF.reserve(sizeof(double) * (size_t)npts * nm3)) || (e = dBR.reserve(sizeof(double) * (size_t)npts * nm3)))
+        if ((e = need(dBF, sizeof(double) * (size_t)npts * nm3)) || (e = need(dBR, sizeof(double) * (size_t)npts * nm3)))
             return cuda_fail(e, "allocating bispectra");
         bfd = dBF.as<double>();
         brd = dBR.as<double>();
@@ -894,7 +925,13 @@ int Engine::run_points(const double *fi, const double *fj, const double *w, doub
                 zoff[k] = axes && total + need <= cap ? total : -1;
                 if (zoff[k] >= 0) total += need;
             }
-            if ((e = dZoff.reserve(sizeof(long long) * zoff.size())) || (e = dZoneH.reserve(sizeof(double2) * (size_t)total)) ||
+            e = dZoneH.reserve(sizeof(double2) * (size_t)total);
+            if (e == cudaErrorMemoryAllocation) {  // no room: every FRF value at its point
+                std::fill(zoff.begin(), zoff.begin() + nz, -1);
+                total = 0;
+                e = cudaSuccess;
+            }
+            if (e || (e = dZoff.reserve(sizeof(long long) * zoff.size())) ||
                 (e = cudaMemcpyAsync(dZoff.p, zoff.data(), sizeof(long long) * zoff.size(), cudaMemcpyHostToDevice, stream)) ||
                 (e = launch_zone_frf(stream, (int)nz, nme, ps.zones, dZoff.as<long long>(), total, frf(), dZoneH.as<double2>())))
                 return cuda_fail(e, "zone FRF tables");

@@ -644,8 +644,8 @@ __global__ __launch_bounds__(256) void k_bfm_fp64(const double *__restrict__ A,
             const int m = mg + MG * u;
             if (m < nm) {
                 const size_t idx = (size_t)pg * nm3 + m + (size_t)nm * no;
-                part_mf[idx] = PAIR && !pp.first ? part_mf[idx] + smf[u] : smf[u];
-                part_mr[idx] = PAIR && !pp.first ? part_mr[idx] + smr[u] : smr[u];
+                part_mf[idx] = !pp.first ? part_mf[idx] + smf[u] : smf[u];
+                part_mr[idx] = !pp.first ? part_mr[idx] + smr[u] : smr[u];
             }
         }
     }

@@ -27,11 +27,29 @@ namespace bsa {
 //   1000, K = 150, 8: 0.41 / 0.59;  2000, K = 40, 6: 0.21 / 0.59;  300, K = 60, 10: 0.11 / 0.17.
 bool Engine::list64_wanted(long long npts, int nr) const {
     using namespace p64;
-    if (K < 24) return false;
+    // the column digits grow with the rows (5 times the A rows at 16 modes): within 32 GB
+    if (K < 24 || tc_block_bytes(nr, nme, K) > ((size_t)32 << 30)) return false;
     const double nm = nme, rows = (double)std::min<long long>(nr, 2 * npts) * ((nme * nme + kTM - 1) / kTM) * kTM;
     const double point_ms = 2.0 * K * nm * nm * nm * (double)npts / (nme < 8 ? 2.0e8 : 4.2e8);
     const double pair_ms = 0.07 + 1.2e-4 * (double)npts + rows * ((K + 63) / 64 * 64) * 1.0e-8;
     return pair_ms < point_ms;
+}
+
+// The points of a list from p0 on.
+static PointSrc from(PointSrc q, long long p0) {
+    q.ix += p0;
+    q.iy += p0;
+    q.iz += p0;
+    q.f1 += p0;
+    q.f2 += p0;
+    if (q.w) q.w += p0;
+    if (q.zones) {
+        q.zid += p0;
+        q.zi += p0;
+        q.zj += p0;
+    }
+    if (q.cptr) q.cptr += p0;
+    return q;
 }
 
 // Third moments (and bispectra) of a point list; rows: the points' A rows on the host (iz < 0: the sum
@@ -52,8 +70,22 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
     const long long rowb = (long long)tc_row_bytes((long long)tiles_x * kTM, K);
     const long long cap = 8LL << 30;
     const long long batch = std::max(1LL, std::min({npts, cap / (24 * nm3), cap / (2 * rowb)}));
-    if ((e = dMixB.reserve(tc_block_bytes(nr, nm, K))) || (e = dFlag.reserve(256))) return cuda_fail(e, "allocating pair products");
-    if ((e = cudaMemsetAsync(dFlag.as<int>() + 1, 0, sizeof(int), stream)) || (e = tc_prep_blocks(stream, nr, nm, K, dA.as<double>(), dMixB.p)))
+    // no room for the column digits, or later for a batch: the point kernel on what is left
+    PairPts pp;
+    auto rest = [&](long long p0) {
+        PointSrc q = from(ps, p0);
+        pp.E = nullptr;
+        pp.first = p0 == 0;
+        const cudaError_t r = launch_bfm_fp64(stream, dA.as<double>(), dQ.as<double>(), K, nm, q, npts - p0, frf(), G,
+                                              dPartF.as<double>(), dPartR.as<double>(), bfd ? bfd + (size_t)p0 * nm3 : nullptr,
+                                              brd ? brd + (size_t)p0 * nm3 : nullptr, pp);
+        return r ? cuda_fail(r, "FP64 point kernel") : BSA_OK;
+    };
+    if ((e = dFlag.reserve(256)) || (e = cudaMemsetAsync(dFlag.as<int>() + 1, 0, sizeof(int), stream)))
+        return cuda_fail(e, "allocating pair products");
+    if ((e = dMixB.reserve(tc_block_bytes(nr, nm, K))) == cudaErrorMemoryAllocation) return rest(0);
+    if (e) return cuda_fail(e, "allocating pair products");
+    if ((e = tc_prep_blocks(stream, nr, nm, K, dA.as<double>(), dMixB.p)))
         return cuda_fail(e, "pair product operands");
     kernels += 2;
     for (long long p0 = 0; p0 < npts; p0 += batch) {
@@ -132,10 +164,11 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
                     items.push_back(make_int4(row_of[x] * tiles_x + t, q, std::min(slots, start[x + 1] * np - q), 0));
         const size_t ib = sizeof(int4) * items.size(), lb = sizeof(int) * blk.size(), xb = sizeof(int) * xmap.size(),
                      pb = sizeof(int) * pe.size();
-        if ((e = dMixA.reserve(sizeof(double) * (size_t)nu * nm3)) ||
-            (e = dMshT.reserve(tc_row_bytes((long long)xmap.size() * tiles_x * kTM, K))) ||
-            (e = dMshIdx.reserve(ib + 2 * lb + xb + pb)))
-            return cuda_fail(e, "allocating pair products");
+        e = dMixA.reserve(sizeof(double) * (size_t)nu * nm3);
+        if (!e) e = dMshT.reserve(tc_row_bytes((long long)xmap.size() * tiles_x * kTM, K));
+        if (!e) e = dMshIdx.reserve(ib + 2 * lb + xb + pb);
+        if (e == cudaErrorMemoryAllocation) return rest(p0);
+        if (e) return cuda_fail(e, "allocating pair products");
         char *d = (char *)dMshIdx.p;
         int4 *ditems = (int4 *)d;
         int *dblk = (int *)(d + ib), *dpair = (int *)(d + ib + lb), *dx = (int *)(d + ib + 2 * lb), *dpe = (int *)(d + ib + 2 * lb + xb);
@@ -150,20 +183,7 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
         PairList l{ditems, dblk, dpair, np, bw, tiles_x};
         if ((e = tc_list_products(stream, c, l, nr, dA.as<double>(), dQ.as<double>(), dMixB.p, dMshT.p, dFlag.as<int>() + 1)))
             return cuda_fail(e, "pair product kernel");
-        PointSrc q = ps;
-        q.ix += p0;
-        q.iy += p0;
-        q.iz += p0;
-        q.f1 += p0;
-        q.f2 += p0;
-        if (q.w) q.w += p0;
-        if (q.zones) {
-            q.zid += p0;
-            q.zi += p0;
-            q.zj += p0;
-        }
-        if (q.cptr) q.cptr += p0;
-        PairPts pp;
+        const PointSrc q = from(ps, p0);
         pp.E = dMixA.as<double>();
         pp.pe = dpe;
         pp.first = p0 == 0;

@@ -336,7 +336,7 @@ __device__ __forceinline__ double pair_at(const Chunk &c, int x, int y, int a, i
 
 // Force and response bispectra of every grid point from the products: one block per point (i1, i2) =
 // (p % nf - N, p / nf - N), the layout and FRF product of k_bfm_fp64.  65 x 65 points of 60 nodes, 6
-// modes: 0.55 ms by three contractions a point, 0.05 ms with the products.
+// modes: 0.55 ms by three contractions a point, 0.02 ms with the products.
 __global__ __launch_bounds__(256) void k_pair_points(Chunk c, int N, const double2 *__restrict__ H, double *__restrict__ bf,
                                                      double *__restrict__ br) {
     __shared__ double2 h[3][64];
@@ -483,17 +483,17 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     const size_t rtb = sizeof(RowTile) * rts.size(), preb = sizeof(long long) * pre.size();
     const size_t hb = sizeof(double2) * (size_t)(2 * N + 1) * nm, nparts = diag ? G * plans.size() : G;
     const long long plen = diag ? 2 * nb : kKinds * nb;
-    double *o = nullptr;
-    if ((e = dMixA.reserve(sizeof(double) * (size_t)emax)) || (e = dMixH.reserve(hb)) || (e = dMshIdx.reserve(rtb + preb)) ||
-        (e = dPartF.reserve(sizeof(double) * nparts * plen)) || (e = dPartR.reserve(sizeof(double) * (size_t)plen)) ||
-        (e = dOut.reserve(sizeof(double) * (3 * (size_t)dim_psd() + 2 * (size_t)nb))))
-        return cuda_fail(e, "allocating pair products");
-    o = dOut.as<double>() + 3 * (size_t)dim_psd();
     const size_t ptb = sizeof(double) * (size_t)(2 * N + 1) * (2 * N + 1) * nb;
-    if (pts && ((bf_host && (e = dBF.reserve(ptb))) || (br_host && (e = dBR.reserve(ptb))))) return cuda_fail(e, "allocating bispectra");
-    if (tensor && ((e = dMixB.reserve(tc_col_bytes(hi + 1, an, K))) || (e = dMshT.reserve(tc_row_bytes(rmax, K))) ||
-                   (e = dFlag.reserve(256))))
-        return cuda_fail(e, "allocating pair products");
+    auto room = [&](DevBuf &b, size_t bytes) { return !e && (e = b.reserve(bytes)) == cudaErrorMemoryAllocation; };
+    e = cudaSuccess;
+    if (room(dMixA, sizeof(double) * (size_t)emax) || (tensor && room(dMixB, tc_col_bytes(hi + 1, an, K))) ||
+        (tensor && room(dMshT, tc_row_bytes(rmax, K))) || room(dMixH, hb) || room(dMshIdx, rtb + preb) ||
+        room(dPartF, sizeof(double) * nparts * plen) || room(dPartR, sizeof(double) * (size_t)plen) ||
+        room(dOut, sizeof(double) * (3 * (size_t)dim_psd() + 2 * (size_t)nb)) || (tensor && room(dFlag, 256)) ||
+        (bf_host && room(dBF, ptb)) || (br_host && room(dBR, ptb)))
+        return kNoRoom;
+    if (e) return cuda_fail(e, "allocating pair products");
+    double *o = dOut.as<double>() + 3 * (size_t)dim_psd();
     char *idx = (char *)dMshIdx.p;
     if ((e = cudaMemcpyAsync(idx, rts.data(), rtb, cudaMemcpyHostToDevice, stream)) ||
         (e = cudaMemcpyAsync(idx + rtb, pre.data(), preb, cudaMemcpyHostToDevice, stream)))
