@@ -648,11 +648,10 @@ struct BatchCase {
     int nnl = 0, psd_type = 0, nme = 0, K = 0;
     bool trunc = true;
     std::vector<int> modes;
-    std::vector<double> hL, hQ, hCorr, hM, hK, hC, hWd3, hWd2;
+    std::vector<double> hWfc, hPhi, hCorr, hM, hK, hC;
     std::vector<int> hNodes;
-    int hNn = 0;
+    int hNn = 0, hNl = 0;
     std::vector<unsigned char> hPack;
-    std::vector<float> hL32;
     std::vector<PsdNode> hPsd;
     std::vector<double> f;  // Classic grid
 };
@@ -675,12 +674,11 @@ int Engine::batch_add(int *id) {
     c.K = K;
     c.trunc = classic_trunc;
     c.modes = modes;
-    c.hL = hL; c.hQ = hQ; c.hCorr = hCorr;
+    c.hWfc = hWfc; c.hPhi = hPhi; c.hNl = hNl; c.hCorr = hCorr;
     if (c.hCorr.empty())  // the caller's arrays may be gone when the sweep runs
         for (int tc : set.tc)
             c.hCorr.insert(c.hCorr.end(), in.corr + (size_t)in.ncorr * (tc - 1), in.corr + (size_t)in.ncorr * tc);
-    c.hNodes = hNodes; c.hNn = hNn; c.hM = hM; c.hK = hK; c.hC = hC; c.hWd3 = hWd3; c.hWd2 = hWd2;
-    c.hL32 = hL32; c.hPsd = hPsd;
+    c.hNodes = hNodes; c.hNn = hNn; c.hM = hM; c.hK = hK; c.hC = hC; c.hPsd = hPsd;
     g_batch.push_back(std::move(c));
     if (id) *id = (int)g_batch.size() - 1;
     return BSA_OK;
@@ -690,17 +688,15 @@ int Engine::batch_add(int *id) {
 // vectors, which stay where they are until the sweep is over.
 void Engine::batch_swap(BatchCase &c) {
     modes.swap(c.modes);
-    hL.swap(c.hL);
-    hQ.swap(c.hQ);
+    hWfc.swap(c.hWfc);
+    hPhi.swap(c.hPhi);
+    std::swap(hNl, c.hNl);
     hCorr.swap(c.hCorr);
     hNodes.swap(c.hNodes);
     std::swap(hNn, c.hNn);
     hM.swap(c.hM);
     hK.swap(c.hK);
     hC.swap(c.hC);
-    hWd3.swap(c.hWd3);
-    hWd2.swap(c.hWd2);
-    hL32.swap(c.hL32);
     hPsd.swap(c.hPsd);
     hPack.swap(c.hPack);
 }

@@ -169,19 +169,19 @@ struct Engine {
     // derived (validate)
     std::vector<int> modes;
     int nme = 0, K = 0;
-    std::vector<double> phitc, hL, hQ, hM, hK, hC;
+    std::vector<double> hM, hK, hC;
+    std::vector<double> hWfc, hPhi;    // what the projection reads: [2 ntc][nnl][hNl], [nme][nnl][hNl]
+    int hNl = 0;                       // loaded DOFs of a node; 0: hWfc is the projection itself, [2 ntc][nnl][nme]
     std::vector<double> hCorr;         // packed coherences [comp][hNn (hNn + 1) / 2], or empty: the caller's array
     std::vector<int> hNodes;           // loaded nodes
     int hNn = 0;                       // nodes the packing counts
     std::vector<unsigned char> hPack;  // the derived tables as they go to the device, in one copy
-    std::vector<double> hWd3, hWd2;  // diagonal-only weights Q L^2 and L^2, [k][m]
-    std::vector<float> hL32;         // FP32 copy of L for the split-precision A(f) table
     std::vector<PsdNode> hPsd;
 
     // device
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
-    DevView dNodes, dL, dQ, dPsdPar, dFrfM, dFrfK, dFrfC, dWd3, dWd2, dL32;  // parts of dProb
+    DevView dNodes, dL, dQ, dPsdPar, dFrfM, dFrfK, dFrfC, dWd3, dWd2, dL32;  // parts of dProb (dWd3, dWd2: Q L^2 and L^2; dL32: L in FP32)
     DevBuf dProb, dLogc, dFreq, dS, dA, dPartF, dPartR, dOut, dPsdF, dWf, dPts,
         dPtsD, dBF, dBR, dMixA, dMixB, dMixH, dMixPart, dA32, dZones, dZidx, dMshT, dMshIdx, dLogc32,
         dPod, dFlag, dSlot, dHash, dCptr, dCq, dZoneH, dZoff, dCorr;

