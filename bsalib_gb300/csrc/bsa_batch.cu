@@ -406,12 +406,6 @@ __global__ void __launch_bounds__(ecls::ELayout<RS>::threads, 1)  // 128 registe
     int *err = p.err;
     if (blockIdx.x == 0 && threadIdx.x == 0) *p.t_start = gtime();
 
-    for (int s = 0; s < ecls::kStages; ++s)
-        for (int t = 2; t < 6; ++t) {
-            uint8_t *tile = smem + s * ecls::kStageBytes + t * kTileBytes;
-            for (int x = threadIdx.x; x < (128 - BROWS) * 128 / 16; x += blockDim.x)
-                ((uint4 *)(tile + BROWS * 128))[x] = make_uint4(0, 0, 0, 0);
-        }
     if (threadIdx.x == 0) {
         for (int s = 0; s < ecls::kStages; ++s) {
             mbar_init(&full[s], 1);
@@ -462,8 +456,8 @@ __global__ void __launch_bounds__(ecls::ELayout<RS>::threads, 1)  // 128 registe
                         tma_2d(st + 1 * kTileBytes, &tmUl, &full[s], x, yu);
                         tma_2d(st + 2 * kTileBytes, &tmGh, &full[s], x, yg);
                         tma_2d(st + 4 * kTileBytes, &tmGl, &full[s], x, yg);
-                        tma_2d(st + 3 * kTileBytes, &tmGh, &full[s], x, yg + BROWS);
-                        tma_2d(st + 5 * kTileBytes, &tmGl, &full[s], x, yg + BROWS);
+                        tma_2d(st + 2 * kTileBytes + BROWS * 128, &tmGh, &full[s], x, yg + BROWS);
+                        tma_2d(st + 4 * kTileBytes + BROWS * 128, &tmGl, &full[s], x, yg + BROWS);
                     }
             }
             const uint32_t last = it;
@@ -503,9 +497,9 @@ __global__ void __launch_bounds__(ecls::ELayout<RS>::threads, 1)  // 128 registe
                             const uint64_t uh = sdesc(base + 0 * kTileBytes + off), ul = sdesc(base + 1 * kTileBytes + off);
                             const uint64_t bh = sdesc(base + 2 * kTileBytes + off), bl = sdesc(base + 4 * kTileBytes + off);
                             const uint32_t acc = (kc > 0 || ks > 0) ? 1u : 0u;
-                            mma256(d, uh, bh, acc);
-                            mma256(d, uh, bl, 1u);
-                            mma256(d, ul, bh, 1u);
+                            mma_n<2 * BROWS>(d, uh, bh, acc);
+                            mma_n<2 * BROWS>(d, uh, bl, 1u);
+                            mma_n<2 * BROWS>(d, ul, bh, 1u);
                         }
                         mma_commit(&empty[s]);
                     }
@@ -581,7 +575,7 @@ __global__ void __launch_bounds__(ecls::ELayout<RS>::threads, 1)  // 128 registe
                 fence_after();
                 const UT &hb = hbs[buf];
                 for (int h2 = 0; h2 < 2; ++h2)
-                    unit_half<NMT, JH>(hb, lane_base + buf * 256 + h2 * 128, wg, a, b, h2 * NC, acc, jh * NMT);
+                    unit_half<NMT, JH>(hb, lane_base + buf * 256 + h2 * BROWS, wg, a, b, h2 * NC, acc, jh * NMT);
                 fence_before();
                 mbar_arrive(&tempty[buf]);
                 since += 2;

@@ -21,7 +21,9 @@
 // element (q = p) feeds all six at half weight (its transpose is in the same tile).
 //
 // The kernel is bsa_mixed.cu's pipeline (a TMA warp, a tcgen05 MMA warp, BF16x3, FP32 TMEM
-// accumulators, 2 stages of 96 KB, N = 256 MMAs over two N tiles of grid columns) with three
+// accumulators, 2 stages of 96 KB, one MMA over two N tiles of whole grid columns, their rows one
+// behind the other in shared memory: N = 240 at widths 12 and 24, where two tiles padded to 256
+// took 25.4 instead of 24.9 ms for the 24-mode building on the 1025^2 grid) with three
 // epilogue warpgroups on the same TMEM buffer, one per weight: the first accumulates (i), (iv)
 // and their force moment, the second (iii), (v) and theirs, the third (ii), (vi) and theirs
 // (warp layouts, plain or register split: ELayout in bsa_eform.cuh).  The FRF values a unit
@@ -71,12 +73,6 @@ __global__ void __launch_bounds__(ELayout<RS>::threads, 1)  // 128 registers a t
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int *err = P.err;
 
-    for (int s = 0; s < kStages; ++s)
-        for (int t = 2; t < 6; ++t) {
-            uint8_t *tile = smem + s * kStageBytes + t * kTileBytes;
-            for (int x = threadIdx.x; x < (128 - BROWS) * 128 / 16; x += blockDim.x)
-                ((uint4 *)(tile + BROWS * 128))[x] = make_uint4(0, 0, 0, 0);
-        }
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(&full[s], 1);
@@ -132,8 +128,8 @@ __global__ void __launch_bounds__(ELayout<RS>::threads, 1)  // 128 registers a t
                         tma_2d(st + 1 * kTileBytes, &tmUl, &full[s], x, yu);
                         tma_2d(st + 2 * kTileBytes, &tmGh, &full[s], x, yg);
                         tma_2d(st + 4 * kTileBytes, &tmGl, &full[s], x, yg);
-                        tma_2d(st + 3 * kTileBytes, &tmGh, &full[s], x, yg + BROWS);
-                        tma_2d(st + 5 * kTileBytes, &tmGl, &full[s], x, yg + BROWS);
+                        tma_2d(st + 2 * kTileBytes + BROWS * 128, &tmGh, &full[s], x, yg + BROWS);
+                        tma_2d(st + 4 * kTileBytes + BROWS * 128, &tmGl, &full[s], x, yg + BROWS);
                     }
             }
             const uint32_t last = it;
@@ -173,9 +169,9 @@ __global__ void __launch_bounds__(ELayout<RS>::threads, 1)  // 128 registers a t
                             const uint64_t uh = sdesc(base + 0 * kTileBytes + off), ul = sdesc(base + 1 * kTileBytes + off);
                             const uint64_t bh = sdesc(base + 2 * kTileBytes + off), bl = sdesc(base + 4 * kTileBytes + off);
                             const uint32_t acc = (kc > 0 || ks > 0) ? 1u : 0u;
-                            mma256(d, uh, bh, acc);
-                            mma256(d, uh, bl, 1u);
-                            mma256(d, ul, bh, 1u);
+                            mma_n<2 * BROWS>(d, uh, bh, acc);
+                            mma_n<2 * BROWS>(d, uh, bl, 1u);
+                            mma_n<2 * BROWS>(d, ul, bh, 1u);
                         }
                         mma_commit(&empty[s]);
                     }
@@ -235,13 +231,13 @@ __global__ void __launch_bounds__(ELayout<RS>::threads, 1)  // 128 registers a t
                         fence_after();
                         const UT &hb = hbs[buf];
                         const int q0 = (nt0 + 2 * u) * NC;
-                        // two N tiles: TMEM columns 0-127 hold columns q0 .., 128-255 q0 + NC ..
+                        // two N tiles: TMEM columns from 0 hold grid columns q0 .., from BROWS q0 + NC ..
                         for (int h2 = 0; h2 < 2; ++h2) {
                             if constexpr (SAMPLE)
-                                unit_half_sample<NMT, JH>(hb, lane_base + buf * 256 + h2 * 128, wg, a, b, p, q0,
+                                unit_half_sample<NMT, JH>(hb, lane_base + buf * 256 + h2 * BROWS, wg, a, b, p, q0,
                                                           h2 * NC, P, jh * NMT, vrow);
                             else
-                                unit_half<NMT, JH>(hb, lane_base + buf * 256 + h2 * 128, wg, a, b, h2 * NC, acc,
+                                unit_half<NMT, JH>(hb, lane_base + buf * 256 + h2 * BROWS, wg, a, b, h2 * NC, acc,
                                                    jh * NMT);
                         }
                         fence_before();

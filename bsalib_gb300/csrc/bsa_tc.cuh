@@ -97,6 +97,16 @@ __device__ __forceinline__ void mma256(uint32_t d, uint64_t a, uint64_t b, uint3
         "l"(a), "l"(b), "r"(kIdesc256), "r"(acc)
         : "memory");
 }
+// N a multiple of 16 up to 256
+template <int N>
+__device__ __forceinline__ void mma_n(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+    static_assert(N % 16 == 0 && N <= 256, "columns of one MMA");
+    constexpr uint32_t idesc = (kIdesc256 & ~(0x3fu << 17)) | ((uint32_t)(N / 8) << 17);
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
 __device__ __forceinline__ void mma_commit(uint64_t *b) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(b)) : "memory");
 }
