@@ -136,6 +136,19 @@ __device__ __forceinline__ void get_point(const PointSrc &ps, long long p, int &
 // Lanes (threadIdx.y) that share the partials of one third moment in the reduction kernels of the
 // split Classic forms: one lane walking every CTA's partial of seven kinds was a chain of dependent
 // loads (0.20 ms for the 64 moments of a 4-mode structure).
+// Error flags that a run's last kernel copies behind its results (null: none), so that one transfer brings
+// both: a second one to pageable memory stops the host for 8 us.
+struct EndFlags {
+    const int *a = nullptr, *b = nullptr;
+    int *out = nullptr;
+};
+__device__ __forceinline__ void end_flags(const EndFlags &f) {
+    if (f.out && blockIdx.x == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
+        f.out[0] = f.a ? *f.a : 0;
+        f.out[1] = f.b ? *f.b : 0;
+    }
+}
+
 constexpr int kRedLanes = 16;
 
 // Sum of a and b over the lanes threadIdx.y of a 32 x kRedLanes block, into lane 0 (fixed order).

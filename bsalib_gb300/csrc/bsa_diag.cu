@@ -230,7 +230,7 @@ int Engine::contract_diag(const PointSrc &ps, long long npts, int msh_form, doub
     const int G = diag::groups(npts);
     if ((e = dPartF.reserve(sizeof(double) * (size_t)G * nme)) || (e = dPartR.reserve(sizeof(double) * (size_t)G * nme)))
         return cuda_fail(e, "allocating partial sums");
-    if ((e = dOut.reserve(sizeof(double) * 5 * (size_t)nme))) return cuda_fail(e, "out");
+    if ((e = dOut.reserve(sizeof(double) * out_doubles()))) return cuda_fail(e, "out");
     double *bfd = nullptr, *brd = nullptr;
     if (bf_host || br_host) {
         if ((e = dBF.reserve(sizeof(double) * (size_t)npts * nme)) || (e = dBR.reserve(sizeof(double) * (size_t)npts * nme)))
@@ -247,20 +247,16 @@ int Engine::contract_diag(const PointSrc &ps, long long npts, int msh_form, doub
     if ((e = launch_reduce_groups(stream, G, nme, dPartF.as<double>(), o, dPartR.as<double>(), o + nme)))
         return cuda_fail(e, "reduction kernel");
     kernels += 2;
-    std::vector<double> h(2 * (size_t)nme);
-    if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)))
-        return cuda_fail(e, "moment copy");
     if (bf_host && (e = fetch(stream, bf_host, bfd, sizeof(double) * (size_t)npts * nme))) return cuda_fail(e, "bispectrum copy");
     if (br_host && (e = fetch(stream, br_host, brd, sizeof(double) * (size_t)npts * nme))) return cuda_fail(e, "bispectrum copy");
-    if ((e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream))) return cuda_fail(e, "sync");
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, ev2, ev1);
+    float ms = 0.f, ms_gemm = 0.f;
+    if ((e = results(&ms, &ms_gemm))) return cuda_fail(e, "moment copy");
     last_ms_contraction = ms;
-    cudaEventElapsedTime(&ms, evg0, evg1);
-    last_ms_gemm = ms;
-    d2h += (double)sizeof(double) * h.size() + (bf_host ? 8.0 * npts * nme : 0.0) + (br_host ? 8.0 * npts * nme : 0.0);
-    if (m3mf) std::memcpy(m3mf, h.data(), sizeof(double) * nme);
-    if (m3mr) std::memcpy(m3mr, h.data() + nme, sizeof(double) * nme);
+    last_ms_gemm = ms_gemm;
+    const double *h = hRes.data() + 3 * (size_t)nme;
+    d2h += 2.0 * sizeof(double) * nme + (bf_host ? 8.0 * npts * nme : 0.0) + (br_host ? 8.0 * npts * nme : 0.0);
+    if (m3mf) std::memcpy(m3mf, h, sizeof(double) * nme);
+    if (m3mr) std::memcpy(m3mr, h + nme, sizeof(double) * nme);
     return BSA_OK;
 }
 

@@ -214,6 +214,12 @@ struct Engine {
     int atable_check();
     cudaError_t need(DevBuf &b, size_t bytes);
     int pipeline_flags(const int *flags, bool atable, bool pairs);
+    // dOut: [second-order moments 3 dim_psd][third-order 2 dim_bisp][the last kernel's EndFlags]
+    size_t out_doubles() const { return 3 * (size_t)dim_psd() + 2 * (size_t)dim_bisp() + 1; }
+    int *out_flags() { return (int *)(dOut.as<double>() + out_doubles() - 1); }
+    cudaError_t results(float *ms_contraction, float *ms_gemm);
+    std::vector<double> hRes;  // dOut on the host, after results()
+    bool res_fresh = false;    // of the current run
     // dimM_psd_ / dimM_bisp_ (src/bsa/BsaLibImpl.F90:313-355): nm / nm for the diagonal-only
     // spectra, nm^2 / nm^3 otherwise.
     long long dim_psd() const { return set.onlyd ? nme : (long long)nme * nme; }

@@ -483,6 +483,19 @@ cudaError_t Engine::need(DevBuf &b, size_t bytes) {
     return b.reserve(bytes);
 }
 
+// Every result of a run in one transfer, and the wait for it; the times from ev2 and between evg0 and evg1.
+cudaError_t Engine::results(float *ms_contraction, float *ms_gemm) {
+    cudaError_t e;
+    hRes.resize(out_doubles());
+    if ((e = cudaMemcpyAsync(hRes.data(), dOut.p, sizeof(double) * hRes.size(), cudaMemcpyDeviceToHost, stream)) ||
+        (e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream)))
+        return e;
+    cudaEventElapsedTime(ms_contraction, ev2, ev1);
+    cudaEventElapsedTime(ms_gemm, evg0, evg1);
+    res_fresh = true;
+    return cudaSuccess;
+}
+
 // Flags read behind a run: [0] the A kernel's, [1] the pair products'.
 int Engine::pipeline_flags(const int *flags, bool atable, bool pairs) {
     if (atable) atable_pending = false;
@@ -636,8 +649,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
         }
         if ((e = upload(dWf, wf, stream))) return cuda_fail(e, "weights");
         if ((e = dPsdF.reserve(sizeof(double) * (size_t)nf * nm2))) return cuda_fail(e, "psd");
-        if ((e = dOut.reserve(sizeof(double) * (3 * (size_t)nm2 + 2 * (size_t)dim_bisp()))))
-            return cuda_fail(e, "out");
+        if ((e = dOut.reserve(sizeof(double) * out_doubles()))) return cuda_fail(e, "out");
         e = diagonal ? launch_force_psd_diag(stream, np, K, nme, dS.as<double>(), dWd2.as<double>(), dPsdF.as<double>())
             : mixed  ? launch_force_psd32(stream, np, (int)set.tc.size(), in.nnl, nme, dL32.as<float>(),
                                           dA32.as<float>(), dPsdF.as<double>())
@@ -651,6 +663,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
         kernels += 2;
     }
     last_points = 0;
+    res_fresh = false;
     if (set.ibisp && (m3mf || m3mr || bf_host || br_host)) {
         PointSrc ps{};
         ps.mode = kPointsGrid;
@@ -718,17 +731,20 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
         if (rc) return rc;
         last_points = (double)npts;
     }
-    // the second-order moments wait on the device until here, so that nothing stops the launches
-    std::vector<double> h(m2 ? 3 * (size_t)nm2 : 0);
-    if (m2 && (e = cudaMemcpyAsync(h.data(), dOut.p, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)))
-        return cuda_fail(e, "m2 copy");
-    if ((e = cudaEventRecord(ev1, stream)) || (e = cudaEventSynchronize(ev1))) return cuda_fail(e, "event");
+    // the second-order moments wait on the device until here, so that nothing stops the launches; the
+    // third-order ones brought them along
+    if (!res_fresh) {
+        hRes.resize(3 * (size_t)nm2);
+        if (m2 && (e = cudaMemcpyAsync(hRes.data(), dOut.p, sizeof(double) * hRes.size(), cudaMemcpyDeviceToHost, stream)))
+            return cuda_fail(e, "m2 copy");
+        if ((e = cudaEventRecord(ev1, stream)) || (e = cudaEventSynchronize(ev1))) return cuda_fail(e, "event");
+    }
     if ((rc = atable_check())) return rc;
     if (m2) {
-        d2h += (double)sizeof(double) * h.size();
-        if (m2mf) std::memcpy(m2mf, h.data(), sizeof(double) * nm2);
-        if (m2mr) std::memcpy(m2mr, h.data() + nm2, sizeof(double) * nm2);
-        if (m2o2mr) std::memcpy(m2o2mr, h.data() + 2 * nm2, sizeof(double) * nm2);
+        d2h += 3.0 * sizeof(double) * (double)nm2;
+        if (m2mf) std::memcpy(m2mf, hRes.data(), sizeof(double) * nm2);
+        if (m2mr) std::memcpy(m2mr, hRes.data() + nm2, sizeof(double) * nm2);
+        if (m2o2mr) std::memcpy(m2o2mr, hRes.data() + 2 * nm2, sizeof(double) * nm2);
     }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev0, ev1);
@@ -787,7 +803,7 @@ int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m
     const int G = bfm_fp64_groups(npts, nme);
     if ((e = need(dPartF, sizeof(double) * (size_t)G * nm3)) || (e = need(dPartR, sizeof(double) * (size_t)G * nm3)))
         return cuda_fail(e, "allocating partial sums");
-    if ((e = dOut.reserve(sizeof(double) * (3 * (size_t)nme * nme + 2 * (size_t)nm3)))) return cuda_fail(e, "out");
+    if ((e = dOut.reserve(sizeof(double) * out_doubles()))) return cuda_fail(e, "out");
     double *bfd = nullptr, *brd = nullptr;
     if (bf_host || br_host) {
         if ((e = need(dBF, sizeof(double) * (size_t)npts * nm3)) || (e = need(dBR, sizeof(double) * (size_t)npts * nm3)))
@@ -809,27 +825,23 @@ int Engine::contract(const PointSrc &ps, long long npts, double *m3mf, double *m
     }
     if ((e = cudaEventRecord(evg1, stream))) return cuda_fail(e, "event");
     double *o = dOut.as<double>() + 3 * (size_t)nme * nme;
-    if ((e = launch_reduce_groups(stream, G, nm3, dPartF.as<double>(), o, dPartR.as<double>(), o + nm3)))
+    const bool pend = atable_pending;
+    if ((e = launch_reduce_groups(stream, G, nm3, dPartF.as<double>(), o, dPartR.as<double>(), o + nm3,
+                                  EndFlags{pend ? dFlag.as<int>() : nullptr, list64 ? dFlag.as<int>() + 1 : nullptr, out_flags()})))
         return cuda_fail(e, "reduction kernel");
     kernels += 2;
-    std::vector<double> h(2 * (size_t)nm3);
-    int flags[2] = {0, 0};  // A table, pair products
-    const bool pend = atable_pending;
-    if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
-        ((list64 || pend) && (e = cudaMemcpyAsync(flags, dFlag.p, sizeof flags, cudaMemcpyDeviceToHost, stream))))
-        return cuda_fail(e, "moment copy");
     if (bf_host && (e = fetch(stream, bf_host, bfd, sizeof(double) * (size_t)npts * nm3))) return cuda_fail(e, "bispectrum copy");
     if (br_host && (e = fetch(stream, br_host, brd, sizeof(double) * (size_t)npts * nm3))) return cuda_fail(e, "bispectrum copy");
-    if ((e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream))) return cuda_fail(e, "sync");
+    float ms = 0.f, ms_gemm = 0.f;
+    if ((e = results(&ms, &ms_gemm))) return cuda_fail(e, "moment copy");
+    const int *flags = (const int *)(hRes.data() + out_doubles() - 1);
     if ((rc = pipeline_flags(flags, pend, list64))) return rc;
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, ev2, ev1);
     last_ms_contraction = ms;
-    cudaEventElapsedTime(&ms, evg0, evg1);
-    last_ms_gemm = ms;
-    d2h += (double)sizeof(double) * h.size() + (bf_host ? 8.0 * npts * nm3 : 0.0) + (br_host ? 8.0 * npts * nm3 : 0.0);
-    if (m3mf) std::memcpy(m3mf, h.data(), sizeof(double) * nm3);
-    if (m3mr) std::memcpy(m3mr, h.data() + nm3, sizeof(double) * nm3);
+    last_ms_gemm = ms_gemm;
+    const double *h = hRes.data() + 3 * (size_t)nme * nme;
+    d2h += 2.0 * sizeof(double) * (double)nm3 + (bf_host ? 8.0 * npts * nm3 : 0.0) + (br_host ? 8.0 * npts * nm3 : 0.0);
+    if (m3mf) std::memcpy(m3mf, h, sizeof(double) * nm3);
+    if (m3mr) std::memcpy(m3mr, h + nm3, sizeof(double) * nm3);
     return BSA_OK;
 }
 

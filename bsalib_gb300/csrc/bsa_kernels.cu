@@ -789,7 +789,8 @@ cudaError_t launch_bfm_fp64(cudaStream_t st, const double *A, const double *Q, i
 // latency: the 30-node tower's 1216 groups of 64 elements took 0.50 ms.
 __global__ void k_reduce_groups(int n_groups, long long len, const double *__restrict__ part,
                                 double *__restrict__ out, const double *__restrict__ part2,
-                                double *__restrict__ out2) {
+                                double *__restrict__ out2, EndFlags fl) {
+    end_flags(fl);
     __shared__ double red[2][32][33];
     const long long x = (long long)blockIdx.x * 32 + threadIdx.x;
     const int ty = threadIdx.y;
@@ -815,12 +816,12 @@ __global__ void k_reduce_groups(int n_groups, long long len, const double *__res
 }
 
 cudaError_t launch_reduce_groups(cudaStream_t st, int n_groups, long long len, const double *part,
-                                 double *out, const double *part2, double *out2) {
+                                 double *out, const double *part2, double *out2, EndFlags fl) {
     if (len == 0) return cudaSuccess;
     // a lane sums at most four groups where the block allows it
     int ny = 1;
     while (ny < 32 && 4 * ny < n_groups) ny *= 2;
-    k_reduce_groups<<<(unsigned)((len + 31) / 32), dim3(32, ny), 0, st>>>(n_groups, len, part, out, part2, out2);
+    k_reduce_groups<<<(unsigned)((len + 31) / 32), dim3(32, ny), 0, st>>>(n_groups, len, part, out, part2, out2, fl);
     return cudaGetLastError();
 }
 

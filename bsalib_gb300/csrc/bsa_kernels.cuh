@@ -87,6 +87,6 @@ cudaError_t launch_zone_frf(cudaStream_t st, int nz, int nm, const ZoneDev *zone
 
 // out[x] = sum_g part[g * len + x] (fixed order); optional second array.
 cudaError_t launch_reduce_groups(cudaStream_t st, int n_groups, long long len, const double *part,
-                                 double *out, const double *part2, double *out2);
+                                 double *out, const double *part2, double *out2, EndFlags fl = EndFlags());
 
 }  // namespace bsa

@@ -460,7 +460,8 @@ __global__ void k_prep_h(int nf, int nm, int NMT, const double *__restrict__ f, 
 // m3[m + nm n + nm^2 o] from the per-CTA FP64 partials: three term contributions each, and
 // with the symmetric D1 (kinds 7) term 1's mirror, kept at (m, o, n).
 __global__ void k_mixed_reduce(int nm, int NMT, int MT, int grid, int kinds, const double *__restrict__ part,
-                               double *__restrict__ m3mf, double *__restrict__ m3mr) {
+                               double *__restrict__ m3mf, double *__restrict__ m3mr, EndFlags fl) {
+    end_flags(fl);
     const int x = blockIdx.x * 32 + threadIdx.x;
     const int nm3 = nm * nm * nm;
     const int xe = x < nm3 ? x : 0;
@@ -620,26 +621,25 @@ int Engine::contract_mixed(const PointSrc &ps, long long npts, double *m3mf, dou
     if (e) return cuda_fail(e, "BF16x3 tcgen05 contraction kernel");
     if ((e = cudaEventRecord(evg1, stream))) return cuda_fail(e, "event");
     const long long nm3 = (long long)nm * nm * nm;
-    if ((e = dOut.reserve(sizeof(double) * (3 * (size_t)nm * nm + 2 * (size_t)nm3)))) return cuda_fail(e, "out");
+    if ((e = dOut.reserve(sizeof(double) * out_doubles()))) return cuda_fail(e, "out");
     double *o = dOut.as<double>() + 3 * (size_t)nm * nm;
-    k_mixed_reduce<<<(unsigned)((nm3 + 31) / 32), dim3(32, kRedLanes), 0, stream>>>(nm, W, MT, grid, kinds, prm.part, o, o + nm3);
+    const bool pend = atable_pending;
+    k_mixed_reduce<<<(unsigned)((nm3 + 31) / 32), dim3(32, kRedLanes), 0, stream>>>(nm, W, MT, grid, kinds, prm.part, o, o + nm3,
+        EndFlags{derr, pend ? dFlag.as<int>() : nullptr, out_flags()});
     if ((e = cudaGetLastError())) return cuda_fail(e, "BF16x3 reduction");
     kernels += 2;
-    std::vector<double> h(2 * (size_t)nm3);
-    int herr = 0;
-    if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
-        (e = cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, stream)) ||
-        (e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream)))
-        return cuda_fail(e, "BF16x3 contraction");
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, ev2, ev1);
+    float ms = 0.f, ms_gemm = 0.f;
+    if ((e = results(&ms, &ms_gemm))) return cuda_fail(e, "BF16x3 contraction");
     last_ms_contraction = ms;
-    cudaEventElapsedTime(&ms, evg0, evg1);
-    last_ms_gemm = ms;
-    d2h += (double)sizeof(double) * h.size() + sizeof(int);
+    last_ms_gemm = ms_gemm;
+    d2h += 2.0 * sizeof(double) * (double)nm3 + sizeof(int);
+    const int *flags = (const int *)(hRes.data() + out_doubles() - 1), herr = flags[0];
+    int rc;
+    if ((rc = pipeline_flags(flags + 1, pend, false))) return rc;
     if (herr) return fail(BSA_ERR_TIMEOUT, "BF16x3 kernel: a pipeline wait ran out of its budget (role %d)", herr);
-    if (m3mf) std::memcpy(m3mf, h.data(), sizeof(double) * nm3);
-    if (m3mr) std::memcpy(m3mr, h.data() + nm3, sizeof(double) * nm3);
+    const double *h = hRes.data() + 3 * (size_t)nm * nm;
+    if (m3mf) std::memcpy(m3mf, h, sizeof(double) * nm3);
+    if (m3mr) std::memcpy(m3mr, h + nm3, sizeof(double) * nm3);
     return BSA_OK;
 }
 

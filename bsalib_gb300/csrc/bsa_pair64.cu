@@ -307,16 +307,25 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
     }
 }
 
-// m3[m + nm n + nm^2 o] from the summed kinds [kKinds][(a, b)][j]; w4 = 2 (the BFM's factor) x 2 (a
-// point and its mirror) x d^2.
-__global__ void k_pair_finish(int nm, double w4, const double *__restrict__ S, double *__restrict__ m3mf,
-                              double *__restrict__ m3mr) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x, nm2 = nm * nm, nm3 = nm2 * nm;
-    if (x >= nm3) return;
-    const int m = x % nm, n = (x / nm) % nm, o = x / nm2;
-    auto at = [&](int kind, int a, int b, int j) { return S[((size_t)kind * nm2 + a * nm + b) * nm + j]; };
-    m3mr[x] = w4 * (at(0, m, n, o) + at(1, m, o, n) + at(2, n, m, o) + at(3, o, n, m) + at(4, n, o, m) + at(5, o, m, n));
-    m3mf[x] = w4 * (at(6, m, n, o) + at(6, m, o, n) + at(7, n, m, o) + at(7, o, m, n) + at(8, o, n, m) + at(8, n, o, m));
+// m3[m + nm n + nm^2 o] from the groups' partials [group][kKinds][(a, b)][j], lanes over the groups;
+// w4 = 2 (the BFM's factor) x 2 (a point and its mirror) x d^2.
+__global__ void k_pair_finish(int nm, int G, double w4, const double *__restrict__ S, double *__restrict__ m3mf,
+                              double *__restrict__ m3mr, EndFlags fl) {
+    end_flags(fl);
+    const int x = blockIdx.x * 32 + threadIdx.x, nm2 = nm * nm, nm3 = nm2 * nm, xe = x < nm3 ? x : 0;
+    const int m = xe % nm, n = (xe / nm) % nm, o = xe / nm2;
+    double mr = 0.0, mf = 0.0;
+    for (int g = threadIdx.y; g < G; g += kRedLanes) {
+        const double *s = S + (size_t)g * kKinds * nm3;
+        auto at = [&](int kind, int a, int b, int j) { return s[((size_t)kind * nm2 + a * nm + b) * nm + j]; };
+        mr += ((at(0, m, n, o) + at(1, m, o, n)) + (at(2, n, m, o) + at(3, o, n, m))) + (at(4, n, o, m) + at(5, o, m, n));
+        mf += ((at(6, m, n, o) + at(6, m, o, n)) + (at(7, n, m, o) + at(7, o, m, n))) + (at(8, o, n, m) + at(8, n, o, m));
+    }
+    red_lanes(mr, mf);
+    if (threadIdx.y == 0 && x < nm3) {
+        m3mr[x] = w4 * mr;
+        m3mf[x] = w4 * mf;
+    }
 }
 
 // E(x, y)[(a, b), j] of a chunk that holds every product.
@@ -484,20 +493,22 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     const size_t hb = sizeof(double2) * (size_t)(2 * N + 1) * nm, nparts = diag ? G * plans.size() : G;
     const long long plen = diag ? 2 * nb : kKinds * nb;
     const size_t ptb = sizeof(double) * (size_t)(2 * N + 1) * (2 * N + 1) * nb;
+    const bool two = !diag && G > 64;
     auto room = [&](DevBuf &b, size_t bytes) { return !e && (e = b.reserve(bytes)) == cudaErrorMemoryAllocation; };
     e = cudaSuccess;
     if (room(dMixA, sizeof(double) * (size_t)emax) || (tensor && room(dMixB, tc_col_bytes(hi + 1, an, K))) ||
         (tensor && room(dMshT, tc_row_bytes(rmax, K))) || room(dMixH, hb) || room(dMshIdx, rtb + preb) ||
-        room(dPartF, sizeof(double) * nparts * plen) || room(dPartR, sizeof(double) * (size_t)plen) ||
-        room(dOut, sizeof(double) * (3 * (size_t)dim_psd() + 2 * (size_t)nb)) || (tensor && room(dFlag, 256)) ||
+        room(dPartF, sizeof(double) * nparts * plen) || (two && room(dPartR, sizeof(double) * (size_t)plen)) ||
+        room(dOut, sizeof(double) * out_doubles()) || (tensor && room(dFlag, 256)) ||
         (bf_host && room(dBF, ptb)) || (br_host && room(dBR, ptb)))
         return kNoRoom;
     if (e) return cuda_fail(e, "allocating pair products");
     double *o = dOut.as<double>() + 3 * (size_t)dim_psd();
     char *idx = (char *)dMshIdx.p;
-    if ((e = cudaMemcpyAsync(idx, rts.data(), rtb, cudaMemcpyHostToDevice, stream)) ||
-        (e = cudaMemcpyAsync(idx + rtb, pre.data(), preb, cudaMemcpyHostToDevice, stream)))
-        return cuda_fail(e, "pair lists");
+    std::vector<char> lists(rtb + preb);
+    std::memcpy(lists.data(), rts.data(), rtb);
+    std::memcpy(lists.data() + rtb, pre.data(), preb);
+    if ((e = cudaMemcpyAsync(idx, lists.data(), lists.size(), cudaMemcpyHostToDevice, stream))) return cuda_fail(e, "pair lists");
     h2d += (double)(rtb + preb);
     if ((e = cudaEventRecord(ev2, stream)) || (e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
     const int nh = (2 * N + 1) * nm;
@@ -548,27 +559,31 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
         d2h += (double)bytes * ((bf_host ? 1 : 0) + (br_host ? 1 : 0));
         return pipeline_flags(flags, pend, tensor);
     }
-    if ((e = launch_reduce_groups(stream, (int)nparts, plen, dPartF.as<double>(), diag ? o : dPartR.as<double>(), nullptr, nullptr)))
-        return cuda_fail(e, "reduction kernel");
-    if (!diag) k_pair_finish<<<(unsigned)((nb + 127) / 128), 128, 0, stream>>>(nm, 4.0 * wval, dPartR.as<double>(), o, o + nb);
-    if ((e = cudaGetLastError())) return cuda_fail(e, "reduction kernel");
-    kernels += diag ? 2 : 3;
-    std::vector<double> h(2 * (size_t)nb);
-    int flags[2] = {0, 0}, rc;  // A table, pair products
     const bool pend = atable_pending;
-    if ((e = cudaMemcpyAsync(h.data(), o, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream)) ||
-        ((tensor || pend) && (e = cudaMemcpyAsync(flags, dFlag.p, sizeof flags, cudaMemcpyDeviceToHost, stream))) ||
-        (e = cudaEventRecord(ev1, stream)) || (e = cudaStreamSynchronize(stream)))
-        return cuda_fail(e, "moment copy");
-    if ((rc = pipeline_flags(flags, pend, tensor))) return rc;
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, ev2, ev1);
+    const EndFlags fl{pend ? dFlag.as<int>() : nullptr, tensor ? dFlag.as<int>() + 1 : nullptr, out_flags()};
+    if (diag) {
+        if ((e = launch_reduce_groups(stream, (int)nparts, plen, dPartF.as<double>(), o, nullptr, nullptr, fl)))
+            return cuda_fail(e, "reduction kernel");
+    } else {
+        // many groups (few outputs) are summed kind by kind first: 304 groups of 4 modes 9 + 4 us, by
+        // k_pair_finish alone 39; from 64 groups down it is the other way
+        if (two && (e = launch_reduce_groups(stream, G, plen, dPartF.as<double>(), dPartR.as<double>(), nullptr, nullptr)))
+            return cuda_fail(e, "reduction kernel");
+        k_pair_finish<<<(unsigned)((nb + 31) / 32), dim3(32, kRedLanes), 0, stream>>>(
+            nm, two ? 1 : G, 4.0 * wval, two ? dPartR.as<double>() : dPartF.as<double>(), o, o + nb, fl);
+    }
+    if ((e = cudaGetLastError())) return cuda_fail(e, "reduction kernel");
+    kernels += two ? 3 : 2;
+    float ms = 0.f, ms_gemm = 0.f;
+    if ((e = results(&ms, &ms_gemm))) return cuda_fail(e, "moment copy");
+    int rc;
+    if ((rc = pipeline_flags((const int *)(hRes.data() + out_doubles() - 1), pend, tensor))) return rc;
     last_ms_contraction = ms;
-    cudaEventElapsedTime(&ms, evg0, evg1);
-    last_ms_gemm = ms;
-    d2h += (double)sizeof(double) * h.size();
-    if (m3mf) std::memcpy(m3mf, h.data(), sizeof(double) * nb);
-    if (m3mr) std::memcpy(m3mr, h.data() + nb, sizeof(double) * nb);
+    last_ms_gemm = ms_gemm;
+    d2h += 2.0 * sizeof(double) * (double)nb;
+    const double *h = hRes.data() + 3 * (size_t)dim_psd();
+    if (m3mf) std::memcpy(m3mf, h, sizeof(double) * nb);
+    if (m3mr) std::memcpy(m3mr, h + nb, sizeof(double) * nb);
     return BSA_OK;
 }
 
