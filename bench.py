@@ -443,7 +443,7 @@ def accuracy_leg(prob, r_mixed, sk_mixed):
            "bars": {"bispectra": 1e-4, "skewness": 1e-3}}
     npts = nf * nf
     full = {"ms_device": ms64, "wall_s": wall64, "value": npts / (ms64 / 1e3), "unit": UNIT,
-            "form": "FP64 kernel, central symmetry of the grid (rows f1 <= 0 evaluated, mirrored weights)"}
+            "form": "products of distinct frequency pairs (every quantity on the grid is even in f), FP64 moments"}
     return acc, full
 
 
