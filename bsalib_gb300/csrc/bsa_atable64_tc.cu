@@ -187,6 +187,7 @@ __device__ __forceinline__ unsigned long long pow2neg(long long t57, const unsig
 // Column exponent of B: |s_j L_jm| < 2^e from the factors' exponents.  Block: one (f, itc).
 __global__ __launch_bounds__(256) void k_wexp(int ntc, int n, int nm, const double *__restrict__ rootS,
                                               const double *__restrict__ L, int *__restrict__ we) {
+    after_previous();
     __shared__ int mx[64];
     const int fc = blockIdx.x, itc = fc % ntc;
     if (threadIdx.x < 64) mx[threadIdx.x] = 0;
@@ -205,6 +206,7 @@ __global__ __launch_bounds__(256) void k_wexp(int ntc, int n, int nm, const doub
 __global__ __launch_bounds__(256) void k_wdigits(int ntc, int n, int nm, int np, int bw, int Kp,
                                                  const double *__restrict__ rootS, const double *__restrict__ L,
                                                  const int *__restrict__ we, __nv_bfloat16 *__restrict__ D) {
+    after_previous();
     const int blk = blockIdx.x, fc = blk / np, itc = fc % ntc, col = threadIdx.x & 31;
     const int k0 = blockIdx.y * 128 + (threadIdx.x >> 5) * 16, m = (blk - fc * np) * bw + col;
     if (k0 >= Kp || col >= bw) return;
@@ -223,6 +225,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     k_atable64_tc(const __grid_constant__ CUtensorMap tmB, int ntc, int n, int nm, int bw, int MT, int nk, int ks_last,
                   const double *__restrict__ f, const double *__restrict__ logc, const double *__restrict__ rootS,
                   const int *__restrict__ we, const int *__restrict__ bad, double *__restrict__ A, int *err) {
+    after_previous();
     if (*bad) return;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -402,7 +405,7 @@ static cudaError_t launch(cudaStream_t st, const CUtensorMap &mb, int nf, const 
     const int MT = (n + 127) / 128, nk = (n + kBK - 1) / kBK, ks_last = (n - (nk - 1) * kBK + 15) / 16;
     cudaError_t e = cudaFuncSetAttribute(k_atable64_tc<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<NP>());
     if (e != cudaSuccess) return e;
-    k_atable64_tc<NP><<<(unsigned)(nf * ntc * MT), kThreads, smem_bytes<NP>(), st>>>(mb, ntc, n, nm, bw, MT, nk, ks_last, f, logc,
+    launch_next(k_atable64_tc<NP>, (unsigned)(nf * ntc * MT), kThreads, smem_bytes<NP>(), st, mb, ntc, n, nm, bw, MT, nk, ks_last, f, logc,
                                                                                    rootS, we, bad, A, err);
     return cudaGetLastError();
 }
@@ -422,8 +425,8 @@ cudaError_t launch_atable64_tc(cudaStream_t st, int nf, const double *f, int ntc
     const size_t nb = (size_t)nf * ntc * np;
     __nv_bfloat16 *D = (__nv_bfloat16 *)scratch;
     int *we = (int *)((char *)scratch + ((nb * kDig * bw * Kp * 2 + 255) & ~(size_t)255));
-    k_wexp<<<nf * ntc, 256, 0, st>>>(ntc, nnl, nm, rootS, L, we);
-    k_wdigits<<<dim3((unsigned)nb, (Kp + 127) / 128), 256, 0, st>>>(ntc, nnl, nm, np, bw, Kp, rootS, L, we, D);
+    launch_next(k_wexp, nf * ntc, 256, 0, st, ntc, nnl, nm, rootS, L, we);
+    launch_next(k_wdigits, dim3((unsigned)nb, (Kp + 127) / 128), 256, 0, st, ntc, nnl, nm, np, bw, Kp, rootS, L, we, D);
     CUtensorMap mb;
     if (!make_map(&mb, D, Kp, (uint64_t)nb * kDig * bw, (uint32_t)bw)) return cudaErrorInvalidValue;
     return np == 1 ? launch<1>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, err)

@@ -61,6 +61,7 @@ constexpr int kThreads = 256;
 // as tf32 hi and lo (zero for m >= nm or j >= n), rows of 128 bytes in plain order.
 __global__ void k_atable_btab(int ntc, int n, int nm, int N, int nk, const float *__restrict__ L,
                               uint32_t *__restrict__ Bh, uint32_t *__restrict__ Bl) {
+    after_previous();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long tot = (long long)ntc * nk * N * kKc;
     if (t >= tot) return;
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_atable_tc(int ntc, int n, int n
                                                         const uint32_t *__restrict__ Bth,
                                                         const uint32_t *__restrict__ Btl, float *__restrict__ A,
                                                         int *err) {
+    after_previous();
     using LY = Layout<N>;
     constexpr float LOG2E = 1.4426950408889634f;
     extern __shared__ uint8_t smem_raw[];
@@ -257,13 +259,13 @@ cudaError_t launch(cudaStream_t st, int nf, const double *f, int ntc, int nnl, i
     const int MT = (nnl + kRows - 1) / kRows, nk = (nnl + kKc - 1) / kKc;
     const long long nb = (long long)ntc * nk * N * kKc;
     uint32_t *Bh = btab, *Bl = btab + nb;
-    k_atable_btab<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(ntc, nnl, nm, N, nk, L, Bh, Bl);
+    launch_next(k_atable_btab, (unsigned)((nb + 255) / 256), 256, 0, st, ntc, nnl, nm, N, nk, L, Bh, Bl);
     const size_t smem = (size_t)Layout<N>::kBars + 64 + sizeof(float) * (size_t)nk * kKc + 1024;
     cudaError_t e = cudaFuncSetAttribute(k_atable_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const long long nblk = (long long)nf * ntc * MT;
     if (nblk > 0x7fffffffLL) return cudaErrorInvalidValue;
-    k_atable_tc<N><<<(unsigned)nblk, kThreads, smem, st>>>(ntc, nnl, nm, MT, f, logc, S, Bh, Bl, A, err);
+    launch_next(k_atable_tc<N>, (unsigned)nblk, kThreads, smem, st, ntc, nnl, nm, MT, f, logc, S, Bh, Bl, A, err);
     return cudaGetLastError();
 }
 

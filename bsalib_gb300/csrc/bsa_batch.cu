@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(192, 1)
     k_bfm_batch(const __grid_constant__ CUtensorMap tmUh, const __grid_constant__ CUtensorMap tmUl,
                 const __grid_constant__ CUtensorMap tmGh, const __grid_constant__ CUtensorMap tmGl,
                 const __grid_constant__ CUtensorMap tmSh, const __grid_constant__ CUtensorMap tmSl, const BParams p) {
+    after_previous();
     constexpr int NC = kBN / NMT;
     constexpr int BROWS = NC * NMT;
     constexpr int W = NMT * JH;
@@ -363,6 +364,7 @@ __global__ void __launch_bounds__(192, 1)
 template <int NMT, int KINDS>
 __global__ void k_batch_reduce(const CaseP *__restrict__ cases, const long long *__restrict__ out_off,
                                const double *__restrict__ part, double *__restrict__ m3mf, double *__restrict__ m3mr) {
+    after_previous();
     const CaseP cs = cases[blockIdx.y];
     const int nm = cs.nm, nm3 = nm * nm * nm;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -390,6 +392,7 @@ template <int NMT, int JH, bool RS = ecls::use_regsplit(NMT, JH)>
 __global__ void __launch_bounds__(ecls::ELayout<RS>::threads, 1)  // 128 registers a thread at launch
     k_bfm_e_batch(const __grid_constant__ CUtensorMap tmUh, const __grid_constant__ CUtensorMap tmUl,
                   const __grid_constant__ CUtensorMap tmGh, const __grid_constant__ CUtensorMap tmGl, const BParams p) {
+    after_previous();
     using namespace ecls;
     constexpr int NC = kBN / NMT;
     constexpr int BROWS = NC * NMT;
@@ -619,6 +622,7 @@ __global__ void __launch_bounds__(ecls::ELayout<RS>::threads, 1)  // 128 registe
 template <int W>
 __global__ void k_batch_reduce_e(const CaseP *__restrict__ cases, const long long *__restrict__ out_off,
                                  const double *__restrict__ part, double *__restrict__ m3mf, double *__restrict__ m3mr) {
+    after_previous();
     const CaseP cs = cases[blockIdx.y];
     const int nm = cs.nm, nm3 = nm * nm * nm;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -955,7 +959,7 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
         if ((e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
         auto launch = [&](auto kern) {
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<grid, 192, smem, stream>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], prm);
+            launch_next(kern, grid, 192, smem, stream, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], prm);
         };
         // the warp layout of each instantiation (register split for the 48-mode width) is its
         // template default; a split kernel is launched only at its full launch registers
@@ -963,7 +967,7 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
             const size_t sm = (size_t)ecls::kStages * ecls::kStageBytes + 1024 + ecls::kBarBytes + 2 * ut;
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             if (rs && ecls::regsplit_check(kern) != cudaSuccess) return false;
-            kern<<<grid, rs ? ecls::ELayout<true>::threads : ecls::ELayout<false>::threads, sm, stream>>>(
+            launch_next(kern, grid, rs ? ecls::ELayout<true>::threads : ecls::ELayout<false>::threads, sm, stream,
                 maps[0], maps[1], maps[2], maps[3], prm);
             return true;
         };
@@ -997,18 +1001,18 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
         for (const CaseP &q : cp) maxnm3 = std::max(maxnm3, q.nm * q.nm * q.nm);
         dim3 rg((maxnm3 + 127) / 128, (unsigned)cp.size());
         if (eform) switch (Wd) {
-        case 8: k_batch_reduce_e<8><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
-        case 16: k_batch_reduce_e<16><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
-        case 24: k_batch_reduce_e<24><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
-        case 32: k_batch_reduce_e<32><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
-        default: k_batch_reduce_e<48><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
+        case 8: launch_next(k_batch_reduce_e<8>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
+        case 16: launch_next(k_batch_reduce_e<16>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
+        case 24: launch_next(k_batch_reduce_e<24>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
+        case 32: launch_next(k_batch_reduce_e<32>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
+        default: launch_next(k_batch_reduce_e<48>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
         }
         else switch (Wd) {
-        case 8: k_batch_reduce<8, kKinds + 2><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
-        case 16: k_batch_reduce<16, kKinds + 2><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
-        case 24: k_batch_reduce<24, kKinds + 2><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
-        case 32: k_batch_reduce<32, kKinds><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
-        default: k_batch_reduce<64, kKinds><<<rg, 128, 0, stream>>>(d_cases, d_off, part, o, o + t3); break;
+        case 8: launch_next(k_batch_reduce<8, kKinds + 2>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
+        case 16: launch_next(k_batch_reduce<16, kKinds + 2>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
+        case 24: launch_next(k_batch_reduce<24, kKinds + 2>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
+        case 32: launch_next(k_batch_reduce<32, kKinds>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
+        default: launch_next(k_batch_reduce<64, kKinds>, rg, 128, 0, stream, d_cases, d_off, part, o, o + t3); break;
         }
         if ((e = cudaGetLastError())) return cuda_fail(e, "batch reduction");
         kernels += 2;

@@ -60,6 +60,7 @@ template <int NMT, int JH, bool SAMPLE, bool RS = use_regsplit(NMT, JH)>
 __global__ void __launch_bounds__(ELayout<RS>::threads, 1)  // 128 registers a thread at launch
     k_bfm_e(const __grid_constant__ CUtensorMap tmUh, const __grid_constant__ CUtensorMap tmUl,
             const __grid_constant__ CUtensorMap tmGh, const __grid_constant__ CUtensorMap tmGl, const EParams P) {
+    after_previous();
     constexpr int NC = kBN / NMT;
     constexpr int BROWS = NC * NMT;
     constexpr int W = NMT * JH;
@@ -281,6 +282,7 @@ namespace ecls {
 // 2 F14, 3 K_iii, 4 K_v, 5 F35, 6 K_ii, 7 K_vi, 8 F26, each kept at the lane's (a, b) and j).
 __global__ void k_e_reduce(int nm, int W, int MT, int grid, const double *__restrict__ part,
                            double *__restrict__ m3mf, double *__restrict__ m3mr, EndFlags fl) {
+    after_previous();
     end_flags(fl);
     const int x = blockIdx.x * 32 + threadIdx.x;
     const int nm3 = nm * nm * nm;
@@ -318,7 +320,7 @@ static cudaError_t launch_k(cudaStream_t st, const CUtensorMap *maps, const EPar
     if (e != cudaSuccess) return e;
     constexpr bool RS = use_regsplit(NMT, JH);
     if (RS && (e = regsplit_check(k_bfm_e<NMT, JH, SAMPLE>)) != cudaSuccess) return e;
-    k_bfm_e<NMT, JH, SAMPLE><<<grid, ELayout<RS>::threads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], p);
+    launch_next(k_bfm_e<NMT, JH, SAMPLE>, grid, ELayout<RS>::threads, smem, st, maps[0], maps[1], maps[2], maps[3], p);
     return cudaGetLastError();
 }
 
@@ -442,7 +444,7 @@ int Engine::contract_e(const PointSrc &ps, double *m3mf, double *m3mr, const ESa
     if ((e = dOut.reserve(sizeof(double) * out_doubles()))) return cuda_fail(e, "out");
     double *o = dOut.as<double>() + 3 * (size_t)nm * nm;
     const bool pend = atable_pending;
-    k_e_reduce<<<(unsigned)((nm3 + 31) / 32), dim3(32, kRedLanes), 0, stream>>>(nm, W, MT, grid, prm.part, o, o + nm3,
+    launch_next(k_e_reduce, (unsigned)((nm3 + 31) / 32), dim3(32, kRedLanes), 0, stream, nm, W, MT, grid, prm.part, o, o + nm3,
         EndFlags{derr, pend ? dFlag.as<int>() : nullptr, out_flags()});
     if ((e = cudaGetLastError())) return cuda_fail(e, "BF16x3 reduction");
     kernels += 2;

@@ -43,6 +43,7 @@ __global__ __launch_bounds__(256) void k_diag_fp64(const double *__restrict__ S,
                                                    FrfPar frf, double *__restrict__ part_mf,
                                                    double *__restrict__ part_mr, double *__restrict__ bf_out,
                                                    double *__restrict__ br_out) {
+    after_previous();
     __shared__ double buf[kBuf];
     __shared__ int pix[kPts], piy[kPts], piz[kPts];
     __shared__ double pw[kPts], pf1[kPts], pf2[kPts];
@@ -184,6 +185,7 @@ __global__ __launch_bounds__(256) void k_diag_fp64(const double *__restrict__ S,
 // mode walking all k took 0.15 ms for 513 rows of 800 k.
 __global__ __launch_bounds__(256) void k_force_psd_diag(int K, int nm, const double *__restrict__ S,
                                                         const double *__restrict__ W2, double *__restrict__ psd) {
+    after_previous();
     __shared__ double red[8][32];
     const int f = blockIdx.x, m = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
     double s = 0.0;
@@ -216,7 +218,7 @@ int groups(long long npts) {
 
 cudaError_t launch_force_psd_diag(cudaStream_t st, int nf, int K, int nm, const double *S, const double *W2,
                                   double *psd) {
-    diag::k_force_psd_diag<<<dim3(nf, (nm + 31) / 32), 256, 0, st>>>(K, nm, S, W2, psd);
+    launch_next(diag::k_force_psd_diag, dim3(nf, (nm + 31) / 32), 256, 0, st, K, nm, S, W2, psd);
     return cudaGetLastError();
 }
 
@@ -239,7 +241,7 @@ int Engine::contract_diag(const PointSrc &ps, long long npts, int msh_form, doub
         brd = dBR.as<double>();
     }
     if ((e = cudaEventRecord(ev2, stream)) || (e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
-    diag::k_diag_fp64<<<G, 256, 0, stream>>>(dS.as<double>(), dWd3.as<double>(), K, nme, ps, npts, msh_form, frf(),
+    launch_next(diag::k_diag_fp64, G, 256, 0, stream, dS.as<double>(), dWd3.as<double>(), K, nme, ps, npts, msh_form, frf(),
                                              dPartF.as<double>(), dPartR.as<double>(), bfd, brd);
     if ((e = cudaGetLastError())) return cuda_fail(e, "diagonal contraction kernel");
     if ((e = cudaEventRecord(evg1, stream))) return cuda_fail(e, "event");

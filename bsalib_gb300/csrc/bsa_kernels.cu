@@ -22,6 +22,7 @@ template <typename R>
 __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 tcs, int nnl,
                             const PsdNode *__restrict__ par, int psd_type, int scaling, double *__restrict__ S,
                             double *__restrict__ expt) {
+    after_previous();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long tot = (long long)nf * ntc * nnl;
     // expt (FP64 only): sqrt(S) instead of S, and the A kernel's exponential table
@@ -81,9 +82,9 @@ cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, 
     const int blk = kExpTab;
     const unsigned grid = (unsigned)((tot + blk - 1) / blk);
     if (fp32)
-        k_nodal_psd<float><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, S, expt);
+        launch_next(k_nodal_psd<float>, grid, blk, 0, st, nf, f, ntc, tcs, nnl, par, psd_type, scaling, S, expt);
     else
-        k_nodal_psd<double><<<grid, blk, 0, st>>>(nf, f, ntc, tcs, nnl, par, psd_type, scaling, S, expt);
+        launch_next(k_nodal_psd<double>, grid, blk, 0, st, nf, f, ntc, tcs, nnl, par, psd_type, scaling, S, expt);
     return cudaGetLastError();
 }
 
@@ -130,6 +131,7 @@ __global__ __launch_bounds__(256) void k_atable(int nf, const double *__restrict
                                                 const double *__restrict__ rootS,
                                                 const double *__restrict__ L, double *__restrict__ A,
                                                 const int *__restrict__ only) {
+    after_previous();
     if (only && !*only) return;
     constexpr int RI = 64, JT = 32, NML = 4 * MPT;
     const int fi = blockIdx.x / ntc, itc = blockIdx.x % ntc;
@@ -186,6 +188,7 @@ __global__ __launch_bounds__(256) void k_atable(int nf, const double *__restrict
 __global__ void k_log_coh(int ntc, int nnl, int nn, long long ncorr, const int *__restrict__ nodes,
                           const double *__restrict__ corr, double *__restrict__ lc, float *__restrict__ lc32,
                           int *__restrict__ bad) {
+    after_previous();
     const long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= (long long)ntc * nnl * nnl) return;
     const int j = (int)(x % nnl), i = (int)(x / nnl % nnl), c = (int)(x / nnl / nnl);
@@ -206,7 +209,7 @@ cudaError_t launch_log_coh(cudaStream_t st, int ntc, int nnl, int nn, long long 
     int *bad = log_coh_bad(lc, (size_t)n);
     cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
-    k_log_coh<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ntc, nnl, nn, ncorr, nodes, corr, lc, lc32, bad);
+    launch_next(k_log_coh, (unsigned)((n + 255) / 256), 256, 0, st, ntc, nnl, nn, ncorr, nodes, corr, lc, lc32, bad);
     return cudaGetLastError();
 }
 
@@ -216,6 +219,7 @@ cudaError_t launch_log_coh(cudaStream_t st, int ntc, int nnl, int nn, long long 
 __global__ void k_project(int K, int nm, int nl, int nnl, const double *__restrict__ wfc, const double *__restrict__ phi,
                           double *__restrict__ L, double *__restrict__ Q, double *__restrict__ W3, double *__restrict__ W2,
                           float *__restrict__ L32) {
+    after_previous();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= K * nm) return;
     const int k = x / nm, m = x - k * nm;
@@ -239,7 +243,7 @@ __global__ void k_project(int K, int nm, int nl, int nnl, const double *__restri
 
 cudaError_t launch_project(cudaStream_t st, int K, int nm, int nl, const double *wfc, const double *phi, int nnl, double *L,
                            double *Q, double *W3, double *W2, float *L32) {
-    k_project<<<(K * nm + 127) / 128, 128, 0, st>>>(K, nm, nl, nnl, wfc, phi, L, Q, W3, W2, L32);
+    launch_next(k_project, (K * nm + 127) / 128, 128, 0, st, K, nm, nl, nnl, wfc, phi, L, Q, W3, W2, L32);
     return cudaGetLastError();
 }
 
@@ -253,7 +257,7 @@ cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int
     const double *expt = logc + (size_t)ntc * nnl * nnl;
 #define BSA_AT_CASE(V)                                                                          \
     if (nm <= 4 * V) {                                                                          \
-        k_atable<V><<<grid, 256, 0, st>>>(nf, f, ntc, nnl, nm, logc, expt, rootS, L, A, only);  \
+        launch_next(k_atable<V>, grid, 256, 0, st, nf, f, ntc, nnl, nm, logc, expt, rootS, L, A, only);  \
         return cudaGetLastError();                                                              \
     }
     BSA_AT_CASE(1)
@@ -280,6 +284,7 @@ cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int
 // frequency, was bound by load latency: 65 rows of the 400-node, 24-mode building 0.56 -> 0.06 ms.
 __global__ __launch_bounds__(256) void k_force_psd(int ntc, int nnl, int nm, const double *__restrict__ L,
                                                    const double *__restrict__ A, double *__restrict__ psd) {
+    after_previous();
     __shared__ double red[8][32];
     const int fi = blockIdx.x, nm2 = nm * nm, K = ntc * nnl;
     const int pr = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
@@ -302,7 +307,7 @@ __global__ __launch_bounds__(256) void k_force_psd(int ntc, int nnl, int nm, con
 cudaError_t launch_force_psd(cudaStream_t st, int nf, int ntc, int nnl, int nm, const double *L,
                              const double *A, double *psd) {
     if (nf == 0) return cudaSuccess;
-    k_force_psd<<<dim3(nf, (nm * nm + 31) / 32), 256, 0, st>>>(ntc, nnl, nm, L, A, psd);
+    launch_next(k_force_psd, dim3(nf, (nm * nm + 31) / 32), 256, 0, st, ntc, nnl, nm, L, A, psd);
     return cudaGetLastError();
 }
 
@@ -312,6 +317,7 @@ cudaError_t launch_force_psd(cudaStream_t st, int nf, int ntc, int nnl, int nm, 
 // run: 1025 rows of 800 k, 24 modes 0.46 -> 0.21 ms.
 __global__ __launch_bounds__(256) void k_force_psd32(int ntc, int nnl, int nm, const float *__restrict__ L,
                                                      const float *__restrict__ A, double *__restrict__ psd) {
+    after_previous();
     __shared__ double red[8][32];
     const int fi = blockIdx.x, nm2 = nm * nm, K = ntc * nnl;
     const int pr = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
@@ -339,7 +345,7 @@ __global__ __launch_bounds__(256) void k_force_psd32(int ntc, int nnl, int nm, c
 cudaError_t launch_force_psd32(cudaStream_t st, int nf, int ntc, int nnl, int nm, const float *L,
                                const float *A, double *psd) {
     if (nf == 0) return cudaSuccess;
-    k_force_psd32<<<dim3(nf, (nm * nm + 31) / 32), 256, 0, st>>>(ntc, nnl, nm, L, A, psd);
+    launch_next(k_force_psd32, dim3(nf, (nm * nm + 31) / 32), 256, 0, st, ntc, nnl, nm, L, A, psd);
     return cudaGetLastError();
 }
 
@@ -348,6 +354,7 @@ cudaError_t launch_force_psd32(cudaStream_t st, int nf, int ntc, int nnl, int nm
 __global__ void k_m2(int k0, int k1, int nm, int diag, const double *__restrict__ f, const double *__restrict__ wf,
                      const double *__restrict__ psd, FrfPar frf, double *m2mf, double *m2mr,
                      double *m2o2mr) {
+    after_previous();
     const int nm2 = diag ? nm : nm * nm;
     const int pr = blockIdx.x;
     const int n = diag ? pr : pr % nm, o = diag ? pr : pr / nm;
@@ -382,7 +389,7 @@ __global__ void k_m2(int k0, int k1, int nm, int diag, const double *__restrict_
 
 cudaError_t launch_m2(cudaStream_t st, int k0, int k1, int nm, int diag, const double *f, const double *wf,
                       const double *psd, FrfPar frf, double *m2mf, double *m2mr, double *m2o2mr) {
-    k_m2<<<diag ? nm : nm * nm, 256, 0, st>>>(k0, k1, nm, diag, f, wf, psd, frf, m2mf, m2mr, m2o2mr);
+    launch_next(k_m2, diag ? nm : nm * nm, 256, 0, st, k0, k1, nm, diag, f, wf, psd, frf, m2mf, m2mr, m2o2mr);
     return cudaGetLastError();
 }
 
@@ -401,6 +408,7 @@ __global__ __launch_bounds__(256) void k_bfm_fp64(const double *__restrict__ A,
                                                   double *__restrict__ part_mr,
                                                   double *__restrict__ bf_out,
                                                   double *__restrict__ br_out) {
+    after_previous();
     constexpr int MG = 256 / NOT;  // m-groups; thread owns m = mg + MG * u, u < MT
     const int tile = blockIdx.x, pg = blockIdx.y, G = gridDim.y;
     const int t = threadIdx.x, nol = t % NOT, mg = t / NOT;
@@ -707,7 +715,7 @@ static cudaError_t launch_bfm_t(cudaStream_t st, const double *A, const double *
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((nm * nm + NOT - 1) / NOT), (unsigned)n_groups);
-    kern<<<grid, 256, smem, st>>>(A, Q, K, nm, ps, npts, frf, pp, part_mf, part_mr, bf_out, br_out);
+    launch_next(kern, grid, 256, smem, st, A, Q, K, nm, ps, npts, frf, pp, part_mf, part_mr, bf_out, br_out);
     return cudaGetLastError();
 }
 
@@ -735,6 +743,7 @@ static cudaError_t launch_bfm_n(cudaStream_t st, const double *A, const double *
 // The zones' FRF tables (PointSrc::zH): a thread per value.
 __global__ void k_zone_frf(int nz, int nm, const ZoneDev *__restrict__ zones, const long long *__restrict__ zoff,
                            long long total, FrfPar frf, double2 *__restrict__ H) {
+    after_previous();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= total) return;
     int lo = 0, up = nz - 1;  // last zone that has a table starting at or before t (zoff[nz + k]: running starts)
@@ -765,7 +774,7 @@ __global__ void k_zone_frf(int nz, int nm, const ZoneDev *__restrict__ zones, co
 cudaError_t launch_zone_frf(cudaStream_t st, int nz, int nm, const ZoneDev *zones, const long long *zoff, long long total,
                             FrfPar frf, double2 *H) {
     if (total == 0) return cudaSuccess;
-    k_zone_frf<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(nz, nm, zones, zoff, total, frf, H);
+    launch_next(k_zone_frf, (unsigned)((total + 255) / 256), 256, 0, st, nz, nm, zones, zoff, total, frf, H);
     return cudaGetLastError();
 }
 
@@ -790,6 +799,7 @@ cudaError_t launch_bfm_fp64(cudaStream_t st, const double *A, const double *Q, i
 __global__ void k_reduce_groups(int n_groups, long long len, const double *__restrict__ part,
                                 double *__restrict__ out, const double *__restrict__ part2,
                                 double *__restrict__ out2, EndFlags fl) {
+    after_previous();
     end_flags(fl);
     __shared__ double red[2][32][33];
     const long long x = (long long)blockIdx.x * 32 + threadIdx.x;
@@ -821,7 +831,7 @@ cudaError_t launch_reduce_groups(cudaStream_t st, int n_groups, long long len, c
     // a lane sums at most four groups where the block allows it
     int ny = 1;
     while (ny < 32 && 4 * ny < n_groups) ny *= 2;
-    k_reduce_groups<<<(unsigned)((len + 31) / 32), dim3(32, ny), 0, st>>>(n_groups, len, part, out, part2, out2, fl);
+    launch_next(k_reduce_groups, (unsigned)((len + 31) / 32), dim3(32, ny), 0, st, n_groups, len, part, out, part2, out2, fl);
     return cudaGetLastError();
 }
 

@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(192, 1)
     k_bfm_mixed(const __grid_constant__ CUtensorMap tmUh, const __grid_constant__ CUtensorMap tmUl,
                 const __grid_constant__ CUtensorMap tmGh, const __grid_constant__ CUtensorMap tmGl,
                 const __grid_constant__ CUtensorMap tmSh, const __grid_constant__ CUtensorMap tmSl, const Params p) {
+    after_previous();
     constexpr int NC = kBN / NMT;         // grid columns per N tile
     constexpr int BROWS = NC * NMT;       // B rows loaded by TMA per tile
     constexpr int W = NMT * JH;           // FRF table width
@@ -373,6 +374,7 @@ __global__ void __launch_bounds__(192, 1)
 // Each thread writes 8 consecutive k of one row as one 16-byte store per hi / lo table.
 __global__ void k_prep_u(int nm, int K, int Kp, int Mp, const float *__restrict__ A, const double *__restrict__ Q,
                          __nv_bfloat16 *__restrict__ Uh, __nv_bfloat16 *__restrict__ Ul, int fold1) {
+    after_previous();
     const int r = blockIdx.x, k0 = blockIdx.y * 64;
     __shared__ float As[64][65], Qs[64][65];  // nm <= 64
     const float *Ar = A + (size_t)(fold1 ? abs(r + 1 - fold1) : r) * K * nm;
@@ -402,6 +404,7 @@ __global__ void k_prep_u(int nm, int K, int Kp, int Mp, const float *__restrict_
 __global__ void k_prep_b(int nm, int NMT, int j0, int K, int Kp, int nf, int n_pad, int trunc, int sum_base,
                          int is_sum, const float *__restrict__ A, __nv_bfloat16 *__restrict__ Th,
                          __nv_bfloat16 *__restrict__ Tl, int fold1) {
+    after_previous();
     const int t = blockIdx.x, k0 = blockIdx.y * 64;
     int src = t;
     if (is_sum) {
@@ -436,6 +439,7 @@ __global__ void k_prep_b(int nm, int NMT, int j0, int K, int Kp, int nf, int n_p
 // modes' real parts and imaginary parts as FP32 lane pairs.
 __global__ void k_prep_h(int nf, int nm, int NMT, const double *__restrict__ f, FrfPar frf, float2 *__restrict__ Hg,
                          float2 *__restrict__ Hs, int pairs) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int ng = nf * NMT, ns = (2 * nf - 1) * NMT;
     if (t >= ng + ns) return;
@@ -461,6 +465,7 @@ __global__ void k_prep_h(int nf, int nm, int NMT, const double *__restrict__ f, 
 // with the symmetric D1 (kinds 7) term 1's mirror, kept at (m, o, n).
 __global__ void k_mixed_reduce(int nm, int NMT, int MT, int grid, int kinds, const double *__restrict__ part,
                                double *__restrict__ m3mf, double *__restrict__ m3mr, EndFlags fl) {
+    after_previous();
     end_flags(fl);
     const int x = blockIdx.x * 32 + threadIdx.x;
     const int nm3 = nm * nm * nm;
@@ -494,20 +499,20 @@ __global__ void k_mixed_reduce(int nm, int NMT, int MT, int grid, int kinds, con
 
 cudaError_t prep_u(cudaStream_t st, int nf, int nm, int K, int Kp, int Mp, const float *A, const double *Q,
                    __nv_bfloat16 *Uh, __nv_bfloat16 *Ul, int fold1) {
-    k_prep_u<<<dim3(nf, Kp / 64), 256, 0, st>>>(nm, K, Kp, Mp, A, Q, Uh, Ul, fold1);
+    launch_next(k_prep_u, dim3(nf, Kp / 64), 256, 0, st, nm, K, Kp, Mp, A, Q, Uh, Ul, fold1);
     return cudaGetLastError();
 }
 
 cudaError_t prep_b(cudaStream_t st, int rows, int nm, int NMT, int j0, int K, int Kp, int nf, int n_pad, int trunc,
                    int sum_base, int is_sum, const float *A, __nv_bfloat16 *Th, __nv_bfloat16 *Tl, int fold1) {
-    k_prep_b<<<dim3(rows, Kp / 64), 256, 0, st>>>(nm, NMT, j0, K, Kp, nf, n_pad, trunc, sum_base, is_sum, A, Th, Tl, fold1);
+    launch_next(k_prep_b, dim3(rows, Kp / 64), 256, 0, st, nm, NMT, j0, K, Kp, nf, n_pad, trunc, sum_base, is_sum, A, Th, Tl, fold1);
     return cudaGetLastError();
 }
 
 cudaError_t prep_h(cudaStream_t st, int nf, int nm, int NMT, const double *f, FrfPar frf, float2 *Hg, float2 *Hs,
                    bool pairs) {
     const int nh = (nf + 2 * nf - 1) * NMT;
-    k_prep_h<<<(nh + 255) / 256, 256, 0, st>>>(nf, nm, NMT, f, frf, Hg, Hs, pairs ? 1 : 0);
+    launch_next(k_prep_h, (nh + 255) / 256, 256, 0, st, nf, nm, NMT, f, frf, Hg, Hs, pairs ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -517,7 +522,7 @@ static cudaError_t launch_gemm(cudaStream_t st, const CUtensorMap *maps, const P
     cudaError_t e =
         cudaFuncSetAttribute(k_bfm_mixed<NMT, JH, SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_bfm_mixed<NMT, JH, SYM><<<grid, 192, smem, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p);
+    launch_next(k_bfm_mixed<NMT, JH, SYM>, grid, 192, smem, st, maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], p);
     return cudaGetLastError();
 }
 
@@ -570,18 +575,18 @@ int Engine::contract_mixed(const PointSrc &ps, long long npts, double *m3mf, dou
     {
         const float *A = dA32.as<float>();
         dim3 gu(nf, Kp / 64);
-        k_prep_u<<<gu, 256, 0, stream>>>(nm, K, Kp, Mp, A, dQ.as<double>(), Uh, Ul, ps.fold1);
+        launch_next(k_prep_u, gu, 256, 0, stream, nm, K, Kp, Mp, A, dQ.as<double>(), Uh, Ul, ps.fold1);
         dim3 gg(nf, Kp / 64), gs(ns, Kp / 64);
         // B tables: one block of rows per mode half, modes jh NMT .. jh NMT + NMT - 1
         for (int jh = 0; jh < JH; ++jh) {
             const size_t og = (size_t)jh * nf * NMT * Kp, os = (size_t)jh * ns * NMT * Kp;
-            k_prep_b<<<gg, 256, 0, stream>>>(nm, NMT, jh * NMT, K, Kp, nf, ps.n_pad, ps.trunc, ps.sum_base, 0, A,
+            launch_next(k_prep_b, gg, 256, 0, stream, nm, NMT, jh * NMT, K, Kp, nf, ps.n_pad, ps.trunc, ps.sum_base, 0, A,
                                              Gh + og, Gl + og, ps.fold1);
-            k_prep_b<<<gs, 256, 0, stream>>>(nm, NMT, jh * NMT, K, Kp, nf, ps.n_pad, ps.trunc, ps.sum_base, 1, A,
+            launch_next(k_prep_b, gs, 256, 0, stream, nm, NMT, jh * NMT, K, Kp, nf, ps.n_pad, ps.trunc, ps.sum_base, 1, A,
                                              Sh + os, Sl + os, ps.fold1);
         }
         const int nh = (nf + ns) * W;
-        k_prep_h<<<(nh + 255) / 256, 256, 0, stream>>>(nf, nm, W, ps.fgrid, frf(), Hg, Hs, 0);
+        launch_next(k_prep_h, (nh + 255) / 256, 256, 0, stream, nf, nm, W, ps.fgrid, frf(), Hg, Hs, 0);
         if ((e = cudaGetLastError())) return cuda_fail(e, "BF16x3 operand preparation");
         kernels += 2 + 2 * JH;
     }
@@ -624,7 +629,7 @@ int Engine::contract_mixed(const PointSrc &ps, long long npts, double *m3mf, dou
     if ((e = dOut.reserve(sizeof(double) * out_doubles()))) return cuda_fail(e, "out");
     double *o = dOut.as<double>() + 3 * (size_t)nm * nm;
     const bool pend = atable_pending;
-    k_mixed_reduce<<<(unsigned)((nm3 + 31) / 32), dim3(32, kRedLanes), 0, stream>>>(nm, W, MT, grid, kinds, prm.part, o, o + nm3,
+    launch_next(k_mixed_reduce, (unsigned)((nm3 + 31) / 32), dim3(32, kRedLanes), 0, stream, nm, W, MT, grid, kinds, prm.part, o, o + nm3,
         EndFlags{derr, pend ? dFlag.as<int>() : nullptr, out_flags()});
     if ((e = cudaGetLastError())) return cuda_fail(e, "BF16x3 reduction");
     kernels += 2;

@@ -56,6 +56,7 @@ constexpr int kRow = 10;            // doubles of a row's factors
 // 30-node tower's 45 tiles: 40 -> 20 us).
 template <int ROWS>
 __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__restrict__ A, const double *__restrict__ Q) {
+    after_previous();
     constexpr int RPT = ROWS / 32, KS = 256 / ROWS;
     __shared__ double As[kKT][ROWS], Bs[kKT][kTN];
     const int t = threadIdx.x, qn = c.qn, an = c.an, rx = c.rx(), K = c.K;
@@ -115,6 +116,7 @@ __global__ __launch_bounds__(256) void k_pair_gemm(Chunk c, const double *__rest
 
 // H of the kept modes at i df, i = 0 .. 2 N.
 __global__ void k_frf_rows(int n, int nm, double df, FrfPar frf, double2 *__restrict__ H) {
+    after_previous();
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= n * nm) return;
     const int m = u % nm;
@@ -176,6 +178,7 @@ __device__ __forceinline__ PairInfo pair_info(int x, int y, int N, int vect) {
 // the FP64 pipe (84 % busy): 2145 pairs of 24 modes 0.88 ms, the sums of row factors formed
 // once a row.
 __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
+    after_previous();
     extern __shared__ double sm[];
     const int t = threadIdx.x, nm = c.an, nm2 = nm * nm;
     const int PB = P.PB, RT = P.RT, EL = RT * nm;
@@ -311,6 +314,7 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
 // w4 = 2 (the BFM's factor) x 2 (a point and its mirror) x d^2.
 __global__ void k_pair_finish(int nm, int G, double w4, const double *__restrict__ S, double *__restrict__ m3mf,
                               double *__restrict__ m3mr, EndFlags fl) {
+    after_previous();
     end_flags(fl);
     const int x = blockIdx.x * 32 + threadIdx.x, nm2 = nm * nm, nm3 = nm2 * nm, xe = x < nm3 ? x : 0;
     const int m = xe % nm, n = (xe / nm) % nm, o = xe / nm2;
@@ -348,6 +352,7 @@ __device__ __forceinline__ double pair_at(const Chunk &c, int x, int y, int a, i
 // modes: 0.55 ms by three contractions a point, 0.02 ms with the products.
 __global__ __launch_bounds__(256) void k_pair_points(Chunk c, int N, const double2 *__restrict__ H, double *__restrict__ bf,
                                                      double *__restrict__ br) {
+    after_previous();
     __shared__ double2 h[3][64];
     const int nm = c.an, nm2 = nm * nm, nm3 = nm2 * nm, nf = 2 * N + 1, p = blockIdx.x;
     const int i1 = p % nf - N, i2 = p / nf - N, i3 = i1 + i2, x = abs(i1), y = abs(i2), z = abs(i3);
@@ -376,6 +381,7 @@ __global__ __launch_bounds__(256) void k_pair_points(Chunk c, int N, const doubl
 // x with its lanes over y; part[group][0: force, 1: response][m].
 __global__ __launch_bounds__(256) void k_pair_moments_diag(Chunk c, int N, int analytic, int vect, double w4,
                                                            const double2 *__restrict__ H, double *__restrict__ part) {
+    after_previous();
     __shared__ double red[2][8];
     const int m = blockIdx.x, nm = c.qn, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double sf = 0.0, sr = 0.0;
@@ -512,7 +518,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     h2d += (double)(rtb + preb);
     if ((e = cudaEventRecord(ev2, stream)) || (e = cudaEventRecord(evg0, stream))) return cuda_fail(e, "event");
     const int nh = (2 * N + 1) * nm;
-    k_frf_rows<<<(nh + 127) / 128, 128, 0, stream>>>(2 * N + 1, nm, df, frf(), dMixH.as<double2>());
+    launch_next(k_frf_rows, (nh + 127) / 128, 128, 0, stream, 2 * N + 1, nm, df, frf(), dMixH.as<double2>());
     if (tensor && ((e = cudaMemsetAsync(dFlag.as<int>() + 1, 0, sizeof(int), stream)) ||
                    (e = tc_prep_cols(stream, hi + 1, an, K, A, dMixB.p))))
         return cuda_fail(e, "pair product operands");
@@ -525,19 +531,19 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
                 return cuda_fail(e, "pair product kernel");
             kernels += 2;
         } else {
-            if (p.items < 304) k_pair_gemm<32><<<dim3((unsigned)p.items, kTM / 32), 256, 0, stream>>>(c, A, Q);
-            else k_pair_gemm<kTM><<<dim3((unsigned)p.items, 1), 256, 0, stream>>>(c, A, Q);
+            if (p.items < 304) launch_next(k_pair_gemm<32>, dim3((unsigned)p.items, kTM / 32), 256, 0, stream, c, A, Q);
+            else launch_next(k_pair_gemm<kTM>, dim3((unsigned)p.items, 1), 256, 0, stream, c, A, Q);
         }
         if (pts) {
-            k_pair_points<<<(2 * N + 1) * (2 * N + 1), 256, 0, stream>>>(c, N, dMixH.as<double2>(), bf_host ? dBF.as<double>() : nullptr,
+            launch_next(k_pair_points, (2 * N + 1) * (2 * N + 1), 256, 0, stream, c, N, dMixH.as<double2>(), bf_host ? dBF.as<double>() : nullptr,
                                                                          br_host ? dBR.as<double>() : nullptr);
         } else if (diag) {
-            k_pair_moments_diag<<<dim3(nm, G), 256, 0, stream>>>(c, N, analytic ? 1 : 0, vect ? 1 : 0, 4.0 * wval,
+            launch_next(k_pair_moments_diag, dim3(nm, G), 256, 0, stream, c, N, analytic ? 1 : 0, vect ? 1 : 0, 4.0 * wval,
                                                                   dMixH.as<double2>(), dPartF.as<double>() + q * G * plen);
         } else {
             MomPar mp{N, vect ? 1 : 0, p.npairs, (const long long *)(idx + rtb) + p.pre0, dMixH.as<double2>(),
                       dPartF.as<double>(), q == 0 ? 1 : 0, RT, PL, PB};
-            k_pair_moments<<<dim3((unsigned)tiles, (unsigned)G), 256, smem, stream>>>(c, mp);
+            launch_next(k_pair_moments, dim3((unsigned)tiles, (unsigned)G), 256, smem, stream, c, mp);
         }
         kernels += 2;
     }
@@ -569,7 +575,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
         // k_pair_finish alone 39; from 64 groups down it is the other way
         if (two && (e = launch_reduce_groups(stream, G, plen, dPartF.as<double>(), dPartR.as<double>(), nullptr, nullptr)))
             return cuda_fail(e, "reduction kernel");
-        k_pair_finish<<<(unsigned)((nb + 31) / 32), dim3(32, kRedLanes), 0, stream>>>(
+        launch_next(k_pair_finish, (unsigned)((nb + 31) / 32), dim3(32, kRedLanes), 0, stream,
             nm, two ? 1 : G, 4.0 * wval, two ? dPartR.as<double>() : dPartF.as<double>(), o, o + nb, fl);
     }
     if ((e = cudaGetLastError())) return cuda_fail(e, "reduction kernel");

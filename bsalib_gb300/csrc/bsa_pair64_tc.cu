@@ -41,6 +41,7 @@ constexpr size_t kTcSmem = 1024 + (size_t)kRingA * kTileA + (size_t)kRingB * kTi
 
 // Column operand: exponent e[c] with |A[y][k][j]| < 2^e[c], c = y an + j.
 __global__ __launch_bounds__(256) void k_col_exp(int an, int K, const double *__restrict__ A, int *__restrict__ ec) {
+    after_previous();
     __shared__ int mx[64];
     const int y = blockIdx.x;
     if (threadIdx.x < 64) mx[threadIdx.x] = 0;
@@ -63,6 +64,7 @@ __global__ __launch_bounds__(256) void k_col_exp(int an, int K, const double *__
 // 32 rows by 8 lanes over k per block.
 __global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restrict__ A, const double *__restrict__ Q,
                                                  int *__restrict__ er) {
+    after_previous();
     __shared__ int mx[8][32];
     const int qn = c.qn, an = c.an, rx = c.rx(), ab = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
     const int x = c.xmap ? c.xmap[blockIdx.x] : c.x0 + blockIdx.x, a = ab / an, b = ab - a * an;
@@ -86,6 +88,7 @@ __global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restri
 // Column digits [ct][digit][32 columns][Kp]; block: one column tile, 128 k.
 __global__ __launch_bounds__(256) void k_col_digits(int nr, int an, int K, int Kp, const double *__restrict__ A,
                                                     const int *__restrict__ ec, __nv_bfloat16 *__restrict__ D) {
+    after_previous();
     const int ct = blockIdx.x, col = threadIdx.x & 31, k0 = blockIdx.y * 128 + (threadIdx.x >> 5) * 16;
     if (k0 >= Kp) return;
     const int c = ct * kTN + col, y = c / an, j = c - y * an;
@@ -102,6 +105,7 @@ __global__ __launch_bounds__(256) void k_col_digits(int nr, int an, int K, int K
 __global__ __launch_bounds__(256) void k_block_digits(int nm, int np, int bw, int K, int Kp, const double *__restrict__ A,
                                                       const int *__restrict__ ec, int *__restrict__ eb,
                                                       __nv_bfloat16 *__restrict__ D) {
+    after_previous();
     const int blk = blockIdx.x, col = threadIdx.x & 31, k0 = blockIdx.y * 128 + (threadIdx.x >> 5) * 16;
     const int y = blk / np, j = (blk - y * np) * bw + col;
     const bool ok = col < bw && j < nm;
@@ -121,6 +125,7 @@ __global__ __launch_bounds__(256) void k_block_digits(int nm, int np, int bw, in
 __global__ __launch_bounds__(256) void k_row_digits(Chunk c, int Kp, const double *__restrict__ A,
                                                     const double *__restrict__ Q, const int *__restrict__ er,
                                                     __nv_bfloat16 *__restrict__ D) {
+    after_previous();
     constexpr int LD = 66;  // [mode][64 k] with 16-byte aligned, staggered rows
     extern __shared__ __align__(16) double sm[];
     const int qn = c.qn, an = c.an, rx = c.rx(), K = c.K, xl = blockIdx.x, kb = blockIdx.y * 64;
@@ -153,6 +158,7 @@ template <bool LIST>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_pair_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Chunk c, PairList pl,
               int nk, int ks_last, const int *__restrict__ er, const int *__restrict__ ec, int *err) {
+    after_previous();
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t *sa = smem, *sb = smem + (size_t)kRingA * kTileA;
@@ -383,8 +389,8 @@ size_t tc_row_bytes(long long nrows, int K) {
 cudaError_t tc_prep_cols(cudaStream_t st, int nr, int an, int K, const double *A, void *cols) {
     const int Kp = kpad(K), nct = (nr * an + kTN - 1) / kTN;
     int *ec = (int *)((char *)cols + up256((size_t)nct * kDig * kTN * Kp * 2));
-    k_col_exp<<<nr, 256, 0, st>>>(an, K, A, ec);
-    k_col_digits<<<dim3(nct, (Kp + 127) / 128), 256, 0, st>>>(nr, an, K, Kp, A, ec, (__nv_bfloat16 *)cols);
+    launch_next(k_col_exp, nr, 256, 0, st, an, K, A, ec);
+    launch_next(k_col_digits, dim3(nct, (Kp + 127) / 128), 256, 0, st, nr, an, K, Kp, A, ec, (__nv_bfloat16 *)cols);
     return cudaGetLastError();
 }
 
@@ -394,18 +400,18 @@ static cudaError_t products(cudaStream_t st, const Chunk &c, const PairList &l, 
                             const double *A, const double *Q, const int *ec, void *rows, int *err) {
     const int Kp = kpad(c.K), nx = c.x1 - c.x0;
     int *er = (int *)((char *)rows + up256(ntiles * kDig * kTM * Kp * 2));
-    k_row_exp<<<dim3(nx, (c.rx() + 31) / 32), 256, 0, st>>>(c, A, Q, er);
+    launch_next(k_row_exp, dim3(nx, (c.rx() + 31) / 32), 256, 0, st, c, A, Q, er);
     const size_t sm = sizeof(double) * 66 * (c.qn + c.an);
     cudaError_t e = cudaFuncSetAttribute(k_row_digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_row_digits<<<dim3(nx, Kp / 64), 256, sm, st>>>(c, Kp, A, Q, er, (__nv_bfloat16 *)rows);
+    launch_next(k_row_digits, dim3(nx, Kp / 64), 256, sm, st, c, Kp, A, Q, er, (__nv_bfloat16 *)rows);
     CUtensorMap ma;
     if (!make_map(&ma, rows, Kp, (uint64_t)ntiles * kDig * kTM, kTM)) return cudaErrorInvalidValue;
     if ((e = cudaFuncSetAttribute(k_pair_tc<LIST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem))) return e;
     int dev = 0, nsm = 0;
     if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev))) return e;
     const int nk = Kp / kBK, ks_last = (c.K - (nk - 1) * kBK + 15) / 16;
-    k_pair_tc<LIST><<<(unsigned)std::min<long long>(nsm, c.items), kTcThreads, kTcSmem, st>>>(ma, mb, c, l, nk, ks_last, er,
+    launch_next(k_pair_tc<LIST>, (unsigned)std::min<long long>(nsm, c.items), kTcThreads, kTcSmem, st, ma, mb, c, l, nk, ks_last, er,
                                                                                              ec, err);
     return cudaGetLastError();
 }
@@ -431,8 +437,8 @@ cudaError_t tc_prep_blocks(cudaStream_t st, int nr, int nm, int K, const double 
     const size_t nb = (size_t)nr * np;
     int *eb = (int *)((char *)cols + up256(nb * kDig * bw * Kp * 2));
     int *ec = (int *)((char *)eb + up256(nb * 32 * sizeof(int)));
-    k_col_exp<<<nr, 256, 0, st>>>(nm, K, A, ec);
-    k_block_digits<<<dim3((unsigned)nb, (Kp + 127) / 128), 256, 0, st>>>(nm, np, bw, K, Kp, A, ec, eb, (__nv_bfloat16 *)cols);
+    launch_next(k_col_exp, nr, 256, 0, st, nm, K, A, ec);
+    launch_next(k_block_digits, dim3((unsigned)nb, (Kp + 127) / 128), 256, 0, st, nm, np, bw, K, Kp, A, ec, eb, (__nv_bfloat16 *)cols);
     return cudaGetLastError();
 }
 
