@@ -18,6 +18,19 @@ constexpr int kExpTab = 256;  // 2^(k / 256), k = 0 .. 255
 // split-precision paths, whose A(f) tables take sqrt(S) in FP32, evaluate the same formulas
 // in FP32 (R = float: relative error ~1e-7, where FP64's pow costs ~100 FP64 instructions).
 // ------------------------------------------------------------------------------------
+// y^(5/6) and y^(4/3): in FP64 from the square and cube roots (45 and 25 FP64 instructions, the general
+// power about 100; 205 600 spectra of Davenport's form 62 us by pow, 29 so), within its 2 ulp.
+template <typename R>
+__device__ __forceinline__ R pow56(R y) {
+    if constexpr (sizeof(R) == 8) return sqrt(y) * cbrt(y);
+    else return pow(y, R(5.0 / 6.0));
+}
+template <typename R>
+__device__ __forceinline__ R pow43(R y) {
+    if constexpr (sizeof(R) == 8) return y * cbrt(y);
+    else return pow(y, R(4.0 / 3.0));
+}
+
 template <typename R>
 __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 tcs, int nnl,
                             const PsdNode *__restrict__ par, int psd_type, int scaling, double *__restrict__ S,
@@ -36,6 +49,8 @@ __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 
     const PsdNode p = par[itc * nnl + i];
     const R fr = (R)f[fi], Ls = (R)p.Ls, U = (R)p.U, Uref = (R)p.Uref, sg = (R)p.sigma;
     const R sig2 = sg * sg;
+    // FP64: the scaling goes into each form's denominator, a division less
+    const R sc = sizeof(R) == 8 && scaling == 1 ? R(kPi4) : R(1);
     R v = 0;
     switch (psd_type) {
     case 1:
@@ -43,12 +58,13 @@ __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 
             const R rt = Ls / U;
             R x = fabs(fr) * rt;
             x = x * x;
-            x = pow(R(1) + R(70.7) * x, R(5.0 / 6.0));
-            v = R(4) * (rt * sig2) / x;
+            x = pow56(R(1) + R(70.7) * x);
+            v = R(4) * (rt * sig2) / (x * sc);
         } else {
             R d = R(2) * (fr * (Ls / U));
             d = d * d;
-            const R r2 = pow(R(1) + R(70.7) * d, R(11.0 / 6.0)) * U;
+            const R y = R(1) + R(70.7) * d;
+            const R r2 = (sizeof(R) == 8 ? y * pow56(y) : pow(y, R(11.0 / 6.0))) * U * sc;
             const R r3 = Ls * (R(1) + R(188.4) * d) / r2 * sig2;
             const R a = r3 + r3;
             v = a + a;
@@ -60,17 +76,17 @@ __global__ void k_nodal_psd(int nf, const double *__restrict__ f, int ntc, int4 
     case 3: {
         const R cst1 = R(0.65 * 1200.0);
         const R x = cst1 * fr / Uref;
-        v = cst1 * sig2 / Uref / pow(R(1) + x * x, R(5.0 / 6.0));
+        v = cst1 * sig2 / Uref / (pow56(R(1) + x * x) * sc);
     } break;
     case 5: {
         const R clu = Ls / U;
         const R cf = fabs(fr) * clu;
-        v = ((R(2.0 / 3.0)) * cf * clu * sig2) / pow(R(1) + cf * cf, R(4.0 / 3.0));
+        v = ((R(2.0 / 3.0)) * cf * clu * sig2) / (pow43(R(1) + cf * cf) * sc);
     } break;
     default:
         v = 0;
     }
-    if (scaling == 1) v = v / R(kPi4);
+    if (sizeof(R) == 4 && scaling == 1) v = v / R(kPi4);
     S[t] = (sizeof(R) == 8 && expt) ? sqrt((double)v) : (double)v;
 }
 
