@@ -136,37 +136,43 @@ struct MomPar {
 };
 
 // Relative weight of grid point (i1, i2) (BsaClassicImpl.F90:596-632, vertex -1/2), 0 beyond it.
-__device__ __forceinline__ double wrel(int i1, int i2, int N, int vect) {
+template <typename T>
+__device__ __forceinline__ T wrel(int i1, int i2, int N, int vect) {
     const int u = abs(i1), v = abs(i2);
-    if (u > N || v > N) return 0.0;
-    if (!vect) return 1.0;
-    return u == N ? (v == N ? -0.5 : 0.5) : (v == N ? 0.5 : 1.0);
+    if (u > N || v > N) return T(0);
+    if (!vect) return T(1);
+    return u == N ? (v == N ? T(-0.5) : T(0.5)) : (v == N ? T(0.5) : T(1));
 }
 
-struct PairInfo {
+// T: double, or float where the weights (multiples of 1/8, exact in either) are formed per element
+template <typename T>
+struct PairWeights {
     int x, y, region;        // 0: every weight 1; 1: w1 = w2p = w3p = 1, w2m = w3m = 0; 2: general
-    double w1, w2p, w2m, w3p, w3m, wm1, wm2, wm3;
+    T w1, w2p, w2m, w3p, w3m, wm1, wm2, wm3;
 };
 
-__device__ __forceinline__ PairInfo pair_info(int x, int y, int N, int vect) {
-    PairInfo f;
+using PairInfo = PairWeights<double>;
+
+template <typename T>
+__device__ __forceinline__ PairWeights<T> pair_info(int x, int y, int N, int vect) {
+    PairWeights<T> f;
     f.x = x;
     f.y = y;
-    const double s = (x == y ? 0.5 : 1.0) * (x == 0 && y == 0 ? 0.5 : 1.0), sm = x == 0 ? 0.0 : s;
+    const T s = (x == y ? T(0.5) : T(1)) * (x == 0 && y == 0 ? T(0.5) : T(1)), sm = x == 0 ? T(0) : s;
     // plus partners (x, y), (x - y, y), (x, y - x); minus partners (x, -y), (x + y, -y), (x, -x - y)
-    const double a1 = wrel(x, y, N, vect);
+    const T a1 = wrel<T>(x, y, N, vect);
     f.w1 = s * a1;
-    f.w2p = s * wrel(x - y, y, N, vect);
-    f.w3p = s * wrel(x, y - x, N, vect);
-    f.w2m = sm * wrel(x + y, y, N, vect);
-    f.w3m = sm * wrel(x, x + y, N, vect);
+    f.w2p = s * wrel<T>(x - y, y, N, vect);
+    f.w3p = s * wrel<T>(x, y - x, N, vect);
+    f.w2m = sm * wrel<T>(x + y, y, N, vect);
+    f.w3m = sm * wrel<T>(x, x + y, N, vect);
     f.wm1 = f.w1 + sm * a1;
     f.wm2 = f.w2p + f.w2m;
     f.wm3 = f.w3p + f.w3m;
     f.region = 2;
-    if (x > 0 && x < y && f.w1 == 1.0 && f.w2p == 1.0 && f.w3p == 1.0) {
-        if (f.w2m == 1.0 && f.w3m == 1.0) f.region = 0;
-        else if (f.w2m == 0.0 && f.w3m == 0.0) f.region = 1;
+    if (x > 0 && x < y && f.w1 == T(1) && f.w2p == T(1) && f.w3p == T(1)) {
+        if (f.w2m == T(1) && f.w3m == T(1)) f.region = 0;
+        else if (f.w2m == T(0) && f.w3m == T(0)) f.region = 1;
     }
     return f;
 }
@@ -202,7 +208,7 @@ __global__ __launch_bounds__(256) void k_pair_moments(Chunk c, MomPar P) {
                 if (P.pre[mid] <= p) lo = mid; else up = mid - 1;
             }
             const int x = c.x0 + lo;
-            PairInfo f = pair_info(x, x + (int)(p - P.pre[lo]), P.N, P.vect);
+            PairInfo f = pair_info<double>(x, x + (int)(p - P.pre[lo]), P.N, P.vect);
             info[t] = f;
         }
         __syncthreads();
@@ -378,7 +384,8 @@ __global__ __launch_bounds__(256) void k_pair_points(Chunk c, int N, const doubl
 // Diagonal-only spectra: the products are P_m(x, y) = sum_k Q_km L_km^2 S_k(x) S_k(y), rows (x, m),
 // columns y, and with a = b = j = m the twelve contributions collapse to
 // 2 (w1 + w2m + w3m) alpha + 2 (w1- + w2p + w3p) beta.  One block per (mode, group of x), a warp per
-// x with its lanes over y; part[group][0: force, 1: response][m].
+// x with its lanes over y; part[group][0: force, 1: response][m].  Bound by the FP64 pipe (20
+// instructions an element): 513 x 513 points of 24 modes 60 us with the weights formed in FP64, 44 in FP32.
 __global__ __launch_bounds__(256) void k_pair_moments_diag(Chunk c, int N, int analytic, int vect, double w4,
                                                            const double2 *__restrict__ H, double *__restrict__ part) {
     after_previous();
@@ -391,14 +398,14 @@ __global__ __launch_bounds__(256) void k_pair_moments_diag(Chunk c, int N, int a
         const double *e = c.E + rt.base + (size_t)(r - mt * kTM) * rt.nct * kTN - rt.ct0 * kTN;
         const double2 hx = H[(size_t)x * nm + m];
         for (int y = x + lane; y <= y1; y += 32) {
-            const PairInfo f = pair_info(x, y, N, vect);
+            const PairWeights<float> f = pair_info<float>(x, y, N, vect);
             const double2 hy = H[(size_t)y * nm + m], p = H[(size_t)min(x + y, 2 * N) * nm + m], d = H[(size_t)(y - x) * nm + m];
             const double qr = hx.x * hy.x, qi = hx.y * hy.y, ur = hx.x * hy.y, ui = hx.y * hy.x;
             const double al = (qr - qi) * p.x + (ur + ui) * p.y, be = (qr + qi) * d.x - (ui - ur) * d.y;
-            const double g = (f.w1 + f.w2m + f.w3m) * al + (f.wm1 - f.w1 + f.w2p + f.w3p) * be;
+            const double g = (double)(f.w1 + f.w2m + f.w3m) * al + (double)(f.wm1 - f.w1 + f.w2p + f.w3p) * be;
             const double v = 2.0 * e[y];
             sr = fma(v, g, sr);
-            sf = fma(v, f.wm1 + f.wm2 + f.wm3, sf);
+            sf = fma(v, (double)(f.wm1 + f.wm2 + f.wm3), sf);
         }
     }
     for (int h = 16; h > 0; h >>= 1) {

@@ -61,18 +61,21 @@ __global__ __launch_bounds__(256) void k_col_exp(int an, int K, const double *__
 }
 
 // Row operand: |Q[k][a] A(x)[k][b]| < 2^e[r] from the factors' exponents (at most a bit above).
-// 32 rows by 8 lanes over k per block.
-__global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restrict__ A, const double *__restrict__ Q,
+// 32 rows by 16 or 8 lanes over k per block: where the blocks fit the chip at once a lane's chain of loads
+// is the time and 16 lanes halve it (K = 800, 24 rows of 257 frequencies: 26 -> 17 us; 576 rows of 65:
+// 40 -> 36), where they do not the lanes' join counts (K = 150, 144 rows of 2222: 67 us by 8, 81 by 16).
+template <int LANES>
+__global__ __launch_bounds__(32 * LANES) void k_row_exp(Chunk c, const double *__restrict__ A, const double *__restrict__ Q,
                                                  int *__restrict__ er) {
     after_previous();
-    __shared__ int mx[8][32];
+    __shared__ int mx[LANES][32];
     const int qn = c.qn, an = c.an, rx = c.rx(), ab = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
     const int x = c.xmap ? c.xmap[blockIdx.x] : c.x0 + blockIdx.x, a = ab / an, b = ab - a * an;
     const int *q = reinterpret_cast<const int *>(Q + a) + 1, *p = reinterpret_cast<const int *>(A + (size_t)x * c.K * an + b) + 1;
     int m = 0;
     if (ab < rx)
 #pragma unroll 8
-        for (int k = lane; k < c.K; k += 8) {
+        for (int k = lane; k < c.K; k += LANES) {
             const int u = (q[(size_t)2 * k * qn] >> 20) & 0x7ff, v = (p[(size_t)2 * k * an] >> 20) & 0x7ff;
             m = max(m, expo_pair(u, v));
         }
@@ -80,7 +83,7 @@ __global__ __launch_bounds__(256) void k_row_exp(Chunk c, const double *__restri
     __syncthreads();
     if (lane == 0 && ab < rx) {
 #pragma unroll
-        for (int z = 1; z < 8; ++z) m = max(m, mx[z][threadIdx.x]);
+        for (int z = 1; z < LANES; ++z) m = max(m, mx[z][threadIdx.x]);
         er[(size_t)blockIdx.x * c.rpad + ab] = expo_of_pairs(m);
     }
 }
@@ -400,7 +403,9 @@ static cudaError_t products(cudaStream_t st, const Chunk &c, const PairList &l, 
                             const double *A, const double *Q, const int *ec, void *rows, int *err) {
     const int Kp = kpad(c.K), nx = c.x1 - c.x0;
     int *er = (int *)((char *)rows + up256(ntiles * kDig * kTM * Kp * 2));
-    launch_next(k_row_exp, dim3(nx, (c.rx() + 31) / 32), 256, 0, st, c, A, Q, er);
+    const long long eb = (long long)nx * ((c.rx() + 31) / 32);
+    if (eb <= 1216) launch_next(k_row_exp<16>, dim3(nx, (c.rx() + 31) / 32), 512, 0, st, c, A, Q, er);
+    else launch_next(k_row_exp<8>, dim3(nx, (c.rx() + 31) / 32), 256, 0, st, c, A, Q, er);
     const size_t sm = sizeof(double) * 66 * (c.qn + c.an);
     cudaError_t e = cudaFuncSetAttribute(k_row_digits, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
