@@ -181,23 +181,23 @@ __global__ __launch_bounds__(256) void k_diag_fp64(const double *__restrict__ S,
     }
 }
 
-// psd[f][m] = sum_k W2[k][m] S[f][k], W2 = L^2: 32 modes by 8 lanes over k per block.  One thread a
-// mode walking all k took 0.15 ms for 513 rows of 800 k.
-__global__ __launch_bounds__(256) void k_force_psd_diag(int K, int nm, const double *__restrict__ S,
+// psd[f][m] = sum_k W2[k][m] S[f][k], W2 = L^2: 32 modes by 16 lanes over k per block.  One thread a
+// mode walking all k took 0.15 ms for 513 rows of 800 k; 257 rows 26 us by 8 lanes, 22 by 16.
+__global__ __launch_bounds__(512) void k_force_psd_diag(int K, int nm, const double *__restrict__ S,
                                                         const double *__restrict__ W2, double *__restrict__ psd) {
     after_previous();
-    __shared__ double red[8][32];
+    __shared__ double red[16][32];
     const int f = blockIdx.x, m = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
     double s = 0.0;
     if (m < nm)
 #pragma unroll 4
-        for (int k = lane; k < K; k += 8) s = fma(W2[(size_t)k * nm + m], S[(size_t)f * K + k], s);
+        for (int k = lane; k < K; k += 16) s = fma(W2[(size_t)k * nm + m], S[(size_t)f * K + k], s);
     red[lane][threadIdx.x & 31] = s;
     __syncthreads();
     if (lane == 0 && m < nm) {
         double v = 0.0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v += red[q][threadIdx.x];
+        for (int q = 0; q < 16; ++q) v += red[q][threadIdx.x];
         psd[(size_t)f * nm + m] = v;
     }
 }
@@ -218,7 +218,7 @@ int groups(long long npts) {
 
 cudaError_t launch_force_psd_diag(cudaStream_t st, int nf, int K, int nm, const double *S, const double *W2,
                                   double *psd) {
-    launch_next(diag::k_force_psd_diag, dim3(nf, (nm + 31) / 32), 256, 0, st, K, nm, S, W2, psd);
+    launch_next(diag::k_force_psd_diag, dim3(nf, (nm + 31) / 32), 512, 0, st, K, nm, S, W2, psd);
     return cudaGetLastError();
 }
 

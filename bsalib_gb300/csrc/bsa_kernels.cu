@@ -295,35 +295,45 @@ cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int
 // Second-order path: force PSD and m2 moments (functionsImpl.F90:1548-1560, 1653-1676;
 // BsaClassicImpl.F90:149-154, 197-210).
 // ------------------------------------------------------------------------------------
-// psd[f][n + nm o] = sum_k L[k][o] A[f][k][n]: 32 pairs (n, o) by 8 lanes over k per block, the lanes'
-// sums added in shared memory in a fixed order.  One thread a pair walking all k, in one block a
-// frequency, was bound by load latency: 65 rows of the 400-node, 24-mode building 0.56 -> 0.06 ms.
-__global__ __launch_bounds__(256) void k_force_psd(int ntc, int nnl, int nm, const double *__restrict__ L,
+// psd[f][n + nm o] = sum_k L[k][o] A[f][k][n]: 32 pairs (n, o) by 8 lanes over k per block (16 where the
+// blocks are few: 291 blocks of 173 k 11 -> 8 us, 650 of 800 43 -> 50), the lanes' sums added in shared
+// memory in a fixed order.  One thread a pair walking all k, in one block a frequency, was bound by load
+// latency: 65 rows of the 400-node, 24-mode building 0.56 -> 0.06 ms.  L^T S(f) L is symmetric, so the
+// pairs n <= o stand for both: 59 -> 43 us there.
+template <int LANES>
+__global__ __launch_bounds__(32 * LANES) void k_force_psd(int ntc, int nnl, int nm, const double *__restrict__ L,
                                                    const double *__restrict__ A, double *__restrict__ psd) {
     after_previous();
-    __shared__ double red[8][32];
+    __shared__ double red[LANES][32];
     const int fi = blockIdx.x, nm2 = nm * nm, K = ntc * nnl;
-    const int pr = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
-    const int n = pr % nm, o = pr / nm;
+    const int pr = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5, np = nm * (nm + 1) / 2;
+    // pr = o (o + 1) / 2 + n, at most 2080 pairs: the root is right to less than one
+    int o = (int)((sqrtf(8.f * (float)pr + 1.f) - 1.f) * 0.5f);
+    if (o * (o + 1) / 2 > pr) --o;
+    if ((o + 1) * (o + 2) / 2 <= pr) ++o;
+    const int n = pr - o * (o + 1) / 2;
     const double *Af = A + (size_t)fi * K * nm + n, *Lo = L + o;
     double s = 0.0;
-    if (pr < nm2)
+    if (pr < np)
 #pragma unroll 4
-        for (int k = lane; k < K; k += 8) s = fma(Lo[(size_t)k * nm], Af[(size_t)k * nm], s);
+        for (int k = lane; k < K; k += LANES) s = fma(Lo[(size_t)k * nm], Af[(size_t)k * nm], s);
     red[lane][threadIdx.x & 31] = s;
     __syncthreads();
-    if (lane == 0 && pr < nm2) {
+    if (lane == 0 && pr < np) {
         double v = 0.0;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v += red[q][threadIdx.x];
-        psd[(size_t)fi * nm2 + pr] = v;
+        for (int q = 0; q < LANES; ++q) v += red[q][threadIdx.x];
+        psd[(size_t)fi * nm2 + n + nm * o] = v;
+        psd[(size_t)fi * nm2 + o + nm * n] = v;
     }
 }
 
 cudaError_t launch_force_psd(cudaStream_t st, int nf, int ntc, int nnl, int nm, const double *L,
                              const double *A, double *psd) {
     if (nf == 0) return cudaSuccess;
-    launch_next(k_force_psd, dim3(nf, (nm * nm + 31) / 32), 256, 0, st, ntc, nnl, nm, L, A, psd);
+    const dim3 grid(nf, (nm * (nm + 1) / 2 + 31) / 32);
+    if ((long long)grid.x * grid.y <= 304) launch_next(k_force_psd<16>, grid, 512, 0, st, ntc, nnl, nm, L, A, psd);
+    else launch_next(k_force_psd<8>, grid, 256, 0, st, ntc, nnl, nm, L, A, psd);
     return cudaGetLastError();
 }
 
