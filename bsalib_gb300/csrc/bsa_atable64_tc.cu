@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
-    constexpr int kPassK = 512 / kBK;  // K blocks of one exact pass
+    constexpr int kPassK = kPassMax / kBK;  // K blocks of one exact pass
 
     if (warp == 16) {
         // ---------------- B loads and MMAs ----------------
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         const int e = we[fc * nm + m];
                         out[m] = e == kBad ? __longlong_as_double(0x7ff8000000000000ll)
                                  : e == kNone ? 0.0
-                                              : si * combine(hi[p][q], lo[p][q], e - 61);
+                                              : si * combine(hi[p][q], lo[p][q], e - 62);
                     }
                 }
         }

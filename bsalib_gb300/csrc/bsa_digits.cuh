@@ -1,4 +1,4 @@
-// bsa_digits.cuh -- FP64 operands as base-128 digits for the tensor cores (the error-free splitting of
+// bsa_digits.cuh -- FP64 operands as base-256 digits for the tensor cores (the error-free splitting of
 // bsa_pair64_tc.cu, which derives it): cutting values into digits, the stacked digit MMA and the
 // combination of the level sums.
 #pragma once
@@ -14,7 +14,8 @@ namespace p64 {
 
 using namespace tc;
 
-constexpr int kDig = 8;            // digits per operand
+constexpr int kDig = 7;            // digits per operand
+constexpr int kPassMax = 128;      // k of one exact pass: 7 x 128 products of at most 2^14 within 2^24
 constexpr int kBad = 1 << 20;      // row exponent of a row that holds an infinity or a NaN
 constexpr int kNone = -(1 << 20);  // of a row of zeros
 
@@ -27,15 +28,16 @@ __device__ __forceinline__ int expo_pair(int u, int v) { return (u == 2047 || v 
 __device__ __forceinline__ int expo_of_pairs(int m) { return m == kBad ? kBad : m == 0 ? kNone : m - 2044; }
 
 // Balanced digits of an integer of at most 55 bits and sign, as floats that are exact in bf16 (low half
-// zero): add 64 to every digit, cut into 7 bits, take 64 away.
+// zero): add 128 to every digit, read the bytes (2^55 has 256 in the first), take 128 away.
 __device__ __forceinline__ void digits_of(unsigned long long x, uint32_t *f) {
-    constexpr unsigned long long kHalf = 64ull * ((1ull << 56) - 1) / 127ull;
-    const unsigned long long u = x + kHalf;
+    const unsigned long long u = x + 0x80808080808080ull;
+    const uint32_t h = (uint32_t)(u >> 32), l = (uint32_t)u;
+    f[0] = __float_as_uint(__uint_as_float(0x4B400000u + (h >> 16)) - 12583040.f);
 #pragma unroll
-    for (int s = 0; s < kDig; ++s) {
-        const int sft = 7 * (kDig - 1 - s);
-        const uint32_t d = s == 0 ? (uint32_t)(u >> sft) : (uint32_t)(u >> sft) & 127u;
-        f[s] = __float_as_uint(__uint_as_float(0x4B400000u + d - 64u) - 12582912.f);
+    for (int s = 1; s < kDig; ++s) {
+        const uint32_t b = s < 3 ? 2 - s : 6 - s;  // byte of h or l
+        const uint32_t w = __byte_perm(s < 3 ? h : l, 0x4B400000u, 0x7640u | b);
+        f[s] = __float_as_uint(__uint_as_float(w) - 12583040.f);
     }
 }
 
@@ -80,29 +82,29 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v) {
                  : "r"(taddr));
 }
 
-// Level sums (exact integers) joined: hi of levels 0 .. 3, lo of 4 .. 7.
+// Level sums (exact integers) joined: hi of levels 0 .. 3, lo of 4 .. 6.
 __device__ __forceinline__ void add_levels(const int *D, long long &hi, long long &lo) {
-    hi += (((long long)D[0] * 128 + D[1]) * 128 + D[2]) * 128 + D[3];
-    lo += (((long long)D[4] * 128 + D[5]) * 128 + D[6]) * 128 + D[7];
+    hi += (((long long)D[0] * 256 + D[1]) * 256 + D[2]) * 256 + D[3];
+    lo += ((long long)D[4] * 256 + D[5]) * 256 + D[6];
 }
 
-// (hi 2^28 + lo) 2^ex rounded once to FP64, in integer instructions.
+// (hi 2^24 + lo) 2^ex rounded once to FP64, in integer instructions.
 __device__ __forceinline__ double combine(long long hi, long long lo, int ex) {
-    long long h = hi + (lo >> 28);
-    uint32_t l = (uint32_t)lo & 0xfffffffu;
+    long long h = hi + (lo >> 24);
+    uint32_t l = (uint32_t)lo & 0xffffffu;
     const bool neg = h < 0;
     if (neg) {
         h = -h - (l != 0);
-        l = (0x10000000u - l) & 0xfffffffu;
+        l = (0x1000000u - l) & 0xffffffu;
     }
     if (h == 0 && l == 0) return 0.0;
-    const int lz = __clzll(h), E = 91 - lz + ex;
+    const int lz = __clzll(h), E = 87 - lz + ex;
     if (lz > 35 || E < -1022 || E > 1022) {  // small sums (28 bits of h at least otherwise) and the ends of the range
-        const double v = scalbn(fma((double)h, 268435456.0, (double)l), ex);
+        const double v = scalbn(fma((double)h, 16777216.0, (double)l), ex);
         return neg ? -v : v;
     }
     const unsigned long long w = ((unsigned long long)h << lz) |
-                                 (lz >= 28 ? (unsigned long long)l << (lz - 28) : (unsigned long long)(l >> (28 - lz)));
+                                 (lz >= 24 ? (unsigned long long)l << (lz - 24) : (unsigned long long)(l >> (24 - lz)));
     // top bit of w at 63: 53 bits and the rounding bit
     unsigned long long b = (w >> 11) + ((w >> 10) & 1ull) + ((unsigned long long)(E + 1022) << 52);
     if (neg) b |= 0x8000000000000000ull;

@@ -32,11 +32,12 @@ namespace p64 {
 
 using namespace tc;
 
-constexpr int kPassK = 512 / kBK;        // K blocks of one exact pass
+constexpr int kPassK = kPassMax / kBK;   // K blocks of one exact pass
 constexpr int kRingA = 8;                // A digit tiles in flight (16 KB each)
-constexpr int kRingB = 2;                // B tiles in flight (32 KB each)
+constexpr int kRingB = 2;                // B tiles in flight (28 KB each)
 constexpr int kTileA = kTM * 128, kTileB = kDig * kTN * 128;
-constexpr int kTcThreads = 192;
+constexpr int kEpiW = 8;                 // epilogue warps: two a TMEM lane quarter, half the columns each
+constexpr int kTcThreads = 64 + 32 * kEpiW, kEpiC = kTN * 4 / kEpiW;
 constexpr size_t kTcSmem = 1024 + (size_t)kRingA * kTileA + (size_t)kRingB * kTileB + 512;
 
 // Column operand: exponent e[c] with |A[y][k][j]| < 2^e[c], c = y an + j.
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
-            mbar_init(&tempty[b], 128);
+            mbar_init(&tempty[b], 32 * kEpiW);
         }
         mbar_init(done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -271,7 +272,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                             if (!mbar_wait(&fa[sA], (ia / kRingA) & 1u, err, 3)) { ok = false; break; }
                             fence_after();
                             const uint32_t ab = su32(sa + sA * kTileA);
-                            // N = (8 - s) 32 columns from level s on
+                            // N = (7 - s) 32 columns from level s on
                             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                                                    ((uint32_t)((kDig - s) * kTN >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
 #pragma unroll
@@ -293,9 +294,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
         __syncwarp();
     } else {
-        // ---------------- epilogue: 128 rows, one a thread ----------------
-        const int quarter = warp & 3, row = quarter * 32 + lane;
-        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16);
+        // ---------------- epilogue: 128 rows, kEpiC columns of one a thread ----------------
+        const int quarter = warp & 3, row = quarter * 32 + lane, c0 = ((warp - 2) >> 2) * kEpiC;
+        const uint32_t lane_base = tmem + ((uint32_t)(quarter * 32) << 16) + c0;
         const int nrows = (c.x1 - c.x0) * c.rx(), ncols = (c.hi + 1) * c.an;
         uint32_t tile = 0;
         bool ok = true;
@@ -311,16 +312,16 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 rt = c.rt[mt];
                 ct = rt.ct0 + (int)(item - rt.item0);
             }
-            long long hi[kTN], lo[kTN];
+            long long hi[kEpiC], lo[kEpiC];
 #pragma unroll
-            for (int q = 0; q < kTN; ++q) hi[q] = lo[q] = 0;
+            for (int q = 0; q < kEpiC; ++q) hi[q] = lo[q] = 0;
             for (int k0 = 0; k0 < nk && ok; k0 += kPassK, ++tile) {
                 const int buf = tile & 1;
                 ok = __all_sync(0xffffffffu, mbar_wait(&tfull[buf], (tile >> 1) & 1u, err, 4));
                 if (!ok) break;
                 fence_after();
 #pragma unroll
-                for (int cg = 0; cg < kTN / 8; ++cg) {
+                for (int cg = 0; cg < kEpiC / 8; ++cg) {
                     uint32_t v[kDig][8];
 #pragma unroll
                     for (int l = 0; l < kDig; ++l) tmem_ld8(lane_base + buf * 256 + l * kTN + cg * 8, v[l]);
@@ -336,21 +337,21 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 fence_before();
                 mbar_arrive(&tempty[buf]);
             }
-            // value = 2^(er + ec - 61) (hi 2^28 + lo)
+            // value = 2^(er + ec - 62) (hi 2^24 + lo)
             auto value = [&](int q, int eu, int ev) {
                 return (eu == kBad || ev == kBad)     ? __longlong_as_double(0x7ff8000000000000ll)
                        : (eu == kNone || ev == kNone) ? 0.0
-                                                      : combine(hi[q], lo[q], eu + ev - 61);
+                                                      : combine(hi[q], lo[q], eu + ev - 62);
             };
             if (LIST) {
                 const int nm = c.an, r = (mt % pl.tiles_x) * kTM + row;
                 if (ok && r < c.rx()) {
                     const int eu = er[mt * kTM + row];
 #pragma unroll
-                    for (int q = 0; q < kTN; ++q) {
-                        const int s = (q >= pl.bw) + (q >= 2 * pl.bw) + (q >= 3 * pl.bw);
+                    for (int q = 0; q < kEpiC; ++q) {
+                        const int cc = c0 + q, s = (cc >= pl.bw) + (cc >= 2 * pl.bw) + (cc >= 3 * pl.bw);
                         if (s >= it.z) continue;
-                        const int blk = pl.blk[it.y + s], cq = q - s * pl.bw, j = (blk % pl.np) * pl.bw + cq;
+                        const int blk = pl.blk[it.y + s], cq = cc - s * pl.bw, j = (blk % pl.np) * pl.bw + cq;
                         if (j < nm)
                             c.E[((size_t)pl.pair[it.y + s] * c.rx() + r) * nm + j] = value(q, eu, ec[blk * 32 + cq]);
                     }
@@ -360,10 +361,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             const int r = mt * kTM + row;
             if (ok && r < nrows) {
                 const int eu = er[r];
-                double *o = c.E + rt.base + (size_t)row * rt.nct * kTN + (size_t)(ct - rt.ct0) * kTN;
+                double *o = c.E + rt.base + (size_t)row * rt.nct * kTN + (size_t)(ct - rt.ct0) * kTN + c0;
 #pragma unroll
-                for (int q = 0; q < kTN; q += 2) {
-                    const int col = ct * kTN + q;
+                for (int q = 0; q < kEpiC; q += 2) {
+                    const int col = ct * kTN + c0 + q;
                     *reinterpret_cast<double2 *>(o + q) = make_double2(value(q, eu, col < ncols ? ec[col] : kNone),
                                                                        value(q + 1, eu, col + 1 < ncols ? ec[col + 1] : kNone));
                 }
