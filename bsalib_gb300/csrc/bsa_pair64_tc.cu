@@ -3,21 +3,23 @@
 // D. Mukunoki, K. Ozaki, T. Ogita, T. Imamura, ISC 2020).
 //
 // Each operand row (fixed x, a, b or y, j; contiguous k) is scaled by a power of two above its
-// largest magnitude, rounded to a 56-bit integer and cut into eight balanced base-128 digits
-// |d| <= 64, stored as bf16 (exact).  The digit products s + t = l < 8 are summed in FP32 in TMEM:
-// at most 8 x 512 products of at most 2^12, so every partial sum is an integer within 2^24 and
-// exact; longer K is cut into passes of 512 whose sums meet in 64-bit integers.  The eight level
+// largest magnitude, rounded to a 56-bit integer and cut into seven balanced base-256 digits
+// |d| <= 128, stored as bf16 (exact).  The digit products s + t = l < 7 are summed in FP32 in TMEM:
+// at most 7 x 128 products of at most 2^14, so every partial sum is an integer within 2^24 and
+// exact; longer K is cut into passes of 128 whose sums meet in 64-bit integers.  The seven level
 // sums combine exactly in integers and round once to FP64, with no FP64 instruction (the pipe is
 // two lanes an SM and clock).  Rounding the rows at 2^-55 of their scale and leaving out the levels
-// s + t >= 8 is an error of about sqrt(8 K) 2^-57 of the row scales' product, below that of K
+// s + t >= 7 is an error of about sqrt(6 K) 2^-57 of the row scales' product, below that of K
 // FP64 FMAs.
 //
-// Cost: 36 digit products of bf16 against the DFMA kernel's one FP64 FMA: 36 / 4096 clocks of an SM
-// against 1 / 2.  Tile: 128 rows by 32 columns; the B digits of the tile are stacked along N (256
-// rows), so A digit s meets B digits 0 .. 7 - s in one MMA of N = (8 - s) 32 whose columns land on
-// levels s .. 7: 8 MMAs a K step instead of 36, and 512 TMEM columns hold two tiles.
-// 400 nodes x 2 components, 24 modes, 65 rows: FP64 pipe 40.5 ms; 1.33 ms here (8.5e11 digit FMAs,
-// 0.65 of the bf16 rate), row digits 0.11 ms.
+// Cost: 28 digit products of bf16 against the DFMA kernel's one FP64 FMA: 28 / 4096 clocks of an SM
+// against 1 / 2.  Tile: 128 rows by 32 columns; the B digits of the tile are stacked along N (224
+// rows), so A digit s meets B digits 0 .. 6 - s in one MMA of N = (7 - s) 32 whose columns land on
+// levels s .. 6: 7 MMAs a K step instead of 28, and 512 TMEM columns hold two tiles.  Bound by shared
+// memory at long K (operand reads and TMA writes take 1.6 times the MMA clocks), by the drain of the
+// level sums at short K: 16 warps share it.  400 nodes x 2 components, 24 modes, 65 rows: FP64 pipe
+// 40.5 ms; 1.19 ms here (6.6e11 digit FMAs), row digits 0.09 ms.  With eight base-128 digits (36
+// products, passes of 512) and 4 drain warps: 1.35 ms; 173 nodes, 11 modes, 97 rows 0.181 -> 0.079.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -33,10 +35,10 @@ namespace p64 {
 using namespace tc;
 
 constexpr int kPassK = kPassMax / kBK;   // K blocks of one exact pass
-constexpr int kRingA = 8;                // A digit tiles in flight (16 KB each)
+constexpr int kRingA = kDig;             // A digit tiles in flight (16 KB each): digit s in slot s
 constexpr int kRingB = 2;                // B tiles in flight (28 KB each)
 constexpr int kTileA = kTM * 128, kTileB = kDig * kTN * 128;
-constexpr int kEpiW = 8;                 // epilogue warps: two a TMEM lane quarter, half the columns each
+constexpr int kEpiW = 16;                // epilogue warps: four a TMEM lane quarter, a quarter of the columns each
 constexpr int kTcThreads = 64 + 32 * kEpiW, kEpiC = kTN * 4 / kEpiW;
 constexpr size_t kTcSmem = 1024 + (size_t)kRingA * kTileA + (size_t)kRingB * kTileB + 512;
 
@@ -227,10 +229,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         tma_2d(sb + sB * kTileB, &tmB, &fb[sB], kb * kBK, ct * kDig * kTN);
                     }
                     for (int s = 0; s < kDig; ++s, ++ia) {
-                        const int sA = ia % kRingA;
-                        if (!mbar_wait(&ea[sA], ((ia / kRingA) & 1u) ^ 1u, err, 1)) { ok = false; break; }
-                        mbar_expect_tx(&fa[sA], kTileA);
-                        tma_2d(sa + sA * kTileA, &tmA, &fa[sA], kb * kBK, (mt * kDig + s) * kTM);
+                        if (!mbar_wait(&ea[s], (ib & 1u) ^ 1u, err, 1)) { ok = false; break; }
+                        mbar_expect_tx(&fa[s], kTileA);
+                        tma_2d(sa + s * kTileA, &tmA, &fa[s], kb * kBK, (mt * kDig + s) * kTM);
                     }
                 }
             }
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            uint32_t ia = 0, ib = 0, tile = 0;
+            uint32_t ib = 0, tile = 0;
             bool ok = true;
             for (long long item = blockIdx.x; item < c.items && ok; item += gridDim.x) {
                 for (int k0 = 0; k0 < nk && ok; k0 += kPassK, ++tile) {
@@ -267,11 +268,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         // unrolled: with the loops kept, issuing took longer than the MMAs (a product
                         // of 400 nodes x 2 components, 24 modes, 65 rows 1.80 ms, unrolled 1.33 ms)
 #pragma unroll
-                        for (int s = 0; s < kDig; ++s, ++ia) {
-                            const int sA = ia % kRingA;
-                            if (!mbar_wait(&fa[sA], (ia / kRingA) & 1u, err, 3)) { ok = false; break; }
+                        for (int s = 0; s < kDig; ++s) {
+                            if (!mbar_wait(&fa[s], ib & 1u, err, 3)) { ok = false; break; }
                             fence_after();
-                            const uint32_t ab = su32(sa + sA * kTileA);
+                            const uint32_t ab = su32(sa + s * kTileA);
                             // N = (7 - s) 32 columns from level s on
                             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                                                    ((uint32_t)((kDig - s) * kTN >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                 if (ks < nks)
                                     mma_n(d + s * kTN, sdesc(ab + ks * 32), sdesc(bb + ks * 32), idesc,
                                           (kb > k0 || ks > 0 || s > 0) ? 1u : 0u);
-                            mma_commit(&ea[sA]);
+                            mma_commit(&ea[s]);
                         }
                         if (ok) mma_commit(&eb[sB]);
                     }
