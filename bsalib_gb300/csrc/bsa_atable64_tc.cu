@@ -7,14 +7,15 @@
 //   * t = -|f| log2 c in 57 fraction bits (one FP64 multiply and one conversion), 2^-t = 2^-n T1[k1]
 //     T2[k2] (1 - e): two tables of 2^(-k / 256) and 2^(-k / 65536) in 63 bits and
 //     e = x - x^2/2 + x^3/6, x < 2^-16 ln 2, in 64-bit integer products; the next term is below 2^-70;
-//   * c_ij^|f| <= 1 and c_ii = 1, so the row scale is 1: eight balanced base-128 digits of its 55
+//   * c_ij^|f| <= 1 and c_ii = 1, so the row scale is 1: seven balanced base-256 digits of its 55
 //     fraction bits go straight to shared memory as bf16;
 //   * B = s_j L_jm has its digits prepared per frequency and component (k_wexp, k_wdigits), its column
 //     scale from the exponents.
 // One block per (f, itc, 128 rows): 16 warps generate digits of 32 columns at a time into two halves of
 // the A tiles and drain TMEM at the end, one thread loads B and issues the MMAs.  Bound by the integer
 // instructions of the generation (about 110 an element).  3333 frequencies, 150 nodes, 12 modes: FP64
-// pipe 3.9 ms, here 1.10 ms and 0.09 for the B digits; 65 rows of 400 nodes x 2, 24 modes: 1.70 / 0.27.  Coherences outside [0, 1] or c_ii != 1 (bad
+// pipe 3.9 ms, here 1.10 ms and 0.09 for the B digits; 65 rows of 400 nodes x 2, 24 modes: 1.70 / 0.27
+// (0.23 of it this kernel with passes of K = 512, 0.25 with those of 128 that seven digits need).  Coherences outside [0, 1] or c_ii != 1 (bad
 // flag of the coherence table) leave the table to k_atable.
 #include <cuda.h>
 #include <cuda_bf16.h>
