@@ -20,18 +20,23 @@
 namespace bsa {
 
 // Whether a point set goes this way: the point kernel's time against that of the digits and products
-// plus the listing of the pairs, from measured rates (ms, point kernel / pair products):
-//   zones of 1523 points, K = 400, 16 modes 9.46 / 0.77;  936, K = 200, 14: 2.60 / 0.44;
-//   2594, K = 120, 10: 1.88 / 0.54;  1620, K = 600, 4: 0.52 / 0.20;
-//   scattered points (no pair shared) 1111, K = 150, 12: 1.43 / 1.31;  1000, K = 200, 12: 1.70 / 1.25;
-//   1000, K = 150, 8: 0.41 / 0.59;  2000, K = 40, 6: 0.21 / 0.59;  300, K = 60, 10: 0.11 / 0.17.
+// plus the listing of the pairs, from measured rates.  Contraction in ms, point kernel / pair products
+// (kept modes nm, K):
+//   scattered points (no pair shared): 100, nm 16, K 40: 0.131 / 0.111;  50, 10, 120: 0.091 / 0.074;  200,
+//   10, 120: 0.227 / 0.126;  500, 6, 120: 0.182 / 0.181;  200, 6, 300: 0.204 / 0.158;  100, 6, 120: 0.062 /
+//   0.078;  1000, 8, 40: 0.165 / 0.226;  500, 3, 300: 0.130 / 0.248;  1000, 4, 400: 0.309 / 0.576;
+//   zones of 144 points: nm 8, K 60: 0.060 / 0.068;  3, 600: 0.114 / 0.085;  6, 240: 0.099 / 0.074;  256 points,
+//   4, 120: 0.052 / 0.068;  1600, 4, 120: 0.184 / 0.168;  1600, 3, 60: 0.140 / 0.186;  1024, 8, 60: 0.235 / 0.146;
+//   1523, 16, 400: 9.46 / 0.55.
 bool Engine::list64_wanted(long long npts, int nr) const {
     using namespace p64;
-    // the column digits grow with the rows (5 times the A rows at 16 modes): within 32 GB
-    if (K < 24 || tc_block_bytes(nr, nme, K) > ((size_t)32 << 30)) return false;
+    // the column digits grow with the rows (5 times the A rows at 16 modes): within 32 GB; up to 16 points
+    // both are launches and chains over K
+    if (K < 24 || npts <= 16 || tc_block_bytes(nr, nme, K) > ((size_t)32 << 30)) return false;
     const double nm = nme, rows = (double)std::min<long long>(nr, 2 * npts) * ((nme * nme + kTM - 1) / kTM) * kTM;
-    const double point_ms = 2.0 * K * nm * nm * nm * (double)npts / (nme < 8 ? 2.0e8 : 4.2e8);
-    const double pair_ms = 0.07 + 1.2e-4 * (double)npts + rows * ((K + 63) / 64 * 64) * 1.0e-8;
+    // a point's chain over K, then the FP64 pipe
+    const double point_ms = 0.03 + K * (nme < 8 ? 1.4e-4 : 3.0e-4) + 2.0 * K * nm * nm * nm * (double)npts / (nme < 8 ? 2.0e8 : 4.2e8);
+    const double pair_ms = 0.06 + (4.1e-5 + 1.0e-7 * nm * nm * nm) * (double)npts + rows * ((K + 63) / 64 * 64) * 4.5e-9;
     return pair_ms < point_ms;
 }
 
