@@ -43,7 +43,10 @@ def test_no_room_for_products(bsalib, call, trunc):
 
     want, n0 = run()
     torch.cuda.empty_cache()
-    hold = torch.empty(torch.cuda.mem_get_info()[0] - (224 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - (224 << 20), dtype=torch.uint8, device="cuda")
+    except torch.OutOfMemoryError:
+        pytest.skip("another process took device memory meanwhile")
     try:
         got, n1 = run()
     finally:
