@@ -7,16 +7,15 @@
 //   * t = -|f| log2 c in 57 fraction bits (one FP64 multiply and one conversion), 2^-t = 2^-n T1[k1]
 //     T2[k2] (1 - e): two tables of 2^(-k / 256) and 2^(-k / 65536) in 63 bits and
 //     e = x - x^2/2 + x^3/6, x < 2^-16 ln 2, in 64-bit integer products; the next term is below 2^-70;
-//   * c_ij^|f| <= 1 and c_ii = 1, so the row scale is 1: seven balanced base-256 digits of its 55
+//   * c_ij^|f| <= 1 and c_ii = 1, so the row scale is 1: eight balanced base-256 digits of its 62
 //     fraction bits go straight to shared memory as bf16;
 //   * B = s_j L_jm has its digits prepared per frequency and component (k_wexp, k_wdigits), its column
 //     scale from the exponents.
 // One block per (f, itc, 128 rows): 16 warps generate digits of 32 columns at a time into two halves of
 // the A tiles and drain TMEM at the end, one thread loads B and issues the MMAs.  Bound by the integer
-// instructions of the generation (about 110 an element).  3333 frequencies, 150 nodes, 12 modes: FP64
-// pipe 3.9 ms, here 1.10 ms and 0.09 for the B digits; 65 rows of 400 nodes x 2, 24 modes: 1.70 / 0.27
-// (0.23 of it this kernel with passes of K = 512, 0.25 with those of 128 that seven digits need).  Coherences outside [0, 1] or c_ii != 1 (bad
-// flag of the coherence table) leave the table to k_atable.
+// instructions of the generation (about 110 an element).  65 rows of 400 nodes x 2, 24 modes: FP64 pipe
+// 1.70 ms, here 0.25 and 0.04 for the B digits.  Coherences outside [0, 1] or c_ii != 1 (bad flag of the
+// coherence table) leave the table to k_atable.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -170,7 +169,7 @@ constexpr int kTileA = 128 * 128, kTileB = kDig * 32 * 128;
 template <int NP>
 constexpr size_t smem_bytes() { return 1024 + (size_t)kDig * kTileA + (size_t)NP * kTileB + 4096 + 256; }
 
-// 2^-t as an integer of 55 fraction bits, t57 = t 2^57 >= 0.
+// 2^-t as an integer of 62 fraction bits, t57 = t 2^57 >= 0.
 __device__ __forceinline__ unsigned long long pow2neg(long long t57, const unsigned long long *T) {
     const unsigned long long t = (unsigned long long)t57;
     const int n = (int)(t >> 57);
@@ -181,8 +180,7 @@ __device__ __forceinline__ unsigned long long pow2neg(long long t57, const unsig
     const unsigned long long e = x - (x2 >> 1) + __umulhi(x3, 0x2aaaaaabu);    // 2^80 (x - x^2/2 + x^3/6)
     const unsigned long long v = __umul64hi(T[(t >> 49) & 255], T[256 + ((t >> 41) & 255)]);  // 62 fraction bits
     const unsigned long long p = v - (__umul64hi(v, e) >> 16);
-    const int sh = n + 7;
-    return sh < 64 ? (p + (1ull << (sh - 1))) >> sh : 0ull;
+    return n == 0 ? p : n < 64 ? (p + (1ull << (n - 1))) >> n : 0ull;
 }
 
 // Column exponent of B: |s_j L_jm| < 2^e from the factors' exponents.  Block: one (f, itc).
@@ -336,7 +334,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         for (int z = 0; z < 2; ++z) {
                             const int j = j0 + 2 * q + z;
                             const unsigned long long x = j >= n       ? 0ull
-                                                         : af == 0.0 ? 1ull << 55
+                                                         : af == 0.0 ? 1ull << 62
                                                                      : pow2neg(__double2ll_rn(l[2 * q + z] * k57), T);
                             digits_of(x, d[z]);
                         }
@@ -358,17 +356,20 @@ __global__ void __launch_bounds__(kThreads, 1)
                 if (ok) {
 #pragma unroll
                     for (int p = 0; p < NP; ++p) {
-                        uint32_t v[kDig][8];
 #pragma unroll
-                        for (int t = 0; t < kDig; ++t)
-                            tmem_ld8(tmem + ((uint32_t)(quarter * 32) << 16) + p * 256 + t * 32 + cg * 8, v[t]);
-                        tmem_wait_ld();
+                        for (int z = 0; z < 2; ++z) {
+                            uint32_t v[4][8];
 #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            int D[kDig];
+                            for (int t = 0; t < 4; ++t)
+                                tmem_ld8(tmem + ((uint32_t)(quarter * 32) << 16) + p * 256 + (4 * z + t) * 32 + cg * 8, v[t]);
+                            tmem_wait_ld();
 #pragma unroll
-                            for (int t = 0; t < kDig; ++t) D[t] = __float2int_rn(__uint_as_float(v[t][q]));
-                            add_levels(D, hi[p][q], lo[p][q]);
+                            for (int q = 0; q < 8; ++q) {
+                                int D[4];
+#pragma unroll
+                                for (int t = 0; t < 4; ++t) D[t] = __float2int_rn(__uint_as_float(v[t][q]));
+                                (z ? lo : hi)[p][q] += join_levels(D);
+                            }
                         }
                     }
                 }
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         const int e = we[fc * nm + m];
                         out[m] = e == kBad ? __longlong_as_double(0x7ff8000000000000ll)
                                  : e == kNone ? 0.0
-                                              : si * combine(hi[p][q], lo[p][q], e - 62);
+                                              : si * combine(hi[p][q], lo[p][q], e - 68);
                     }
                 }
         }

@@ -14,8 +14,8 @@ namespace p64 {
 
 using namespace tc;
 
-constexpr int kDig = 7;            // digits per operand
-constexpr int kPassMax = 128;      // k of one exact pass: 7 x 128 products of at most 2^14 within 2^24
+constexpr int kDig = 8;            // digits per operand
+constexpr int kPassMax = 128;      // k of one exact pass: 8 x 128 products of at most 2^14 within 2^24
 constexpr int kBad = 1 << 20;      // row exponent of a row that holds an infinity or a NaN
 constexpr int kNone = -(1 << 20);  // of a row of zeros
 
@@ -27,21 +27,19 @@ __device__ __forceinline__ int expo(double v) { return (__double2hiint(v) >> 20)
 __device__ __forceinline__ int expo_pair(int u, int v) { return (u == 2047 || v == 2047) ? kBad : (u && v) ? u + v : 0; }
 __device__ __forceinline__ int expo_of_pairs(int m) { return m == kBad ? kBad : m == 0 ? kNone : m - 2044; }
 
-// Balanced digits of an integer of at most 55 bits and sign, as floats that are exact in bf16 (low half
-// zero): add 128 to every digit, read the bytes (2^55 has 256 in the first), take 128 away.
+// Balanced digits of an integer of at most 62 bits and sign, as floats that are exact in bf16 (low half
+// zero): add 128 to every digit, read the bytes, take 128 away.
 __device__ __forceinline__ void digits_of(unsigned long long x, uint32_t *f) {
-    const unsigned long long u = x + 0x80808080808080ull;
+    const unsigned long long u = x + 0x8080808080808080ull;
     const uint32_t h = (uint32_t)(u >> 32), l = (uint32_t)u;
-    f[0] = __float_as_uint(__uint_as_float(0x4B400000u + (h >> 16)) - 12583040.f);
 #pragma unroll
-    for (int s = 1; s < kDig; ++s) {
-        const uint32_t b = s < 3 ? 2 - s : 6 - s;  // byte of h or l
-        const uint32_t w = __byte_perm(s < 3 ? h : l, 0x4B400000u, 0x7640u | b);
+    for (int s = 0; s < kDig; ++s) {
+        const uint32_t w = __byte_perm(s < 4 ? h : l, 0x4B400000u, 0x7640u | (uint32_t)(3 - (s & 3)));
         f[s] = __float_as_uint(__uint_as_float(w) - 12583040.f);
     }
 }
 
-// NV (8 or 16) values of one row, scaled by 2^(55 - e), as digits: dst[s plane + 0 .. NV - 1].
+// NV (8 or 16) values of one row, scaled by 2^(62 - e), as digits: dst[s plane + 0 .. NV - 1].
 template <int NV>
 __device__ __forceinline__ void put_digits(const double *v, int e, __nv_bfloat16 *dst, size_t plane) {
     uint32_t w[kDig][NV / 2];
@@ -51,7 +49,7 @@ __device__ __forceinline__ void put_digits(const double *v, int e, __nv_bfloat16
 #pragma unroll
         for (int z = 0; z < 2; ++z) {
             const double x = v[2 * q + z];
-            const int ex = expo(x), sh = 3 + (ex - 1023) - e;
+            const int ex = expo(x), sh = 10 + (ex - 1023) - e;
             unsigned long long m = ((unsigned long long)__double_as_longlong(x) & 0xfffffffffffffull) | 0x10000000000000ull;
             if (sh >= 0) m <<= sh;
             else if (sh > -60) m = (m + (1ull << (-sh - 1))) >> -sh;
@@ -82,29 +80,28 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v) {
                  : "r"(taddr));
 }
 
-// Level sums (exact integers) joined: hi of levels 0 .. 3, lo of 4 .. 6.
-__device__ __forceinline__ void add_levels(const int *D, long long &hi, long long &lo) {
-    hi += (((long long)D[0] * 256 + D[1]) * 256 + D[2]) * 256 + D[3];
-    lo += ((long long)D[4] * 256 + D[5]) * 256 + D[6];
+// Level sums (exact integers) joined: hi of levels 0 .. 3, lo of 4 .. 7.
+__device__ __forceinline__ long long join_levels(const int *D) {
+    return (((long long)D[0] * 256 + D[1]) * 256 + D[2]) * 256 + D[3];
 }
 
-// (hi 2^24 + lo) 2^ex rounded once to FP64, in integer instructions.
+// (hi 2^32 + lo) 2^ex rounded once to FP64, in integer instructions.
 __device__ __forceinline__ double combine(long long hi, long long lo, int ex) {
-    long long h = hi + (lo >> 24);
-    uint32_t l = (uint32_t)lo & 0xffffffu;
+    long long h = hi + (lo >> 32);
+    uint32_t l = (uint32_t)lo;
     const bool neg = h < 0;
     if (neg) {
         h = -h - (l != 0);
-        l = (0x1000000u - l) & 0xffffffu;
+        l = 0u - l;
     }
     if (h == 0 && l == 0) return 0.0;
-    const int lz = __clzll(h), E = 87 - lz + ex;
-    if (lz > 35 || E < -1022 || E > 1022) {  // small sums (28 bits of h at least otherwise) and the ends of the range
-        const double v = scalbn(fma((double)h, 16777216.0, (double)l), ex);
+    const int lz = __clzll(h), E = 95 - lz + ex;
+    if (lz > 35 || E < -1022 || E > 1022) {  // small sums (29 bits of h at least otherwise) and the ends of the range
+        const double v = scalbn(fma((double)h, 4294967296.0, (double)l), ex);
         return neg ? -v : v;
     }
     const unsigned long long w = ((unsigned long long)h << lz) |
-                                 (lz >= 24 ? (unsigned long long)l << (lz - 24) : (unsigned long long)(l >> (24 - lz)));
+                                 (lz >= 32 ? (unsigned long long)l << (lz - 32) : (unsigned long long)l >> (32 - lz));
     // top bit of w at 63: 53 bits and the rounding bit
     unsigned long long b = (w >> 11) + ((w >> 10) & 1ull) + ((unsigned long long)(E + 1022) << 52);
     if (neg) b |= 0x8000000000000000ull;

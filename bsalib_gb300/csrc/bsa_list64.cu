@@ -30,8 +30,8 @@ namespace bsa {
 //   1523, 16, 400: 9.46 / 0.55.
 bool Engine::list64_wanted(long long npts, int nr) const {
     using namespace p64;
-    // the column digits grow with the rows (5 times the A rows at 16 modes): within 32 GB; up to 16 points
-    // both are launches and chains over K
+    // the column digits grow with the rows (twice the A rows, modes padded to eights and K to 64): within
+    // 32 GB; up to 16 points both are launches and chains over K
     if (K < 24 || npts <= 16 || tc_block_bytes(nr, nme, K) > ((size_t)32 << 30)) return false;
     const double nm = nme, rows = (double)std::min<long long>(nr, 2 * npts) * ((nme * nme + kTM - 1) / kTM) * kTM;
     // a point's chain over K, then the FP64 pipe
@@ -72,7 +72,7 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
     const long long nm3 = (long long)rx * nm;
     cudaError_t e;
     // products of a batch: at most 8 GB, and the row digits at most 8 GB (two row operands a point at most)
-    const long long rowb = (long long)tc_row_bytes((long long)tiles_x * kTM, K);
+    const long long rowb = (long long)tc_row_bytes((long long)tiles_x * kTM, K, 0);
     const long long cap = 8LL << 30;
     const long long batch = std::max(1LL, std::min({npts, cap / (24 * nm3), cap / (2 * rowb)}));
     // no room for the column digits, or later for a batch: the point kernel on what is left
@@ -170,7 +170,7 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
         const size_t ib = sizeof(int4) * items.size(), lb = sizeof(int) * blk.size(), xb = sizeof(int) * xmap.size(),
                      pb = sizeof(int) * pe.size();
         e = dMixA.reserve(sizeof(double) * (size_t)nu * nm3);
-        if (!e) e = dMshT.reserve(tc_row_bytes((long long)xmap.size() * tiles_x * kTM, K));
+        if (!e) e = dMshT.reserve(tc_row_bytes((long long)xmap.size() * tiles_x * kTM, K, (long long)items.size()));
         if (!e) e = dMshIdx.reserve(ib + 2 * lb + xb + pb);
         if (e == cudaErrorMemoryAllocation) return rest(p0);
         if (e) return cuda_fail(e, "allocating pair products");
@@ -196,7 +196,7 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
                                  dPartR.as<double>(), bfd ? bfd + (size_t)p0 * nm3 : nullptr,
                                  brd ? brd + (size_t)p0 * nm3 : nullptr, pp)))
             return cuda_fail(e, "FP64 point kernel");
-        kernels += 4;
+        kernels += 5;
         if (p0 + n < npts && (e = cudaStreamSynchronize(stream))) return cuda_fail(e, "pair products");  // the lists are rewritten
     }
     return BSA_OK;

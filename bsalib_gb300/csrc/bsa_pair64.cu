@@ -471,7 +471,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     std::vector<Plan> plans;
     std::vector<RowTile> rts;
     std::vector<long long> pre;
-    long long emax = 0, rmax = 0;
+    long long emax = 0, rmax = 0, imax = 0;
     const bool pts = bf_host || br_host;
     for (int x0 = 0; x0 <= N;) {
         Plan p{x0, x0, 0, 0, 0, 0, rts.size(), pre.size()};
@@ -499,6 +499,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
         p.ntiles = (int)(rts.size() - p.rt0);
         emax = std::max(emax, p.elems);
         rmax = std::max(rmax, rows);
+        imax = std::max(imax, p.items);
         plans.push_back(p);
         x0 = p.x1;
     }
@@ -510,7 +511,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     auto room = [&](DevBuf &b, size_t bytes) { return !e && (e = b.reserve(bytes)) == cudaErrorMemoryAllocation; };
     e = cudaSuccess;
     if (room(dMixA, sizeof(double) * (size_t)emax) || (tensor && room(dMixB, tc_col_bytes(hi + 1, an, K))) ||
-        (tensor && room(dMshT, tc_row_bytes(rmax, K))) || room(dMixH, hb) || room(dMshIdx, rtb + preb) ||
+        (tensor && room(dMshT, tc_row_bytes(rmax, K, imax))) || room(dMixH, hb) || room(dMshIdx, rtb + preb) ||
         room(dPartF, sizeof(double) * nparts * plen) || (two && room(dPartR, sizeof(double) * (size_t)plen)) ||
         room(dOut, sizeof(double) * out_doubles()) || (tensor && room(dFlag, 256)) ||
         (bf_host && room(dBF, ptb)) || (br_host && room(dBR, ptb)))
@@ -536,7 +537,7 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
         if (tensor) {
             if ((e = tc_products(stream, c, hi + 1, A, Q, dMixB.p, dMshT.p, dFlag.as<int>() + 1)))
                 return cuda_fail(e, "pair product kernel");
-            kernels += 2;
+            kernels += 3;
         } else {
             if (p.items < 304) launch_next(k_pair_gemm<32>, dim3((unsigned)p.items, kTM / 32), 256, 0, stream, c, A, Q);
             else launch_next(k_pair_gemm<kTM>, dim3((unsigned)p.items, 1), 256, 0, stream, c, A, Q);

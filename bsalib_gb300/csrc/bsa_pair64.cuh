@@ -53,10 +53,10 @@ __device__ __forceinline__ int tile_row(const Chunk &c, long long item) {
 }
 
 // Tensor-core products.  tc_col_bytes / tc_row_bytes: scratch of the column operand (nr rows of the A
-// table) and of the row operand of nrows product rows.  tc_prep_cols once per analysis, then
+// table) and of the row operand of nrows product rows in items tiles.  tc_prep_cols once per analysis, then
 // tc_products per chunk.  err receives a nonzero code if a pipeline wait ran out of its budget.
 size_t tc_col_bytes(int nr, int an, int K);
-size_t tc_row_bytes(long long nrows, int K);
+size_t tc_row_bytes(long long nrows, int K, long long items);
 cudaError_t tc_prep_cols(cudaStream_t st, int nr, int an, int K, const double *A, void *cols);
 cudaError_t tc_products(cudaStream_t st, const Chunk &c, int nr, const double *A, const double *Q, void *cols,
                         void *rows, int *err);

@@ -3,23 +3,28 @@
 // D. Mukunoki, K. Ozaki, T. Ogita, T. Imamura, ISC 2020).
 //
 // Each operand row (fixed x, a, b or y, j; contiguous k) is scaled by a power of two above its
-// largest magnitude, rounded to a 56-bit integer and cut into seven balanced base-256 digits
-// |d| <= 128, stored as bf16 (exact).  The digit products s + t = l < 7 are summed in FP32 in TMEM:
-// at most 7 x 128 products of at most 2^14, so every partial sum is an integer within 2^24 and
-// exact; longer K is cut into passes of 128 whose sums meet in 64-bit integers.  The seven level
+// largest magnitude, rounded to a 62-bit integer and cut into eight balanced base-256 digits
+// |d| <= 128, stored as bf16 (exact).  The digit products s + t = l < 8 are summed in FP32 in TMEM:
+// at most 8 x 128 products of at most 2^14, so every partial sum is an integer within 2^24 and
+// exact; longer K is cut into passes of 128 whose sums meet in 64-bit integers.  The eight level
 // sums combine exactly in integers and round once to FP64, with no FP64 instruction (the pipe is
-// two lanes an SM and clock).  Rounding the rows at 2^-55 of their scale and leaving out the levels
-// s + t >= 7 is an error of about sqrt(6 K) 2^-57 of the row scales' product, below that of K
-// FP64 FMAs.
+// two lanes an SM and clock).
 //
-// Cost: 28 digit products of bf16 against the DFMA kernel's one FP64 FMA: 28 / 4096 clocks of an SM
-// against 1 / 2.  Tile: 128 rows by 32 columns; the B digits of the tile are stacked along N (224
-// rows), so A digit s meets B digits 0 .. 6 - s in one MMA of N = (7 - s) 32 whose columns land on
-// levels s .. 6: 7 MMAs a K step instead of 28, and 512 TMEM columns hold two tiles.  Bound by shared
-// memory at long K (operand reads and TMA writes take 1.6 times the MMA clocks), by the drain of the
+// Error: rounding the rows at 2^-63 of their scale and leaving out the levels s + t >= 8 is an absolute
+// error of at most K 2^-59 of the row's scale times the column's.  Against the FP64 FMAs' bound K 2^-53
+// sum |a_k b_k| that is no more wherever the sum is at least 2^-6 of the scales; an element whose terms are
+// all smaller (two modes that move different nodes) is found and computed again on the FP64 pipe
+// (k_pair_mend), so every element keeps FP64's own precision.  With seven digits the bound was met only from
+// four times the scales up: elements between two groups of nodes 50 m apart were off by 2e-11 of themselves.
+//
+// Cost: 36 digit products of bf16 against the DFMA kernel's one FP64 FMA: 36 / 4096 clocks of an SM
+// against 1 / 2.  Tile: 128 rows by 32 columns; the B digits of the tile are stacked along N (256
+// rows), so A digit s meets B digits 0 .. 7 - s in one MMA of N = (8 - s) 32 whose columns land on
+// levels s .. 7: 8 MMAs a K step instead of 36, and 512 TMEM columns hold two tiles.  Bound by shared
+// memory at long K (operand reads and TMA writes exceed the MMA clocks), by the drain of the
 // level sums at short K: 16 warps share it.  400 nodes x 2 components, 24 modes, 65 rows: FP64 pipe
-// 40.5 ms; 1.19 ms here (6.6e11 digit FMAs), row digits 0.09 ms.  With eight base-128 digits (36
-// products, passes of 512) and 4 drain warps: 1.35 ms; 173 nodes, 11 modes, 97 rows 0.181 -> 0.079.
+// 40.5 ms; 1.32 ms here (8.5e11 digit FMAs), row digits 0.10 ms, the search for small elements 0.09 ms; 173
+// nodes, 11 modes, 97 rows 86 us, 13 and 28.  Seven digits: 1.19 ms and 79 us.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -36,10 +41,12 @@ using namespace tc;
 
 constexpr int kPassK = kPassMax / kBK;   // K blocks of one exact pass
 constexpr int kRingA = kDig;             // A digit tiles in flight (16 KB each): digit s in slot s
-constexpr int kRingB = 2;                // B tiles in flight (28 KB each)
+constexpr int kRingB = 2;                // B tiles in flight (32 KB each)
 constexpr int kTileA = kTM * 128, kTileB = kDig * kTN * 128;
 constexpr int kEpiW = 16;                // epilogue warps: four a TMEM lane quarter, a quarter of the columns each
 constexpr int kTcThreads = 64 + 32 * kEpiW, kEpiC = kTN * 4 / kEpiW;
+constexpr float kSmall = 1.f / 64;       // k_pair_mend
+constexpr long long kSmallHi = 1LL << 30;
 constexpr size_t kTcSmem = 1024 + (size_t)kRingA * kTileA + (size_t)kRingB * kTileB + 512;
 
 // Column operand: exponent e[c] with |A[y][k][j]| < 2^e[c], c = y an + j.
@@ -163,7 +170,7 @@ __global__ __launch_bounds__(256) void k_row_digits(Chunk c, int Kp, const doubl
 template <bool LIST>
 __global__ void __launch_bounds__(kTcThreads, 1)
     k_pair_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Chunk c, PairList pl,
-              int nk, int ks_last, const int *__restrict__ er, const int *__restrict__ ec, int *err) {
+              int nk, int ks_last, const int *__restrict__ er, const int *__restrict__ ec, uint8_t *__restrict__ small, int *err) {
     after_previous();
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -272,7 +279,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                             if (!mbar_wait(&fa[s], ib & 1u, err, 3)) { ok = false; break; }
                             fence_after();
                             const uint32_t ab = su32(sa + s * kTileA);
-                            // N = (7 - s) 32 columns from level s on
+                            // N = (8 - s) 32 columns from level s on
                             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
                                                    ((uint32_t)((kDig - s) * kTN >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
 #pragma unroll
@@ -322,26 +329,32 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 fence_after();
 #pragma unroll
                 for (int cg = 0; cg < kEpiC / 8; ++cg) {
-                    uint32_t v[kDig][8];
 #pragma unroll
-                    for (int l = 0; l < kDig; ++l) tmem_ld8(lane_base + buf * 256 + l * kTN + cg * 8, v[l]);
-                    tmem_wait_ld();
+                    for (int z = 0; z < 2; ++z) {  // levels 0 .. 3, then 4 .. 7
+                        uint32_t v[4][8];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        int D[kDig];
+                        for (int l = 0; l < 4; ++l) tmem_ld8(lane_base + buf * 256 + (4 * z + l) * kTN + cg * 8, v[l]);
+                        tmem_wait_ld();
 #pragma unroll
-                        for (int l = 0; l < kDig; ++l) D[l] = __float2int_rn(__uint_as_float(v[l][q]));
-                        add_levels(D, hi[cg * 8 + q], lo[cg * 8 + q]);
+                        for (int q = 0; q < 8; ++q) {
+                            int D[4];
+#pragma unroll
+                            for (int l = 0; l < 4; ++l) D[l] = __float2int_rn(__uint_as_float(v[l][q]));
+                            (z ? lo : hi)[cg * 8 + q] += join_levels(D);
+                        }
                     }
                 }
                 fence_before();
                 mbar_arrive(&tempty[buf]);
             }
-            // value = 2^(er + ec - 62) (hi 2^24 + lo)
+            // value = 2^(er + ec - 68) (hi 2^32 + lo); bit q of the mask: |value| < kSmall 2^(er + ec), k_pair_mend looks
+            uint32_t mask = 0;
             auto value = [&](int q, int eu, int ev) {
-                return (eu == kBad || ev == kBad)     ? __longlong_as_double(0x7ff8000000000000ll)
-                       : (eu == kNone || ev == kNone) ? 0.0
-                                                      : combine(hi[q], lo[q], eu + ev - 62);
+                if (eu == kBad || ev == kBad) return __longlong_as_double(0x7ff8000000000000ll);
+                if (eu == kNone || ev == kNone) return 0.0;
+                const long long h = hi[q] + (lo[q] >> 32);
+                if (h < kSmallHi && h >= -kSmallHi) mask |= 1u << q;
+                return combine(hi[q], lo[q], eu + ev - 68);
             };
             if (LIST) {
                 const int nm = c.an, r = (mt % pl.tiles_x) * kTM + row;
@@ -356,19 +369,20 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                             c.E[((size_t)pl.pair[it.y + s] * c.rx() + r) * nm + j] = value(q, eu, ec[blk * 32 + cq]);
                     }
                 }
-                continue;
-            }
-            const int r = mt * kTM + row;
-            if (ok && r < nrows) {
-                const int eu = er[r];
-                double *o = c.E + rt.base + (size_t)row * rt.nct * kTN + (size_t)(ct - rt.ct0) * kTN + c0;
+            } else {
+                const int r = mt * kTM + row;
+                if (ok && r < nrows) {
+                    const int eu = er[r];
+                    double *o = c.E + rt.base + (size_t)row * rt.nct * kTN + (size_t)(ct - rt.ct0) * kTN + c0;
 #pragma unroll
-                for (int q = 0; q < kEpiC; q += 2) {
-                    const int col = ct * kTN + c0 + q;
-                    *reinterpret_cast<double2 *>(o + q) = make_double2(value(q, eu, col < ncols ? ec[col] : kNone),
-                                                                       value(q + 1, eu, col + 1 < ncols ? ec[col + 1] : kNone));
+                    for (int q = 0; q < kEpiC; q += 2) {
+                        const int col = ct * kTN + c0 + q;
+                        *reinterpret_cast<double2 *>(o + q) = make_double2(value(q, eu, col < ncols ? ec[col] : kNone),
+                                                                           value(q + 1, eu, col + 1 < ncols ? ec[col + 1] : kNone));
+                    }
                 }
             }
+            if (ok) small[((size_t)item * kTM + row) * (kTN / kEpiC) + (c0 / kEpiC)] = (uint8_t)mask;
         }
     }
     fence_before();
@@ -377,17 +391,177 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// |v| 2^-e as FP32 from below, at least 2^-60 unless v is zero.
+__device__ __forceinline__ float scaled_abs(double v, int e) {
+    const int h = __double2hiint(v) & 0x7fffffff, l = __double2loint(v);
+    if ((h | l) == 0) return 0.f;
+    const int d = min(max((h >> 20) - 1023 - e, -60), 0);
+    return __int_as_float(((d + 127) << 23) | ((h & 0xfffff) << 3) | ((uint32_t)l >> 29));
+}
+
+// Products whose terms are all small against the scales: k_pair_tc's error is absolute, at most
+// K 2^-59 2^(er + ec) (a term's two roundings at 2^-63 and the seven products of level 8), where K FP64
+// FMAs are within K 2^-53 sum |a_k b_k|.  So an element keeps its digits only where sum |a_k b_k| >=
+// 2^-6 2^(er + ec) = kSmall 2^(er + ec): there the bound is the FMAs' own.  |E| is a lower bound of that
+// sum; for the elements below it (mask) the sum itself is formed in FP32, over 16 k spread along K at a time until it
+// suffices, and what stays below is computed again as k_pair_gemm does it.  Measured error relative to
+// the sum at the threshold, digits / FMAs: K = 24 6e-17 / 1.4e-16, 173 1.0e-16 / 3.6e-16, 800 2.0e-16 /
+// 7.9e-16; at 2^-10 of the scales the digits are 4 times the FMAs' error, at 2^-20 4000 times.
+// One block per product tile, most of which end at the first test.
+template <bool LIST>
+__global__ __launch_bounds__(256) void k_pair_mend(Chunk c, PairList pl, const double *__restrict__ A, const double *__restrict__ Q,
+                                                   const int *__restrict__ er, const int *__restrict__ ec,
+                                                   const uint32_t *__restrict__ small) {
+    after_previous();
+    constexpr int KT = 16;
+    __shared__ __align__(16) double As[KT][kTM], Bs[KT][kTN];
+    const int t = threadIdx.x, tr = (t >> 3) * 4, tc = (t & 7) * 4, qn = c.qn, an = c.an, rx = c.rx(), K = c.K;
+    const long long item = blockIdx.x;
+    uint32_t bits = 0;  // element (i, q) of this thread: bit 4 i + q
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bits |= ((small[item * kTM + tr + i] >> tc) & 15u) << (4 * i);
+    if (!__syncthreads_or(bits != 0)) return;
+    int4 it = make_int4(0, 0, 0, 0);
+    RowTile rt{};
+    int mt, ct = 0;
+    if (LIST) {
+        it = pl.items[item];
+        mt = it.x;
+    } else {
+        mt = tile_row(c, item);
+        rt = c.rt[mt];
+        ct = rt.ct0 + (int)(item - rt.item0);
+    }
+    // row of the tile: its A row and its place among the rows (a, b) of that; column: A row and mode
+    auto row_of = [&](int row, int &x, int &ab) {
+        if (LIST) {
+            x = c.xmap[mt / pl.tiles_x];
+            ab = (mt % pl.tiles_x) * kTM + row;
+            return ab < rx;
+        }
+        const int r = mt * kTM + row;
+        x = c.x0 + r / rx;
+        ab = r % rx;
+        return x < c.x1;
+    };
+    auto col_of = [&](int cc, int &y, int &j, int &e) {
+        if (LIST) {
+            const int s = cc / pl.bw;
+            if (s >= it.z) return false;
+            const int blk = pl.blk[it.y + s], cq = cc - s * pl.bw;
+            y = blk / pl.np;
+            j = (blk - y * pl.np) * pl.bw + cq;
+            e = blk * 32 + cq;
+            return j < an;
+        }
+        e = ct * kTN + cc;
+        y = e / an;
+        j = e - y * an;
+        return y <= c.hi;
+    };
+    // this thread's staging row and column
+    const int sr = t & (kTM - 1), kr = t >> 7, sc = t & (kTN - 1), kc = t >> 5;
+    int x, ab, y, j, e;
+    const bool rv = row_of(sr, x, ab), cv = col_of(sc, y, j, e);
+    const int a = rv ? ab / an : 0, b = rv ? ab - a * an : 0, eu = rv ? er[mt * kTM + sr] : 0, ev = cv ? ec[e] : 0;
+    const double *Qa = Q + a, *Ab = A + (size_t)(rv ? x : 0) * K * an + b, *Aj = A + (size_t)(cv ? y : 0) * K * an + (cv ? j : 0);
+    float(*Af)[kTM] = reinterpret_cast<float(*)[kTM]>(As);
+    float(*Bf)[kTN] = reinterpret_cast<float(*)[kTN]>(Bs);
+    float sum[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) sum[i][q] = 0.f;
+    // elements of the tile that are none of the product's (the mask of a tile that timed out is not written)
+    uint32_t pend = bits;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        int u, v, w;
+        if (!row_of(tr + i, u, v)) pend &= ~(15u << (4 * i));
+        if (!col_of(tc + i, u, v, w)) pend &= ~(0x1111u << i);
+    }
+    const int nch = (K + KT - 1) / KT;
+    for (int ch = 0; ch < nch; ++ch) {
+        for (int u = kr; u < KT; u += 2) {
+            const int k = ch + nch * u;
+            Af[u][sr] = (rv && k < K) ? scaled_abs(Qa[(size_t)k * qn] * Ab[(size_t)k * an], eu) : 0.f;
+        }
+        for (int u = kc; u < KT; u += 8) {
+            const int k = ch + nch * u;
+            Bf[u][sc] = (cv && k < K) ? scaled_abs(Aj[(size_t)k * an], ev) : 0.f;
+        }
+        __syncthreads();
+        if (pend) {
+#pragma unroll 4
+            for (int u = 0; u < KT; ++u) {
+                const float4 p = *reinterpret_cast<const float4 *>(&Af[u][tr]), q = *reinterpret_cast<const float4 *>(&Bf[u][tc]);
+                const float ar[4] = {p.x, p.y, p.z, p.w}, br[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int z = 0; z < 4; ++z) sum[i][z] = fmaf(ar[i], br[z], sum[i][z]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int z = 0; z < 4; ++z)
+                    if (sum[i][z] >= kSmall) pend &= ~(1u << (4 * i + z));
+        }
+        if (!__syncthreads_or(pend != 0)) return;
+    }
+    // every term zero: so are the digits' product and the FMAs'
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int z = 0; z < 4; ++z)
+            if (sum[i][z] == 0.f) pend &= ~(1u << (4 * i + z));
+    if (!__syncthreads_or(pend != 0)) return;
+    double acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[i][q] = 0.0;
+    for (int k0 = 0; k0 < K; k0 += KT) {
+        const int kn = min(KT, K - k0);
+        for (int u = kr; u < kn; u += 2) As[u][sr] = rv ? Qa[(size_t)(k0 + u) * qn] * Ab[(size_t)(k0 + u) * an] : 0.0;
+        for (int u = kc; u < kn; u += 8) Bs[u][sc] = cv ? Aj[(size_t)(k0 + u) * an] : 0.0;
+        __syncthreads();
+        if (pend)
+            for (int u = 0; u < kn; ++u) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (pend >> (4 * i + q) & 1u) acc[i][q] = fma(As[u][tr + i], Bs[u][tc + q], acc[i][q]);
+            }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (!(pend >> (4 * i + q) & 1u)) continue;
+            if (LIST) {
+                int y2, j2, e2;
+                col_of(tc + q, y2, j2, e2);
+                c.E[((size_t)pl.pair[it.y + (tc + q) / pl.bw] * rx + (mt % pl.tiles_x) * kTM + tr + i) * an + j2] = acc[i][q];
+            } else {
+                c.E[rt.base + (size_t)(tr + i) * rt.nct * kTN + (size_t)(ct - rt.ct0) * kTN + tc + q] = acc[i][q];
+            }
+        }
+}
+
 static int kpad(int K) { return (K + kBK - 1) / kBK * kBK; }
 static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-// [digits][exponents]
+// [digits][exponents], the row operand's followed by the items' masks
 size_t tc_col_bytes(int nr, int an, int K) {
     const size_t ct = ((size_t)nr * an + kTN - 1) / kTN;
     return up256(ct * kDig * kTN * kpad(K) * 2) + up256(sizeof(int) * (size_t)nr * an);
 }
-size_t tc_row_bytes(long long nrows, int K) {
+size_t tc_row_bytes(long long nrows, int K, long long items) {
     const size_t mt = (size_t)((nrows + kTM - 1) / kTM);
-    return up256(mt * kDig * kTM * kpad(K) * 2) + up256(sizeof(int) * (size_t)nrows);
+    return up256(mt * kDig * kTM * kpad(K) * 2) + up256(sizeof(int) * mt * kTM) + (size_t)items * kTM * kTN / 8;
 }
 
 cudaError_t tc_prep_cols(cudaStream_t st, int nr, int an, int K, const double *A, void *cols) {
@@ -404,6 +578,7 @@ static cudaError_t products(cudaStream_t st, const Chunk &c, const PairList &l, 
                             const double *A, const double *Q, const int *ec, void *rows, int *err) {
     const int Kp = kpad(c.K), nx = c.x1 - c.x0;
     int *er = (int *)((char *)rows + up256(ntiles * kDig * kTM * Kp * 2));
+    uint8_t *small = (uint8_t *)er + up256(sizeof(int) * ntiles * kTM);  // a bit an element of the items' tiles
     const long long eb = (long long)nx * ((c.rx() + 31) / 32);
     if (eb <= 1216) launch_next(k_row_exp<16>, dim3(nx, (c.rx() + 31) / 32), 512, 0, st, c, A, Q, er);
     else launch_next(k_row_exp<8>, dim3(nx, (c.rx() + 31) / 32), 256, 0, st, c, A, Q, er);
@@ -418,7 +593,8 @@ static cudaError_t products(cudaStream_t st, const Chunk &c, const PairList &l, 
     if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev))) return e;
     const int nk = Kp / kBK, ks_last = (c.K - (nk - 1) * kBK + 15) / 16;
     launch_next(k_pair_tc<LIST>, (unsigned)std::min<long long>(nsm, c.items), kTcThreads, kTcSmem, st, ma, mb, c, l, nk, ks_last, er,
-                                                                                             ec, err);
+                                                                                             ec, small, err);
+    launch_next(k_pair_mend<LIST>, (unsigned)c.items, 256, 0, st, c, l, A, Q, er, ec, (const uint32_t *)small);
     return cudaGetLastError();
 }
 
