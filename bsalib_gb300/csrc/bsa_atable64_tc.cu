@@ -14,8 +14,9 @@
 // One block per (f, itc, 128 rows): 16 warps generate digits of 32 columns at a time into two halves of
 // the A tiles and drain TMEM at the end, one thread loads B and issues the MMAs.  Bound by the integer
 // instructions of the generation (about 110 an element).  65 rows of 400 nodes x 2, 24 modes: FP64 pipe
-// 1.70 ms, here 0.25 and 0.04 for the B digits.  Coherences outside [0, 1] or c_ii != 1 (bad flag of the
-// coherence table) leave the table to k_atable.
+// 1.70 ms, here 0.25, 0.04 for the B digits and 0.06 for the elements far below their column's scale,
+// which k_atable64_mend sums on the FP64 pipe; 3333 rows of 150 nodes, 12 modes: 3.9 ms, here 1.13, 0.09 and
+// 0.06.  Coherences outside [0, 1] or c_ii != 1 (bad flag of the coherence table) leave the table to k_atable.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -166,6 +167,9 @@ constexpr unsigned long long kLn2 = 0xb17217f7d1cf79acull;  // round(2^64 ln 2)
 constexpr int kGen = 512, kThreads = kGen + 32;
 constexpr int kTileA = 128 * 128, kTileB = kDig * 32 * 128;
 
+constexpr float kSmall = 1.f / 256;  // k_atable64_mend
+constexpr long long kSmallHi = 1LL << 28;
+
 template <int NP>
 constexpr size_t smem_bytes() { return 1024 + (size_t)kDig * kTileA + (size_t)NP * kTileB + 4096 + 256; }
 
@@ -223,7 +227,8 @@ template <int NP>
 __global__ void __launch_bounds__(kThreads, 1)
     k_atable64_tc(const __grid_constant__ CUtensorMap tmB, int ntc, int n, int nm, int bw, int MT, int nk, int ks_last,
                   const double *__restrict__ f, const double *__restrict__ logc, const double *__restrict__ rootS,
-                  const int *__restrict__ we, const int *__restrict__ bad, double *__restrict__ A, int *err) {
+                  const int *__restrict__ we, const int *__restrict__ bad, double *__restrict__ A, uint8_t *__restrict__ small,
+                  int *err) {
     after_previous();
     if (*bad) return;
     extern __shared__ uint8_t smem_raw[];
@@ -382,17 +387,22 @@ __global__ void __launch_bounds__(kThreads, 1)
             const double si = rootS[(size_t)fc * n + ri];
             double *out = A + ((size_t)fc * n + ri) * nm;
 #pragma unroll
-            for (int p = 0; p < NP; ++p)
+            for (int p = 0; p < NP; ++p) {
+                if (cg * 8 >= bw) continue;
+                uint32_t mask = 0;  // bit q: the sum is below kSmall of its scale, k_atable64_mend looks
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    const int c = cg * 8 + q, m = p * bw + c;
-                    if (c < bw && m < nm) {
-                        const int e = we[fc * nm + m];
-                        out[m] = e == kBad ? __longlong_as_double(0x7ff8000000000000ll)
-                                 : e == kNone ? 0.0
-                                              : si * combine(hi[p][q], lo[p][q], e - 68);
-                    }
+                    const int m = p * bw + cg * 8 + q;
+                    if (m >= nm) continue;
+                    const int e = we[fc * nm + m];
+                    const long long h = hi[p][q] + (lo[p][q] >> 32);
+                    if (e != kBad && e != kNone && h < kSmallHi && h >= -kSmallHi) mask |= 1u << q;
+                    out[m] = e == kBad    ? __longlong_as_double(0x7ff8000000000000ll)
+                             : e == kNone ? 0.0
+                                          : si * combine(hi[p][q], lo[p][q], e - 68);
                 }
+                small[((size_t)fc * n + ri) * 8 + p * (bw / 8) + cg] = (uint8_t)mask;
+            }
         }
     }
     fence_before();
@@ -401,38 +411,108 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp == 16) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256 * NP) : "memory");
 }
 
+// Rows where c_ij^|f| decays between i and the nodes that a mode moves: the digits' error is absolute
+// against the largest s_j L_jm (2^-62 a term), so an element keeps them only where sum_j c_ij^|f| |s_j
+// L_jm| >= kSmall of the scale; at that line their measured error is 2.1e-16 of the sum against the FP64
+// pipe's 2.7e-16 (200 nodes; 400: 2.7e-16 / 3.5e-16), half of it a factor 2 above.  The element itself and
+// then the 32 nodes around i bound that sum from below; what is left is summed on the FP64 pipe, lanes over j.
+// A warp scans the masks of eight rows, far apart (those near the foot of a tower come together: 32
+// neighbouring rows a warp took twice the time).
+__global__ __launch_bounds__(256) void k_atable64_mend(int rows, int ntc, int n, int nm, const double *__restrict__ f,
+                                                       const double *__restrict__ logc, const double *__restrict__ expt,
+                                                       const double *__restrict__ rootS, const double *__restrict__ L,
+                                                       const int *__restrict__ we, const int *__restrict__ bad,
+                                                       const unsigned long long *__restrict__ small, double *__restrict__ A) {
+    after_previous();
+    if (*bad) return;
+    __shared__ double T[kExpTab];
+    T[threadIdx.x] = expt[threadIdx.x];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, first = blockIdx.x * 8 + (threadIdx.x >> 5), step = gridDim.x * 8;
+    const unsigned long long own = lane < 8 && first + lane * step < rows ? small[first + lane * step] & (~0ull >> (64 - nm)) : 0ull;
+    for (unsigned todo = __ballot_sync(0xffffffffu, own != 0); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1, row = first + src * step, fc = row / n, i = row - fc * n, itc = fc % ntc;
+        unsigned long long mk = __shfl_sync(0xffffffffu, own, src);
+        const double af = fabs(f[fc / ntc]);
+        const double *lc = logc + ((size_t)itc * n + i) * n, *s = rootS + (size_t)fc * n, *l = L + (size_t)itc * n * nm;
+        const int jw = max(0, min(i - 16, n - 32)) + lane;
+        const float cw = jw >= n ? 0.f : af == 0.0 ? 1.f : expf((float)(af * lc[jw]));
+        for (unsigned long long b = mk; b; b &= b - 1) {
+            const int m = __ffsll(b) - 1;
+            float v = jw < n ? cw * scaled_abs(s[jw] * l[(size_t)jw * nm + m], we[fc * nm + m]) : 0.f;
+#pragma unroll
+            for (int h = 16; h > 0; h >>= 1) v += __shfl_xor_sync(0xffffffffu, v, h);
+            if (v >= kSmall) mk &= ~(1ull << m);
+        }
+        while (mk) {
+            int m[8], cnt = 0;
+            double acc[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                m[q] = 0;
+                acc[q] = 0.0;
+                if (mk) {
+                    m[q] = __ffsll(mk) - 1;
+                    mk &= mk - 1;
+                    ++cnt;
+                }
+            }
+            for (int j = lane; j < n; j += 32) {
+                const double c = af == 0.0 ? 1.0 : expc(af * lc[j], T), sj = s[j];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (q < cnt) acc[q] = fma(c, sj * l[(size_t)j * nm + m[q]], acc[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                if (q >= cnt) continue;
+                for (int h = 16; h > 0; h >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], h);
+                if (lane == 0) A[(size_t)row * nm + m[q]] = s[i] * acc[q];
+            }
+        }
+    }
+}
+
 template <int NP>
 static cudaError_t launch(cudaStream_t st, const CUtensorMap &mb, int nf, const double *f, int ntc, int n, int nm, int bw,
-                          const double *logc, const double *rootS, const int *we, const int *bad, double *A, int *err) {
+                          const double *logc, const double *rootS, const int *we, const int *bad, double *A, uint8_t *small,
+                          int *err) {
     const int MT = (n + 127) / 128, nk = (n + kBK - 1) / kBK, ks_last = (n - (nk - 1) * kBK + 15) / 16;
     cudaError_t e = cudaFuncSetAttribute(k_atable64_tc<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<NP>());
     if (e != cudaSuccess) return e;
     launch_next(k_atable64_tc<NP>, (unsigned)(nf * ntc * MT), kThreads, smem_bytes<NP>(), st, mb, ntc, n, nm, bw, MT, nk, ks_last, f, logc,
-                                                                                   rootS, we, bad, A, err);
+                                                                                   rootS, we, bad, A, small, err);
     return cudaGetLastError();
 }
 
 }  // namespace at64
 
-// [digits][exponents] of nf frequencies
+// [digits][exponents][masks, 8 bytes a row] of nf frequencies
+static size_t up256(size_t n) { return (n + 255) & ~(size_t)255; }
 size_t atable64_tc_scratch(int nf, int ntc, int nnl, int nm) {
     const size_t nb = (size_t)nf * ntc * p64::blocks_of(nm), Kp = (nnl + tc::kBK - 1) / tc::kBK * tc::kBK;
-    return ((nb * p64::kDig * p64::block_width(nm) * Kp * 2 + 255) & ~(size_t)255) + sizeof(int) * (size_t)nf * ntc * nm;
+    return up256(nb * p64::kDig * p64::block_width(nm) * Kp * 2) + up256(sizeof(int) * (size_t)nf * ntc * nm) +
+           (size_t)8 * nf * ntc * nnl;
 }
 
 cudaError_t launch_atable64_tc(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm, const double *logc,
                                const double *rootS, const double *L, const int *bad, double *A, void *scratch, int *err) {
     using namespace at64;
-    const int np = blocks_of(nm), bw = block_width(nm), Kp = (nnl + kBK - 1) / kBK * kBK;
+    const int np = blocks_of(nm), bw = block_width(nm), Kp = (nnl + kBK - 1) / kBK * kBK, rows = nf * ntc * nnl;
     const size_t nb = (size_t)nf * ntc * np;
     __nv_bfloat16 *D = (__nv_bfloat16 *)scratch;
-    int *we = (int *)((char *)scratch + ((nb * kDig * bw * Kp * 2 + 255) & ~(size_t)255));
+    int *we = (int *)((char *)scratch + up256(nb * kDig * bw * Kp * 2));
+    uint8_t *small = (uint8_t *)we + up256(sizeof(int) * (size_t)nf * ntc * nm);
     launch_next(k_wexp, nf * ntc, 256, 0, st, ntc, nnl, nm, rootS, L, we);
     launch_next(k_wdigits, dim3((unsigned)nb, (Kp + 127) / 128), 256, 0, st, ntc, nnl, nm, np, bw, Kp, rootS, L, we, D);
     CUtensorMap mb;
     if (!make_map(&mb, D, Kp, (uint64_t)nb * kDig * bw, (uint32_t)bw)) return cudaErrorInvalidValue;
-    return np == 1 ? launch<1>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, err)
-                   : launch<2>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, err);
+    const cudaError_t e = np == 1 ? launch<1>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, small, err)
+                                  : launch<2>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, small, err);
+    if (e != cudaSuccess) return e;
+    launch_next(k_atable64_mend, (unsigned)((rows + 63) / 64), 256, 0, st, rows, ntc, nnl, nm, f, logc,
+                logc + (size_t)ntc * nnl * nnl, rootS, L, we, bad, (const unsigned long long *)small, A);
+    return cudaGetLastError();
 }
 
 }  // namespace bsa

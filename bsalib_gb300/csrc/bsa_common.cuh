@@ -191,6 +191,31 @@ __device__ __forceinline__ void red_lanes(double &a, double &b) {
     b = red[1][0][x];
 }
 
+constexpr int kExpTab = 256;  // 2^(k / 256), k = 0 .. 255
+
+// e^x by table and polynomial (P. T. P. Tang, ACM TOMS 15, 1989): x = (256 q + k) ln2 / 256 + r,
+// |r| <= ln2 / 512, e^x = 2^q T[k] (1 + r + r^2/2 + r^3/6 + r^4/24); the next term is below 2^-54.
+// ln2 / 256 = hi + lo with hi of 25 bits, so that its product with the integer (18 bits) is exact.
+// Beyond |x| = 700, for infinities and for NaN: exp().
+__device__ __forceinline__ double expc(double x, const double *T) {
+    if (!(fabs(x) < 700.0)) return exp(x);
+    constexpr double kInv = 256.0 / 0.693147180559945309417232121458;
+    constexpr double kHi = 23258160.0 / 8589934592.0;  // round(2^33 ln2 / 256) / 2^33
+    constexpr double kLo = -7.4400558592100307755539978e-12;
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52: adding it rounds to an integer
+    const double z = fma(x, kInv, kMagic);
+    const int n = __double2loint(z);
+    const double kd = z - kMagic;
+    double r = fma(kd, -kHi, x);
+    r = fma(kd, -kLo, r);
+    double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
+    p = fma(p, r, 0.5);
+    p = fma(p, r * r, r);
+    const double t = T[n & (kExpTab - 1)];
+    const double v = fma(t, p, t);
+    return __hiloint2double(__double2hiint(v) + ((n >> 8) << 20), __double2loint(v));
+}
+
 // Two FP32 lanes in one 64-bit register.  The paired FP32 instructions of sm_100 and later
 // (fma.rn.f32x2, mul.rn.f32x2) run both lanes from one issue slot, each lane rounded as the
 // scalar fma.rn / mul.rn would round it.

@@ -27,6 +27,14 @@ __device__ __forceinline__ int expo(double v) { return (__double2hiint(v) >> 20)
 __device__ __forceinline__ int expo_pair(int u, int v) { return (u == 2047 || v == 2047) ? kBad : (u && v) ? u + v : 0; }
 __device__ __forceinline__ int expo_of_pairs(int m) { return m == kBad ? kBad : m == 0 ? kNone : m - 2044; }
 
+// |v| 2^-e as FP32 from below, at least 2^-60 unless v is zero.
+__device__ __forceinline__ float scaled_abs(double v, int e) {
+    const int h = __double2hiint(v) & 0x7fffffff, l = __double2loint(v);
+    if ((h | l) == 0) return 0.f;
+    const int d = min(max((h >> 20) - 1023 - e, -60), 0);
+    return __int_as_float(((d + 127) << 23) | ((h & 0xfffff) << 3) | ((uint32_t)l >> 29));
+}
+
 // Balanced digits of an integer of at most 62 bits and sign, as floats that are exact in bf16 (low half
 // zero): add 128 to every digit, read the bytes, take 128 away.
 __device__ __forceinline__ void digits_of(unsigned long long x, uint32_t *f) {

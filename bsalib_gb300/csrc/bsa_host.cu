@@ -464,7 +464,7 @@ int Engine::build_atable_dev(int nf, bool fp32, int f0) {
                                    dS.as<double>() + (size_t)q * K, dL.as<double>(), bad, dA.as<double>() + (size_t)q * K * nme,
                                    dMshT.p, dFlag.as<int>());
             if (e) return cuda_fail(e, "A-table kernel");
-            kernels += 3;
+            kernels += 4;
         }
     }
     e = launch_atable(stream, nf, fp, ntc, in.nnl, nme, dLogc.as<double>(), dS.as<double>(), dL.as<double>(), dA.as<double>(),

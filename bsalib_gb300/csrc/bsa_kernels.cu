@@ -7,8 +7,6 @@
 
 namespace bsa {
 
-constexpr int kExpTab = 256;  // 2^(k / 256), k = 0 .. 255
-
 // ------------------------------------------------------------------------------------
 // Stage (a): nodal turbulence PSD.  One thread per (f, itc, node), node fastest so the
 // stores are coalesced.  Model formulas: vonKarmanPSD_ (WindPSDImpl.F90:149-226, u form
@@ -117,29 +115,6 @@ cudaError_t launch_nodal_psd(cudaStream_t st, int nf, const double *f, int ntc, 
 // where exp() spends about 25, and sqrt(S) comes from k_nodal_psd.  150 nodes, 12 modes, 3333
 // frequencies: 13.1 -> 3.9 ms.
 // ------------------------------------------------------------------------------------
-// e^x by table and polynomial (P. T. P. Tang, ACM TOMS 15, 1989): x = (256 q + k) ln2 / 256 + r,
-// |r| <= ln2 / 512, e^x = 2^q T[k] (1 + r + r^2/2 + r^3/6 + r^4/24); the next term is below 2^-54.
-// ln2 / 256 = hi + lo with hi of 25 bits, so that its product with the integer (18 bits) is exact.
-// Beyond |x| = 700, for infinities and for NaN: exp().
-__device__ __forceinline__ double expc(double x, const double *T) {
-    if (!(fabs(x) < 700.0)) return exp(x);
-    constexpr double kInv = 256.0 / 0.693147180559945309417232121458;
-    constexpr double kHi = 23258160.0 / 8589934592.0;  // round(2^33 ln2 / 256) / 2^33
-    constexpr double kLo = -7.4400558592100307755539978e-12;
-    constexpr double kMagic = 6755399441055744.0;  // 1.5 2^52: adding it rounds to an integer
-    const double z = fma(x, kInv, kMagic);
-    const int n = __double2loint(z);
-    const double kd = z - kMagic;
-    double r = fma(kd, -kHi, x);
-    r = fma(kd, -kLo, r);
-    double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
-    p = fma(p, r, 0.5);
-    p = fma(p, r * r, r);
-    const double t = T[n & (kExpTab - 1)];
-    const double v = fma(t, p, t);
-    return __hiloint2double(__double2hiint(v) + ((n >> 8) << 20), __double2loint(v));
-}
-
 template <int MPT>
 __global__ __launch_bounds__(256) void k_atable(int nf, const double *__restrict__ f, int ntc, int nnl,
                                                 int nm, const double *__restrict__ logc,

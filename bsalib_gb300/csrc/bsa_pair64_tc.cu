@@ -391,14 +391,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
-// |v| 2^-e as FP32 from below, at least 2^-60 unless v is zero.
-__device__ __forceinline__ float scaled_abs(double v, int e) {
-    const int h = __double2hiint(v) & 0x7fffffff, l = __double2loint(v);
-    if ((h | l) == 0) return 0.f;
-    const int d = min(max((h >> 20) - 1023 - e, -60), 0);
-    return __int_as_float(((d + 127) << 23) | ((h & 0xfffff) << 3) | ((uint32_t)l >> 29));
-}
-
 // Products whose terms are all small against the scales: k_pair_tc's error is absolute, at most
 // K 2^-59 2^(er + ec) (a term's two roundings at 2^-63 and the seven products of level 8), where K FP64
 // FMAs are within K 2^-53 sum |a_k b_k|.  So an element keeps its digits only where sum |a_k b_k| >=

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from bsalib_gb300 import api
-from bsalib_gb300.problem import packed_coherence, tall_building
+from bsalib_gb300.problem import packed_coherence, random_structure, tall_building
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,39 @@ def test_listed_elements(bsalib, nodes, modes, gap):
     finally:
         s.close()
     _within(bf, want, 2 * nodes)
+
+
+def _force_psd(p, f):
+    """L^T A(f), A = s (c^|f|) s L, in extended precision (Davenport-Uliege spectra, one component)."""
+    X = np.longdouble
+    n = p.nn
+    lin = (p.wfc[0, 0, :][:, None] * p.phi).astype(X)
+    c = np.zeros((n, n), X)
+    iu = np.triu_indices(n)
+    c[iu] = p.nod_corr[:, 0]
+    c.T[iu] = p.nod_corr[:, 0]
+    r, sg = (p.L[0, 0, p.wz_node - 1] / p.u_node).astype(X), p.sigma[0, p.wz_node - 1].astype(X)
+    s = np.sqrt(X(2) / 3 * f * r * r * sg ** 2 / (1 + (f * r) ** 2) ** (X(4) / 3) / (4 * X(np.pi)))
+    return lin.T @ (s[:, None] * (c ** X(f) @ (s[:, None] * lin)))
+
+
+@pytest.mark.parametrize("nodes,modes", [(80, 8), (129, 12), (200, 33), (100, 64), (600, 5)])
+@pytest.mark.parametrize("gap", [0.0, 20.0, 60.0, 150.0])
+def test_force_spectra_elements(bsalib, nodes, modes, gap):
+    """The A table, one frequency at a time.  Tolerance: sums over the nodes in A and in L^T A, the exponent's
+    two roundings of x = |f log c|, and 60 roundings for the spectrum and the weights."""
+    p = random_structure(nodes, nodes=(nodes, nodes), modes=(modes, modes), nfreq_grid=(9, 9))
+    q = _groups(nodes, modes, gap)
+    p.phi[:], p.nod_corr[:] = q.phi, q.nod_corr
+    p.settings.ibisp, p.settings.df, h = 0, 0.4, p.settings.nfreqs - 1
+    for k in range(1, h):
+        s = api.BsaSession(p)
+        try:
+            s.set_rows(h + k, h + k + 1)
+            got = s.run()["m2mf_cls"].reshape(modes, modes)
+        finally:
+            s.close()
+        f = k * p.settings.df
+        want = (_force_psd(p, f) * 2 * np.pi * p.settings.df).astype(float)
+        x = -f * np.log(p.nod_corr[:, 0].min())
+        assert np.all(np.abs(got - want) <= (2 * nodes + 2 * x + 60) * U * want)
