@@ -396,10 +396,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (m >= nm) continue;
                     const int e = we[fc * nm + m];
                     const long long h = hi[p][q] + (lo[p][q] >> 32);
-                    if (e != kBad && e != kNone && h < kSmallHi && h >= -kSmallHi) mask |= 1u << q;
-                    out[m] = e == kBad    ? __longlong_as_double(0x7ff8000000000000ll)
-                             : e == kNone ? 0.0
-                                          : si * combine(hi[p][q], lo[p][q], e - 68);
+                    if (e == kBad || (e != kNone && h < kSmallHi && h >= -kSmallHi)) mask |= 1u << q;
+                    out[m] = e == kBad || e == kNone ? 0.0 : si * combine(hi[p][q], lo[p][q], e - 68);
                 }
                 small[((size_t)fc * n + ri) * 8 + p * (bw / 8) + cg] = (uint8_t)mask;
             }
@@ -438,8 +436,9 @@ __global__ __launch_bounds__(256) void k_atable64_mend(int rows, int ntc, int n,
         const int jw = max(0, min(i - 16, n - 32)) + lane;
         const float cw = jw >= n ? 0.f : af == 0.0 ? 1.f : expf((float)(af * lc[jw]));
         for (unsigned long long b = mk; b; b &= b - 1) {
-            const int m = __ffsll(b) - 1;
-            float v = jw < n ? cw * scaled_abs(s[jw] * l[(size_t)jw * nm + m], we[fc * nm + m]) : 0.f;
+            const int m = __ffsll(b) - 1, e = we[fc * nm + m];
+            if (e == kBad) continue;  // the whole column
+            float v = jw < n ? cw * scaled_abs(s[jw] * l[(size_t)jw * nm + m], e) : 0.f;
 #pragma unroll
             for (int h = 16; h > 0; h >>= 1) v += __shfl_xor_sync(0xffffffffu, v, h);
             if (v >= kSmall) mk &= ~(1ull << m);

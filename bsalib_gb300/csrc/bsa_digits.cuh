@@ -16,16 +16,30 @@ using namespace tc;
 
 constexpr int kDig = 8;            // digits per operand
 constexpr int kPassMax = 128;      // k of one exact pass: 8 x 128 products of at most 2^14 within 2^24
-constexpr int kBad = 1 << 20;      // row exponent of a row that holds an infinity or a NaN
+constexpr int kBad = 1 << 20;      // exponent of a row left to the FP64 pipe
 constexpr int kNone = -(1 << 20);  // of a row of zeros
 
-// Biased exponent field (0 for zeros and denormals, 2047 for infinities and NaN).
-__device__ __forceinline__ int expo(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+// Biased exponent field, 1 for denormals and 0 for zeros only; 2047 for infinities and NaN.
+__device__ __forceinline__ int expo(double v) {
+    const int h = __double2hiint(v) & 0x7fffffff, e = h >> 20;
+    return e ? e : (h | __double2loint(v)) != 0;
+}
 
-// Exponent field sum of a product's factors: 0 where one is zero or denormal, kBad where one is not
-// finite; expo_of_pairs: the exponent e with |u v| < 2^e from the largest such sum.
+// Row exponents.  Digits are cut from finite, normal numbers: a row that holds an infinity or a NaN, one
+// whose entries are products of two factors and may overflow, and one whose smaller entries are near the
+// denormals is kBad, and its elements are formed on the FP64 pipe as they come.
+__device__ __forceinline__ int expo_row(int e) { return e > 1024 || e < -900 ? kBad : e; }
+// Exponent field sum of a product's factors: 0 where one is zero, kBad where one is not finite;
+// expo_of_pairs: the exponent e with |u v| < 2^e from the largest such sum.
 __device__ __forceinline__ int expo_pair(int u, int v) { return (u == 2047 || v == 2047) ? kBad : (u && v) ? u + v : 0; }
-__device__ __forceinline__ int expo_of_pairs(int m) { return m == kBad ? kBad : m == 0 ? kNone : m - 2044; }
+__device__ __forceinline__ int expo_of_pairs(int m) { return m == kBad ? kBad : m == 0 ? kNone : expo_row(m - 2044); }
+
+// Whether an element of these row and column exponents is the FP64 pipe's: also where the result itself
+// may leave the normal range.
+__device__ __forceinline__ bool fp64_only(int eu, int ev) {
+    if (eu == kBad || ev == kBad) return true;
+    return eu != kNone && ev != kNone && (eu + ev < -900 || eu + ev > 1000);
+}
 
 // |v| 2^-e as FP32 from below, at least 2^-60 unless v is zero.
 __device__ __forceinline__ float scaled_abs(double v, int e) {

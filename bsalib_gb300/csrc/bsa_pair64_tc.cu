@@ -66,14 +66,15 @@ __global__ __launch_bounds__(256) void k_col_exp(int an, int K, const double *__
     __syncthreads();
     if ((int)threadIdx.x < an) {
         const int e = mx[threadIdx.x];
-        ec[y * an + threadIdx.x] = e == 2047 ? kBad : e == 0 ? kNone : e - 1022;
+        ec[y * an + threadIdx.x] = e == 2047 ? kBad : e == 0 ? kNone : expo_row(e - 1022);
     }
 }
 
 // Row operand: |Q[k][a] A(x)[k][b]| < 2^e[r] from the factors' exponents (at most a bit above).
 // 32 rows by 16 or 8 lanes over k per block: where the blocks fit the chip at once a lane's chain of loads
-// is the time and 16 lanes halve it (K = 800, 24 rows of 257 frequencies: 26 -> 17 us; 576 rows of 65:
-// 40 -> 36), where they do not the lanes' join counts (K = 150, 144 rows of 2222: 67 us by 8, 81 by 16).
+// is the time and 16 lanes halve it (K = 800, 24 rows of 257 frequencies: 26 -> 17 us), where they do not the
+// lanes' join counts (K = 150, 144 rows of 2222: 67 us by 8, 81 by 16; these by the high words alone, which do
+// not tell the smallest denormals from zero: 86 us by 8 with both words, 55 instead of 36 for 576 rows of 65).
 template <int LANES>
 __global__ __launch_bounds__(32 * LANES) void k_row_exp(Chunk c, const double *__restrict__ A, const double *__restrict__ Q,
                                                  int *__restrict__ er) {
@@ -81,14 +82,11 @@ __global__ __launch_bounds__(32 * LANES) void k_row_exp(Chunk c, const double *_
     __shared__ int mx[LANES][32];
     const int qn = c.qn, an = c.an, rx = c.rx(), ab = blockIdx.y * 32 + (threadIdx.x & 31), lane = threadIdx.x >> 5;
     const int x = c.xmap ? c.xmap[blockIdx.x] : c.x0 + blockIdx.x, a = ab / an, b = ab - a * an;
-    const int *q = reinterpret_cast<const int *>(Q + a) + 1, *p = reinterpret_cast<const int *>(A + (size_t)x * c.K * an + b) + 1;
+    const double *q = Q + a, *p = A + (size_t)x * c.K * an + b;
     int m = 0;
     if (ab < rx)
 #pragma unroll 8
-        for (int k = lane; k < c.K; k += LANES) {
-            const int u = (q[(size_t)2 * k * qn] >> 20) & 0x7ff, v = (p[(size_t)2 * k * an] >> 20) & 0x7ff;
-            m = max(m, expo_pair(u, v));
-        }
+        for (int k = lane; k < c.K; k += LANES) m = max(m, expo_pair(expo(q[(size_t)k * qn]), expo(p[(size_t)k * an])));
     mx[lane][threadIdx.x & 31] = m;
     __syncthreads();
     if (lane == 0 && ab < rx) {
@@ -347,10 +345,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 fence_before();
                 mbar_arrive(&tempty[buf]);
             }
-            // value = 2^(er + ec - 68) (hi 2^32 + lo); bit q of the mask: |value| < kSmall 2^(er + ec), k_pair_mend looks
+            // value = 2^(er + ec - 68) (hi 2^32 + lo); bit q of the mask: |value| < kSmall 2^(er + ec) or fp64_only, k_pair_mend looks
             uint32_t mask = 0;
             auto value = [&](int q, int eu, int ev) {
-                if (eu == kBad || ev == kBad) return __longlong_as_double(0x7ff8000000000000ll);
+                if (fp64_only(eu, ev)) {
+                    mask |= 1u << q;
+                    return 0.0;
+                }
                 if (eu == kNone || ev == kNone) return 0.0;
                 const long long h = hi[q] + (lo[q] >> 32);
                 if (h < kSmallHi && h >= -kSmallHi) mask |= 1u << q;
@@ -399,6 +400,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // suffices, and what stays below is computed again as k_pair_gemm does it.  Measured error relative to
 // the sum at the threshold, digits / FMAs: K = 24 6e-17 / 1.4e-16, 173 1.0e-16 / 3.6e-16, 800 2.0e-16 /
 // 7.9e-16; at 2^-10 of the scales the digits are 4 times the FMAs' error, at 2^-20 4000 times.
+// Elements whose row or column exponent is kBad go there at once (fp64_only).
 // One block per product tile, most of which end at the first test.
 template <bool LIST>
 __global__ __launch_bounds__(256) void k_pair_mend(Chunk c, PairList pl, const double *__restrict__ A, const double *__restrict__ Q,
@@ -472,8 +474,19 @@ __global__ __launch_bounds__(256) void k_pair_mend(Chunk c, PairList pl, const d
         if (!row_of(tr + i, u, v)) pend &= ~(15u << (4 * i));
         if (!col_of(tc + i, u, v, w)) pend &= ~(0x1111u << i);
     }
+    uint32_t only = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        int u, v, w;
+        if (!col_of(tc + q, u, v, w)) continue;
+        const int eq = ec[w];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if ((pend >> (4 * i + q) & 1u) && fp64_only(er[mt * kTM + tr + i], eq)) only |= 1u << (4 * i + q);
+    }
+    pend &= ~only;
     const int nch = (K + KT - 1) / KT;
-    for (int ch = 0; ch < nch; ++ch) {
+    for (int ch = 0; ch < nch && __syncthreads_or(pend != 0); ++ch) {
         for (int u = kr; u < KT; u += 2) {
             const int k = ch + nch * u;
             Af[u][sr] = (rv && k < K) ? scaled_abs(Qa[(size_t)k * qn] * Ab[(size_t)k * an], eu) : 0.f;
@@ -499,7 +512,6 @@ __global__ __launch_bounds__(256) void k_pair_mend(Chunk c, PairList pl, const d
                 for (int z = 0; z < 4; ++z)
                     if (sum[i][z] >= kSmall) pend &= ~(1u << (4 * i + z));
         }
-        if (!__syncthreads_or(pend != 0)) return;
     }
     // every term zero: so are the digits' product and the FMAs'
 #pragma unroll
@@ -507,6 +519,7 @@ __global__ __launch_bounds__(256) void k_pair_mend(Chunk c, PairList pl, const d
 #pragma unroll
         for (int z = 0; z < 4; ++z)
             if (sum[i][z] == 0.f) pend &= ~(1u << (4 * i + z));
+    pend |= only;
     if (!__syncthreads_or(pend != 0)) return;
     double acc[4][4];
 #pragma unroll

@@ -101,3 +101,59 @@ def test_force_spectra_elements(bsalib, nodes, modes, gap):
         want = (_force_psd(p, f) * 2 * np.pi * p.settings.df).astype(float)
         x = -f * np.log(p.nod_corr[:, 0].min())
         assert np.all(np.abs(got - want) <= (2 * nodes + 2 * x + 60) * U * want)
+
+
+# factors of the quadratic and linear coefficients, and node 7's quadratic one for the mode that moves it:
+# products Q A over the largest number, Q and A near its root, denormal Q, results among the denormals.  Grid
+# points whose sum is on the grid: the point kernel multiplies a sum that reads zero by Q A
+@pytest.mark.parametrize("quad,lin,at7", [(1.0, 1e120, 1e200), (1e200, 1e100, 1e7), (1e155, 1e70, 1e84), (1e-313, 1e145, 1e2),
+                                          (1e-200, 1e-40, 1.0), (1e-160, 1e-74, 1e9)])
+def test_ends_of_the_range(bsalib, quad, lin, at7):
+    p = _groups(60, 8, 10.0)
+    p.phi[7, :] = np.where(np.arange(8) == 3, 0.5, 0.0)
+    p.wfc[0, :3] *= lin
+    p.wfc[0, 3:] *= quad
+    p.wfc[0, 3:, 7] *= at7
+    rng = np.random.default_rng(4)
+    f1, f2 = rng.uniform(-2, 2, 400), rng.uniform(-2, 2, 400)
+    s = api.BsaSession(p)
+    try:
+        f, bf, _ = s.classic_bispectra()
+        n = f.size
+        i1, i2 = (v.ravel() for v in np.meshgrid(np.arange(n), np.arange(n), indexing="ij"))
+        on = np.abs(i1 + i2 - (n - 1)) <= (n - 1) // 2
+        i1, i2 = i1[on], i2[on]
+        want = np.concatenate([s.classic_points(i1[k:k + 15], i2[k:k + 15])[0] for k in range(0, i1.size, 15)])
+        lst, _ = s.msh_bispectra(f1, f2)
+        pieces = np.concatenate([s.msh_bispectra(f1[k:k + 2], f2[k:k + 2])[0] for k in range(0, 400, 2)])
+    finally:
+        s.close()
+    for a, b in ((bf.reshape(n * n, -1)[on], want.reshape(on.sum(), -1)), (lst, pieces)):
+        ok = np.isfinite(b)
+        assert np.array_equal(a[~ok], b[~ok], equal_nan=True)
+        # a denormal's rounding is 2^-1075 at every term
+        assert np.all(np.abs(a[ok] - b[ok]) <= 2 * (120 + 4) * (U * np.abs(b[ok]) + 2.0 ** -1074))
+
+
+@pytest.mark.parametrize("at7", [1e306, 1e308, np.inf, 1e-320])
+def test_force_spectra_ends_of_the_range(bsalib, at7):
+    """Against the same table formed by the general kernel, which a node's own coherence one rounding below 1
+    selects (that moves an element by a rounding at most)."""
+    got = []
+    for own in (1.0, 1.0 - 2.0 ** -53):
+        p = random_structure(90, nodes=(90, 90), modes=(6, 6), nfreq_grid=(9, 9))
+        q = _groups(90, 6, 20.0)
+        p.phi[:], p.nod_corr[:] = q.phi, q.nod_corr
+        p.phi[7, :] = np.where(np.arange(6) == 1, 0.5, 0.0)
+        p.wfc[0, :3, 7] *= at7 / 1e3 if np.isfinite(at7) else at7
+        p.nod_corr[0, 0] = own
+        p.settings.ibisp = 0
+        s = api.BsaSession(p)
+        try:
+            got.append(s.run()["m2mf_cls"])
+        finally:
+            s.close()
+    a, b = got
+    ok = np.isfinite(b)
+    assert np.array_equal(a[~ok], b[~ok], equal_nan=True)
+    assert np.all(np.abs(a[ok] - b[ok]) <= 4 * (90 + 20) * U * np.abs(b[ok]))
