@@ -721,6 +721,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
                         for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back(2.0 * f[0] + s * (f[1] - f[0]));
                     const int r = diagonal ? build_psd(ftab) : build_atable(ftab, false);
                     if (r) return r;
+                    ps.fgrid = dFreq.as<double>();  // a longer table than that of f >= 0: the block may have moved
                 }
             }
             if (rc == kNoRoom)
