@@ -26,6 +26,8 @@ Engine &eng() {
 }
 
 int Engine::fail(int code, const char *fmt, ...) {
+    // copies still queued read tables that the failing call is about to give up
+    if (stream) cudaStreamSynchronize(stream);
     if (!halted) {
         char buf[512];
         va_list ap;
