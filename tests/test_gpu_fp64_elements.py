@@ -145,7 +145,7 @@ def test_force_spectra_ends_of_the_range(bsalib, at7):
         q = _groups(90, 6, 20.0)
         p.phi[:], p.nod_corr[:] = q.phi, q.nod_corr
         p.phi[7, :] = np.where(np.arange(6) == 1, 0.5, 0.0)
-        p.wfc[0, :3, 7] *= at7 / 1e3 if np.isfinite(at7) else at7
+        p.wfc[0, 0, 7] *= at7 / 1e3 if np.isfinite(at7) else at7
         p.nod_corr[0, 0] = own
         p.settings.ibisp = 0
         s = api.BsaSession(p)
@@ -157,3 +157,28 @@ def test_force_spectra_ends_of_the_range(bsalib, at7):
     ok = np.isfinite(b)
     assert np.array_equal(a[~ok], b[~ok], equal_nan=True)
     assert np.all(np.abs(a[ok] - b[ok]) <= 4 * (90 + 20) * U * np.abs(b[ok]))
+
+
+# K at the edges of a 16-wide step, of a 64-wide block and of the 128-wide exact pass
+@pytest.mark.parametrize("nodes", [24, 31, 32, 33, 63, 64, 65, 128, 129])
+@pytest.mark.parametrize("modes", [11, 12])
+def test_elements_around_a_pass(bsalib, nodes, modes):
+    test_bispectra_elements(bsalib, nodes, modes, 10.0)
+    test_listed_elements(bsalib, nodes, modes, 10.0)
+
+
+def test_elements_over_a_wide_range(bsalib):
+    """Forces over twelve decades along the height, and a mode that is 1e-60 of the others but at one node."""
+    p = _groups(64, 8, 0.0, nfreqs=40, df=0.05)
+    p.wfc[0, :3, :] *= np.logspace(0, -12, p.nn)
+    p.phi[:, 3] *= np.where(p.phi[:, 3] == 1.0, 1.0, 1e-60)
+    s = api.BsaSession(p)
+    try:
+        f, bf, _ = s.classic_bispectra()
+        n = f.size
+        i1, i2 = (v.ravel() for v in np.meshgrid(np.arange(n), np.arange(n), indexing="ij"))
+        i1, i2 = i1[::7], i2[::7]
+        want = np.concatenate([s.classic_points(i1[k:k + 15], i2[k:k + 15])[0] for k in range(0, i1.size, 15)])
+    finally:
+        s.close()
+    _within(bf.reshape(n * n, -1)[::7], want.reshape(i1.size, -1), 128)
