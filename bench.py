@@ -47,16 +47,21 @@ def algorithmic_flops_per_point(nnl, nm, ntc):
 
 
 def issued_flops_e(nf, nm, nnl, ntc):
-    """BF16 flop the E-form kernel issues per launch: per grid row p the units (pairs of N tiles
-    of NC columns from the tile holding column p), per unit and row tile 3 MMAs (hi*hi, hi*lo,
-    lo*hi) of M = 128, N = 256 over K rounded up to 16."""
-    nmt = 8 if nm <= 8 else 16 if nm <= 16 else 24
+    """BF16 flop the E-form kernel issues per launch, in the width and mode passes the library plans: per grid
+    row p the units (pairs of N tiles of NC columns from the tile holding column p) of every mode pass, per
+    unit and row tile 3 MMAs (hi*hi, hi*lo, lo*hi) of M = 128 rows by the 2 NC columns of NMT modes, over K
+    rounded up to 16."""
+    from bsalib_gb300 import api
+    from bsalib_gb300.autotune import FAMILY
+    width = api.tile_plan(FAMILY["cls_e_width"], nm, ntc * nnl, nf)
+    passes = api.tile_plan(FAMILY["cls_e_split"], nm, ntc * nnl, nf)
+    nmt = width // passes
     nc = 128 // nmt
     ntl = (nf + nc - 1) // nc
-    units = sum((ntl - p // nc + 1) // 2 for p in range(nf))
+    units = passes * sum((ntl - p // nc + 1) // 2 for p in range(nf))
     mt = (nm * nm + 127) // 128
     k_eff = ((ntc * nnl + 15) // 16) * 16
-    return units * mt * 3 * 2 * 128 * 256 * k_eff
+    return units * mt * 3 * 2 * 128 * (2 * nc * nmt) * k_eff
 
 
 class Clocks:
