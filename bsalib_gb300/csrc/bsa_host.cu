@@ -443,10 +443,11 @@ int Engine::build_atable_dev(int nf, bool fp32, int f0) {
     if ((e = need(dA, sizeof(double) * (size_t)nf * K * nme))) return cuda_fail(e, "allocating A");
     const double *fp = dFreq.as<double>() + f0;
     const int *bad = log_coh_bad(dLogc.as<double>(), (size_t)ntc * in.nnl * in.nnl);
-    // On the tensor cores from 80 nodes on.  Second-order analyses, FP64 pipe / tensor cores (ms): 40
-    // nodes, 12 modes, 65 rows 0.071 / 0.075; 64, 12, 65: 0.078 / 0.078; 100, 12, 65: 0.107 / 0.091;
-    // 150, 12, 129: 0.229 / 0.139; 400, 24, 33: 0.564 / 0.157; 520, 8, 17: 0.258 / 0.165.
-    bool tensor = in.nnl >= 80;
+    // On the tensor cores from 112 nodes on, and from 80 where the modes are many enough.  Second-order
+    // analyses, FP64 pipe / tensor cores (ms): 64 nodes, 12 modes, 65 rows: 0.078 / 0.077; 80, 12, 65: 0.091 /
+    // 0.088; 80, 24, 33: 0.110 / 0.091; 96, 8, 65: 0.081 / 0.087; 130, 6, 33: 0.116 / 0.102; 150, 12, 129: 0.239 /
+    // 0.150; 400, 24, 33: 0.585 / 0.177; 520, 8, 17: 0.284 / 0.193; 130, 60, 17: 0.300 / 0.169.
+    bool tensor = in.nnl >= 112 || (in.nnl >= 80 && in.nnl * nme >= 960);
     int step = 0;
     if (tensor) {
         // frequencies in chunks of at most 1 GB of B digits; without room for them the FP64 pipe

@@ -22,12 +22,12 @@ namespace bsa {
 // Whether a point set goes this way: the point kernel's time against that of the digits and products
 // plus the listing of the pairs, from measured rates.  Contraction in ms, point kernel / pair products
 // (kept modes nm, K):
-//   scattered points (no pair shared): 100, nm 16, K 40: 0.131 / 0.111;  50, 10, 120: 0.091 / 0.074;  200,
-//   10, 120: 0.227 / 0.126;  500, 6, 120: 0.182 / 0.181;  200, 6, 300: 0.204 / 0.158;  100, 6, 120: 0.062 /
-//   0.078;  1000, 8, 40: 0.165 / 0.226;  500, 3, 300: 0.130 / 0.248;  1000, 4, 400: 0.309 / 0.576;
-//   zones of 144 points: nm 8, K 60: 0.060 / 0.068;  3, 600: 0.114 / 0.085;  6, 240: 0.099 / 0.074;  256 points,
-//   4, 120: 0.052 / 0.068;  1600, 4, 120: 0.184 / 0.168;  1600, 3, 60: 0.140 / 0.186;  1024, 8, 60: 0.235 / 0.146;
-//   1523, 16, 400: 9.46 / 0.55.
+//   scattered points (no pair shared): 100, nm 16, K 40: 0.133 / 0.131;  50, 10, 120: 0.092 / 0.087;  200,
+//   10, 120: 0.227 / 0.160;  500, 6, 120: 0.183 / 0.227;  200, 6, 300: 0.205 / 0.192;  100, 6, 120: 0.068 /
+//   0.088;  1000, 8, 40: 0.168 / 0.291;  500, 3, 300: 0.134 / 0.290;  1000, 4, 400: 0.307 / 0.673;
+//   zones of 144 points: nm 8, K 60: 0.057 / 0.076;  3, 600: 0.117 / 0.094;  6, 240: 0.099 / 0.086;  256 points,
+//   4, 120: 0.050 / 0.076;  1600, 4, 120: 0.184 / 0.187;  1600, 3, 60: 0.141 / 0.184;  1024, 8, 60: 0.234 / 0.161;
+//   1523, 16, 400: 9.46 / 0.58.
 bool Engine::list64_wanted(long long npts, int nr) const {
     using namespace p64;
     // the column digits grow with the rows (twice the A rows, modes padded to eights and K to 64): within
@@ -36,7 +36,7 @@ bool Engine::list64_wanted(long long npts, int nr) const {
     const double nm = nme, rows = (double)std::min<long long>(nr, 2 * npts) * ((nme * nme + kTM - 1) / kTM) * kTM;
     // a point's chain over K, then the FP64 pipe
     const double point_ms = 0.03 + K * (nme < 8 ? 1.4e-4 : 3.0e-4) + 2.0 * K * nm * nm * nm * (double)npts / (nme < 8 ? 2.0e8 : 4.2e8);
-    const double pair_ms = 0.06 + (4.1e-5 + 1.0e-7 * nm * nm * nm) * (double)npts + rows * ((K + 63) / 64 * 64) * 4.5e-9;
+    const double pair_ms = 0.07 + (5.0e-5 + 1.0e-7 * nm * nm * nm) * (double)npts + rows * ((K + 63) / 64 * 64) * 5.0e-9;
     return pair_ms < point_ms;
 }
 

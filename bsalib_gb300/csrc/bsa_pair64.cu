@@ -460,10 +460,10 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     const int G = diag ? std::min(64, (N + 8) / 8) : (int)std::max(1LL, std::min(want, (pairs_all + PB - 1) / PB));
     const size_t smem = smem_of(PB);
     // Products on the tensor cores (bsa_pair64_tc.cu) where they outweigh the digits' preparation.
-    // Measured contraction, FP64 pipe / tensor cores: 4.1e6 FMAs, K = 30: 0.097 / 0.108 ms; 7.3e6,
-    // K = 60: 0.126 / 0.109; 1.9e7, K = 20: 0.137 / 0.167; 5.4e7, K = 12: 0.353 / 0.447; 6.9e7,
-    // K = 30: 0.285 / 0.240 (K is padded to 16, and the moments do not get faster).
-    const bool tensor = K >= 24 && pairs_all * nb * K >= 7000000LL;
+    // Measured contraction in ms, FP64 pipe / tensor cores: 4.1e6 FMAs, K = 30: 0.069 / 0.080; 1.1e7, K = 24:
+    // 0.096 / 0.103; 1.6e7, K = 30: 0.115 / 0.102; from K = 40 on 7.3e6, K = 60: 0.082 / 0.080; 1.2e7, K = 40:
+    // 0.090 / 0.089; 1.4e7, K = 400: 0.168 / 0.091.  (K is padded to 16 and the moments do not get faster.)
+    const bool tensor = K >= 24 && pairs_all * nb * K >= (K < 40 ? 15000000LL : 7000000LL);
     // chunks of first rows: at most 4 GB of products and of row digits each
     const long long cap = 1LL << 29;
     const int Kd = (K + 63) / 64 * 64 * 2;  // digits of a row in doubles
