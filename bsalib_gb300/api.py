@@ -128,7 +128,7 @@ def load(path: Optional[str] = None):
         "bsa_Run": [vp] * 7, "bsa_computeSkewness": [i, vp, vp, vp],
         "bsa_gpu_setPrecision": [i], "bsa_gpu_setClassicTruncation": [i], "bsa_gpu_setClassicRows": [i, i],
         "bsa_gpu_clsBispectra": [vp, i, vp, vp, vp], "bsa_gpu_mshBispectra": [vp, vp, i, vp, vp],
-        "bsa_gpu_clsBispectraAt": [vp, vp, i, vp, vp], "bsa_gpu_setWaitTest": [i],
+        "bsa_gpu_clsBispectraAt": [vp, vp, i, vp, vp], "bsa_gpu_setWaitTest": [i], "bsa_gpu_setWaitTestFP64": [i, i],
         "bsa_gpu_setMesherGraphs": [i], "bsa_gpu_setMesherExpansion": [i], "bsa_gpu_setMesherPassBytes": [d], "bsa_gpu_setClassicShard": [i, i], "bsa_enableVisualMode": [], "bsa_setVisualIndexes": [vp, i], "bsa_setBRMExportDefaultMode": [i],
         "bsa_gpu_setTilePlan": [i] * 8, "bsa_gpu_clearTilePlans": [], "bsa_gpu_loadTilePlans": [C.c_char_p],
         "bsa_gpu_getTilePlan": [i, i, i, i, vp],

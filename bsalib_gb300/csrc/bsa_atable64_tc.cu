@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     k_atable64_tc(const __grid_constant__ CUtensorMap tmB, int ntc, int n, int nm, int bw, int MT, int nk, int ks_last,
                   const double *__restrict__ f, const double *__restrict__ logc, const double *__restrict__ rootS,
                   const int *__restrict__ we, const int *__restrict__ bad, double *__restrict__ A, uint8_t *__restrict__ small,
-                  int *err) {
+                  int *err, int test_skip1) {
     after_previous();
     if (*bad) return;
     extern __shared__ uint8_t smem_raw[];
@@ -298,7 +298,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                     mma_commit(&aempty[h]);
                 }
-                if (ok && (kb % kPassK == kPassK - 1 || kb == nk - 1)) mma_commit(done);
+                if (ok && (kb % kPassK == kPassK - 1 || kb == nk - 1) && !(test_skip1 == pass + 1 && blockIdx.x == 0))
+                    mma_commit(done);
             }
             if (!ok) {  // what is in flight lands before the block leaves
                 mma_commit(done);
@@ -354,6 +355,8 @@ __global__ void __launch_bounds__(kThreads, 1)
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 mbar_arrive(&afull[h]);
             }
+            // where a wait failed the lanes may differ: leave together, the warp-wide steps below need them all
+            ok = __all_sync(0xffffffffu, ok);
             if (kb % kPassK == kPassK - 1 || kb == nk - 1) {
                 const uint32_t ph = (uint32_t)(kb / kPassK) & 1u;
                 ok = __all_sync(0xffffffffu, mbar_wait(done, ph, err, 26)) && ok;
@@ -475,12 +478,12 @@ __global__ __launch_bounds__(256) void k_atable64_mend(int rows, int ntc, int n,
 template <int NP>
 static cudaError_t launch(cudaStream_t st, const CUtensorMap &mb, int nf, const double *f, int ntc, int n, int nm, int bw,
                           const double *logc, const double *rootS, const int *we, const int *bad, double *A, uint8_t *small,
-                          int *err) {
+                          int *err, int test_skip1) {
     const int MT = (n + 127) / 128, nk = (n + kBK - 1) / kBK, ks_last = (n - (nk - 1) * kBK + 15) / 16;
     cudaError_t e = cudaFuncSetAttribute(k_atable64_tc<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<NP>());
     if (e != cudaSuccess) return e;
     launch_next(k_atable64_tc<NP>, (unsigned)(nf * ntc * MT), kThreads, smem_bytes<NP>(), st, mb, ntc, n, nm, bw, MT, nk, ks_last, f, logc,
-                                                                                   rootS, we, bad, A, small, err);
+                                                                                   rootS, we, bad, A, small, err, test_skip1);
     return cudaGetLastError();
 }
 
@@ -495,7 +498,8 @@ size_t atable64_tc_scratch(int nf, int ntc, int nnl, int nm) {
 }
 
 cudaError_t launch_atable64_tc(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm, const double *logc,
-                               const double *rootS, const double *L, const int *bad, double *A, void *scratch, int *err) {
+                               const double *rootS, const double *L, const int *bad, double *A, void *scratch, int *err,
+                               int test_skip1) {
     using namespace at64;
     const int np = blocks_of(nm), bw = block_width(nm), Kp = (nnl + kBK - 1) / kBK * kBK, rows = nf * ntc * nnl;
     const size_t nb = (size_t)nf * ntc * np;
@@ -506,8 +510,8 @@ cudaError_t launch_atable64_tc(cudaStream_t st, int nf, const double *f, int ntc
     launch_next(k_wdigits, dim3((unsigned)nb, (Kp + 127) / 128), 256, 0, st, ntc, nnl, nm, np, bw, Kp, rootS, L, we, D);
     CUtensorMap mb;
     if (!make_map(&mb, D, Kp, (uint64_t)nb * kDig * bw, (uint32_t)bw)) return cudaErrorInvalidValue;
-    const cudaError_t e = np == 1 ? launch<1>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, small, err)
-                                  : launch<2>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, small, err);
+    const cudaError_t e = np == 1 ? launch<1>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, small, err, test_skip1)
+                                  : launch<2>(st, mb, nf, f, ntc, nnl, nm, bw, logc, rootS, we, bad, A, small, err, test_skip1);
     if (e != cudaSuccess) return e;
     launch_next(k_atable64_mend, (unsigned)((rows + 63) / 64), 256, 0, st, rows, ntc, nnl, nm, f, logc,
                 logc + (size_t)ntc * nnl * nnl, rootS, L, we, bad, (const unsigned long long *)small, A);

@@ -142,6 +142,7 @@ struct Engine {
     std::vector<std::vector<double>> own_d;
     bool classic_sym = false;   // bsa_gpu_setClassicSymmetry: evaluate half the Classic grid
     bool use_e_form = true;     // bsa_gpu_setClassicForm: E form of the split contraction where it applies
+    int wait_test_atable1 = 0, wait_test_pair1 = 0;  // bsa_gpu_setWaitTestFP64: the same for the FP64 A table and pair products
     int wait_test_tile1 = 0;    // bsa_gpu_setWaitTest: tile + 1 whose ready signal CTA 0 omits (0 = off)
     bool msh_graphs = true;     // bsa_gpu_setMesherGraphs: each Mesher zone pass as one CUDA graph
     bool msh_dev_expand = true; // bsa_gpu_setMesherExpansion: zone passes expanded on the device

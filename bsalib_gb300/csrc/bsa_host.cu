@@ -465,7 +465,8 @@ int Engine::build_atable_dev(int nf, bool fp32, int f0) {
         for (int q = 0; q < nf; q += step) {
             e = launch_atable64_tc(stream, std::min(step, nf - q), fp + q, ntc, in.nnl, nme, dLogc.as<double>(),
                                    dS.as<double>() + (size_t)q * K, dL.as<double>(), bad, dA.as<double>() + (size_t)q * K * nme,
-                                   dMshT.p, dFlag.as<int>());
+                                   dMshT.p, dFlag.as<int>(), wait_test_atable1);
+            wait_test_atable1 = 0;  // one launch only
             if (e) return cuda_fail(e, "A-table kernel");
             kernels += 4;
         }
@@ -1430,6 +1431,13 @@ int bsa_gpu_setWaitTest(int tile) {
     GUARD();
     if (tile < -1) return eng().fail(BSA_ERR_ARG, "tile must be >= -1");
     eng().wait_test_tile1 = tile + 1;
+    return BSA_OK;
+}
+
+int bsa_gpu_setWaitTestFP64(int kernel, int tile) {
+    GUARD();
+    if (tile < -1 || kernel < 0 || kernel > 1) return eng().fail(BSA_ERR_ARG, "kernel 0 or 1, tile >= -1");
+    (kernel == 0 ? eng().wait_test_atable1 : eng().wait_test_pair1) = tile + 1;
     return BSA_OK;
 }
 

@@ -27,10 +27,11 @@ cudaError_t launch_atable(cudaStream_t st, int nf, const double *f, int ntc, int
 
 // The same on the tensor cores (bsa_atable64_tc.cu); leaves A alone where *bad is set (then launch_atable
 // with only = bad forms it).  scratch: atable64_tc_scratch(nf, ntc, nnl, nm) bytes; err receives a
-// nonzero code if a pipeline wait ran out of its budget.
+// nonzero code if a pipeline wait ran out of its budget.  test_skip1: pass + 1 whose ready signal block 0 omits.
 size_t atable64_tc_scratch(int nf, int ntc, int nnl, int nm);
 cudaError_t launch_atable64_tc(cudaStream_t st, int nf, const double *f, int ntc, int nnl, int nm, const double *logc,
-                               const double *rootS, const double *L, const int *bad, double *A, void *scratch, int *err);
+                               const double *rootS, const double *L, const int *bad, double *A, void *scratch, int *err,
+                               int test_skip1 = 0);
 
 
 // The FP32 table on the tensor cores (bsa_atable_tc.cu): tf32 hi/lo split, FP32 accumulation;

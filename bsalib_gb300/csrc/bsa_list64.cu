@@ -184,7 +184,8 @@ int Engine::contract_list64(const PointSrc &ps, long long npts, const HostRows &
             (e = cudaMemcpyAsync(dpe, pe.data(), pb, cudaMemcpyHostToDevice, stream)))
             return cuda_fail(e, "pair lists");
         h2d += (double)(ib + 2 * lb + xb + pb);
-        Chunk c{0, (int)xmap.size(), nm, nm, K, nr - 1, 0, (long long)items.size(), nullptr, dMixA.as<double>(), tiles_x * kTM, dx};
+        Chunk c{0, (int)xmap.size(), nm, nm, K, nr - 1, 0, (long long)items.size(), nullptr, dMixA.as<double>(), tiles_x * kTM, dx, wait_test_pair1};
+        wait_test_pair1 = 0;  // one launch only
         PairList l{ditems, dblk, dpair, np, bw, tiles_x};
         if ((e = tc_list_products(stream, c, l, nr, dA.as<double>(), dQ.as<double>(), dMixB.p, dMshT.p, dFlag.as<int>() + 1)))
             return cuda_fail(e, "pair product kernel");

@@ -533,7 +533,8 @@ int Engine::contract_pair64(int N, double df, bool analytic, bool vect, double w
     if (tensor) kernels += 2;
     for (size_t q = 0; q < plans.size(); ++q) {
         const Plan &p = plans[q];
-        Chunk c{p.x0, p.x1, nm, an, K, hi, p.ntiles, p.items, (const RowTile *)idx + p.rt0, dMixA.as<double>(), rx, nullptr};
+        Chunk c{p.x0, p.x1, nm, an, K, hi, p.ntiles, p.items, (const RowTile *)idx + p.rt0, dMixA.as<double>(), rx, nullptr, wait_test_pair1};
+        wait_test_pair1 = 0;  // one launch only
         if (tensor) {
             if ((e = tc_products(stream, c, hi + 1, A, Q, dMixB.p, dMshT.p, dFlag.as<int>() + 1)))
                 return cuda_fail(e, "pair product kernel");

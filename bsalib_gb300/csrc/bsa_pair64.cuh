@@ -27,6 +27,7 @@ struct Chunk {
     double *E;
     int rpad;         // rows of one x in the row operand (rx, or whole tiles in a pair list)
     const int *xmap;  // pair list: A row of x (x0 = 0); null: x itself
+    int test_skip1 = 0;  // tile pass + 1 whose ready signal block 0 omits (bsa_gpu_setWaitTestFP64)
     __host__ __device__ int rx() const { return qn * an; }  // rows of one x
 };
 

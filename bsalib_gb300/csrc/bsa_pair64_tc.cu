@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         }
                         if (ok) mma_commit(&eb[sB]);
                     }
-                    if (ok) mma_commit(&tfull[buf]);
+                    if (ok && !(c.test_skip1 == (int)tile + 1 && blockIdx.x == 0)) mma_commit(&tfull[buf]);
                 }
             }
             mma_commit(done);

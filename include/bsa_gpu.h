@@ -475,6 +475,9 @@ int bsa_gpu_getTilePlan(int family, int nm, int K, int nf, int *value);
  * accumulator-ready signal of that CTA's accumulator tile, so the epilogue's wait runs out (no
  * fault, no copy left in flight); -1 switches it off.  Applies to one analysis. */
 int bsa_gpu_setWaitTest(int tile);
+/* The same for the FP64 kernels: kernel 0, the A(f) table on the tensor cores, block 0 omits the signal of its
+ * K pass `tile`; kernel 1, the pair products, that of its accumulator tile.  Applies to one launch. */
+int bsa_gpu_setWaitTestFP64(int kernel, int tile);
 
 /* No counterpart in the reference.  on != 0 (default): each split-precision Mesher zone pass
  * (every refinement level of an adaptive refinement) runs its device work -- operand rows, the
