@@ -899,8 +899,7 @@ int Engine::batch_run(double *m3mf, double *m3mr, double *m2mr, double *case_ms,
             } else {
                 hostv.push_back(c.f);
                 std::vector<double> &ftab = hostv.back();
-                if (!c.trunc)
-                    for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back(2.0 * c.f[0] + s * (c.f[1] - c.f[0]));
+                if (!c.trunc) push_sums(ftab, c.f);
                 rc = build_atable(ftab, true);
             }
             if (rc) return rc;

@@ -226,6 +226,7 @@ struct Engine {
     long long dim_psd() const { return set.onlyd ? nme : (long long)nme * nme; }
     long long dim_bisp() const { return set.onlyd ? nme : (long long)nme * nme * nme; }
     int classic_grid(std::vector<double> &f);
+    static void push_sums(std::vector<double> &ftab, const std::vector<double> &f);
     int run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf, double *m3mr, double *bf_host,
                     double *br_host, std::vector<double> *grid_out);
     int classic_export(PointSrc ps, const std::vector<double> &f, double *m3mf, double *m3mr);

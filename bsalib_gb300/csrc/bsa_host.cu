@@ -562,6 +562,15 @@ int Engine::classic_grid(std::vector<double> &f) {
     return BSA_OK;
 }
 
+// f1 + f2 of the index sums s = i1 + i2 behind the rows of the grid f: multiples of the step as the grid's own
+// frequencies, so that f1 = -f2 is f = 0 (2 f[0] + s (f[1] - f[0]) is that but for a rounding, and c^|f| of a
+// zero coherence is 1 at 0 and 0 beside it).
+void Engine::push_sums(std::vector<double> &ftab, const std::vector<double> &f) {
+    const int nf = (int)f.size(), zero = f[0] != 0.0 ? (nf - 1) / 2 : 0;
+    const double df = f[zero + 1] - f[zero];
+    for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back((s - 2 * zero) * df);
+}
+
 // Classic analysis on the GPU (mainClassic_, BsaClassicImpl.F90:39-376): every grid point,
 // moments reduced in the kernel epilogue.  Optional materialised bispectra (nf, nf, nm^3).
 int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf, double *m3mr, double *bf_host,
@@ -600,9 +609,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
     const bool analytic = !classic_trunc;
     std::vector<double> ftab = f;
     if (analytic) {
-        // s-table: f1 + f2 = 2 f[0] + s df, s = i1 + i2.
-        const double d = f[1] - f[0];
-        for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back(2.0 * f[0] + s * d);
+        push_sums(ftab, f);
     }
     // Diagonal-only spectra read the nodal PSD table alone and stay FP64 (O(K nm) per point).
     const bool diagonal = set.onlyd != 0;
@@ -721,8 +728,7 @@ int Engine::run_classic(double *m2mf, double *m2mr, double *m2o2mr, double *m3mf
                     // no room for the products and their operands: the point kernel on the rows of every f
                     for (DevBuf *b : {&dMixA, &dMixB, &dMshT}) b->release();
                     ftab = f;
-                    if (analytic)
-                        for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back(2.0 * f[0] + s * (f[1] - f[0]));
+                    if (analytic) push_sums(ftab, f);
                     const int r = diagonal ? build_psd(ftab) : build_atable(ftab, false);
                     if (r) return r;
                     ps.fgrid = dFreq.as<double>();  // a longer table than that of f >= 0: the block may have moved
@@ -766,8 +772,7 @@ int Engine::classic_export(PointSrc ps, const std::vector<double> &f, double *m3
     int rc;
     if (precision == BSA_PREC_BF16X3 && !set.onlyd) {
         std::vector<double> ftab = f;
-        if (!ps.trunc)
-            for (int s = 0; s < 2 * nf - 1; ++s) ftab.push_back(2.0 * f[0] + s * (f[1] - f[0]));
+        if (!ps.trunc) push_sums(ftab, f);
         if ((rc = build_atable(ftab, false))) return rc;
         ps.fgrid = dFreq.as<double>();
     }
@@ -1041,8 +1046,7 @@ int Engine::classic_points(const int *i1, const int *i2, long long npts, double 
         }
     } else {
         std::vector<double> ftab = f;
-        if (analytic)
-            for (int s2 = 0; s2 < 2 * nf - 1; ++s2) ftab.push_back(2.0 * f[0] + s2 * (f[1] - f[0]));
+        if (analytic) push_sums(ftab, f);
         if ((rc = build_atable(ftab, false))) return rc;
         const size_t n = (size_t)npts;
         std::vector<int> iz(n);

@@ -182,3 +182,24 @@ def test_elements_over_a_wide_range(bsalib):
     finally:
         s.close()
     _within(bf.reshape(n * n, -1)[::7], want.reshape(i1.size, -1), 128)
+
+
+@pytest.mark.parametrize("gap", [0.0, 40.0, None])
+@pytest.mark.parametrize("trunc", [True, False])
+def test_moment_elements(bsalib, gap, trunc):
+    """Third moments of the force: sums of positive products over the grid (but for its four corners), within
+    the products' bound and one rounding a grid point, twice for the corners' sign."""
+    p = _groups(60, 8, gap)
+    nf = p.classic_nf()
+
+    def run(rows=None):
+        s = api.BsaSession(p, classic_truncation=trunc)
+        try:
+            if rows:
+                s.set_rows(*rows)
+            return s.run()["m3mf_cls"]
+        finally:
+            s.close()
+
+    a, b = run(), run((0, nf // 2)) + run((nf // 2, nf))
+    assert np.all(np.abs(a - b) <= 4 * (120 + nf * nf) * U * np.abs(b))
