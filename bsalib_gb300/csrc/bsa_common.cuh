@@ -133,9 +133,6 @@ __device__ __forceinline__ void get_point(const PointSrc &ps, long long p, int &
     }
 }
 
-// Lanes (threadIdx.y) that share the partials of one third moment in the reduction kernels of the
-// split Classic forms: one lane walking every CTA's partial of seven kinds was a chain of dependent
-// loads (0.20 ms for the 64 moments of a 4-mode structure).
 // A kernel's launch while the kernel before it on the stream still runs: its blocks wait in
 // after_previous(), first of all, until that kernel has ended and its writes are visible.  A chain of
 // small kernels costs 3.5 us each instead of 6.2 (12 kernels of 4000 threads, 42 for 74 us).  A
@@ -172,6 +169,9 @@ __device__ __forceinline__ void end_flags(const EndFlags &f) {
     }
 }
 
+// Lanes (threadIdx.y) that share the partials of one third moment in the reduction kernels of the
+// split Classic forms: one lane walking every CTA's partial of seven kinds was a chain of dependent
+// loads (0.20 ms for the 64 moments of a 4-mode structure).
 constexpr int kRedLanes = 16;
 
 // Sum of a and b over the lanes threadIdx.y of a 32 x kRedLanes block, into lane 0 (fixed order).
