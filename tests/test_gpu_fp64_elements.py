@@ -203,3 +203,27 @@ def test_moment_elements(bsalib, gap, trunc):
 
     a, b = run(), run((0, nf // 2)) + run((nf // 2, nf))
     assert np.all(np.abs(a - b) <= 4 * (120 + nf * nf) * U * np.abs(b))
+
+
+def test_factors_below_every_high_word(bsalib):
+    """Quadratic coefficients whose high word is zero (below 2^-1042) at one node, whose products with large
+    linear forces are the largest of their rows, and for one mode the only ones."""
+    p = _groups(60, 8, 10.0)
+    i, j = np.triu_indices(p.nn)
+    p.nod_corr[i != j] = 0.0
+    p.phi[:, 1] = np.arange(p.nn) == 7
+    p.wfc[0, :3] *= 1e-10
+    p.wfc[0, 3:] *= 1e-220
+    p.wfc[0, :3, 7] *= 1e157
+    p.wfc[0, 3:, 7] = 3e-320
+    rng = np.random.default_rng(4)
+    f1, f2 = rng.uniform(-2, 2, (2, 400))
+    s = api.BsaSession(p)
+    try:
+        lst, _ = s.msh_bispectra(f1, f2)
+        pieces = np.concatenate([s.msh_bispectra(f1[k:k + 2], f2[k:k + 2])[0] for k in range(0, 400, 2)])
+    finally:
+        s.close()
+    ok = np.isfinite(pieces)
+    assert np.array_equal(lst[~ok], pieces[~ok], equal_nan=True)
+    assert np.all(np.abs(lst[ok] - pieces[ok]) <= 2 * (120 + 4) * U * np.abs(pieces[ok]))
