@@ -229,7 +229,9 @@ void bsaclFinalise(void);                                                 /* bsa
 /* 3. Plugin-level entries and controls                                                */
 /* ---------------------------------------------------------------------------------- */
 
-/* Contraction precision for the Classic grid (BSA_PREC_FP64 default, or BSA_PREC_BF16X3). */
+/* Contraction precision for the Classic grid (BSA_PREC_FP64 default, or BSA_PREC_BF16X3).  FP64 holds element by
+ * element: what the tensor cores form as sums of digits is formed on the FP64 pipe where an element lies
+ * so far below its scales that their error would exceed FP64's. */
 int bsa_gpu_setPrecision(int prec);
 
 /* Classic S(f1+f2) beyond the grid: 1 (default) reads zero, as the reference's padded
