@@ -146,6 +146,7 @@ void Engine::reset_inputs() {
     pod_nmodes = 0;
     export_fn = nullptr;
     export_user = nullptr;
+    wait_test_atable1 = wait_test_pair1 = 0;
     brm_file_close(-1);
     visual = false;
     visual_modal = true;
