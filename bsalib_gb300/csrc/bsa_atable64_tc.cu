@@ -14,9 +14,9 @@
 // One block per (f, itc, 128 rows): 16 warps generate digits of 32 columns at a time into two halves of
 // the A tiles and drain TMEM at the end, one thread loads B and issues the MMAs.  Bound by the integer
 // instructions of the generation (about 110 an element).  65 rows of 400 nodes x 2, 24 modes: FP64 pipe
-// 1.70 ms, here 0.25, 0.04 for the B digits and 0.06 for the elements far below their column's scale,
+// 1.70 ms, here 0.25, 0.04 for the B digits and 0.04 for the elements far below their column's scale,
 // which k_atable64_mend sums on the FP64 pipe; 3333 rows of 150 nodes, 12 modes: 3.9 ms, here 1.13, 0.09 and
-// 0.06.  Coherences outside [0, 1] or c_ii != 1 (bad flag of the coherence table) leave the table to k_atable.
+// 0.08.  Coherences outside [0, 1] or c_ii != 1 (bad flag of the coherence table) leave the table to k_atable.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -167,8 +167,8 @@ constexpr unsigned long long kLn2 = 0xb17217f7d1cf79acull;  // round(2^64 ln 2)
 constexpr int kGen = 512, kThreads = kGen + 32;
 constexpr int kTileA = 128 * 128, kTileB = kDig * 32 * 128;
 
-constexpr float kSmall = 1.f / 256;  // k_atable64_mend
-constexpr long long kSmallHi = 1LL << 28;
+constexpr float kSmall = 1.f / 128;  // k_atable64_mend
+constexpr long long kSmallHi = 1LL << 29;
 
 template <int NP>
 constexpr size_t smem_bytes() { return 1024 + (size_t)kDig * kTileA + (size_t)NP * kTileB + 4096 + 256; }
@@ -414,9 +414,11 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // Rows where c_ij^|f| decays between i and the nodes that a mode moves: the digits' error is absolute
 // against the largest s_j L_jm (2^-62 a term), so an element keeps them only where sum_j c_ij^|f| |s_j
-// L_jm| >= kSmall of the scale; at that line their measured error is 2.1e-16 of the sum against the FP64
-// pipe's 2.7e-16 (200 nodes; 400: 2.7e-16 / 3.5e-16), half of it a factor 2 above.  The element itself and
-// then the 32 nodes around i bound that sum from below; what is left is summed on the FP64 pipe, lanes over j.
+// L_jm| >= kSmall of the scale.  Measured error relative to that sum from the line to twice it, digits / FP64
+// pipe: 200 nodes 1.2e-16 / 2.8e-16, 400 1.4e-16 / 3.7e-16, 1000 with local modes 3.7e-16 / 8.3e-16, 1200 1.4e-16
+// / 2.7e-16; below half of it the digits' is the larger.  The element itself and then the 32 nodes around i
+// bound the sum from below; what is left is summed on the FP64 pipe, lanes over j, without the nodes that add
+// less than 2^-60 of it (zones of 200 nodes 85 -> 35 us, 400 nodes x 2 100 -> 44).
 // A warp scans the masks of eight rows, far apart (those near the foot of a tower come together: 32
 // neighbouring rows a warp took twice the time).
 __global__ __launch_bounds__(256) void k_atable64_mend(int rows, int ntc, int n, int nm, const double *__restrict__ f,
@@ -438,14 +440,21 @@ __global__ __launch_bounds__(256) void k_atable64_mend(int rows, int ntc, int n,
         const double *lc = logc + ((size_t)itc * n + i) * n, *s = rootS + (size_t)fc * n, *l = L + (size_t)itc * n * nm;
         const int jw = max(0, min(i - 16, n - 32)) + lane;
         const float cw = jw >= n ? 0.f : af == 0.0 ? 1.f : expf((float)(af * lc[jw]));
+        float least = 1.f;  // of the sums that are too small, over the 32 nodes
         for (unsigned long long b = mk; b; b &= b - 1) {
             const int m = __ffsll(b) - 1, e = we[fc * nm + m];
-            if (e == kBad) continue;  // the whole column
+            if (e == kBad) {  // the whole column
+                least = 0.f;
+                continue;
+            }
             float v = jw < n ? cw * scaled_abs(s[jw] * l[(size_t)jw * nm + m], e) : 0.f;
 #pragma unroll
             for (int h = 16; h > 0; h >>= 1) v += __shfl_xor_sync(0xffffffffu, v, h);
             if (v >= kSmall) mk &= ~(1ull << m);
+            else least = fminf(least, v);
         }
+        // nodes that add less than 2^-60 of every sum are passed over, 32 at a time (scaled_abs is true to 2^-60)
+        const float skip = least >= 0x1p-40f ? least * 0x1p-60f / (float)n : -1.f;
         while (mk) {
             int m[8], cnt = 0;
             double acc[8];
@@ -459,11 +468,15 @@ __global__ __launch_bounds__(256) void k_atable64_mend(int rows, int ntc, int n,
                     ++cnt;
                 }
             }
-            for (int j = lane; j < n; j += 32) {
-                const double c = af == 0.0 ? 1.0 : expc(af * lc[j], T), sj = s[j];
+            for (int j0 = 0; j0 < n; j0 += 32) {
+                const int j = j0 + lane;
+                const bool in = j < n;
+                const double x = in ? af * lc[j] : 0.0;
+                if (!__any_sync(0xffffffffu, in && (af == 0.0 || expf((float)x) > skip))) continue;
+                const double c = !in ? 0.0 : af == 0.0 ? 1.0 : expc(x, T), sj = in ? s[j] : 0.0;
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    if (q < cnt) acc[q] = fma(c, sj * l[(size_t)j * nm + m[q]], acc[q]);
+                    if (in && q < cnt) acc[q] = fma(c, sj * l[(size_t)j * nm + m[q]], acc[q]);
             }
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
